@@ -264,10 +264,10 @@ struct sfg_context {
     bool any_bc = false;                // boundary-aware lattice kernel in use
     RowItem* d_zh_rows = nullptr;       // Zou-He rows (channel, y)
     int n_zh = 0;
-    // independent launch groups at the start of a step (contact cell list,
-    // force tiles + tile moments) run on side streams, joined by events
+    // independent launch groups at the start of a step (contact cells and
+    // force tiles, tile moments) run on side streams, joined by events
     cudaStream_t side[3] = {nullptr, nullptr, nullptr};
-    cudaEvent_t ev_fork = nullptr, ev_contact = nullptr, ev_tiles = nullptr, ev_mom = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_tiles = nullptr, ev_mom = nullptr;
     cudaEvent_t ev_lat1 = nullptr;      // the lattice pass over untouched force tiles
     cudaEvent_t ev_slots = nullptr;     // the step's slot records exist
     // the learned gate's fallback flag beside the last spread, the step's
@@ -427,15 +427,13 @@ static void free_all(sfg_context* c) {
     F(c->mb.rest_len); F(c->mb.rest_ang); F(c->mb.rest_ds); F(c->mb.prev_len);
     F(c->mb.mk_cap); F(c->mb.mk_chan); F(c->mb.ix0); F(c->mb.iy0); F(c->mb.valid);
     F(c->mb.pair_count); F(c->mb.wx); F(c->mb.wy);
-    F(c->tb.tile_chan); F(c->tb.tile_flag); F(c->tb.tile_cnt); F(c->tb.cursor);
-    F(c->tb.slot_scan); F(c->tb.list_off); F(c->tb.slot_tile); F(c->tb.n_slots);
-    F(c->tb.list); F(c->tb.scan_tmp); F(c->tb.acc); F(c->tb.gsnap); F(c->tb.capped);
-    F(c->tb.fluid_touched); F(c->tb.acc0); F(c->tb.mom); F(c->tb.slot_info); F(c->tb.slot_order); F(c->tb.slot_rank); F(c->tb.cls_cnt); F(c->tb.spread_ctr); F(c->tb.resid_gate); F(c->tb.resid_plain);
+    F(c->tb.tile_chan); F(c->tb.tile_cnt); F(c->tb.tile_pos); F(c->tb.ctr);
+    F(c->tb.list); F(c->tb.acc); F(c->tb.gsnap); F(c->tb.capped);
+    F(c->tb.fluid_touched); F(c->tb.acc0); F(c->tb.mom); F(c->tb.slot_info); F(c->tb.slot_order); F(c->tb.resid_gate); F(c->tb.resid_plain);
     F(c->mb.u0); F(c->mb.dFsum); F(c->mb.dFprev); F(c->mb.slot8);
     F(c->d_model); F(c->d_learned_steps); F(c->d_fallbacks);
     F(c->d_hfeat); F(c->d_hlab); F(c->d_hvalid); F(c->d_feat); F(c->d_frame); F(c->d_plain_needed);
-    F(c->cb.cell_of); F(c->cb.cell_cnt); F(c->cb.cell_start); F(c->cb.cursor); F(c->cb.list);
-    F(c->cb.scan_tmp);
+    F(c->cb.cell_of); F(c->cb.cell); F(c->cb.next); F(c->cb.list); F(c->cb.lpos);
     F(c->d_phi); F(c->d_stepped); F(c->d_adr_pending); F(c->d_c_fresh); F(c->d_status);
     F(c->d_step_ctr);
     F(c->d_io);
@@ -479,7 +477,7 @@ static void free_all(sfg_context* c) {
         }
         c->side[i] = nullptr;
     }
-    for (cudaEvent_t* e : {&c->ev_fork, &c->ev_contact, &c->ev_tiles, &c->ev_mom, &c->ev_lat1, &c->ev_slots,
+    for (cudaEvent_t* e : {&c->ev_fork, &c->ev_tiles, &c->ev_mom, &c->ev_lat1, &c->ev_slots,
                            &c->ev_gate, &c->ev_pn, &c->ev_lat, &c->ev_flags}) {
         if (*e) cudaEventDestroy(*e);
         *e = nullptr;
@@ -1061,27 +1059,19 @@ extern "C" int sfg_initialize(sfg_context* c) {
     const int T = tb.T;
     CU(dalloc(&tb.tile_chan, T));
     CU(cudaMemcpy(tb.tile_chan, tile_chan.data(), sizeof(int) * T, cudaMemcpyHostToDevice));
-    CU(dalloc(&tb.tile_flag, T));
     CU(dalloc(&tb.tile_cnt, T));
-    CU(dalloc(&tb.cursor, T));
-    CU(dalloc(&tb.slot_scan, T));
-    CU(dalloc(&tb.list_off, T));
+    CU(cudaMemset(tb.tile_cnt, 0, sizeof(int) * std::max(T, 1)));
+    CU(dalloc(&tb.tile_pos, T));
     for (int i = 0; i < 2; ++i) {
         CU(dalloc(&tb.tile_slot[i], T));
         CU(cudaMemset(tb.tile_slot[i], 0xff, sizeof(int) * std::max(T, 1)));
         CU(cudaMalloc(&tb.fin[i], (size_t)tb.max_slots * 2 * TILE_CELLS * c->real_size()));
     }
-    CU(dalloc(&tb.slot_tile, tb.max_slots));
     CU(dalloc(&tb.slot_info, tb.max_slots));
-    CU(dalloc(&tb.slot_order, tb.max_slots));
-    CU(dalloc(&tb.slot_rank, tb.max_slots));
-    CU(dalloc(&tb.cls_cnt, SLOT_CLASSES));
-    tb.n_spread_ctr = c->Kmax + 3;
-    CU(dalloc(&tb.spread_ctr, tb.n_spread_ctr));
-    CU(dalloc(&tb.n_slots, 1));
-    CU(cudaMemset(tb.n_slots, 0, sizeof(int)));
+    CU(dalloc(&tb.slot_order, (size_t)SLOT_CLASSES * tb.max_slots));
+    CU(dalloc(&tb.ctr, NUM_STEP_CTR));
+    CU(cudaMemset(tb.ctr, 0, sizeof(int) * NUM_STEP_CTR));
     CU(dalloc(&tb.list, 8LL * M));
-    CU(dalloc(&tb.scan_tmp, scan_tmp_ints(T)));
     CU(dalloc(&tb.acc, (size_t)tb.max_slots * 2 * TILE_CELLS));
     CU(cudaMalloc(&tb.gsnap, (size_t)tb.max_slots * 2 * TILE_CELLS * c->real_size()));
     if (c->Kmax > 1) CU(cudaMalloc(&tb.mom, (size_t)tb.max_slots * TILE_CELLS * 4 * c->real_size()));
@@ -1110,13 +1100,11 @@ extern "C" int sfg_initialize(sfg_context* c) {
 
     // contact cells
     CU(dalloc(&c->cb.cell_of, M));
-    CU(dalloc(&c->cb.cell_cnt, c->ncells));
-    CU(dalloc(&c->cb.cell_start, c->ncells));
-    CU(dalloc(&c->cb.cursor, c->ncells));
+    CU(dalloc(&c->cb.cell, c->ncells));
+    CU(dalloc(&c->cb.next, M));
     CU(dalloc(&c->cb.list, M));
-    CU(dalloc(&c->cb.scan_tmp, scan_tmp_ints(c->ncells)));
-    CU(cudaMemset(c->cb.cell_cnt, 0, sizeof(int) * std::max(c->ncells, 1)));
-    CU(cudaMemset(c->cb.cell_start, 0, sizeof(int) * std::max(c->ncells, 1)));
+    CU(dalloc(&c->cb.lpos, M));
+    CU(cudaMemset(c->cb.cell, 0, sizeof(int2) * std::max(c->ncells, 1)));
 
     // Peskin table (delta_function.h:29-37)
     {
@@ -1143,7 +1131,7 @@ extern "C" int sfg_initialize(sfg_context* c) {
     CU(cudaStreamSynchronize(c->stream));
     if (c->M > 0 && !c->side[0]) {
         for (int i = 0; i < 3; ++i) CU(cudaStreamCreateWithFlags(&c->side[i], cudaStreamNonBlocking));
-        for (cudaEvent_t* e : {&c->ev_fork, &c->ev_contact, &c->ev_tiles, &c->ev_mom, &c->ev_lat1, &c->ev_slots,
+        for (cudaEvent_t* e : {&c->ev_fork, &c->ev_tiles, &c->ev_mom, &c->ev_lat1, &c->ev_slots,
                            &c->ev_gate, &c->ev_pn, &c->ev_lat, &c->ev_flags})
             CU(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
@@ -1192,27 +1180,19 @@ static int enqueue_step_t(sfg_context* c, int p) {
     const bool split = c->M > 0 && !c->profiling && c->side[0] != nullptr && c->split_lattice &&
                        c->use_vec8 && !L.any_adr && !c->any_bc;
     if (c->M > 0) {
-        cudaMemsetAsync(c->tb.capped, 0, sizeof(int) * nch, st);
-        cudaMemsetAsync(c->tb.fluid_touched, 0, sizeof(int) * nch, st);
-        cudaMemsetAsync(c->tb.resid_gate, 0, sizeof(unsigned) * nch, st);
-        cudaMemsetAsync(c->tb.resid_plain, 0, sizeof(unsigned) * nch, st);
-        cudaMemsetAsync(c->tb.spread_ctr, 0, sizeof(int) * c->tb.n_spread_ctr, st);
         const S* fp = static_cast<const S*>(c->f[p]);
-        // The contact cell list and the force tiles read positions only, the
-        // tile moments the populations: with profiling off they run beside
-        // the membrane forces on side streams and join before their users.
+        // The contact cells and the force tiles read positions only, the tile
+        // moments the populations: with profiling off they run beside the
+        // membrane forces on side streams and join before their users.
         const bool par = !c->profiling && c->side[0] != nullptr;
         if (par) {
             CU(cudaEventRecord(c->ev_fork, st));
-            CU(cudaStreamWaitEvent(c->side[0], c->ev_fork, 0));
             CU(cudaStreamWaitEvent(c->side[1], c->ev_fork, 0));
-            launch_contact_prep(c->d_chans, c->M, c->mb, c->cb, c->ncells, c->side[0]);
-            CU(cudaEventRecord(c->ev_contact, c->side[0]));
-            launch_tiles(c->d_chans, c->d_caps, c->M, c->mb, c->tb, c->tb.T, p, c->d_phi,
-                         c->d_status, c->side[1], c->Kmax > 1 ? c->ev_slots : nullptr);
+            launch_tiles(c->d_chans, nch, c->d_caps, c->M, c->mb, c->tb, c->cb, c->ncells, p,
+                         c->d_phi, c->d_status, c->side[1], c->ev_slots);
             CU(cudaEventRecord(c->ev_tiles, c->side[1]));
             // the tile moments need the slot records only: they run beside
-            // the work order and the marker lists
+            // the marker lists
             if (c->Kmax > 1) {
                 CU(cudaStreamWaitEvent(c->side[2], c->ev_slots, 0));
                 launch_tile_moments<S, R>(c->d_chans, fp, c->tb, c->spread_grid, c->side[2]);
@@ -1227,33 +1207,33 @@ static int enqueue_step_t(sfg_context* c, int p) {
                 launches += 1;
             }
             launch_membrane(c->d_caps, c->NC, c->mb, c->d_has_prev, c->maxn, c->d_status, st);
-            CU(cudaStreamWaitEvent(st, c->ev_contact, 0));
+            CU(cudaStreamWaitEvent(st, c->ev_slots, 0));
             launch_contact_force(c->d_chans, c->M, c->mb, c->cb, st);
             if (c->pillar_repulsion) {
                 launch_obstacle_repulsion(c->d_chans, c->M, c->mb, st);
                 launches += 1;
             }
             CU(cudaStreamWaitEvent(st, c->ev_tiles, 0));
-            launch_spread<R>(c->d_chans, c->mb, c->tb, p, 0, MDF_PLAIN, 0, c->spread_grid,
+            launch_spread<R>(c->d_chans, c->mb, c->tb, p, 0, MDF_PLAIN, c->spread_grid,
                              c->d_status, st);
             if (c->Kmax > 1) CU(cudaStreamWaitEvent(st, c->ev_mom, 0));
-            launches += 1 + (c->ncells > 0 ? 7 : 1) + 10 + 1 + (c->Kmax > 1 ? 1 : 0);
+            launches += 1 + 1 + 3 + 1 + (c->Kmax > 1 ? 1 : 0);
         } else {
+            launch_tiles(c->d_chans, nch, c->d_caps, c->M, c->mb, c->tb, c->cb, c->ncells, p,
+                         c->d_phi, c->d_status, st);
+            mark(c, SFG_PHASE_IBM_TILES);
             launch_membrane(c->d_caps, c->NC, c->mb, c->d_has_prev, c->maxn, c->d_status, st);
             mark(c, SFG_PHASE_MEMBRANE);
-            launch_contact(c->d_chans, c->M, c->mb, c->cb, c->ncells, st);
+            launch_contact_force(c->d_chans, c->M, c->mb, c->cb, st);
             if (c->pillar_repulsion) {
                 launch_obstacle_repulsion(c->d_chans, c->M, c->mb, st);
                 launches += 1;
             }
             mark(c, SFG_PHASE_CONTACT);
-            launch_tiles(c->d_chans, c->d_caps, c->M, c->mb, c->tb, c->tb.T, p, c->d_phi,
-                         c->d_status, st);
-            mark(c, SFG_PHASE_IBM_TILES);
-            launch_spread<R>(c->d_chans, c->mb, c->tb, p, 0, MDF_PLAIN, 0, c->spread_grid,
+            launch_spread<R>(c->d_chans, c->mb, c->tb, p, 0, MDF_PLAIN, c->spread_grid,
                              c->d_status, st);
             mark(c, SFG_PHASE_IBM_SPREAD);
-            launches += 1 + (c->ncells > 0 ? 7 : 1) + 10 + 1;
+            launches += 1 + 1 + 3 + 1;
             if (c->Kmax > 1) {
                 launch_tile_moments<S, R>(c->d_chans, fp, c->tb, c->spread_grid, st);
                 mark(c, SFG_PHASE_MDF_INTERP);
@@ -1267,7 +1247,7 @@ static int enqueue_step_t(sfg_context* c, int p) {
                                      c->d_model, c->d_feat, c->d_frame, c->learned_grid,
                                      c->d_status, st);
             mark(c, SFG_PHASE_MDF_LEARNED);
-            launch_spread<R>(c->d_chans, c->mb, c->tb, p, 1, MDF_SEED, 1, c->spread_grid,
+            launch_spread<R>(c->d_chans, c->mb, c->tb, p, 1, MDF_SEED, c->spread_grid,
                              c->d_status, st);
             mark(c, SFG_PHASE_IBM_SPREAD);
             launch_mdf_interp<S, R>(c->d_chans, c->M, c->mb, fp, c->tb, p, 2, MDF_LEARNED, st);
@@ -1282,7 +1262,7 @@ static int enqueue_step_t(sfg_context* c, int p) {
             } else {
                 launch_plain_needed(c->d_chans, nch, c->tb, st);
             }
-            launch_spread<R>(c->d_chans, c->mb, c->tb, p, 2, MDF_LEARNED, 2, c->spread_grid,
+            launch_spread<R>(c->d_chans, c->mb, c->tb, p, 2, MDF_LEARNED, c->spread_grid,
                              c->d_status, st);
             if (par) CU(cudaStreamWaitEvent(st, c->ev_pn, 0));
             mark(c, SFG_PHASE_IBM_SPREAD);
@@ -1291,7 +1271,7 @@ static int enqueue_step_t(sfg_context* c, int p) {
         for (int k = 1; k < c->Kmax; ++k) {
             launch_mdf_interp<S, R>(c->d_chans, c->M, c->mb, fp, c->tb, p, k, MDF_PLAIN, st);
             mark(c, SFG_PHASE_MDF_INTERP);
-            launch_spread<R>(c->d_chans, c->mb, c->tb, p, k, MDF_PLAIN, 2 + k, c->spread_grid,
+            launch_spread<R>(c->d_chans, c->mb, c->tb, p, k, MDF_PLAIN, c->spread_grid,
                              c->d_status, st);
             mark(c, SFG_PHASE_IBM_SPREAD);
             launches += 2;
@@ -1339,7 +1319,7 @@ static int enqueue_step_t(sfg_context* c, int p) {
     mark(c, SFG_PHASE_BOOKKEEPING);
     launches += 2;
     if (c->M > 0) {
-        launch_interp_move<S, R>(c->d_chans, c->d_caps, c->NC, c->M, c->mb,
+        launch_interp_move<S, R>(c->d_chans, c->d_caps, c->NC, c->M, c->mb, c->cb,
                                  static_cast<const S*>(c->f[1 - p]), c->tb, p, c->d_phi, st);
         mark(c, SFG_PHASE_INTERP_MOVE);
         launches += 1;

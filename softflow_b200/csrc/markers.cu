@@ -310,47 +310,73 @@ __device__ __forceinline__ double2 pair_force(const ChannelDev& ch, double2 pa, 
     return make_double2(nrm.x * F_n + F_t.x, nrm.y * F_n + F_t.y);
 }
 
-__global__ void k_contact_bin(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
-                              int* __restrict__ cell_of, int* __restrict__ cell_cnt) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    const ChannelDev& ch = chans[mb.mk_chan[m]];
-    if (ch.brute_contact) return;
-    const int c = ch.cell_base + contact_cell(ch, mb.pos[m]);
-    cell_of[m] = c;
-    atomicAdd(&cell_cnt[c], 1);
-}
-
-__global__ void k_contact_fill(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
-                               const int* __restrict__ cell_of, const int* __restrict__ cell_start,
-                               int* __restrict__ cursor, int* __restrict__ list) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    const ChannelDev& ch = chans[mb.mk_chan[m]];
-    if (ch.brute_contact) return;
-    const int c = cell_of[m];
-    list[cell_start[c] + atomicAdd(&cursor[c], 1)] = m;
-}
-
-// Cells hold a handful of markers: insertion sort restores the reference's
-// insertion order (capsule-major, node-minor = ascending marker index).
-__global__ void k_contact_sort(int ncells, const int* __restrict__ cell_start,
-                               const int* __restrict__ cell_cnt, int* __restrict__ list) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncells) return;
-    int* a = list + cell_start[c];
-    const int n = cell_cnt[c];
-    for (int i = 1; i < n; ++i) {
-        const int v = a[i];
-        int j = i - 1;
-        while (j >= 0 && a[j] > v) { a[j + 1] = a[j]; --j; }
-        a[j + 1] = v;
+// The cell list without a scan: k_marker_prep pushes every marker onto its
+// cell's linked list (CellRec.head, CellRec::next by marker); here the marker
+// that reached its empty cell first walks that list, takes list space for the
+// cell (one atomic per warp), sorts the cell's markers into the reference's
+// insertion order (capsule-major, node-minor = ascending marker index) and
+// replaces the cell's record by (start, count).  Where a cell's markers lie
+// in the list does not matter, only their order within the cell.  The work
+// follows the markers instead of the cells (5 to 20 times as many), and the
+// records of visited cells are cleared again by the marker move, so nothing
+// runs over all cells: on 30 capsules the binning, three-kernel scan, fill
+// and sort with their two memsets were nine graph nodes in a row.
+constexpr int CONTACT_BUF = 32;   // markers of a cell sorted in thread-local memory
+__device__ __forceinline__ void contact_cells(int m, int M, const ChannelDev* __restrict__ chans,
+                                              const MarkerBufs& mb, const ContactBufs& cb,
+                                              int* __restrict__ total) {
+    bool owner = m < M;
+    int c = 0, n = 0, head = 0;
+    int buf[CONTACT_BUF];
+    if (owner) {
+        owner = !chans[mb.mk_chan[m]].brute_contact && cb.next[m] == 0;
+        if (owner) {
+            c = cb.cell_of[m];
+            head = cb.cell[c].x;
+            for (int i = head; i != 0; i = cb.next[i - 1]) {
+                if (n < CONTACT_BUF) buf[n] = i - 1;
+                ++n;
+            }
+        }
     }
+    const int lane = threadIdx.x & 31;
+    int inc = n;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    int base = 0;
+    if (lane == 31 && inc > 0) base = atomicAdd(total, inc);
+    base = __shfl_sync(0xffffffffu, base, 31) + inc - n;
+    if (!owner) return;
+    if (n <= CONTACT_BUF) {
+        for (int i = 1; i < n; ++i) {
+            const int v = buf[i];
+            int j = i - 1;
+            while (j >= 0 && buf[j] > v) { buf[j + 1] = buf[j]; --j; }
+            buf[j + 1] = v;
+        }
+        for (int i = 0; i < n; ++i) cb.list[base + i] = make_int2(buf[i], mb.mk_cap[buf[i]]);
+    } else {   // a crowded cell: sorted in place
+        int k = 0;
+        for (int i = head; i != 0; i = cb.next[i - 1], ++k) {
+            const int v = i - 1;
+            int j = k - 1;
+            while (j >= 0 && cb.list[base + j].x > v) { cb.list[base + j + 1] = cb.list[base + j]; --j; }
+            cb.list[base + j + 1] = make_int2(v, mb.mk_cap[v]);
+        }
+    }
+    for (int i = 0; i < n; ++i) cb.lpos[base + i] = mb.pos[cb.list[base + i].x];
+    cb.cell[c] = make_int2(base, n);
 }
 
+// One thread per marker.  The nine cell records of its 3 x 3 neighbourhood
+// are loaded together; an entry of the same capsule (most of them) costs one
+// 8-byte load, another capsule's entry also the position copied into the
+// list.  Velocities are read only where damping or friction use them.
 __global__ void k_contact_force(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
-                                const int* __restrict__ cell_of, const int* __restrict__ cell_start,
-                                const int* __restrict__ cell_cnt, const int* __restrict__ list) {
+                                ContactBufs cb) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M) return;
     const ChannelDev& ch = chans[mb.mk_chan[m]];
@@ -367,25 +393,29 @@ __global__ void k_contact_force(const ChannelDev* __restrict__ chans, int M, Mar
             ++count;
         }
     } else {
-        const int ci = cell_of[m] - ch.cell_base;
+        const int ci = cb.cell_of[m] - ch.cell_base;
         const int cx = ci % ch.ncx, cy = ci / ch.ncx;
-        for (int dy = -1; dy <= 1; ++dy) {
-            const int yy = cy + dy;
-            if (yy < 0 || yy >= ch.ncy) continue;
-            for (int dx = -1; dx <= 1; ++dx) {
-                int xx = cx + dx;
-                if (xx < 0) xx += ch.ncx;
-                if (xx >= ch.ncx) xx -= ch.ncx;
-                const int cell = ch.cell_base + yy * ch.ncx + xx;
-                const int s = cell_start[cell], e = s + cell_cnt[cell];
-                for (int k = s; k < e; ++k) {
-                    const int b = list[k];
-                    if (mb.mk_cap[b] == cap) continue;
-                    const double2 f = pair_force(ch, pa, va, mb.pos[b], mb.vel[b]);
-                    F.x = F.x + f.x;
-                    F.y = F.y + f.y;
-                    ++count;
-                }
+        const bool moving = ch.rep_damping > 0.0 || ch.rep_friction > 0.0;
+        int2 rec[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            const int yy = cy + k / 3 - 1;
+            int xx = cx + k % 3 - 1;
+            if (xx < 0) xx += ch.ncx;
+            if (xx >= ch.ncx) xx -= ch.ncx;
+            rec[k] = yy < 0 || yy >= ch.ncy ? make_int2(0, 0)
+                                            : cb.cell[ch.cell_base + yy * ch.ncx + xx];
+        }
+#pragma unroll
+        for (int k = 0; k < 9; ++k) {
+            for (int e = rec[k].x; e < rec[k].x + rec[k].y; ++e) {
+                const int2 o = cb.list[e];   // marker, capsule
+                if (o.y == cap) continue;
+                const double2 f = pair_force(ch, pa, va, cb.lpos[e],
+                                             moving ? mb.vel[o.x] : make_double2(0.0, 0.0));
+                F.x = F.x + f.x;
+                F.y = F.y + f.y;
+                ++count;
             }
         }
     }
@@ -427,15 +457,30 @@ __device__ __forceinline__ int stencil_tiles(const ChannelDev& ch, int ix0, int 
     return n;
 }
 
-// Per-marker preparation: arc length ds (min-image, immersed_boundary.cpp:
-// 164-173), stencil origin, validity, and the tile occupancy counts.
-__global__ void k_ibm_prep(const ChannelDev* __restrict__ chans,
-                           const CapsuleDev* __restrict__ caps, int M, MarkerBufs mb,
-                           const double* __restrict__ phi_tbl, int* __restrict__ tile_flag,
-                           int* __restrict__ tile_cnt, unsigned* status) {
+// Per-marker preparation: contact cell, arc length ds (min-image,
+// immersed_boundary.cpp:164-173), stencil origin, validity, and the tile
+// occupancy counts.  Also starts the step's counters and per-channel
+// results at zero (nothing else of the step runs before it, and the previous
+// step's have been read): as memsets these were five graph nodes in a row.
+__global__ void k_marker_prep(const ChannelDev* __restrict__ chans, int nch,
+                              const CapsuleDev* __restrict__ caps, int M, MarkerBufs mb,
+                              const double* __restrict__ phi_tbl, TileBufs tb, ContactBufs cb,
+                              unsigned* status) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int c = m; c < nch; c += gridDim.x * blockDim.x) {
+        tb.capped[c] = 0;
+        tb.fluid_touched[c] = 0;
+        tb.resid_gate[c] = 0u;
+        tb.resid_plain[c] = 0u;
+    }
+    if (m < NUM_STEP_CTR) tb.ctr[m] = 0;
     if (m >= M) return;
     const ChannelDev& ch = chans[mb.mk_chan[m]];
+    if (!ch.brute_contact) {
+        const int c = ch.cell_base + contact_cell(ch, mb.pos[m]);
+        cb.cell_of[m] = c;
+        cb.next[m] = atomicExch(&cb.cell[c].x, m + 1);
+    }
     const CapsuleDev& cp = caps[mb.mk_cap[m]];
     const int k = m - cp.off, n = cp.n;
     const int kp = cp.off + (k - 1 + n) % n, kn = cp.off + (k + 1) % n;
@@ -475,29 +520,54 @@ __global__ void k_ibm_prep(const ChannelDev* __restrict__ chans,
     for (int a = 0; a < 8; ++a) {
         const int key = a < nt ? t[a] : -1;
         const unsigned peers = __match_any_sync(__activemask(), key);
-        if (key >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1) {
-            tile_flag[key] = 1;
-            atomicAdd(&tile_cnt[key], __popc(peers));
-        }
+        if (key >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1)
+            atomicAdd(&tb.tile_cnt[key], __popc(peers));
     }
 }
 
 // Slot map of the step, and per slot the record the spread reads first
 // (SlotInfo: tile, channel, tile origin, list length and offset, nx, ny), so
-// that a spread warp starts a slot with one 32-byte load.
-__global__ void k_tile_slots(int T, const int* __restrict__ tile_flag,
-                             const int* __restrict__ slot_scan, int* __restrict__ tile_slot,
-                             int* __restrict__ slot_tile, const ChannelDev* __restrict__ chans,
-                             const int* __restrict__ tile_chan, const int* __restrict__ tile_cnt,
-                             const int* __restrict__ list_off, SlotInfo* __restrict__ info,
-                             int* __restrict__ cls_cnt, int* __restrict__ slot_rank) {
-    const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= T) return;
-    if (tile_flag[t]) {
-        const int s = slot_scan[t];
+// that a spread warp starts a slot with one 32-byte load.  One thread per
+// tile: a warp takes slots and list space for its touched tiles with one
+// atomic each (which numbers they get does not matter to any result), so no
+// scan runs before it.  The tile's count is cleared for the next step and
+// tile_pos[t] is left at the tile's first list entry for k_tile_fill.
+// Each slot is also entered under its list-length class (slot_order), for the
+// spread's work order.  The blocks after the tiles' build the contact cells.
+__global__ void k_tile_slots(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
+                             TileBufs tb, int* __restrict__ tile_slot, ContactBufs cb,
+                             int tile_blocks) {
+    if ((int)blockIdx.x >= tile_blocks) {
+        contact_cells((blockIdx.x - tile_blocks) * blockDim.x + threadIdx.x, M, chans, mb, cb,
+                      &tb.ctr[CTR_CONTACT]);
+        return;
+    }
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const int cnt = t < tb.T ? tb.tile_cnt[t] : 0;
+    const unsigned touched = __ballot_sync(0xffffffffu, cnt > 0);
+    if (touched == 0u) {                       // warp-uniform
+        if (t < tb.T) tile_slot[t] = -1;
+        return;
+    }
+    int inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    int sbase = 0, lbase = 0;
+    if (lane == 31) {
+        sbase = atomicAdd(&tb.ctr[CTR_SLOTS], __popc(touched));
+        lbase = atomicAdd(&tb.ctr[CTR_LIST], inc);
+    }
+    sbase = __shfl_sync(0xffffffffu, sbase, 31);
+    lbase = __shfl_sync(0xffffffffu, lbase, 31);
+    if (cnt > 0) {
+        const int s = sbase + __popc(touched & ((1u << lane) - 1u)), off = lbase + inc - cnt;
+        tb.tile_cnt[t] = 0;
+        tb.tile_pos[t] = off;
         tile_slot[t] = s;
-        slot_tile[s] = t;
-        const int chan = tile_chan[t];
+        const int chan = tb.tile_chan[t];
         const ChannelDev& ch = chans[chan];
         const int local = t - ch.tile_base;
         SlotInfo si;
@@ -505,46 +575,53 @@ __global__ void k_tile_slots(int T, const int* __restrict__ tile_flag,
         si.chan = chan;
         si.x0 = (local % ch.tiles_x) * TILE_W;
         si.y0 = (local / ch.tiles_x) * TILE_H;
-        si.cnt = tile_cnt[t];
-        si.off = list_off[t];
+        si.cnt = cnt;
+        si.off = off;
         si.nx = ch.nx;
         si.ny = ch.ny;
-        info[s] = si;
+        tb.slot_info[s] = si;
         // rank within the list-length class: one atomic per class and warp
-        const int cls = slot_class(si.cnt);
+        const int cls = slot_class(cnt);
         const unsigned peers = __match_any_sync(__activemask(), cls);
-        const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+        const int leader = __ffs(peers) - 1;
         int base = 0;
-        if (lane == leader) base = atomicAdd(&cls_cnt[cls], __popc(peers));
+        if (lane == leader) base = atomicAdd(&tb.ctr[CTR_CLASS + cls], __popc(peers));
         base = __shfl_sync(peers, base, leader);
-        slot_rank[s] = base + __popc(peers & ((1u << lane) - 1u));
-    } else {
+        tb.slot_order[(size_t)cls * tb.max_slots + base + __popc(peers & ((1u << lane) - 1u))] = s;
+    } else if (t < tb.T) {
         tile_slot[t] = -1;
     }
 }
 
 // The spread's work order: slots by descending class, any order within a
 // class (every slot's result is independent of the warp and of the order).
-__global__ void k_slot_order(const int* __restrict__ n_slots_p, const SlotInfo* __restrict__ info,
-                             const int* __restrict__ cls_cnt, const int* __restrict__ slot_rank,
-                             int* __restrict__ order) {
-    __shared__ int start[SLOT_CLASSES];
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int c = SLOT_CLASSES - 1; c >= 0; --c) {
-            start[c] = acc;
-            acc += cls_cnt[c];
+// Lane l holds the first position of class SLOT_CLASSES - 1 - l, so a
+// position's class is the last lane whose start does not exceed it.
+struct WorkOrder {
+    int start;
+    __device__ __forceinline__ explicit WorkOrder(const int* __restrict__ ctr) {
+        const int lane = threadIdx.x & 31;
+        const int n = lane < SLOT_CLASSES ? ctr[CTR_CLASS + SLOT_CLASSES - 1 - lane] : 0;
+        int inc = n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
         }
+        start = inc - n;
     }
-    __syncthreads();
-    const int n = *n_slots_p;
-    for (int s = blockIdx.x * blockDim.x + threadIdx.x; s < n; s += gridDim.x * blockDim.x)
-        order[start[slot_class(info[s].cnt)] + slot_rank[s]] = s;
-}
+    // (all lanes of the warp call it with the same position)
+    __device__ __forceinline__ int slot(const int* __restrict__ order, int max_slots, int p) const {
+        const bool below = (threadIdx.x & 31) < SLOT_CLASSES && start <= p;
+        const int l = __popc(__ballot_sync(0xffffffffu, below)) - 1;
+        const int s0 = __shfl_sync(0xffffffffu, start, l);
+        return order[(size_t)(SLOT_CLASSES - 1 - l) * max_slots + p - s0];
+    }
+};
 
 __global__ void k_tile_fill(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
-                            const int* __restrict__ list_off, int* __restrict__ cursor,
-                            int* __restrict__ list, const int* __restrict__ tile_slot) {
+                            int* __restrict__ tile_pos, int* __restrict__ list,
+                            const int* __restrict__ tile_slot) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M || !mb.valid[m]) return;
     const ChannelDev& ch = chans[mb.mk_chan[m]];
@@ -559,9 +636,9 @@ __global__ void k_tile_fill(const ChannelDev* __restrict__ chans, int M, MarkerB
         const unsigned peers = __match_any_sync(__activemask(), key);
         const int leader = __ffs(peers) - 1;
         int base = 0;
-        if (key >= 0 && lane == leader) base = atomicAdd(&cursor[key], __popc(peers));
+        if (key >= 0 && lane == leader) base = atomicAdd(&tile_pos[key], __popc(peers));
         base = __shfl_sync(peers, base, leader);
-        if (key >= 0) list[list_off[key] + base + __popc(peers & ((1u << lane) - 1u))] = m;
+        if (key >= 0) list[base + __popc(peers & ((1u << lane) - 1u))] = m;
     }
     // the slot of every stencil cell, by row tile and stencil column, for the
     // interpolations of the step (one 32-byte record instead of 16 lookups)
@@ -674,8 +751,7 @@ constexpr int spread_min_ctas() { return sizeof(R) == 4 ? 4 : 3; }
 template <typename R>
 __global__ void __launch_bounds__(SPREAD_WARPS * 32, spread_min_ctas<R>())
 k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot_info,
-         const int* __restrict__ slot_order, const int* __restrict__ n_slots_p,
-         int* __restrict__ slot_ctr,
+         const int* __restrict__ slot_order, const int* __restrict__ ctr, int max_slots,
          int* __restrict__ list, MarkerBufs mb, double* __restrict__ acc,
          double* __restrict__ acc0, R* __restrict__ gsnap, R* __restrict__ fin, int sweep,
          int mode, const unsigned* __restrict__ resid_gate,
@@ -690,7 +766,8 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
     A* ax = W.ax;
     A* ay = W.ay;
     int* sl = W.ck.list;
-    const int n_slots = *n_slots_p;
+    const int n_slots = ctr[CTR_SLOTS];
+    const WorkOrder wo(ctr);
     // slots are dealt to the warps in rounds over the work order (longest
     // lists first, alternating direction, so each warp's share sums to
     // about the same work; a shared claim counter serialises on one L2
@@ -701,7 +778,7 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
     // the warps in reverse order on odd rounds
     const int wid = blockIdx.x * SPREAD_WARPS + warp;
     int round = 0, next = wid;
-    int nslot = next < n_slots ? slot_order[next] : 0;
+    int nslot = next < n_slots ? wo.slot(slot_order, max_slots, next) : 0;
     SlotInfo nfo{};
     if (next < n_slots) nfo = slot_info[nslot];
     while (next < n_slots) {
@@ -710,7 +787,7 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
         ++round;
         next = round * nwarps + ((round & 1) ? nwarps - 1 - wid : wid);
         if (next < n_slots) {
-            nslot = slot_order[next];
+            nslot = wo.slot(slot_order, max_slots, next);
             nfo = slot_info[nslot];
         }
         const int chan = si.chan;
@@ -1063,7 +1140,7 @@ __device__ __forceinline__ float fx_value(unsigned lo, int hi) {
 
 __global__ void __launch_bounds__(SPREAD_WARPS * 32, 4)
 k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot_info,
-            const int* __restrict__ slot_order, const int* __restrict__ n_slots_p,
+            const int* __restrict__ slot_order, const int* __restrict__ ctr, int max_slots,
             const int* __restrict__ list, MarkerBufs mb,
             double* __restrict__ acc, double* __restrict__ acc0, float* __restrict__ gsnap,
             float* __restrict__ fin, int sweep, int mode, const unsigned* __restrict__ resid_gate,
@@ -1079,13 +1156,14 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
         W.hit[i] = 0;
     }
     __syncwarp();
-    const int n_slots = *n_slots_p;
+    const int n_slots = ctr[CTR_SLOTS];
+    const WorkOrder wo(ctr);
     const int nwarps = gridDim.x * SPREAD_WARPS;
     // round k takes work-order positions k nwarps .. (k + 1) nwarps - 1,
     // the warps in reverse order on odd rounds
     const int wid = blockIdx.x * SPREAD_WARPS + warp;
     int round = 0, next = wid;
-    int nslot = next < n_slots ? slot_order[next] : 0;
+    int nslot = next < n_slots ? wo.slot(slot_order, max_slots, next) : 0;
     SlotInfo nfo{};
     if (next < n_slots) nfo = slot_info[nslot];
     while (next < n_slots) {
@@ -1094,7 +1172,7 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
         ++round;
         next = round * nwarps + ((round & 1) ? nwarps - 1 - wid : wid);
         if (next < n_slots) {
-            nslot = slot_order[next];
+            nslot = wo.slot(slot_order, max_slots, next);
             nfo = slot_info[nslot];
         }
         const int chan = si.chan;
@@ -1396,8 +1474,11 @@ __global__ void k_tile_moments(const ChannelDev* __restrict__ chans,
 
 // Move marker m with its interpolated velocity u (simulation.cpp:656-675,
 // capsule.cpp:267-297).
-__device__ __forceinline__ void move_marker(const ChannelDev& ch, const MarkerBufs& mb, int m,
-                                            double2 u) {
+// The record of the marker's contact cell goes back to empty for the next
+// step (every marker of a cell stores the same zeros).
+__device__ __forceinline__ void move_marker(const ChannelDev& ch, const MarkerBufs& mb,
+                                            const ContactBufs& cb, int m, double2 u) {
+    if (!ch.brute_contact) cb.cell[cb.cell_of[m]] = make_int2(0, 0);
     double2 p = mb.pos[m];
     const double ux = u.x, uy = u.y;
     mb.vel[m] = make_double2(ux, uy);
@@ -1432,14 +1513,14 @@ __device__ __forceinline__ void move_marker(const ChannelDev& ch, const MarkerBu
 // thread per marker.
 template <typename S, typename R>
 __global__ void k_interp_move(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
-                              const S* __restrict__ f, const int* __restrict__ tile_slot,
+                              ContactBufs cb, const S* __restrict__ f, const int* __restrict__ tile_slot,
                               const R* __restrict__ fin, const double* __restrict__ phi_tbl) {
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M) return;
     const ChannelDev& ch = chans[mb.mk_chan[m]];
     double2 u = make_double2(0.0, 0.0);
     if (mb.valid[m]) u = interp_u_acc<S, R, R>(ch, mb, m, f, tile_slot, fin);
-    move_marker(ch, mb, m, u);
+    move_marker(ch, mb, cb, m, u);
 }
 
 // The marker move of the FP32-arithmetic modes, one warp per capsule: the
@@ -1469,8 +1550,9 @@ struct MoveBox {
 template <typename S>
 __global__ void __launch_bounds__(MOVE_WARPS * 32)
 k_interp_move_caps(const CapsuleDev* __restrict__ caps, int ncaps,
-                   const ChannelDev* __restrict__ chans, MarkerBufs mb, const S* __restrict__ f,
-                   const int* __restrict__ tile_slot, const float* __restrict__ fin) {
+                   const ChannelDev* __restrict__ chans, MarkerBufs mb, ContactBufs cb,
+                   const S* __restrict__ f, const int* __restrict__ tile_slot,
+                   const float* __restrict__ fin) {
     extern __shared__ __align__(16) unsigned char move_smem[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int c = blockIdx.x * MOVE_WARPS + warp;
@@ -1575,7 +1657,7 @@ k_interp_move_caps(const CapsuleDev* __restrict__ caps, int ncaps,
                 u = make_double2((double)ux, (double)uy);
             }
         }
-        move_marker(ch, mb, m, u);
+        move_marker(ch, mb, cb, m, u);
     }
 }
 
@@ -1856,79 +1938,44 @@ void launch_obstacle_repulsion(const ChannelDev* chans, int M, const MarkerBufs&
     k_obstacle_repulsion<<<(M + 255) / 256, 256, 0, st>>>(chans, M, mb);
 }
 
-void launch_contact(const ChannelDev* chans, int M, const MarkerBufs& mb, ContactBufs& cb,
-                    int ncells, cudaStream_t st) {
-    launch_contact_prep(chans, M, mb, cb, ncells, st);
-    launch_contact_force(chans, M, mb, cb, st);
-}
-
-void launch_contact_force(const ChannelDev* chans, int M, const MarkerBufs& mb, ContactBufs& cb,
-                          cudaStream_t st) {
+void launch_contact_force(const ChannelDev* chans, int M, const MarkerBufs& mb,
+                          const ContactBufs& cb, cudaStream_t st) {
     if (M == 0) return;
     const int B = 256, G = (M + B - 1) / B;
-    k_contact_force<<<G, B, 0, st>>>(chans, M, mb, cb.cell_of, cb.cell_start, cb.cell_cnt,
-                                     cb.list);
+    k_contact_force<<<G, B, 0, st>>>(chans, M, mb, cb);
 }
 
-void launch_contact_prep(const ChannelDev* chans, int M, const MarkerBufs& mb, ContactBufs& cb,
-                         int ncells, cudaStream_t st) {
-    if (M == 0) return;
-    const int B = 256, G = (M + B - 1) / B;
-    if (ncells > 0) {
-        cudaMemsetAsync(cb.cell_cnt, 0, sizeof(int) * ncells, st);
-        cudaMemsetAsync(cb.cursor, 0, sizeof(int) * ncells, st);
-        k_contact_bin<<<G, B, 0, st>>>(chans, M, mb, cb.cell_of, cb.cell_cnt);
-        scan_exclusive(cb.cell_cnt, cb.cell_start, ncells, cb.scan_tmp, nullptr, st);
-        k_contact_fill<<<G, B, 0, st>>>(chans, M, mb, cb.cell_of, cb.cell_start, cb.cursor,
-                                        cb.list);
-        k_contact_sort<<<(ncells + B - 1) / B, B, 0, st>>>(ncells, cb.cell_start, cb.cell_cnt,
-                                                           cb.list);
-    }
-}
-
-void launch_tiles(const ChannelDev* chans, const CapsuleDev* caps, int M, const MarkerBufs& mb,
-                  TileBufs& tb, int T, int parity, const double* phi_tbl, unsigned* status,
-                  cudaStream_t st, cudaEvent_t slots_ready) {
-    const int B = 256, G = (M + B - 1) / B;
-    cudaMemsetAsync(tb.tile_flag, 0, sizeof(int) * T, st);
-    cudaMemsetAsync(tb.tile_cnt, 0, sizeof(int) * T, st);
-    cudaMemsetAsync(tb.cursor, 0, sizeof(int) * T, st);
-    cudaMemsetAsync(tb.cls_cnt, 0, sizeof(int) * SLOT_CLASSES, st);
-    k_ibm_prep<<<G, B, 0, st>>>(chans, caps, M, mb, phi_tbl, tb.tile_flag, tb.tile_cnt, status);
-    scan_exclusive(tb.tile_flag, tb.slot_scan, T, tb.scan_tmp, tb.n_slots, st);
-    scan_exclusive(tb.tile_cnt, tb.list_off, T, tb.scan_tmp, nullptr, st);
-    k_tile_slots<<<(T + B - 1) / B, B, 0, st>>>(T, tb.tile_flag, tb.slot_scan,
-                                                tb.tile_slot[parity], tb.slot_tile, chans,
-                                                tb.tile_chan, tb.tile_cnt, tb.list_off,
-                                                tb.slot_info, tb.cls_cnt, tb.slot_rank);
+void launch_tiles(const ChannelDev* chans, int nch, const CapsuleDev* caps, int M,
+                  const MarkerBufs& mb, TileBufs& tb, const ContactBufs& cb, int ncells, int parity,
+                  const double* phi_tbl, unsigned* status, cudaStream_t st,
+                  cudaEvent_t slots_ready) {
+    const int B = 256, G = (M + B - 1) / B, TB = (tb.T + B - 1) / B;
+    k_marker_prep<<<G, B, 0, st>>>(chans, nch, caps, M, mb, phi_tbl, tb, cb, status);
+    k_tile_slots<<<TB + (ncells > 0 ? G : 0), B, 0, st>>>(chans, M, mb, tb, tb.tile_slot[parity],
+                                                          cb, TB);
     if (slots_ready) cudaEventRecord(slots_ready, st);
-    k_slot_order<<<148, 256, 0, st>>>(tb.n_slots, tb.slot_info, tb.cls_cnt, tb.slot_rank,
-                                      tb.slot_order);
-    k_tile_fill<<<G, B, 0, st>>>(chans, M, mb, tb.list_off, tb.cursor, tb.list,
-                                 tb.tile_slot[parity]);
+    k_tile_fill<<<G, B, 0, st>>>(chans, M, mb, tb.tile_pos, tb.list, tb.tile_slot[parity]);
 }
 
 template <typename R>
 void launch_spread(const ChannelDev* chans, const MarkerBufs& mb, TileBufs& tb, int parity,
-                   int sweep, int mode, int launch_idx, int grid, unsigned* status,
-                   cudaStream_t st) {
+                   int sweep, int mode, int grid, unsigned* status, cudaStream_t st) {
     if constexpr (sizeof(R) == 4) {
         k_spread_fx<<<grid, SPREAD_WARPS * 32, spread_fx_smem(), st>>>(
-            chans, tb.slot_info, tb.slot_order, tb.n_slots, tb.list, mb, tb.acc, tb.acc0,
+            chans, tb.slot_info, tb.slot_order, tb.ctr, tb.max_slots, tb.list, mb, tb.acc, tb.acc0,
             static_cast<float*>(tb.gsnap), static_cast<float*>(tb.fin[parity]), sweep, mode,
             tb.resid_gate, tb.plain_needed, tb.capped, tb.fluid_touched, status);
     } else {
         k_spread<R><<<grid, SPREAD_WARPS * 32, spread_smem<R>(), st>>>(
-            chans, tb.slot_info, tb.slot_order, tb.n_slots, tb.spread_ctr + launch_idx, tb.list,
-            mb, tb.acc,
+            chans, tb.slot_info, tb.slot_order, tb.ctr, tb.max_slots, tb.list, mb, tb.acc,
             tb.acc0, static_cast<R*>(tb.gsnap), static_cast<R*>(tb.fin[parity]), sweep, mode,
             tb.resid_gate, tb.plain_needed, tb.capped, tb.fluid_touched, status);
     }
 }
 template void launch_spread<double>(const ChannelDev*, const MarkerBufs&, TileBufs&, int, int,
-                                    int, int, int, unsigned*, cudaStream_t);
+                                    int, int, unsigned*, cudaStream_t);
 template void launch_spread<float>(const ChannelDev*, const MarkerBufs&, TileBufs&, int, int, int,
-                                   int, int, unsigned*, cudaStream_t);
+                                   int, unsigned*, cudaStream_t);
 
 template <typename S, typename R>
 void launch_mdf_interp(const ChannelDev* chans, int M, const MarkerBufs& mb, const S* f,
@@ -1944,24 +1991,24 @@ void launch_mdf_interp(const ChannelDev* chans, int M, const MarkerBufs& mb, con
 template <typename S, typename R>
 void launch_tile_moments(const ChannelDev* chans, const S* f, TileBufs& tb, int grid,
                          cudaStream_t st) {
-    k_tile_moments<S, R><<<grid, 256, 0, st>>>(chans, tb.slot_info, tb.n_slots, f,
+    k_tile_moments<S, R><<<grid, 256, 0, st>>>(chans, tb.slot_info, tb.ctr + CTR_SLOTS, f,
                                                static_cast<typename Mom4<R>::T*>(tb.mom));
 }
 
 template <typename S, typename R>
 void launch_interp_move(const ChannelDev* chans, const CapsuleDev* caps, int ncaps, int M,
-                        const MarkerBufs& mb, const S* f, TileBufs& tb, int parity,
-                        const double* phi_tbl, cudaStream_t st) {
+                        const MarkerBufs& mb, const ContactBufs& cb, const S* f, TileBufs& tb,
+                        int parity, const double* phi_tbl, cudaStream_t st) {
     if constexpr (sizeof(R) == 4) {
         (void)phi_tbl;
         if (ncaps == 0) return;
         k_interp_move_caps<S><<<(ncaps + MOVE_WARPS - 1) / MOVE_WARPS, MOVE_WARPS * 32,
                                 MOVE_WARPS * sizeof(MoveBox), st>>>(
-            caps, ncaps, chans, mb, f, tb.tile_slot[parity],
+            caps, ncaps, chans, mb, cb, f, tb.tile_slot[parity],
             static_cast<const float*>(tb.fin[parity]));
     } else {
         const int B = tb.marker_block, G = (M + B - 1) / B;
-        k_interp_move<S, R><<<G, B, 0, st>>>(chans, M, mb, f, tb.tile_slot[parity],
+        k_interp_move<S, R><<<G, B, 0, st>>>(chans, M, mb, cb, f, tb.tile_slot[parity],
                                              static_cast<const R*>(tb.fin[parity]), phi_tbl);
     }
 }
@@ -1972,8 +2019,8 @@ void launch_interp_move(const ChannelDev* chans, const CapsuleDev* caps, int nca
     template void launch_tile_moments<S, R>(const ChannelDev*, const S*, TileBufs&, int,       \
                                             cudaStream_t);                                      \
     template void launch_interp_move<S, R>(const ChannelDev*, const CapsuleDev*, int, int,     \
-                                           const MarkerBufs&, const S*, TileBufs&, int,        \
-                                           const double*, cudaStream_t);
+                                           const MarkerBufs&, const ContactBufs&, const S*,    \
+                                           TileBufs&, int, const double*, cudaStream_t);
 SFG_INST(double, double)
 SFG_INST(float, float)
 SFG_INST(__half, float)

@@ -7,13 +7,24 @@
 
 namespace sfg {
 
+// Contact cells of the step: while the list is built a cell's record is
+// (head marker + 1, 0) and `next` chains its markers; afterwards (start,
+// count) into the list.  Zero between steps.
 struct ContactBufs {
     int* cell_of = nullptr;     // [M] global contact cell of each marker
-    int* cell_cnt = nullptr;    // [ncells]
-    int* cell_start = nullptr;  // [ncells]
-    int* cursor = nullptr;      // [ncells]
-    int* list = nullptr;        // [M]
-    int* scan_tmp = nullptr;
+    int2* cell = nullptr;       // [ncells]
+    int* next = nullptr;        // [M] next marker + 1 of the same cell
+    int2* list = nullptr;       // [M] (marker, capsule), ascending within a cell
+    double2* lpos = nullptr;    // [M] position of each list entry
+};
+
+// Counters of one step (k_marker_prep zeroes them).
+enum StepCtr : int {
+    CTR_SLOTS = 0,              // force-tile slots
+    CTR_LIST = 1,               // marker list entries
+    CTR_CONTACT = 2,            // contact list entries
+    CTR_CLASS = 16,             // [SLOT_CLASSES] slots per list-length class
+    NUM_STEP_CTR = CTR_CLASS + SLOT_CLASSES
 };
 
 // Per-slot record of the step's force tiles (written by k_tile_slots).
@@ -25,16 +36,11 @@ struct TileBufs {
     int T = 0;                  // force tiles over all channels
     int max_slots = 0;
     int* tile_chan = nullptr;   // [T]
-    int* tile_flag = nullptr;   // [T]
-    int* tile_cnt = nullptr;    // [T] markers whose stencil covers the tile
-    int* cursor = nullptr;      // [T]
-    int* slot_scan = nullptr;   // [T]
-    int* list_off = nullptr;    // [T]
+    int* tile_cnt = nullptr;    // [T] markers whose stencil covers the tile (0 between steps)
+    int* tile_pos = nullptr;    // [T] next free list entry of the tile
     int* tile_slot[2] = {nullptr, nullptr};  // [T] per step parity
-    int* slot_tile = nullptr;   // [max_slots]
-    int* n_slots = nullptr;     // [1]
+    int* ctr = nullptr;         // [NUM_STEP_CTR] counters of the step
     int* list = nullptr;        // [8 M]
-    int* scan_tmp = nullptr;
     double* acc = nullptr;      // [max_slots][TILE_CELLS][2]: (x, y) per cell
     void* gsnap = nullptr;      // [max_slots][2][TILE_CELLS] (R)
     void* fin[2] = {nullptr, nullptr};
@@ -47,12 +53,7 @@ struct TileBufs {
     // The order in which the spread warps take the slots: by descending
     // class of list length (passes of 8 markers), so that each warp's share
     // of the step's tiles sums to about the same work.
-    int* slot_order = nullptr;      // [max_slots]
-    int* slot_rank = nullptr;       // [max_slots] rank of the slot within its class
-    int* cls_cnt = nullptr;         // [SLOT_CLASSES] slots per class
-    int* spread_ctr = nullptr;      // [n_spread_ctr] slot counters, one per spread launch of a
-                                    // step (zeroed at the start of the step)
-    int n_spread_ctr = 0;
+    int* slot_order = nullptr;      // [SLOT_CLASSES][max_slots] slots by class
     int* plain_needed = nullptr;  // [1] set when some channel needs the plain sweeps; null
                                   // (always run them) unless a channel is learned
     unsigned* resid_gate = nullptr;   // [nchan] learned form's no-slip residual (float bits)
@@ -73,29 +74,26 @@ cudaError_t prepare_spread();
 int spread_blocks_per_sm(bool fp64);
 void launch_membrane(const CapsuleDev* caps, int ncaps, const MarkerBufs& mb, int* has_prev,
                      int maxn, unsigned* status, cudaStream_t st);
-void launch_contact(const ChannelDev* chans, int M, const MarkerBufs& mb, ContactBufs& cb,
-                    int ncells, cudaStream_t st);
-// The cell list (binning, scan, fill, sort: positions only) and the pair
-// forces (added to the membrane forces) as separate launch groups.
-void launch_contact_prep(const ChannelDev* chans, int M, const MarkerBufs& mb, ContactBufs& cb,
-                         int ncells, cudaStream_t st);
-void launch_contact_force(const ChannelDev* chans, int M, const MarkerBufs& mb, ContactBufs& cb,
-                          cudaStream_t st);
+// Pair and wall contact forces, added to the membrane forces (after the
+// contact cells of launch_tiles).
+void launch_contact_force(const ChannelDev* chans, int M, const MarkerBufs& mb,
+                          const ContactBufs& cb, cudaStream_t st);
 // Repulsion of markers from the pillars of their channel (after the pairs).
 void launch_obstacle_repulsion(const ChannelDev* chans, int M, const MarkerBufs& mb,
                                cudaStream_t st);
-// `slots_ready` (may be null) is recorded once the slot records exist (the
-// tile moments need no more).
-void launch_tiles(const ChannelDev* chans, const CapsuleDev* caps, int M, const MarkerBufs& mb,
-                  TileBufs& tb, int T, int parity, const double* phi_tbl, unsigned* status,
-                  cudaStream_t st, cudaEvent_t slots_ready = nullptr);
+// The step's bookkeeping from the marker positions: stencils, contact cells,
+// force-tile slots and their marker lists.  `slots_ready` (may be null) is
+// recorded once the slot records and contact cells exist (the tile moments
+// and the contact forces need no more).
+void launch_tiles(const ChannelDev* chans, int nch, const CapsuleDev* caps, int M,
+                  const MarkerBufs& mb, TileBufs& tb, const ContactBufs& cb, int ncells, int parity,
+                  const double* phi_tbl, unsigned* status, cudaStream_t st,
+                  cudaEvent_t slots_ready = nullptr);
 // Spread of sweep `sweep` in forcing mode `mode` (MdfMode); sweep 0 spreads
-// the membrane and contact forces of every channel.  launch_idx: the
-// launch's slot counter in tb.spread_ctr (distinct per launch of a step).
+// the membrane and contact forces of every channel.
 template <typename R>
 void launch_spread(const ChannelDev* chans, const MarkerBufs& mb, TileBufs& tb, int parity,
-                   int sweep, int mode, int launch_idx, int grid, unsigned* status,
-                   cudaStream_t st);
+                   int sweep, int mode, int grid, unsigned* status, cudaStream_t st);
 template <typename S, typename R>
 void launch_mdf_interp(const ChannelDev* chans, int M, const MarkerBufs& mb, const S* f,
                        TileBufs& tb, int parity, int sweep, int mode, cudaStream_t st);
@@ -121,8 +119,8 @@ void launch_tile_moments(const ChannelDev* chans, const S* f, TileBufs& tb, int 
                          cudaStream_t st);
 template <typename S, typename R>
 void launch_interp_move(const ChannelDev* chans, const CapsuleDev* caps, int ncaps, int M,
-                        const MarkerBufs& mb, const S* f, TileBufs& tb, int parity,
-                        const double* phi_tbl, cudaStream_t st);
+                        const MarkerBufs& mb, const ContactBufs& cb, const S* f, TileBufs& tb,
+                        int parity, const double* phi_tbl, cudaStream_t st);
 
 // Lattice kernels (lattice_f64.cu / lattice_f32.cu).
 struct LatticeLaunch {
