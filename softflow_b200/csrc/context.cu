@@ -425,8 +425,9 @@ static void free_all(sfg_context* c) {
     F(c->d_has_prev);
     F(c->mb.pos); F(c->mb.vel); F(c->mb.frc); F(c->mb.dF); F(c->mb.ds);
     F(c->mb.rest_len); F(c->mb.rest_ang); F(c->mb.rest_ds); F(c->mb.prev_len);
-    F(c->mb.mk_cap); F(c->mb.mk_chan); F(c->mb.ix0); F(c->mb.iy0); F(c->mb.valid);
+    F(c->mb.mk_cap); F(c->mb.mk_chan); F(c->mb.org); F(c->mb.valid);
     F(c->mb.pair_count); F(c->mb.wx); F(c->mb.wy);
+    F(c->mb.wxf); F(c->mb.wyf); F(c->mb.wf); F(c->mb.dsf);
     F(c->tb.tile_chan); F(c->tb.tile_cnt); F(c->tb.tile_pos); F(c->tb.ctr);
     F(c->tb.list); F(c->tb.acc); F(c->tb.gsnap); F(c->tb.capped);
     F(c->tb.fluid_touched); F(c->tb.acc0); F(c->tb.mom); F(c->tb.slot_info); F(c->tb.slot_order); F(c->tb.resid_gate); F(c->tb.resid_plain);
@@ -994,19 +995,25 @@ extern "C" int sfg_initialize(sfg_context* c) {
     CU(dalloc(&c->mb.vel, M));
     CU(dalloc(&c->mb.frc, M));
     CU(dalloc(&c->mb.dF, M));
-    CU(dalloc(&c->mb.ds, M));
     CU(dalloc(&c->mb.rest_len, M));
     CU(dalloc(&c->mb.rest_ang, M));
     CU(dalloc(&c->mb.rest_ds, M));
     CU(dalloc(&c->mb.prev_len, M));
     CU(dalloc(&c->mb.mk_cap, M));
     CU(dalloc(&c->mb.mk_chan, M));
-    CU(dalloc(&c->mb.ix0, M));
-    CU(dalloc(&c->mb.iy0, M));
+    CU(dalloc(&c->mb.org, M));
     CU(dalloc(&c->mb.valid, M));
     CU(dalloc(&c->mb.pair_count, M));
-    CU(dalloc(&c->mb.wx, 4LL * M));
-    CU(dalloc(&c->mb.wy, 4LL * M));
+    if (c->precision == SFG_FP64) {
+        CU(dalloc(&c->mb.ds, M));
+        CU(dalloc(&c->mb.wx, 4LL * M));
+        CU(dalloc(&c->mb.wy, 4LL * M));
+    } else {
+        CU(dalloc(&c->mb.dsf, M));
+        CU(dalloc(&c->mb.wxf, M));
+        CU(dalloc(&c->mb.wyf, M));
+        CU(dalloc(&c->mb.wf, 4LL * M));
+    }
     CU(dalloc(&c->d_caps, c->NC));
     CU(dalloc(&c->d_has_prev, c->NC));
     if (c->any_chem) {
@@ -1188,7 +1195,7 @@ static int enqueue_step_t(sfg_context* c, int p) {
         if (par) {
             CU(cudaEventRecord(c->ev_fork, st));
             CU(cudaStreamWaitEvent(c->side[1], c->ev_fork, 0));
-            launch_tiles(c->d_chans, nch, c->d_caps, c->M, c->mb, c->tb, c->cb, c->ncells, p,
+            launch_tiles<R>(c->d_chans, nch, c->d_caps, c->M, c->mb, c->tb, c->cb, c->ncells, p,
                          c->d_phi, c->d_status, c->side[1], c->ev_slots);
             CU(cudaEventRecord(c->ev_tiles, c->side[1]));
             // the tile moments need the slot records only: they run beside
@@ -1219,7 +1226,7 @@ static int enqueue_step_t(sfg_context* c, int p) {
             if (c->Kmax > 1) CU(cudaStreamWaitEvent(st, c->ev_mom, 0));
             launches += 1 + 1 + 3 + 1 + (c->Kmax > 1 ? 1 : 0);
         } else {
-            launch_tiles(c->d_chans, nch, c->d_caps, c->M, c->mb, c->tb, c->cb, c->ncells, p,
+            launch_tiles<R>(c->d_chans, nch, c->d_caps, c->M, c->mb, c->tb, c->cb, c->ncells, p,
                          c->d_phi, c->d_status, st);
             mark(c, SFG_PHASE_IBM_TILES);
             launch_membrane(c->d_caps, c->NC, c->mb, c->d_has_prev, c->maxn, c->d_status, st);

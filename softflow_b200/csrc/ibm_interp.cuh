@@ -37,13 +37,11 @@ __device__ __forceinline__ double2 interp_u_acc(const ChannelDev& ch, const Mark
     // compute type: double in FP64 contexts (the reference's arithmetic),
     // float in the FP32-arithmetic modes
     using C = typename std::conditional<sizeof(R) == 8, double, float>::type;
-    const int ix0 = mb.ix0[m], iy0 = mb.iy0[m];
+    const int2 og = mb.org[m];
+    const int ix0 = og.x, iy0 = og.y;
     const StencilSlots ss(mb, m, iy0);
-    const double2* wx2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
-    const double2* wy2 = reinterpret_cast<const double2*>(mb.wy + 4 * (size_t)m);
-    const double2 wxa = wx2[0], wxb = wx2[1], wya = wy2[0], wyb = wy2[1];
-    const C wxs[4] = {(C)wxa.x, (C)wxa.y, (C)wxb.x, (C)wxb.y};
-    const C wys[4] = {(C)wya.x, (C)wya.y, (C)wyb.x, (C)wyb.y};
+    C wxs[4], wys[4];
+    stencil_weights(mb, m, wxs, wys);
     int jxs[4];
 #pragma unroll
     for (int sx = 0; sx < 4; ++sx) {
@@ -139,13 +137,11 @@ __device__ __forceinline__ double2 interp_u_mom(const ChannelDev& ch, const Mark
     // float in the FP32-arithmetic modes (fewer registers, more resident
     // warps for this latency-bound gather)
     using C = typename std::conditional<sizeof(R) == 8, double, float>::type;
-    const int ix0 = mb.ix0[m], iy0 = mb.iy0[m];
+    const int2 og = mb.org[m];
+    const int ix0 = og.x, iy0 = og.y;
     const StencilSlots ss(mb, m, iy0);
-    const double2* wx2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
-    const double2* wy2 = reinterpret_cast<const double2*>(mb.wy + 4 * (size_t)m);
-    const double2 wxa = wx2[0], wxb = wx2[1], wya = wy2[0], wyb = wy2[1];
-    const C wxs[4] = {(C)wxa.x, (C)wxa.y, (C)wxb.x, (C)wxb.y};
-    const C wys[4] = {(C)wya.x, (C)wya.y, (C)wyb.x, (C)wyb.y};
+    C wxs[4], wys[4];
+    stencil_weights(mb, m, wxs, wys);
     int jxs[4];
 #pragma unroll
     for (int sx = 0; sx < 4; ++sx) {

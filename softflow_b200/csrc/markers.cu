@@ -462,6 +462,7 @@ __device__ __forceinline__ int stencil_tiles(const ChannelDev& ch, int ix0, int 
 // occupancy counts.  Also starts the step's counters and per-channel
 // results at zero (nothing else of the step runs before it, and the previous
 // step's have been read): as memsets these were five graph nodes in a row.
+template <typename R>
 __global__ void k_marker_prep(const ChannelDev* __restrict__ chans, int nch,
                               const CapsuleDev* __restrict__ caps, int M, MarkerBufs mb,
                               const double* __restrict__ phi_tbl, TileBufs tb, ContactBufs cb,
@@ -488,7 +489,7 @@ __global__ void k_marker_prep(const ChannelDev* __restrict__ chans, int nch,
     const double2 p = mb.pos[m];
     const double dp = norm_d(min_image_d(p, mb.pos[kp], Lx));
     const double dn = norm_d(min_image_d(mb.pos[kn], p, Lx));
-    mb.ds[m] = 0.5 * (dp + dn);
+    const double ds = 0.5 * (dp + dn);
     int ok = finite2(p);
     int ix0 = 0, iy0 = 0;
     if (ok) {
@@ -504,15 +505,34 @@ __global__ void k_marker_prep(const ChannelDev* __restrict__ chans, int nch,
     } else if (!finite2(p)) {
         atomicOr(status, (unsigned)ST_NAN_MARKER);
     }
-    mb.ix0[m] = ix0;
-    mb.iy0[m] = iy0;
+    mb.org[m] = make_int2(ix0, iy0);
     mb.valid[m] = ok;
     if (!ok) return;
     // Peskin weights of the stencil, evaluated once per step (delta_function.h:44-59)
+    double wx[4], wy[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
-        mb.wx[4 * m + k] = phi_lut(phi_tbl, p.x - (double)(ix0 - 1 + k));
-        mb.wy[4 * m + k] = phi_lut(phi_tbl, p.y - (double)(iy0 - 1 + k));
+        wx[k] = phi_lut(phi_tbl, p.x - (double)(ix0 - 1 + k));
+        wy[k] = phi_lut(phi_tbl, p.y - (double)(iy0 - 1 + k));
+    }
+    if constexpr (sizeof(R) == 8) {
+        mb.ds[m] = ds;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            mb.wx[4 * (size_t)m + k] = wx[k];
+            mb.wy[4 * (size_t)m + k] = wy[k];
+        }
+    } else {
+        mb.dsf[m] = (float)ds;
+        mb.wxf[m] = make_float4((float)wx[0], (float)wx[1], (float)wx[2], (float)wx[3]);
+        mb.wyf[m] = make_float4((float)wy[0], (float)wy[1], (float)wy[2], (float)wy[3]);
+        auto point = [&](int k, int j) {
+            const double w = wx[k] * wy[j];
+            return w > 1e-15 ? (float)w : (w > 0.5e-15 ? WF_TOUCH_ONLY : WF_NONE);
+        };
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+            mb.wf[4 * (size_t)m + j] = make_float4(point(0, j), point(1, j), point(2, j), point(3, j));
     }
     int t[8];
     const int nt = stencil_tiles(ch, ix0, iy0, t);
@@ -625,7 +645,7 @@ __global__ void k_tile_fill(const ChannelDev* __restrict__ chans, int M, MarkerB
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M || !mb.valid[m]) return;
     const ChannelDev& ch = chans[mb.mk_chan[m]];
-    const int ix0 = mb.ix0[m], iy0 = mb.iy0[m];
+    const int ix0 = mb.org[m].x, iy0 = mb.org[m].y;
     int t[8];
     const int nt = stencil_tiles(ch, ix0, iy0, t);
     // one atomic per distinct tile and warp; the lanes of a tile take
@@ -898,8 +918,8 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
                 if (c + jm < cnt) {
                     const int m = lst[c + jm];
                     rf = sweep == 0 ? mb.frc[m] : mb.dF[m];
-                    rix = mb.ix0[m];
-                    riy = mb.iy0[m];
+                    rix = mb.org[m].x;
+                    riy = mb.org[m].y;
                     rds = mb.ds[m];
                     const double2* wx2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
                     rw0 = wx2[0];
@@ -993,8 +1013,8 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
             if (lane < SPREAD_CHUNK && c + lane < cnt) {
                 const int m = lst[c + lane];
                 rf = sweep == 0 ? mb.frc[m] : mb.dF[m];
-                rix = mb.ix0[m];
-                riy = mb.iy0[m];
+                rix = mb.org[m].x;
+                riy = mb.org[m].y;
                 rds = mb.ds[m];
                 const double2* wx2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
                 const double2* wy2 = reinterpret_cast<const double2*>(mb.wy + 4 * (size_t)m);
@@ -1195,55 +1215,60 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
             (ch.learned && (mode == MDF_SEED || (mode == MDF_PLAIN && sweep == 1))) ? acc0 : acc);
         const size_t base2 = (size_t)slot * TILE_CELLS;
         // four lanes per marker, one stencil row each, eight markers a pass;
-        // the next pass's marker data is loaded before this pass's points
+        // the next pass's marker data is loaded before this pass's points.
+        // Neighbouring list entries are neighbouring markers, whose stencils
+        // overlap: the lanes of marker jm take their four columns in an order
+        // rotated by jm, so that the warp's adds of one instruction meet
+        // fewer of each other's cells (same-address shared atomics serialise;
+        // along a vertical piece of membrane all eight markers share their
+        // columns)
         const int jm = lane >> 2, sy = lane & 3;
+        const bool rot1 = jm & 1, rot2 = jm & 2;
         struct Mk {
-            double2 f, w0, w1;
-            double ds, wy;
-            int ix, iy;
+            float4 w;
+            double2 f;
+            float ds;
+            int2 org;
         };
         auto fetch = [&](int c, Mk& k) {
             if (c + jm < cnt) {
                 const int m = lst[c + jm];
                 k.f = sweep == 0 ? mb.frc[m] : mb.dF[m];
-                k.ix = mb.ix0[m];
-                k.iy = mb.iy0[m];
-                k.ds = mb.ds[m];
-                const double2* wx2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
-                k.w0 = wx2[0];
-                k.w1 = wx2[1];
-                k.wy = mb.wy[4 * (size_t)m + sy];
+                k.org = mb.org[m];
+                k.ds = mb.dsf[m];
+                k.w = mb.wf[4 * (size_t)m + sy];
             }
         };
         Mk cur{}, nxt{};
         fetch(0, cur);
         for (int c0 = 0; c0 < cnt; c0 += 8) {
             fetch(c0 + 8, nxt);
-            if (c0 + jm < cnt) {
+            const int iy = cur.org.y - 1 + sy, cyl = iy - y0;
+            if (c0 + jm < cnt && cyl >= 0 && cyl < TILE_H && iy >= 0 && iy < ny) {
                 const bool ok = !(isnan(cur.f.x) || isnan(cur.f.y));
-                const int iy = cur.iy - 1 + sy, cyl = iy - y0;
-                const bool vrow = cyl >= 0 && cyl < TILE_H && iy >= 0 && iy < ny;
-                const double wxk[4] = {cur.w0.x, cur.w0.y, cur.w1.x, cur.w1.y};
-                const float fx = (float)cur.f.x, fy = (float)cur.f.y, ds = (float)cur.ds;
+                const float fx = (float)cur.f.x, fy = (float)cur.f.y, ds = cur.ds;
+                const float4 a = rot1 ? make_float4(cur.w.y, cur.w.z, cur.w.w, cur.w.x) : cur.w;
+                const float wr[4] = {rot2 ? a.z : a.x, rot2 ? a.w : a.y, rot2 ? a.x : a.z,
+                                     rot2 ? a.y : a.w};
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
-                    int jx = cur.ix - 1 + k;
+                    int jx = cur.org.x - 1 + ((k + jm) & 3);
                     if (jx < 0) jx += nx;
                     if (jx >= nx) jx -= nx;
                     const int cl = jx - x0;
-                    const double w = wxk[k] * cur.wy;
+                    const float wf = wr[k];
                     // touched: a superset of the points that the
                     // interpolations read (they test the weight in float)
-                    if (vrow && jx >= 0 && jx < nx && cl >= 0 && cl < TILE_W && w > 0.5e-15) {
+                    if (jx >= 0 && jx < nx && cl >= 0 && cl < TILE_W && wf != WF_NONE) {
                         const int i = cyl * ACC_W + cl;
                         W.hit[i] = 1;   // (lanes that meet here all store 1)
-                        if (!ok || !(w > 1e-15)) continue;
-                        const float wf = (float)w;
-                        const long long qx = fx_quant(fx * wf * ds), qy = fx_quant(fy * wf * ds);
-                        atomicAdd(&W.lo[0][i], fx_lo(qx));
-                        atomicAdd(&W.hi[0][i], fx_hi(qx));
-                        atomicAdd(&W.lo[1][i], fx_lo(qy));
-                        atomicAdd(&W.hi[1][i], fx_hi(qy));
+                        if (ok && wf != WF_TOUCH_ONLY) {
+                            const long long qx = fx_quant(fx * wf * ds), qy = fx_quant(fy * wf * ds);
+                            atomicAdd(&W.lo[0][i], fx_lo(qx));
+                            atomicAdd(&W.hi[0][i], fx_hi(qx));
+                            atomicAdd(&W.lo[1][i], fx_lo(qy));
+                            atomicAdd(&W.hi[1][i], fx_hi(qy));
+                        }
                     }
                 }
             }
@@ -1564,14 +1589,15 @@ k_interp_move_caps(const CapsuleDev* __restrict__ caps, int ncaps,
     // the stencils' box: x relative to the first marker (minimum image)
     int ref = 0;
     for (int k = 0; k < n; ++k)
-        if (mb.valid[off + k]) { ref = mb.ix0[off + k]; break; }
+        if (mb.valid[off + k]) { ref = mb.org[off + k].x; break; }
     int dmin = INT_MAX, dmax = INT_MIN, ymin = INT_MAX, ymax = INT_MIN;
     for (int k = lane; k < n; k += 32) {
         if (!mb.valid[off + k]) continue;
-        int d = mb.ix0[off + k] - ref;
+        const int2 og = mb.org[off + k];
+        int d = og.x - ref;
         if (2 * d > nx) d -= nx;
         if (2 * d < -nx) d += nx;
-        const int y = mb.iy0[off + k];
+        const int y = og.y;
         dmin = min(dmin, d);
         dmax = max(dmax, d);
         ymin = min(ymin, y);
@@ -1622,15 +1648,12 @@ k_interp_move_caps(const CapsuleDev* __restrict__ caps, int ncaps,
             if (!boxed) {
                 u = interp_u_acc_global<S>(ch, mb, m, f, tile_slot, fin);
             } else {
-                const int ix0 = mb.ix0[m], iy0 = mb.iy0[m];
+                const int ix0 = mb.org[m].x, iy0 = mb.org[m].y;
                 int d = ix0 - ref;
                 if (2 * d > nx) d -= nx;
                 if (2 * d < -nx) d += nx;
-                const double2* wx2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
-                const double2* wy2 = reinterpret_cast<const double2*>(mb.wy + 4 * (size_t)m);
-                const double2 wxa = wx2[0], wxb = wx2[1], wya = wy2[0], wyb = wy2[1];
-                const float wxs[4] = {(float)wxa.x, (float)wxa.y, (float)wxb.x, (float)wxb.y};
-                const float wys[4] = {(float)wya.x, (float)wya.y, (float)wyb.x, (float)wyb.y};
+                float wxs[4], wys[4];
+                stencil_weights(mb, m, wxs, wys);
                 float ux = 0.f, uy = 0.f;
 #pragma unroll
                 for (int sy = 0; sy < 4; ++sy) {
@@ -1945,17 +1968,25 @@ void launch_contact_force(const ChannelDev* chans, int M, const MarkerBufs& mb,
     k_contact_force<<<G, B, 0, st>>>(chans, M, mb, cb);
 }
 
+template <typename R>
 void launch_tiles(const ChannelDev* chans, int nch, const CapsuleDev* caps, int M,
                   const MarkerBufs& mb, TileBufs& tb, const ContactBufs& cb, int ncells, int parity,
                   const double* phi_tbl, unsigned* status, cudaStream_t st,
                   cudaEvent_t slots_ready) {
     const int B = 256, G = (M + B - 1) / B, TB = (tb.T + B - 1) / B;
-    k_marker_prep<<<G, B, 0, st>>>(chans, nch, caps, M, mb, phi_tbl, tb, cb, status);
+    k_marker_prep<R><<<G, B, 0, st>>>(chans, nch, caps, M, mb, phi_tbl, tb, cb, status);
     k_tile_slots<<<TB + (ncells > 0 ? G : 0), B, 0, st>>>(chans, M, mb, tb, tb.tile_slot[parity],
                                                           cb, TB);
     if (slots_ready) cudaEventRecord(slots_ready, st);
     k_tile_fill<<<G, B, 0, st>>>(chans, M, mb, tb.tile_pos, tb.list, tb.tile_slot[parity]);
 }
+
+template void launch_tiles<double>(const ChannelDev*, int, const CapsuleDev*, int, const MarkerBufs&,
+                                   TileBufs&, const ContactBufs&, int, int, const double*,
+                                   unsigned*, cudaStream_t, cudaEvent_t);
+template void launch_tiles<float>(const ChannelDev*, int, const CapsuleDev*, int, const MarkerBufs&,
+                                  TileBufs&, const ContactBufs&, int, int, const double*, unsigned*,
+                                  cudaStream_t, cudaEvent_t);
 
 template <typename R>
 void launch_spread(const ChannelDev* chans, const MarkerBufs& mb, TileBufs& tb, int parity,

@@ -24,12 +24,19 @@ struct MarkerBufs {
     double* prev_len;
     int* mk_cap;        // capsule of each marker
     int* mk_chan;       // channel of each marker
-    int* ix0;           // floor(x), floor(y) of the current step
-    int* iy0;
+    int2* org;          // stencil origin of the step: floor(x), floor(y)
     int* valid;         // finite position with its stencil rows near the lattice
     int* pair_count;    // contact pairs visited per marker (bookkeeping)
-    double* wx;         // [M][4] phi(x - ix) for ix = ix0-1 .. ix0+2 (this step)
-    double* wy;         // [M][4] phi(y - iy) for iy = iy0-1 .. iy0+2
+    // Stencil weights of the step, phi(x - ix) for ix = ix0-1 .. ix0+2 and
+    // phi(y - iy) for iy = iy0-1 .. iy0+2: in FP64 contexts the doubles; in the
+    // FP32-arithmetic modes what their kernels compute with, formed once
+    double* wx;         // [M][4] FP64 contexts
+    double* wy;
+    float4* wxf;        // [M] the weights rounded to float (interpolations)
+    float4* wyf;
+    float4* wf;         // [M][4] spread weight of each stencil row's points: the double
+                        // product rounded to float, or one of the marks below
+    float* dsf;         // [M] arc length rounded to float
     // multi-direct forcing state of the learned form and its training data
     double2* u0;        // velocity interpolated after the membrane-force spread
     double2* dFsum;     // forcing correction of this step summed over its sweeps
@@ -38,6 +45,28 @@ struct MarkerBufs {
     // [row tile (of the first / last stencil row)][stencil column sx]
     int* slot8;
 };
+
+// Marks in MarkerBufs::wf of points that take no part in the spread: a weight
+// of at most 1e-15 that the interpolations may still read (they test a float
+// product), and one that nothing reads.
+constexpr float WF_TOUCH_ONLY = -1.0f;
+constexpr float WF_NONE = -2.0f;
+
+// The marker's stencil weights in the compute type of a context.
+__device__ __forceinline__ void stencil_weights(const MarkerBufs& mb, int m, double wx[4],
+                                                double wy[4]) {
+    const double2* x2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
+    const double2* y2 = reinterpret_cast<const double2*>(mb.wy + 4 * (size_t)m);
+    const double2 xa = x2[0], xb = x2[1], ya = y2[0], yb = y2[1];
+    wx[0] = xa.x; wx[1] = xa.y; wx[2] = xb.x; wx[3] = xb.y;
+    wy[0] = ya.x; wy[1] = ya.y; wy[2] = yb.x; wy[3] = yb.y;
+}
+__device__ __forceinline__ void stencil_weights(const MarkerBufs& mb, int m, float wx[4],
+                                                float wy[4]) {
+    const float4 x = mb.wxf[m], y = mb.wyf[m];
+    wx[0] = x.x; wx[1] = x.y; wx[2] = x.z; wx[3] = x.w;
+    wy[0] = y.x; wy[1] = y.y; wy[2] = y.z; wy[3] = y.w;
+}
 
 // ---------------- Peskin 4-point delta via the 1024-bin table --------------
 // reference delta_function.h:44-54 (table built on the host from :18-26)

@@ -85,6 +85,7 @@ void launch_obstacle_repulsion(const ChannelDev* chans, int M, const MarkerBufs&
 // force-tile slots and their marker lists.  `slots_ready` (may be null) is
 // recorded once the slot records and contact cells exist (the tile moments
 // and the contact forces need no more).
+template <typename R>
 void launch_tiles(const ChannelDev* chans, int nch, const CapsuleDev* caps, int M,
                   const MarkerBufs& mb, TileBufs& tb, const ContactBufs& cb, int ncells, int parity,
                   const double* phi_tbl, unsigned* status, cudaStream_t st,
