@@ -1250,14 +1250,13 @@ static int enqueue_step_t(sfg_context* c, int p) {
         if (c->any_learned) {
             // seed, one plain sweep, gate; the plain sweeps below run only for
             // channels above the threshold
-            launch_mdf_learned<S, R>(c->d_chans, c->d_caps, c->M, c->mb, fp, c->tb, p,
-                                     c->d_model, c->d_feat, c->d_frame, c->learned_grid,
+            launch_mdf_learned<R>(c->d_chans, c->d_caps, c->M, c->mb, c->tb, c->d_model, c->d_feat, c->d_frame, c->learned_grid,
                                      c->d_status, st);
             mark(c, SFG_PHASE_MDF_LEARNED);
             launch_spread<R>(c->d_chans, c->mb, c->tb, p, 1, MDF_SEED, c->spread_grid,
                              c->d_status, st);
             mark(c, SFG_PHASE_IBM_SPREAD);
-            launch_mdf_interp<S, R>(c->d_chans, c->M, c->mb, fp, c->tb, p, 2, MDF_LEARNED, st);
+            launch_mdf_interp<R>(c->d_chans, c->M, c->mb, c->tb, 2, MDF_LEARNED, st);
             mark(c, SFG_PHASE_MDF_INTERP);
             // whether any channel falls back needs the gate residuals only:
             // it is found beside the last spread, and the plain sweeps wait
@@ -1276,7 +1275,7 @@ static int enqueue_step_t(sfg_context* c, int p) {
             launches += 6;
         }
         for (int k = 1; k < c->Kmax; ++k) {
-            launch_mdf_interp<S, R>(c->d_chans, c->M, c->mb, fp, c->tb, p, k, MDF_PLAIN, st);
+            launch_mdf_interp<R>(c->d_chans, c->M, c->mb, c->tb, k, MDF_PLAIN, st);
             mark(c, SFG_PHASE_MDF_INTERP);
             launch_spread<R>(c->d_chans, c->mb, c->tb, p, k, MDF_PLAIN, c->spread_grid,
                              c->d_status, st);

@@ -128,11 +128,9 @@ template <> struct Mom4<float> { using T = float4; };
 // column and row 1 or 2).
 template <typename R, bool NEAR = false>
 __device__ __forceinline__ double2 interp_u_mom(const ChannelDev& ch, const MarkerBufs& mb, int m,
-                                               const int* __restrict__ tile_slot,
                                                const typename Mom4<R>::T* __restrict__ mom,
                                                const double* __restrict__ acc,
                                                double& rho_near) {
-    (void)tile_slot;
     // compute type: double in FP64 contexts (the reference's arithmetic),
     // float in the FP32-arithmetic modes (fewer registers, more resident
     // warps for this latency-bound gather)
@@ -228,6 +226,126 @@ __device__ __forceinline__ double2 interp_u_mom(const ChannelDev& ch, const Mark
     }
     return make_double2((double)ux, (double)uy);
 }
+
+// interp_u_mom with four lanes per marker: lane `row` of the quad loads the four
+// cells of its stencil row at once and forms their terms, then the rows' terms
+// are added in the same order (row by row, the running sum passed from lane to
+// lane), so the result is the one-thread sum bit for bit.  Every lane of the
+// quad gets u and rho_near.  All lanes of the warp call this; a quad with
+// on = false reads nothing.
+template <typename R>
+__device__ __forceinline__ double2 quad_interp(const ChannelDev& ch, const MarkerBufs& mb, int m,
+                                               bool on, int row,
+                                               const typename Mom4<R>::T* __restrict__ mom,
+                                               const double* __restrict__ acc,
+                                               double& rho_near) {
+    // compute type: double in FP64 contexts (the reference's arithmetic),
+    // float in the FP32-arithmetic modes
+    using C = typename std::conditional<sizeof(R) == 8, double, float>::type;
+    C tx[4], ty[4], near = 1;
+    int syn = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) tx[i] = ty[i] = 0;
+    if (on) {
+        const int2 og = mb.org[m];
+        const int jy = og.y - 1 + row;
+        C wx[4], wy;
+        int4 sl4;
+        {
+            const int ty0 = max(og.y - 1, 0) / TILE_H;
+            sl4 = reinterpret_cast<const int4*>(mb.slot8 + 8 * (size_t)m)[jy / TILE_H != ty0 ? 1 : 0];
+        }
+        if constexpr (sizeof(R) == 8) {
+            const double2* x2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
+            const double2 xa = x2[0], xb = x2[1];
+            wx[0] = xa.x; wx[1] = xa.y; wx[2] = xb.x; wx[3] = xb.y;
+            wy = mb.wy[4 * (size_t)m + row];
+        } else {
+            const float4 x = mb.wxf[m];
+            wx[0] = x.x; wx[1] = x.y; wx[2] = x.z; wx[3] = x.w;
+            wy = reinterpret_cast<const float*>(mb.wyf)[4 * (size_t)m + row];
+        }
+        const int sl[4] = {sl4.x, sl4.y, sl4.z, sl4.w};
+        typename Mom4<R>::T q[4];
+        C fx[4], fy[4];
+        bool in[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            int jx = og.x - 1 + i;
+            if (jx < 0) jx += ch.nx;
+            if (jx >= ch.nx) jx -= ch.nx;
+            in[i] = jy >= 0 && jy < ch.ny && jx >= 0 && jx < ch.nx && sl[i] >= 0;
+            if (in[i]) {
+                const size_t at = (size_t)sl[i] * TILE_CELLS + (jy % TILE_H) * TILE_W + (jx % TILE_W);
+                q[i] = mom[at];
+                // (x, y) pairs of R: double2 in FP64 contexts, float2 otherwise
+                if constexpr (sizeof(R) == 8) {
+                    const double2 a = reinterpret_cast<const double2*>(acc)[at];
+                    fx[i] = a.x;
+                    fy[i] = a.y;
+                } else {
+                    const float2 a = reinterpret_cast<const float2*>(acc)[at];
+                    fx[i] = a.x;
+                    fy[i] = a.y;
+                }
+            }
+        }
+        // the nearest node's stencil column and row (always 1 or 2 for a
+        // finite position; otherwise, or outside the lattice, the density is 1)
+        const double2 p = mb.pos[m];
+        int ixr = (int)(p.x + 0.5);
+        const int iyr = (int)(p.y + 0.5), sxn = ixr - og.x + 1;
+        if (ixr < 0) ixr += ch.nx;
+        if (ixr >= ch.nx) ixr -= ch.nx;
+        syn = iyr - (og.y - 1);
+        const bool seen = iyr >= 0 && iyr < ch.ny && ixr >= 0 && ixr < ch.nx && sxn >= 0 &&
+                          sxn <= 3 && syn >= 0 && syn <= 3;
+        syn = syn < 0 ? 0 : (syn > 3 ? 3 : syn);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            if (!in[i]) continue;
+            if (seen && i == sxn) near = (C)q[i].x;
+            const C w = wx[i] * wy;
+            if (w > (C)1e-15) {
+                const C rho = (C)q[i].x;
+                C cu = 0, cv = 0;
+                if (rho > (C)1e-15) {
+                    if constexpr (sizeof(R) == 8) {
+                        cu = ((double)q[i].y + 0.5 * fx[i]) / rho;
+                        cv = ((double)q[i].z + 0.5 * fy[i]) / rho;
+                    } else {
+                        const float inv = __frcp_rn(rho);
+                        cu = (q[i].y + 0.5f * fx[i]) * inv;
+                        cv = (q[i].z + 0.5f * fy[i]) * inv;
+                    }
+                }
+                tx[i] = cu * w;
+                ty[i] = cv * w;
+            }
+        }
+    }
+    rho_near = (double)__shfl_sync(0xffffffffu, near, syn, 4);
+    // a term that takes no part is +0, which leaves the sum as it is (it
+    // starts at +0 and can never become -0)
+    C ux = 0, uy = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+        const C sx = (((ux + tx[0]) + tx[1]) + tx[2]) + tx[3];
+        const C sy = (((uy + ty[0]) + ty[1]) + ty[2]) + ty[3];
+        ux = __shfl_sync(0xffffffffu, sx, r, 4);
+        uy = __shfl_sync(0xffffffffu, sy, r, 4);
+    }
+    return make_double2((double)ux, (double)uy);
+}
+
+// Whether a per-marker interpolation takes four lanes a marker.  Few markers
+// cannot fill the chip and every kernel is one warp's chain of dependent loads
+// and instructions, which the quad shortens (1,455 instructions a warp to a
+// third; 720 markers: 8.6 -> 5.2 us a sweep); with many the one-thread form
+// does the same loads with less work around them (204 k markers: the step's
+// interpolations 111 us against 117).  The line lies where the quads' warps
+// fill one resident wave of the chip.
+inline bool interp_by_quads(int M) { return M <= 32768; }
 
 // Inputs of the forcing network in the marker's local frame (tangent t along
 // e_prev + e_next, normal n = (-t_y, t_x)):

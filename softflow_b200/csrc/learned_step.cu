@@ -33,18 +33,24 @@ __device__ __forceinline__ bool learned_marker(const ChannelDev* __restrict__ ch
 // Interpolation after the membrane spread (with the step's tile moments) and
 // the network inputs of every marker of a learned channel: u0, feat [M][8] and
 // the local tangent frame [M].
-template <typename R>
+template <typename R, bool QUAD>
 __global__ void k_mdf_features(const ChannelDev* __restrict__ chans,
                                const CapsuleDev* __restrict__ caps, int M, MarkerBufs mb,
-                               const int* __restrict__ tile_slot,
                                const typename Mom4<R>::T* __restrict__ mom,
                                const double* __restrict__ acc, float* __restrict__ feat,
                                double2* __restrict__ frame) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M || !learned_marker(chans, mb, m)) return;
-    const ChannelDev& ch = chans[mb.mk_chan[m]];
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, m = QUAD ? tid >> 2 : tid;
+    const bool on = m < M && learned_marker(chans, mb, m);
+    const ChannelDev& ch = chans[on ? mb.mk_chan[m] : 0];
     double unused;
-    const double2 u0 = interp_u_mom<R>(ch, mb, m, tile_slot, mom, acc, unused);
+    double2 u0;
+    if constexpr (QUAD) {
+        u0 = quad_interp<R>(ch, mb, m, on, tid & 3, mom, acc, unused);
+        if (!on || (tid & 3) != 0) return;
+    } else {
+        if (!on) return;
+        u0 = interp_u_mom<R>(ch, mb, m, mom, acc, unused);
+    }
     float fe[8];
     double2 t, nrm;
     mdf_features(ch, caps[mb.mk_cap[m]], mb, m, u0, fe, t, nrm);
@@ -133,16 +139,16 @@ cudaError_t prepare_mdf_learned() {
                                 (int)sizeof(mlp::FwdSmemDual));
 }
 
-template <typename S, typename R>
+template <typename R>
 void launch_mdf_learned(const ChannelDev* chans, const CapsuleDev* caps, int M,
-                        const MarkerBufs& mb, const S* f, TileBufs& tb, int parity,
-                        const void* model, float* feat, double2* frame, int grid,
-                        unsigned* status, cudaStream_t st) {
+                        const MarkerBufs& mb, TileBufs& tb, const void* model, float* feat,
+                        double2* frame, int grid, unsigned* status, cudaStream_t st) {
     if (M <= 0) return;
-    (void)f;
-    k_mdf_features<R><<<(M + tb.marker_block - 1) / tb.marker_block, tb.marker_block, 0, st>>>(
-        chans, caps, M, mb, tb.tile_slot[parity], static_cast<const typename Mom4<R>::T*>(tb.mom),
-        tb.acc0, feat, frame);   // a learned channel's sweep-0 force is in acc0
+    const bool quads = interp_by_quads(M);
+    const int B = tb.marker_block, G = ((quads ? 4 * M : M) + B - 1) / B;
+    // a learned channel's sweep-0 force is in acc0
+    (quads ? k_mdf_features<R, true> : k_mdf_features<R, false>)<<<G, B, 0, st>>>(
+        chans, caps, M, mb, static_cast<const typename Mom4<R>::T*>(tb.mom), tb.acc0, feat, frame);
     const int tiles = (M + mlp::ROWS - 1) / mlp::ROWS;
     const int g = tiles < grid ? tiles : grid;
     k_mdf_seed<<<g, mlp::ROWS, sizeof(mlp::FwdSmemDual), st>>>(
@@ -155,14 +161,11 @@ void launch_harvest(const ChannelDev* chans, const CapsuleDev* caps, int M, cons
     k_harvest<<<(M + 127) / 128, 128, 0, st>>>(chans, caps, M, mb, feat, label, valid);
 }
 
-#define SFG_INST(S, R)                                                                        \
-    template void launch_mdf_learned<S, R>(const ChannelDev*, const CapsuleDev*, int,          \
-                                           const MarkerBufs&, const S*, TileBufs&, int,        \
-                                           const void*, float*, double2*, int, unsigned*,      \
-                                           cudaStream_t);
-SFG_INST(double, double)
-SFG_INST(float, float)
-SFG_INST(__half, float)
-#undef SFG_INST
+template void launch_mdf_learned<double>(const ChannelDev*, const CapsuleDev*, int,
+                                         const MarkerBufs&, TileBufs&, const void*, float*,
+                                         double2*, int, unsigned*, cudaStream_t);
+template void launch_mdf_learned<float>(const ChannelDev*, const CapsuleDev*, int,
+                                        const MarkerBufs&, TileBufs&, const void*, float*,
+                                        double2*, int, unsigned*, cudaStream_t);
 
 }  // namespace sfg

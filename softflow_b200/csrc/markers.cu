@@ -1389,24 +1389,29 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
 // correction (dFsum), the first sweep's interpolation (u0) and the no-slip
 // residual max |U_prev - U_interp| per channel: at the learned form's sweep
 // (resid_gate) and at a plain iteration's last sweep (resid_plain).
-template <typename S, typename R>
+template <typename R, bool QUAD>
 __global__ void k_mdf_interp(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
-                             const int* __restrict__ tile_slot,
                              const typename Mom4<R>::T* __restrict__ mom,
                              const double* __restrict__ acc, const double* __restrict__ acc0,
                              int sweep, int mode, unsigned* __restrict__ resid_gate,
                              unsigned* __restrict__ resid_plain,
                              const int* __restrict__ plain_needed) {
     if (mode == MDF_PLAIN && plain_needed && !*plain_needed) return;  // no channel needs it
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    const int chan = mb.mk_chan[m];
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, m = QUAD ? t >> 2 : t;
+    const int chan = m < M ? mb.mk_chan[m] : 0;
     const ChannelDev& ch = chans[chan];
-    if (sweep >= ch.ibm_iterations || !mb.valid[m]) return;
-    if (!mdf_active(ch, mode, resid_gate, chan)) return;
+    const bool on = m < M && sweep < ch.ibm_iterations && mb.valid[m] &&
+                    mdf_active(ch, mode, resid_gate, chan);
     const double* base = (mode == MDF_PLAIN && ch.learned && sweep == 1) ? acc0 : acc;
     double rho_local;
-    const double2 u = interp_u_mom<R, true>(ch, mb, m, tile_slot, mom, base, rho_local);
+    double2 u;
+    if constexpr (QUAD) {
+        u = quad_interp<R>(ch, mb, m, on, t & 3, mom, base, rho_local);
+        if (!on || (t & 3) != 0) return;
+    } else {
+        if (!on) return;
+        u = interp_u_mom<R, true>(ch, mb, m, mom, base, rho_local);
+    }
     const double2 v = mb.vel[m];
     const double dux = v.x - u.x, duy = v.y - u.y;
     const double2 d = make_double2(dux * (2.0 * rho_local), duy * (2.0 * rho_local));
@@ -2008,16 +2013,19 @@ template void launch_spread<double>(const ChannelDev*, const MarkerBufs&, TileBu
 template void launch_spread<float>(const ChannelDev*, const MarkerBufs&, TileBufs&, int, int, int,
                                    int, unsigned*, cudaStream_t);
 
-template <typename S, typename R>
-void launch_mdf_interp(const ChannelDev* chans, int M, const MarkerBufs& mb, const S* f,
-                       TileBufs& tb, int parity, int sweep, int mode, cudaStream_t st) {
-    (void)f;
-    const int B = tb.marker_block, G = (M + B - 1) / B;
-    k_mdf_interp<S, R><<<G, B, 0, st>>>(chans, M, mb, tb.tile_slot[parity],
-                                        static_cast<const typename Mom4<R>::T*>(tb.mom), tb.acc,
-                                        tb.acc0, sweep, mode, tb.resid_gate, tb.resid_plain,
-                                        tb.plain_needed);
+template <typename R>
+void launch_mdf_interp(const ChannelDev* chans, int M, const MarkerBufs& mb, TileBufs& tb,
+                       int sweep, int mode, cudaStream_t st) {
+    const bool quads = interp_by_quads(M);
+    const int B = tb.marker_block, G = ((quads ? 4 * M : M) + B - 1) / B;
+    (quads ? k_mdf_interp<R, true> : k_mdf_interp<R, false>)<<<G, B, 0, st>>>(
+        chans, M, mb, static_cast<const typename Mom4<R>::T*>(tb.mom), tb.acc, tb.acc0, sweep,
+        mode, tb.resid_gate, tb.resid_plain, tb.plain_needed);
 }
+template void launch_mdf_interp<double>(const ChannelDev*, int, const MarkerBufs&, TileBufs&, int,
+                                        int, cudaStream_t);
+template void launch_mdf_interp<float>(const ChannelDev*, int, const MarkerBufs&, TileBufs&, int,
+                                       int, cudaStream_t);
 
 template <typename S, typename R>
 void launch_tile_moments(const ChannelDev* chans, const S* f, TileBufs& tb, int grid,
@@ -2045,8 +2053,6 @@ void launch_interp_move(const ChannelDev* chans, const CapsuleDev* caps, int nca
 }
 
 #define SFG_INST(S, R)                                                                          \
-    template void launch_mdf_interp<S, R>(const ChannelDev*, int, const MarkerBufs&, const S*,  \
-                                          TileBufs&, int, int, int, cudaStream_t);              \
     template void launch_tile_moments<S, R>(const ChannelDev*, const S*, TileBufs&, int,       \
                                             cudaStream_t);                                      \
     template void launch_interp_move<S, R>(const ChannelDev*, const CapsuleDev*, int, int,     \

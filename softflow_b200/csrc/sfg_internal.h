@@ -95,17 +95,16 @@ void launch_tiles(const ChannelDev* chans, int nch, const CapsuleDev* caps, int 
 template <typename R>
 void launch_spread(const ChannelDev* chans, const MarkerBufs& mb, TileBufs& tb, int parity,
                    int sweep, int mode, int grid, unsigned* status, cudaStream_t st);
-template <typename S, typename R>
-void launch_mdf_interp(const ChannelDev* chans, int M, const MarkerBufs& mb, const S* f,
-                       TileBufs& tb, int parity, int sweep, int mode, cudaStream_t st);
+template <typename R>
+void launch_mdf_interp(const ChannelDev* chans, int M, const MarkerBufs& mb, TileBufs& tb,
+                       int sweep, int mode, cudaStream_t st);
 // Learned forcing: interpolation after the membrane spread and network
 // inputs (feat [M][8], frame [M]), then tensor-core inference and rotation
 // back to the lattice frame -> dF, dFsum, u0 of every marker of a learned
 // channel.  `model` is a mlp::ModelDev.
-template <typename S, typename R>
+template <typename R>
 void launch_mdf_learned(const ChannelDev* chans, const CapsuleDev* caps, int M,
-                        const MarkerBufs& mb, const S* f, TileBufs& tb, int parity,
-                        const void* model, float* feat, double2* frame, int grid,
+                        const MarkerBufs& mb, TileBufs& tb, const void* model, float* feat, double2* frame, int grid,
                         unsigned* status, cudaStream_t st);
 // Training data of the step: inputs [M x 8], labels [M x 2] (the step's total
 // correction in the local frame), valid [M].

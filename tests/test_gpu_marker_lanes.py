@@ -1,0 +1,44 @@
+"""The per-marker kernels with four lanes a marker (contexts of at most 32,768
+markers) and with one thread a marker (larger ones) compute the same sums in the
+same order: a channel run alone, with few markers, equals the same channel inside
+an ensemble on the other side of the line, bit for bit.  Marker counts end at
+odd places of the warps and blocks on both sides."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _build(S, precision, n_copies, nodes):
+    ens = S.Ensemble(precision=precision)
+    for k in range(1 + n_copies):
+        p = S.SimulationParams(nx=72 if k == 0 else 320, ny=44 if k == 0 else 200,
+                               ibm_iterations=4, precision=precision)
+        p.fluid.boundary_type = S.BoundaryType.PERIODIC
+        p.fluid.collision_model = S.CollisionModel.BGK
+        p.fluid.body_force_x = 2e-5
+        i = ens.add_channel(p)
+        mp = S.MembraneParams(model=S.MembraneModel.NEO_HOOKEAN, G_s=0.05)
+        if k == 0:
+            for c in ((1.2, 20.3), (30.4, 9.1), (52.8, 33.9)):     # seam, wall, interior
+                ens.addCapsule(i, c, 4.0, nodes, mp)
+        else:
+            for cy in range(12, 190, 16):
+                for cx in range(10, 316, 16):
+                    ens.addCapsule(i, (cx, cy), 4.0, 32, mp)
+    ens.initialize()
+    return ens
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32", "fp16s"])
+@pytest.mark.parametrize("nodes", [27, 33])
+def test_few_and_many_markers_agree(sfg, precision, nodes):
+    import softflow_b200 as S
+    few, many = _build(S, precision, 0, nodes), _build(S, precision, 5, nodes)
+    assert few.num_markers() <= 32768 < many.num_markers()
+    few.run(6)
+    many.run(6)
+    for a, b in zip(few.field(0).macroscopic(), many.field(0).macroscopic()):
+        assert np.array_equal(a, b)
+    assert np.array_equal(few.capsules(0).positions(), many.capsules(0).positions())
+    assert np.array_equal(few.capsules(0).velocities(), many.capsules(0).velocities())
