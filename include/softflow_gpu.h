@@ -483,7 +483,7 @@ enum sfg_phase {
     SFG_PHASE_IBM_SPREAD = 3,   /* "IBM spread" (all MDF sweeps)              */
     SFG_PHASE_MDF_INTERP = 4,   /* MDF interpolation sweeps                   */
     SFG_PHASE_LATTICE = 5,      /* "LBM step" (+ fused scalar step)           */
-    SFG_PHASE_BOOKKEEPING = 6,  /* per-step flags                             */
+    SFG_PHASE_BOOKKEEPING = 6,  /* unused: the lattice kernel advances the flags */
     SFG_PHASE_INTERP_MOVE = 7,  /* "IBM interpolate" + marker move            */
     SFG_PHASE_MDF_LEARNED = 8,  /* learned forcing: interpolation + network   */
     SFG_NUM_PHASES = 9

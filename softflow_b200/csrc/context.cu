@@ -125,29 +125,6 @@ void build_ibb_links(int chan, const sfg_channel_params& p, const std::vector<un
         }
 }
 
-__global__ void k_step_flags(const ChannelDev* __restrict__ chans, int nch, int* stepped,
-                             int* adr_pending, int* c_fresh, unsigned* step_ctr,
-                             const unsigned* __restrict__ resid_gate,
-                             long long* __restrict__ learned_steps,
-                             long long* __restrict__ fallbacks) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c == 0) *step_ctr += 1u;
-    if (c >= nch) return;
-    if (chans[c].learned && chans[c].cap_end > chans[c].cap_begin) {
-        learned_steps[c] += 1;
-        if (mdf_fallback(resid_gate[c], chans[c].mdf_threshold)) fallbacks[c] += 1;
-    }
-    if (chans[c].adr) {
-        if (chans[c].adr_now) {
-            c_fresh[c] = 0;          // this step's scalar step has run
-        } else {
-            if (adr_pending[c]) c_fresh[c] = 0;
-            adr_pending[c] = 1;
-        }
-    }
-    stepped[c] = 1;
-}
-
 __global__ void k_flush_flags(int nch, int* adr_pending, int* c_fresh) {
     const int c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= nch) return;
@@ -270,9 +247,8 @@ struct sfg_context {
     cudaEvent_t ev_fork = nullptr, ev_tiles = nullptr, ev_mom = nullptr;
     cudaEvent_t ev_lat1 = nullptr;      // the lattice pass over untouched force tiles
     cudaEvent_t ev_slots = nullptr;     // the step's slot records exist
-    // the learned gate's fallback flag beside the last spread, the step's
-    // flags beside the marker move
-    cudaEvent_t ev_gate = nullptr, ev_pn = nullptr, ev_lat = nullptr, ev_flags = nullptr;
+    // the learned gate's fallback flag beside the last spread
+    cudaEvent_t ev_gate = nullptr, ev_pn = nullptr;
     bool split_lattice = false;         // that pass beside the forcing (8-cell kernel; off:
                                         // the concurrent pass slowed the forcing more than it
                                         // saved on the ensemble)
@@ -313,11 +289,9 @@ struct sfg_context {
     ContactBufs cb;
     int ncells = 0;
     double* d_phi = nullptr;
-    int* d_stepped = nullptr;
-    int* d_adr_pending = nullptr;
-    int* d_c_fresh = nullptr;
+    int* d_flags = nullptr;             // both sets of step flags
+    StepFlags flags[2] = {};            // step t reads flags[t & 1]
     unsigned* d_status = nullptr;
-    unsigned* d_step_ctr = nullptr;
     double* d_io = nullptr;
     size_t io_doubles = 0;
     int spread_grid = 0;
@@ -364,6 +338,10 @@ struct sfg_context {
     std::vector<int> pev_phase;
     float phase_ms[SFG_NUM_PHASES] = {0};
 
+    StepFlagArgs flag_args(int p) const {
+        return {flags[p], flags[1 - p], (int)ch.size(), tb.resid_gate, d_learned_steps, d_fallbacks};
+    }
+    const StepFlags& cur_flags() const { return flags[steps & 1]; }
     size_t elem_size() const { return precision == SFG_FP64 ? 8 : (precision == SFG_FP32 ? 4 : 2); }
     size_t real_size() const { return precision == SFG_FP64 ? 8 : 4; }
 };
@@ -435,8 +413,7 @@ static void free_all(sfg_context* c) {
     F(c->d_model); F(c->d_learned_steps); F(c->d_fallbacks);
     F(c->d_hfeat); F(c->d_hlab); F(c->d_hvalid); F(c->d_feat); F(c->d_frame); F(c->d_plain_needed);
     F(c->cb.cell_of); F(c->cb.cell); F(c->cb.next); F(c->cb.list); F(c->cb.lpos);
-    F(c->d_phi); F(c->d_stepped); F(c->d_adr_pending); F(c->d_c_fresh); F(c->d_status);
-    F(c->d_step_ctr);
+    F(c->d_phi); F(c->d_flags); F(c->d_status);
     F(c->d_io);
     F(c->d_zh_rows);
     c->d_zh_rows = nullptr;
@@ -479,7 +456,7 @@ static void free_all(sfg_context* c) {
         c->side[i] = nullptr;
     }
     for (cudaEvent_t* e : {&c->ev_fork, &c->ev_tiles, &c->ev_mom, &c->ev_lat1, &c->ev_slots,
-                           &c->ev_gate, &c->ev_pn, &c->ev_lat, &c->ev_flags}) {
+                           &c->ev_gate, &c->ev_pn}) {
         if (*e) cudaEventDestroy(*e);
         *e = nullptr;
     }
@@ -1120,16 +1097,15 @@ extern "C" int sfg_initialize(sfg_context* c) {
         CU(dalloc(&c->d_phi, 1025));
         CU(cudaMemcpy(c->d_phi, tbl.data(), sizeof(double) * 1025, cudaMemcpyHostToDevice));
     }
-    CU(dalloc(&c->d_stepped, nch));
-    CU(dalloc(&c->d_adr_pending, nch));
-    CU(dalloc(&c->d_c_fresh, nch));
     CU(dalloc(&c->d_status, 1));
-    CU(dalloc(&c->d_step_ctr, 1));
-    CU(cudaMemset(c->d_step_ctr, 0, sizeof(unsigned)));
-    CU(cudaMemset(c->d_stepped, 0, sizeof(int) * nch));
-    CU(cudaMemset(c->d_adr_pending, 0, sizeof(int) * nch));
-    CU(cudaMemset(c->d_c_fresh, 0, sizeof(int) * nch));
     CU(cudaMemset(c->d_status, 0, sizeof(unsigned)));
+    const int set = 3 * nch + 1;
+    CU(dalloc(&c->d_flags, 2 * set));
+    CU(cudaMemset(c->d_flags, 0, sizeof(int) * 2 * set));
+    for (int i = 0; i < 2; ++i) {
+        int* f = c->d_flags + i * set;
+        c->flags[i] = {f, f + nch, f + 2 * nch, reinterpret_cast<unsigned*>(f + 3 * nch)};
+    }
 
     int nsm = 148;
     cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
@@ -1139,7 +1115,7 @@ extern "C" int sfg_initialize(sfg_context* c) {
     if (c->M > 0 && !c->side[0]) {
         for (int i = 0; i < 3; ++i) CU(cudaStreamCreateWithFlags(&c->side[i], cudaStreamNonBlocking));
         for (cudaEvent_t* e : {&c->ev_fork, &c->ev_tiles, &c->ev_mom, &c->ev_lat1, &c->ev_slots,
-                           &c->ev_gate, &c->ev_pn, &c->ev_lat, &c->ev_flags})
+                           &c->ev_gate, &c->ev_pn})
             CU(cudaEventCreateWithFlags(e, cudaEventDisableTiming));
     }
     c->initialized = true;
@@ -1169,8 +1145,7 @@ static int enqueue_step_t(sfg_context* c, int p) {
     int launches = 0;
     mark(c, -1);
     LatticeLaunch L{c->d_items, c->n_items, c->d_chans, c->f[p], c->f[1 - p], c->g[p],
-                    c->g[1 - p], c->cfield, c->d_stepped, c->d_adr_pending, c->d_c_fresh,
-                    c->d_step_ctr, c->any_adr && !c->any_chem, c->d_items4, c->n_items4, c->use_vec4,
+                    c->g[1 - p], c->cfield, c->flag_args(p), c->any_adr && !c->any_chem, c->d_items4, c->n_items4, c->use_vec4,
                     c->persistent_ctas, c->shared_collision, c->any_bc, c->d_zh_rows,
                     c->n_zh, c->d_ibb, c->ibb_level_start.data(),
                     (int)c->ibb_level_start.size() - 1, c->d_items8, c->n_items8, c->use_vec8,
@@ -1308,29 +1283,13 @@ static int enqueue_step_t(sfg_context* c, int p) {
         launches += 2;
     }
     mark(c, SFG_PHASE_LATTICE);
-    // the step's flags and the marker move are independent: the flags run
-    // beside the move and join before the step ends
-    const bool par_flags = c->M > 0 && !c->profiling && c->side[1] != nullptr;
-    cudaStream_t fs = st;
-    if (par_flags) {
-        CU(cudaEventRecord(c->ev_lat, st));
-        CU(cudaStreamWaitEvent(c->side[1], c->ev_lat, 0));
-        fs = c->side[1];
-    }
-    k_step_flags<<<(nch + 127) / 128, 128, 0, fs>>>(c->d_chans, nch, c->d_stepped,
-                                                    c->d_adr_pending, c->d_c_fresh,
-                                                    c->d_step_ctr, c->tb.resid_gate,
-                                                    c->d_learned_steps, c->d_fallbacks);
-    if (par_flags) CU(cudaEventRecord(c->ev_flags, c->side[1]));
-    mark(c, SFG_PHASE_BOOKKEEPING);
-    launches += 2;
+    launches += 1;
     if (c->M > 0) {
         launch_interp_move<S, R>(c->d_chans, c->d_caps, c->NC, c->M, c->mb, c->cb,
                                  static_cast<const S*>(c->f[1 - p]), c->tb, p, c->d_phi, st);
         mark(c, SFG_PHASE_INTERP_MOVE);
         launches += 1;
     }
-    if (par_flags) CU(cudaStreamWaitEvent(st, c->ev_flags, 0));
     c->launches = launches;
     return SFG_OK;
 }
@@ -1839,11 +1798,11 @@ template <typename S, typename R>
 static int flush_scalar_t(sfg_context* c) {
     const int P = (int)(c->steps & 1);
     LatticeLaunch L{c->d_items, c->n_items, c->d_chans, c->f[P], nullptr, c->g[P], c->g[1 - P],
-                    c->cfield, c->d_stepped, c->d_adr_pending, c->d_c_fresh, c->d_step_ctr,
-                    c->any_adr, c->d_items4, c->n_items4, false, 0, -1};
+                    c->cfield, c->flag_args(P), c->any_adr, c->d_items4, c->n_items4, false, 0, -1};
     launch_scalar_flush<S, R>(L, last_view(c), c->stream);
     const int nch = (int)c->ch.size();
-    k_flush_flags<<<(nch + 127) / 128, 128, 0, c->stream>>>(nch, c->d_adr_pending, c->d_c_fresh);
+    k_flush_flags<<<(nch + 127) / 128, 128, 0, c->stream>>>(nch, c->flags[P].adr_pending,
+                                                             c->flags[P].c_fresh);
     CU(cudaGetLastError());
     c->g_cur = 1 - P;
     c->adr_pending_h = false;
@@ -1872,7 +1831,7 @@ extern "C" int sfg_set_concentration(sfg_context* c, int chi, const double* C) {
     else
         k_scalar_set<float><<<io_blocks(N), 256, 0, c->stream>>>(c->d_io, (float*)c->g[0], (float*)c->g[1], (float*)c->cfield, d);
     const int one = 1;
-    CU(cudaMemcpyAsync(c->d_c_fresh + chi, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    CU(cudaMemcpyAsync(c->cur_flags().c_fresh + chi, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     if (c->d_cov) CU(cudaMemsetAsync(c->d_cov + d.cell_off, 0, (size_t)d.plane, c->stream));
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(c->stream));
@@ -1895,7 +1854,7 @@ extern "C" int sfg_set_scalar_state(sfg_context* c, int chi, const double* C, co
     else
         k_scalar_import<float><<<io_blocks(N), 256, 0, c->stream>>>(c->d_io, c->d_io + N, (float*)c->g[0], (float*)c->g[1], (float*)c->cfield, d);
     const int one = 1;
-    CU(cudaMemcpyAsync(c->d_c_fresh + chi, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
+    CU(cudaMemcpyAsync(c->cur_flags().c_fresh + chi, &one, sizeof(int), cudaMemcpyHostToDevice, c->stream));
     if (c->d_cov) CU(cudaMemsetAsync(c->d_cov + d.cell_off, 0, (size_t)d.plane, c->stream));
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(c->stream));
@@ -1910,7 +1869,7 @@ extern "C" int sfg_mark_restored(sfg_context* c) {
     CU(cudaSetDevice(c->device));
     const int nch = (int)c->ch.size();
     std::vector<int> ones(nch, 1);
-    CU(cudaMemcpyAsync(c->d_stepped, ones.data(), sizeof(int) * nch, cudaMemcpyHostToDevice, c->stream));
+    CU(cudaMemcpyAsync(c->cur_flags().stepped, ones.data(), sizeof(int) * nch, cudaMemcpyHostToDevice, c->stream));
     CU(cudaStreamSynchronize(c->stream));
     c->restored = true;
     return SFG_OK;

@@ -217,9 +217,8 @@ template <typename S, typename R, bool ADR>
 __global__ void __launch_bounds__(256)
 k_lattice_step(const RowItem* __restrict__ items, int n_items, const ChannelDev* __restrict__ chans,
                const S* __restrict__ src, S* __restrict__ dst, const R* __restrict__ gsrc,
-               R* __restrict__ gdst, const R* __restrict__ cfield, TileView tv,
-               const int* __restrict__ stepped, const int* __restrict__ adr_pending,
-               const int* __restrict__ c_fresh, const unsigned* __restrict__ step_ctr) {
+               R* __restrict__ gdst, const R* __restrict__ cfield, TileView tv, StepFlagArgs fa) {
+    advance_flags(chans, fa);
     const int item = blockIdx.x * ITEMS_PER_CTA + (threadIdx.x >> 5);
     if (item >= n_items) return;
     const RowItem it = items[item];
@@ -235,7 +234,7 @@ k_lattice_step(const RowItem* __restrict__ items, int n_items, const ChannelDev*
     for (int q = 0; q < 9; ++q) f[q] = PopIO<S, R>::ld(fs + q * plane, q);
     R rho, jx, jy;
     lattice_moments(f, rho, jx, jy);
-    const int st = stepped[it.chan];
+    const int st = fa.cur.stepped[it.chan];
     const CellForces<R> cf = cell_forces<R>(ch, x, y, tv, st);
     R ux, uy;
     cell_velocity(rho, jx, jy, cf.Gx, cf.Gy, ux, uy);
@@ -249,19 +248,19 @@ k_lattice_step(const RowItem* __restrict__ items, int n_items, const ChannelDev*
         collide_bgk(f, rho, ux, uy, cf.Fx, cf.Fy, R(ch.omega));
     }
     const Nbr b = neighbours(x, y, nx, ny, ch.periodic_y ? 1 : 0);
-    const uint32_t seed = mix32((uint32_t)n ^ mix32(*step_ctr + 0x51ED270Bu));
+    const uint32_t seed = mix32((uint32_t)n ^ mix32(*fa.cur.step_ctr + 0x51ED270Bu));
     push_cell<S, R>(dst + ch.f_off, f, x, y, n, pitch, plane, b, seed);
     if (ADR) {
         // Scalar step of the previous lattice step (it needs that step's
         // final velocity, which is only known once its populations have been
         // streamed): advection_diffusion.cpp:84-223.
-        if (ch.adr && adr_pending[it.chan]) {
+        if (ch.adr && fa.cur.adr_pending[it.chan]) {
             R g[9];
             const R* gp = gsrc + ch.g_off + n;
 #pragma unroll
             for (int q = 0; q < 9; ++q) g[q] = gp[q * plane];
             R C;
-            if (c_fresh[it.chan]) C = cfield[ch.cell_off + n];
+            if (fa.cur.c_fresh[it.chan]) C = cfield[ch.cell_off + n];
             else C = g[0] + g[1] + g[2] + g[3] + g[4] + g[5] + g[6] + g[7] + g[8];
             R vx, vy;
             cell_velocity(rho, jx, jy, cf.Px, cf.Py, vx, vy);
@@ -303,8 +302,8 @@ template <typename S, typename R>
 __global__ void __launch_bounds__(256)
 k_lattice_step_bc(const RowItem* __restrict__ items, int n_items,
                   const ChannelDev* __restrict__ chans, const S* __restrict__ src,
-                  S* __restrict__ dst, TileView tv, const int* __restrict__ stepped,
-                  const unsigned* __restrict__ step_ctr) {
+                  S* __restrict__ dst, TileView tv, StepFlagArgs fa) {
+    advance_flags(chans, fa);
     const int item = blockIdx.x * ITEMS_PER_CTA + (threadIdx.x >> 5);
     if (item >= n_items) return;
     const RowItem it = items[item];
@@ -323,7 +322,7 @@ k_lattice_step_bc(const RowItem* __restrict__ items, int n_items,
     R rho, jx, jy;
     lattice_moments(f, rho, jx, jy);
     if (kind == CK_FLUID) {
-        const CellForces<R> cf = cell_forces<R>(ch, x, y, tv, stepped[it.chan]);
+        const CellForces<R> cf = cell_forces<R>(ch, x, y, tv, fa.cur.stepped[it.chan]);
         R ux, uy;
         cell_velocity(rho, jx, jy, cf.Gx, cf.Gy, ux, uy);
         const int coll = ch.collision;
@@ -336,7 +335,7 @@ k_lattice_step_bc(const RowItem* __restrict__ items, int n_items,
             collide_bgk(f, rho, ux, uy, cf.Fx, cf.Fy, R(ch.omega));
         }
     }
-    const uint32_t seed = mix32((uint32_t)n ^ mix32(*step_ctr + 0x51ED270Bu));
+    const uint32_t seed = mix32((uint32_t)n ^ mix32(*fa.cur.step_ctr + 0x51ED270Bu));
     S* __restrict__ fd = dst + ch.f_off;
     const bool per_x = ch.bc_x == 1;
     const bool mw_bot = !ch.periodic_y && fabs(ch.u_bot) > 1e-15;
@@ -1351,8 +1350,8 @@ __global__ void __launch_bounds__(256, 2)
 k_lattice_step8h(const RowItem* __restrict__ items, int n_items,
                  const ChannelDev* __restrict__ chans, int n_chans,
                  const __half* __restrict__ src, __half* __restrict__ dst, TileView tv,
-                 const int* __restrict__ stepped, const unsigned* __restrict__ step_ctr,
-                 int pass, unsigned* __restrict__ status) {
+                 StepFlagArgs fa, int pass, unsigned* __restrict__ status) {
+    if (pass != 1) advance_flags(chans, fa);
     const int lane = threadIdx.x & 31;
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -1360,7 +1359,7 @@ k_lattice_step8h(const RowItem* __restrict__ items, int n_items,
     const int i0 = gwarp * chunk;
     const int i1 = min(n_items, i0 + chunk);
     if (i0 >= i1) return;                      // warp-uniform
-    const uint32_t step_mix = mix32(*step_ctr + 0x51ED270Bu);
+    const uint32_t step_mix = mix32(*fa.cur.step_ctr + 0x51ED270Bu);
     RowItem next = items[i0];
     for (int item = i0; item < i1; ++item) {
         const RowItem it = next;
@@ -1371,7 +1370,7 @@ k_lattice_step8h(const RowItem* __restrict__ items, int n_items,
             continue;
         }
         const ChannelDev& ch = chans[it.chan];
-        lattice_run8h<COLL>(it, ch, stepped[it.chan], src, dst, tv, step_mix, lane, pass,
+        lattice_run8h<COLL>(it, ch, fa.cur.stepped[it.chan], src, dst, tv, step_mix, lane, pass,
                             status);
     }
 }
@@ -1389,9 +1388,8 @@ __global__ void __launch_bounds__(256, lattice_min_ctas<R, ADR>())
 k_lattice_step4(const RowItem* __restrict__ items, int n_items,
                 const ChannelDev* __restrict__ chans, const S* __restrict__ src,
                 S* __restrict__ dst, const R* __restrict__ gsrc, R* __restrict__ gdst,
-                const R* __restrict__ cfield, TileView tv, const int* __restrict__ stepped,
-                const int* __restrict__ adr_pending, const int* __restrict__ c_fresh,
-                const unsigned* __restrict__ step_ctr) {
+                const R* __restrict__ cfield, TileView tv, StepFlagArgs fa) {
+    advance_flags(chans, fa);
     const int lane = threadIdx.x & 31;
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -1399,17 +1397,17 @@ k_lattice_step4(const RowItem* __restrict__ items, int n_items,
     const int i0 = gwarp * chunk;
     const int i1 = min(n_items, i0 + chunk);
     if (i0 >= i1) return;                      // warp-uniform
-    const uint32_t step_mix = mix32(*step_ctr + 0x51ED270Bu);
+    const uint32_t step_mix = mix32(*fa.cur.step_ctr + 0x51ED270Bu);
     RowItem next = items[i0];
     for (int item = i0; item < i1; ++item) {
         const RowItem it = next;
         if (item + 1 < i1) next = items[item + 1];
         const ChannelDev& ch = chans[it.chan];
-        const int st = stepped[it.chan];
+        const int st = fa.cur.stepped[it.chan];
         bool adr_on = false, fresh = false;
         if (ADR) {
-            adr_on = ch.adr && adr_pending[it.chan];
-            fresh = adr_on && c_fresh[it.chan] != 0;
+            adr_on = ch.adr && fa.cur.adr_pending[it.chan];
+            fresh = adr_on && fa.cur.c_fresh[it.chan] != 0;
         }
         lattice_run4<S, R, ADR, COLL>(it, ch, st, src, dst, gsrc, gdst, cfield, tv, adr_on,
                                       fresh, step_mix, lane);

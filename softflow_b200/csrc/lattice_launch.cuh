@@ -25,7 +25,7 @@ static void launch_step4(const LatticeLaunch& L, const TileViewArgs& tv, int gri
     k_lattice_step4<S, R, ADR, COLL><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
         L.items4, L.n_items4, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
         static_cast<const R*>(L.gsrc), static_cast<R*>(L.gdst), static_cast<const R*>(L.cfield),
-        to_view(tv), L.stepped, L.adr_pending, L.c_fresh, L.step_ctr);
+        to_view(tv), L.flags);
 }
 
 template <typename S, typename R, bool ADR>
@@ -48,18 +48,18 @@ void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, cudaStr
         k_lattice_step_bc<S, R><<<(L.n_items + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA,
                                   32 * ITEMS_PER_CTA, 0, st>>>(
             L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
-            to_view(tv), L.stepped, L.step_ctr);
+            to_view(tv), L.flags);
         for (int lv = 0; lv < L.n_ibb_levels; ++lv) {
             const int a = L.ibb_level_start[lv], n = L.ibb_level_start[lv + 1] - a;
             if (n > 0)
                 k_ibb<S, R><<<(n + 127) / 128, 128, 0, st>>>(L.ibb + a, n, L.chans,
                                                              static_cast<S*>(L.dst),
-                                                             L.step_ctr);
+                                                             L.flags.cur.step_ctr);
         }
         if (L.n_zh > 0)
             k_zou_he<S, R><<<(L.n_zh + 127) / 128, 128, 0, st>>>(L.zh_rows, L.n_zh, L.chans,
                                                                  static_cast<S*>(L.dst),
-                                                                 L.step_ctr);
+                                                                 L.flags.cur.step_ctr);
         return;
     }
     if constexpr (std::is_same<S, __half>::value && std::is_same<R, float>::value) {
@@ -72,16 +72,16 @@ void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, cudaStr
             __half* dst = static_cast<__half*>(L.dst);
             switch (L.collision) {
                 case 0: k_lattice_step8h<0><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
-                            L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.stepped, L.step_ctr, L.pass, L.status);
+                            L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.flags, L.pass, L.status);
                         break;
                 case 1: k_lattice_step8h<1><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
-                            L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.stepped, L.step_ctr, L.pass, L.status);
+                            L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.flags, L.pass, L.status);
                         break;
                 case 2: k_lattice_step8h<2><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
-                            L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.stepped, L.step_ctr, L.pass, L.status);
+                            L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.flags, L.pass, L.status);
                         break;
                 default: k_lattice_step8h<-1><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
-                             L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.stepped, L.step_ctr, L.pass, L.status);
+                             L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.flags, L.pass, L.status);
                          break;
             }
             return;
@@ -101,13 +101,11 @@ void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, cudaStr
         k_lattice_step<S, R, true><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
             L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
             static_cast<const R*>(L.gsrc), static_cast<R*>(L.gdst),
-            static_cast<const R*>(L.cfield), to_view(tv), L.stepped, L.adr_pending, L.c_fresh,
-            L.step_ctr);
+            static_cast<const R*>(L.cfield), to_view(tv), L.flags);
     else
         k_lattice_step<S, R, false><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
             L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
-            nullptr, nullptr, nullptr, to_view(tv), L.stepped, L.adr_pending, L.c_fresh,
-            L.step_ctr);
+            nullptr, nullptr, nullptr, to_view(tv), L.flags);
 }
 
 template <typename S, typename R>
@@ -117,7 +115,8 @@ void launch_scalar_now(const LatticeLaunch& L, const TileViewArgs& tv, unsigned 
     k_scalar_now<S, R><<<(L.n_items + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA, 32 * ITEMS_PER_CTA, 0,
                          st>>>(L.items, L.n_items, L.chans, static_cast<const S*>(L.dst),
                                static_cast<const R*>(L.gsrc), static_cast<R*>(L.gdst),
-                               static_cast<const R*>(L.cfield), cov, to_view(tv), L.c_fresh);
+                               static_cast<const R*>(L.cfield), cov, to_view(tv),
+                               L.flags.cur.c_fresh);
 }
 
 template <typename S, typename R>
@@ -127,7 +126,7 @@ void launch_scalar_flush(const LatticeLaunch& L, const TileViewArgs& tv_last, cu
                            32 * ITEMS_PER_CTA, 0, st>>>(
         L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<const R*>(L.gsrc),
         static_cast<R*>(L.gdst), static_cast<const R*>(L.cfield), to_view(tv_last),
-        L.adr_pending, L.c_fresh);
+        L.flags.cur.adr_pending, L.flags.cur.c_fresh);
 }
 
 inline int io_grid(long long n) {

@@ -132,10 +132,7 @@ struct LatticeLaunch {
     const void* gsrc;
     void* gdst;
     const void* cfield;
-    const int* stepped;
-    const int* adr_pending;
-    const int* c_fresh;
-    const unsigned* step_ctr;   // device step counter (stochastic-rounding seed)
+    StepFlagArgs flags;
     bool any_adr;
     const RowItem* items4;      // 128-cell runs for the vectorised kernel
     int n_items4;
