@@ -302,7 +302,8 @@ struct sfg_context {
     bool restored = false;              // state restored before the first step
     bool adr_pending_h = false;
     int g_cur = 0;
-    cudaGraphExec_t gexec[2] = {nullptr, nullptr};
+    cudaGraphExec_t gexec[2] = {nullptr, nullptr};   // one step from parity p
+    cudaGraphExec_t gmulti[2] = {nullptr, nullptr};  // MULTI_STEPS steps from parity p
     bool use_graphs = true;
     bool force_scalar_lattice = false;  // diagnostics: use the one-cell-per-thread kernel
     bool force_vec4_lattice = false;    // diagnostics: four cells per lane in FP16S too
@@ -388,7 +389,8 @@ static void free_all(sfg_context* c) {
     };
     for (int i = 0; i < 2; ++i) {
         if (c->gexec[i]) cudaGraphExecDestroy(c->gexec[i]);
-        c->gexec[i] = nullptr;
+        if (c->gmulti[i]) cudaGraphExecDestroy(c->gmulti[i]);
+        c->gexec[i] = c->gmulti[i] = nullptr;
         F(c->f[i]);
         F(c->g[i]);
         F(c->tb.tile_slot[i]);
@@ -1138,8 +1140,10 @@ static void mark(sfg_context* c, int phase) {
     c->pev_phase.push_back(phase);
 }
 
+// `within`: the stream's previous operation is the previous step of the same
+// captured graph.
 template <typename S, typename R>
-static int enqueue_step_t(sfg_context* c, int p) {
+static int enqueue_step_t(sfg_context* c, int p, bool within) {
     cudaStream_t st = c->stream;
     const int nch = (int)c->ch.size();
     int launches = 0;
@@ -1184,7 +1188,7 @@ static int enqueue_step_t(sfg_context* c, int p) {
                 CU(cudaStreamWaitEvent(c->side[2], c->ev_tiles, 0));
                 LatticeLaunch L1 = L;
                 L1.pass = 1;
-                launch_lattice_step<S, R>(L1, tv, c->side[2]);
+                launch_lattice_step<S, R>(L1, tv, false, c->side[2]);
                 CU(cudaEventRecord(c->ev_lat1, c->side[2]));
                 launches += 1;
             }
@@ -1267,10 +1271,10 @@ static int enqueue_step_t(sfg_context* c, int p) {
     if (c->any_bc && c->ibb_level_start.size() > 1) launches += (int)c->ibb_level_start.size() - 1;
     if (split) {
         L.pass = 2;
-        launch_lattice_step<S, R>(L, tv, st);
+        launch_lattice_step<S, R>(L, tv, false, st);
         CU(cudaStreamWaitEvent(st, c->ev_lat1, 0));
     } else {
-        launch_lattice_step<S, R>(L, tv, st);
+        launch_lattice_step<S, R>(L, tv, within && c->M == 0, st);
     }
     if (c->any_chem) {
         // this step's scalar step, then the capsule chemistry
@@ -1294,38 +1298,51 @@ static int enqueue_step_t(sfg_context* c, int p) {
     return SFG_OK;
 }
 
-static int enqueue_step(sfg_context* c, int p) {
-    if (c->precision == SFG_FP64) return enqueue_step_t<double, double>(c, p);
-    if (c->precision == SFG_FP32) return enqueue_step_t<float, float>(c, p);
-    return enqueue_step_t<__half, float>(c, p);
+static int enqueue_step(sfg_context* c, int p, bool within = false) {
+    if (c->precision == SFG_FP64) return enqueue_step_t<double, double>(c, p, within);
+    if (c->precision == SFG_FP32) return enqueue_step_t<float, float>(c, p, within);
+    return enqueue_step_t<__half, float>(c, p, within);
 }
 
-static int build_graphs(sfg_context* c) {
-    for (int p = 0; p < 2; ++p) {
-        cudaGraph_t g = nullptr;
-        CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
-        enqueue_step(c, p);
-        CU(cudaStreamEndCapture(c->stream, &g));
-        cudaError_t e = cudaGraphInstantiate(&c->gexec[p], g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess)
-            return fail(SFG_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    }
+// Captures `n` steps from parity p into one graph.
+static int build_graph(sfg_context* c, int p, int n, cudaGraphExec_t* out) {
+    cudaGraph_t g = nullptr;
+    CU(cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = SFG_OK;
+    for (int i = 0; i < n && rc == SFG_OK; ++i) rc = enqueue_step(c, (p + i) & 1, i > 0);
+    cudaError_t e = cudaStreamEndCapture(c->stream, &g);
+    if (rc == SFG_OK && e == cudaSuccess) e = cudaGraphInstantiate(out, g, 0);
+    if (g) cudaGraphDestroy(g);
+    if (rc != SFG_OK) return rc;
+    if (e != cudaSuccess)
+        return fail(SFG_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
     return SFG_OK;
 }
+
+// Steps per graph of a context without markers, whose step is one kernel: the
+// kernels of a graph overlap their start-up, those of two graphs do not
+// (even, so that the parity is the same after it).
+constexpr int MULTI_STEPS = 16;
 
 extern "C" int sfg_step(sfg_context* c, int nsteps) {
     if (!c) return fail(SFG_ERR_ARG, "sfg_step: null context");
     if (!c->initialized) return fail(SFG_ERR_STATE, "sfg_step: context not initialized");
     if (nsteps < 0) return fail(SFG_ERR_ARG, "sfg_step: negative step count");
     CU(cudaSetDevice(c->device));
-    if (c->use_graphs && !c->gexec[0]) {
-        int rc = build_graphs(c);
+    if (c->use_graphs && !c->profiling) {   // the graphs these steps take
+        const int p = (int)(c->steps & 1);
+        const bool multi = c->M == 0 && nsteps >= MULTI_STEPS;
+        const int single = multi ? nsteps % MULTI_STEPS : nsteps;
+        int rc = SFG_OK;
+        if (multi && !c->gmulti[p]) rc = build_graph(c, p, MULTI_STEPS, &c->gmulti[p]);
+        for (int k = 0; k < std::min(single, 2) && rc == SFG_OK; ++k)
+            if (!c->gexec[(p + k) & 1]) rc = build_graph(c, (p + k) & 1, 1, &c->gexec[(p + k) & 1]);
         if (rc != SFG_OK) return rc;
     }
     CU(cudaEventRecord(c->ev0, c->stream));
-    for (int i = 0; i < nsteps; ++i) {
+    for (int i = 0, n; i < nsteps; i += n) {
         const int p = (int)(c->steps & 1);
+        n = 1;
         if (c->profiling) {
             c->pev_phase.clear();
             enqueue_step(c, p);
@@ -1337,19 +1354,22 @@ extern "C" int sfg_step(sfg_context* c, int nsteps) {
                 if (ph >= 0 && ph < SFG_NUM_PHASES) c->phase_ms[ph] += ms;
             }
         } else if (c->use_graphs) {
-            CU(cudaGraphLaunch(c->gexec[p], c->stream));
+            const bool multi = c->M == 0 && nsteps - i >= MULTI_STEPS;
+            if (multi) n = MULTI_STEPS;
+            CU(cudaGraphLaunch(multi ? c->gmulti[p] : c->gexec[p], c->stream));
         } else {
             enqueue_step(c, p);
         }
         if (c->any_adr) {
+            const int last = (p + n - 1) & 1;   // parity of the last of the n steps
             if (c->any_chem) {
-                c->g_cur = 1 - p;    // scalar step done inside the step
+                c->g_cur = 1 - last;    // scalar step done inside the step
             } else {
-                if (c->adr_pending_h) c->g_cur = 1 - p;
+                if (c->adr_pending_h || n > 1) c->g_cur = 1 - last;
                 c->adr_pending_h = true;
             }
         }
-        ++c->steps;
+        c->steps += n;
     }
     CU(cudaEventRecord(c->ev1, c->stream));
     CU(cudaGetLastError());
@@ -1386,7 +1406,8 @@ int sfg_mlp_model_device(sfg_mlp* m, const void** model, cudaStream_t st);
 static void drop_graphs(sfg_context* c) {
     for (int i = 0; i < 2; ++i) {
         if (c->gexec[i]) cudaGraphExecDestroy(c->gexec[i]);
-        c->gexec[i] = nullptr;
+        if (c->gmulti[i]) cudaGraphExecDestroy(c->gmulti[i]);
+        c->gexec[i] = c->gmulti[i] = nullptr;
     }
 }
 

@@ -14,6 +14,7 @@
 #include <type_traits>
 
 #include "collide.cuh"
+#include "launch.cuh"
 
 namespace sfg {
 
@@ -218,6 +219,7 @@ __global__ void __launch_bounds__(256)
 k_lattice_step(const RowItem* __restrict__ items, int n_items, const ChannelDev* __restrict__ chans,
                const S* __restrict__ src, S* __restrict__ dst, const R* __restrict__ gsrc,
                R* __restrict__ gdst, const R* __restrict__ cfield, TileView tv, StepFlagArgs fa) {
+    chain_begin();
     advance_flags(chans, fa);
     const int item = blockIdx.x * ITEMS_PER_CTA + (threadIdx.x >> 5);
     if (item >= n_items) return;
@@ -303,6 +305,7 @@ __global__ void __launch_bounds__(256)
 k_lattice_step_bc(const RowItem* __restrict__ items, int n_items,
                   const ChannelDev* __restrict__ chans, const S* __restrict__ src,
                   S* __restrict__ dst, TileView tv, StepFlagArgs fa) {
+    chain_begin();
     advance_flags(chans, fa);
     const int item = blockIdx.x * ITEMS_PER_CTA + (threadIdx.x >> 5);
     if (item >= n_items) return;
@@ -381,6 +384,7 @@ template <typename S, typename R>
 __global__ void k_ibb(const IbbLink* __restrict__ links, int n,
                       const ChannelDev* __restrict__ chans, S* __restrict__ dst,
                       const unsigned* __restrict__ step_ctr) {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const IbbLink L = links[i];
@@ -419,6 +423,7 @@ template <typename S, typename R>
 __global__ void k_zou_he(const RowItem* __restrict__ rows, int n_rows,
                          const ChannelDev* __restrict__ chans, S* __restrict__ dst,
                          const unsigned* __restrict__ step_ctr) {
+    chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_rows) return;
     const RowItem it = rows[i];
@@ -1351,6 +1356,7 @@ k_lattice_step8h(const RowItem* __restrict__ items, int n_items,
                  const ChannelDev* __restrict__ chans, int n_chans,
                  const __half* __restrict__ src, __half* __restrict__ dst, TileView tv,
                  StepFlagArgs fa, int pass, unsigned* __restrict__ status) {
+    chain_begin();
     if (pass != 1) advance_flags(chans, fa);
     const int lane = threadIdx.x & 31;
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1389,6 +1395,7 @@ k_lattice_step4(const RowItem* __restrict__ items, int n_items,
                 const ChannelDev* __restrict__ chans, const S* __restrict__ src,
                 S* __restrict__ dst, const R* __restrict__ gsrc, R* __restrict__ gdst,
                 const R* __restrict__ cfield, TileView tv, StepFlagArgs fa) {
+    chain_begin();
     advance_flags(chans, fa);
     const int lane = threadIdx.x & 31;
     const int gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;

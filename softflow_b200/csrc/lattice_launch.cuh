@@ -20,46 +20,45 @@ inline TileView to_view(const TileViewArgs& a) {
 }
 
 template <typename S, typename R, bool ADR, int COLL>
-static void launch_step4(const LatticeLaunch& L, const TileViewArgs& tv, int grid,
+static void launch_step4(const LatticeLaunch& L, const TileViewArgs& tv, int grid, bool chained,
                          cudaStream_t st) {
-    k_lattice_step4<S, R, ADR, COLL><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
-        L.items4, L.n_items4, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
+    launch_chain(
+        chained, k_lattice_step4<S, R, ADR, COLL>, grid, 32 * ITEMS_PER_CTA, 0, st, L.items4, L.n_items4, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
         static_cast<const R*>(L.gsrc), static_cast<R*>(L.gdst), static_cast<const R*>(L.cfield),
         to_view(tv), L.flags);
 }
 
 template <typename S, typename R, bool ADR>
 static void launch_step4_coll(const LatticeLaunch& L, const TileViewArgs& tv, int grid,
-                              cudaStream_t st) {
+                              bool chained, cudaStream_t st) {
     switch (L.collision) {
-        case 0: launch_step4<S, R, ADR, 0>(L, tv, grid, st); break;
-        case 1: launch_step4<S, R, ADR, 1>(L, tv, grid, st); break;
-        case 2: launch_step4<S, R, ADR, 2>(L, tv, grid, st); break;
-        default: launch_step4<S, R, ADR, -1>(L, tv, grid, st); break;
+        case 0: launch_step4<S, R, ADR, 0>(L, tv, grid, chained, st); break;
+        case 1: launch_step4<S, R, ADR, 1>(L, tv, grid, chained, st); break;
+        case 2: launch_step4<S, R, ADR, 2>(L, tv, grid, chained, st); break;
+        default: launch_step4<S, R, ADR, -1>(L, tv, grid, chained, st); break;
     }
 }
 
 template <typename S, typename R>
-void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, cudaStream_t st) {
+void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, bool chained,
+                         cudaStream_t st) {
     if (L.any_bc) {
         // boundary-aware kernel (no scalar transport in such contexts), then
         // the Zou-He columns on the streamed populations
         if (L.n_items == 0) return;
-        k_lattice_step_bc<S, R><<<(L.n_items + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA,
-                                  32 * ITEMS_PER_CTA, 0, st>>>(
-            L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
+        launch_chain(
+            chained, k_lattice_step_bc<S, R>, (L.n_items + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA,
+            32 * ITEMS_PER_CTA, 0, st, L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
             to_view(tv), L.flags);
         for (int lv = 0; lv < L.n_ibb_levels; ++lv) {
             const int a = L.ibb_level_start[lv], n = L.ibb_level_start[lv + 1] - a;
             if (n > 0)
-                k_ibb<S, R><<<(n + 127) / 128, 128, 0, st>>>(L.ibb + a, n, L.chans,
-                                                             static_cast<S*>(L.dst),
-                                                             L.flags.cur.step_ctr);
+                launch_chain(true, k_ibb<S, R>, (n + 127) / 128, 128, 0, st, L.ibb + a, n, L.chans,
+                             static_cast<S*>(L.dst), L.flags.cur.step_ctr);
         }
         if (L.n_zh > 0)
-            k_zou_he<S, R><<<(L.n_zh + 127) / 128, 128, 0, st>>>(L.zh_rows, L.n_zh, L.chans,
-                                                                 static_cast<S*>(L.dst),
-                                                                 L.flags.cur.step_ctr);
+            launch_chain(true, k_zou_he<S, R>, (L.n_zh + 127) / 128, 128, 0, st, L.zh_rows, L.n_zh,
+                         L.chans, static_cast<S*>(L.dst), L.flags.cur.step_ctr);
         return;
     }
     if constexpr (std::is_same<S, __half>::value && std::is_same<R, float>::value) {
@@ -70,20 +69,12 @@ void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, cudaStr
             const TileView v = to_view(tv);
             const __half* src = static_cast<const __half*>(L.src);
             __half* dst = static_cast<__half*>(L.dst);
-            switch (L.collision) {
-                case 0: k_lattice_step8h<0><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
-                            L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.flags, L.pass, L.status);
-                        break;
-                case 1: k_lattice_step8h<1><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
-                            L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.flags, L.pass, L.status);
-                        break;
-                case 2: k_lattice_step8h<2><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
-                            L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.flags, L.pass, L.status);
-                        break;
-                default: k_lattice_step8h<-1><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
-                             L.items8, L.n_items8, L.chans, L.n_chans, src, dst, v, L.flags, L.pass, L.status);
-                         break;
-            }
+            auto k = L.collision == 0   ? k_lattice_step8h<0>
+                     : L.collision == 1 ? k_lattice_step8h<1>
+                     : L.collision == 2 ? k_lattice_step8h<2>
+                                        : k_lattice_step8h<-1>;
+            launch_chain(chained, k, grid, 32 * ITEMS_PER_CTA, 0, st, L.items8, L.n_items8, L.chans,
+                         L.n_chans, src, dst, v, L.flags, L.pass, L.status);
             return;
         }
     }
@@ -91,21 +82,21 @@ void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, cudaStr
         if (L.n_items4 == 0) return;
         const int grid = std::max(1, std::min(L.persistent_ctas,
                                               (L.n_items4 + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA));
-        if (L.any_adr) launch_step4_coll<S, R, true>(L, tv, grid, st);
-        else launch_step4_coll<S, R, false>(L, tv, grid, st);
+        if (L.any_adr) launch_step4_coll<S, R, true>(L, tv, grid, chained, st);
+        else launch_step4_coll<S, R, false>(L, tv, grid, chained, st);
         return;
     }
     if (L.n_items == 0) return;
     const int grid = (L.n_items + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA;
     if (L.any_adr)
-        k_lattice_step<S, R, true><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
-            L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
+        launch_chain(
+            chained, k_lattice_step<S, R, true>, grid, 32 * ITEMS_PER_CTA, 0, st, L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
             static_cast<const R*>(L.gsrc), static_cast<R*>(L.gdst),
             static_cast<const R*>(L.cfield), to_view(tv), L.flags);
     else
-        k_lattice_step<S, R, false><<<grid, 32 * ITEMS_PER_CTA, 0, st>>>(
-            L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
-            nullptr, nullptr, nullptr, to_view(tv), L.flags);
+        launch_chain(
+            chained, k_lattice_step<S, R, false>, grid, 32 * ITEMS_PER_CTA, 0, st, L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
+            (const R*)nullptr, (R*)nullptr, (const R*)nullptr, to_view(tv), L.flags);
 }
 
 template <typename S, typename R>
@@ -185,7 +176,7 @@ int lattice_ctas_per_sm_t(bool adr, bool vec8) {
 
 #define SFG_LATTICE_INST(S, R)                                                                   \
     template int lattice_ctas_per_sm_t<S, R>(bool, bool);                                            \
-    template void launch_lattice_step<S, R>(const LatticeLaunch&, const TileViewArgs&,           \
+    template void launch_lattice_step<S, R>(const LatticeLaunch&, const TileViewArgs&, bool,     \
                                             cudaStream_t);                                        \
     template void launch_scalar_flush<S, R>(const LatticeLaunch&, const TileViewArgs&,           \
                                             cudaStream_t);                                        \

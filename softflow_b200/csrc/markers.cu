@@ -15,6 +15,7 @@
 #include "lattice.cuh"
 #include "sfg_internal.h"
 #include "ibm_interp.cuh"
+#include "launch.cuh"
 
 namespace sfg {
 
@@ -467,6 +468,7 @@ __global__ void k_marker_prep(const ChannelDev* __restrict__ chans, int nch,
                               const CapsuleDev* __restrict__ caps, int M, MarkerBufs mb,
                               const double* __restrict__ phi_tbl, TileBufs tb, ContactBufs cb,
                               unsigned* status) {
+    chain_begin();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     for (int c = m; c < nch; c += gridDim.x * blockDim.x) {
         tb.capped[c] = 0;
@@ -557,6 +559,7 @@ __global__ void k_marker_prep(const ChannelDev* __restrict__ chans, int nch,
 __global__ void k_tile_slots(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
                              TileBufs tb, int* __restrict__ tile_slot, ContactBufs cb,
                              int tile_blocks) {
+    chain_begin();
     if ((int)blockIdx.x >= tile_blocks) {
         contact_cells((blockIdx.x - tile_blocks) * blockDim.x + threadIdx.x, M, chans, mb, cb,
                       &tb.ctr[CTR_CONTACT]);
@@ -642,6 +645,7 @@ struct WorkOrder {
 __global__ void k_tile_fill(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
                             int* __restrict__ tile_pos, int* __restrict__ list,
                             const int* __restrict__ tile_slot) {
+    chain_begin();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M || !mb.valid[m]) return;
     const ChannelDev& ch = chans[mb.mk_chan[m]];
@@ -1979,11 +1983,13 @@ void launch_tiles(const ChannelDev* chans, int nch, const CapsuleDev* caps, int 
                   const double* phi_tbl, unsigned* status, cudaStream_t st,
                   cudaEvent_t slots_ready) {
     const int B = 256, G = (M + B - 1) / B, TB = (tb.T + B - 1) / B;
-    k_marker_prep<R><<<G, B, 0, st>>>(chans, nch, caps, M, mb, phi_tbl, tb, cb, status);
-    k_tile_slots<<<TB + (ncells > 0 ? G : 0), B, 0, st>>>(chans, M, mb, tb, tb.tile_slot[parity],
-                                                          cb, TB);
+    launch_chain(false, k_marker_prep<R>, G, B, 0, st, chans, nch, caps, M, mb, phi_tbl, tb, cb,
+                 status);
+    launch_chain(true, k_tile_slots, TB + (ncells > 0 ? G : 0), B, 0, st, chans, M, mb, tb,
+                 tb.tile_slot[parity], cb, TB);
     if (slots_ready) cudaEventRecord(slots_ready, st);
-    k_tile_fill<<<G, B, 0, st>>>(chans, M, mb, tb.tile_pos, tb.list, tb.tile_slot[parity]);
+    launch_chain(true, k_tile_fill, G, B, 0, st, chans, M, mb, tb.tile_pos, tb.list,
+                 tb.tile_slot[parity]);
 }
 
 template void launch_tiles<double>(const ChannelDev*, int, const CapsuleDev*, int, const MarkerBufs&,

@@ -164,8 +164,11 @@ struct TileViewArgs {
 int lattice_ctas_per_sm(int precision, bool adr, bool vec8);
 template <typename S, typename R>
 int lattice_ctas_per_sm_t(bool adr, bool vec8);
+// `chained` (launch.cuh): the stream's previous operation is a lattice step of
+// the same graph.
 template <typename S, typename R>
-void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, cudaStream_t st);
+void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, bool chained,
+                         cudaStream_t st);
 template <typename S, typename R>
 void launch_scalar_flush(const LatticeLaunch& L, const TileViewArgs& tv_last, cudaStream_t st);
 // Scalar step of the current step on its streamed populations (L.dst) and
