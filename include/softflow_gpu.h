@@ -491,11 +491,12 @@ enum sfg_phase {
 int sfg_set_profiling(sfg_context* ctx, int on);
 int sfg_get_phase_times(sfg_context* ctx, float* ms, int n);
 int sfg_reset_phase_times(sfg_context* ctx);
-/* Lattice kernel variant, before sfg_initialize: 0 (default) = the widest
- * vectorised form the channels allow (eight cells per lane in FP16-shifted
- * storage without the scalar when every nx % 8 == 0, otherwise four cells
- * per lane when every nx % 4 == 0), 1 = one cell per thread, 2 = four cells
- * per lane, 3 = as 0 with the eight-cell kernel's cells in force tiles
+/* Lattice kernel variant, before sfg_initialize: 0 (default) = the faster form
+ * the channels allow (in FP16-shifted storage eight cells per lane without the
+ * scalar when every nx % 8 == 0, otherwise four cells per lane when every
+ * nx % 4 == 0; in FP32 and FP64 four cells per lane on large lattices with
+ * every nx % 4 == 0, else one cell per thread), 1 = one cell per thread, 2 =
+ * four cells per lane (nx % 4 == 0), 3 = as 0 with the eight-cell kernel's cells in force tiles
  * untouched by the step's markers stepped beside the forcing on a side
  * stream.  FP64 and FP32 results are identical across variants; FP16-shifted
  * results of the four- and eight-cell forms differ only in the stochastic

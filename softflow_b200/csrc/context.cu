@@ -639,6 +639,23 @@ static void apply_launch_config(sfg_context* c) {
     c->learned_grid = c->nsm * std::max(1, std::min(c->learned_cps, 6));
 }
 
+// Whether the one-cell-per-thread lattice kernel is the faster one for `cells`
+// lattice cells.  Few cells leave the chip idle, and a thread's chain of four
+// cells is then the step's length: FP32 400 x 80 3.8 us a step with four cells a
+// lane against 2.6 with one, 1024 x 256 equal (5.5), 2048 x 512 13.6 against 16.3;
+// FP64 BGK 512 x 200 7.0 against 5.3, 1024 x 256 11.9 against 9.9, 2048 x 512 39.8
+// against 42.7.  FP64 regularized, bound by its divisions, keeps too few warps
+// resident with four cells in registers at any size (4096 x 1024: 969 us against
+// 585).  FP32 and FP64 give the same bits either way; the FP16-shifted kernels
+// draw other dither bits, so their form follows from nx alone.
+static bool one_cell_lattice(const sfg_context* c, long long cells) {
+    if (c->precision == SFG_FP32) return cells <= 200 * 1024;
+    if (c->precision != SFG_FP64) return false;
+    for (const ChanHost& h : c->ch)
+        if (h.p.collision != 2) return cells <= 512 * 1024;
+    return true;
+}
+
 extern "C" int sfg_initialize(sfg_context* c) {
     if (!c) return fail(SFG_ERR_ARG, "sfg_initialize: null context");
     if (c->initialized) return fail(SFG_ERR_STATE, "sfg_initialize: already initialized");
@@ -906,7 +923,8 @@ extern "C" int sfg_initialize(sfg_context* c) {
     CU(cudaMemcpy(c->d_chans, dch.data(), sizeof(ChannelDev) * nch, cudaMemcpyHostToDevice));
     CU(dalloc(&c->d_items, items.size()));
     CU(cudaMemcpy(c->d_items, items.data(), sizeof(RowItem) * items.size(), cudaMemcpyHostToDevice));
-    c->use_vec4 = all_vec4 && !c->force_scalar_lattice && !c->any_bc;
+    c->use_vec4 = all_vec4 && !c->force_scalar_lattice && !c->any_bc &&
+                  (c->force_vec4_lattice || !one_cell_lattice(c, cell_off));
     c->use_vec8 = c->use_vec4 && all_vec8 && c->precision == SFG_FP16S && !c->force_vec4_lattice;
     if (c->any_bc && c->any_adr)
         return fail(SFG_ERR_ARG, "sfg_initialize: the scalar cannot share a context with "

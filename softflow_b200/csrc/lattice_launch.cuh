@@ -64,8 +64,7 @@ void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, bool ch
     if constexpr (std::is_same<S, __half>::value && std::is_same<R, float>::value) {
         if (L.use_vec8 && !L.any_adr) {
             if (L.n_items8 == 0) return;
-            const int grid = std::max(1, std::min(L.persistent_ctas,
-                                                  (L.n_items8 + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA));
+            const int grid = std::max(1, std::min(L.persistent_ctas, L.n_items8));
             const TileView v = to_view(tv);
             const __half* src = static_cast<const __half*>(L.src);
             __half* dst = static_cast<__half*>(L.dst);
@@ -80,8 +79,7 @@ void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, bool ch
     }
     if (L.use_vec4) {
         if (L.n_items4 == 0) return;
-        const int grid = std::max(1, std::min(L.persistent_ctas,
-                                              (L.n_items4 + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA));
+        const int grid = std::max(1, std::min(L.persistent_ctas, L.n_items4));
         if (L.any_adr) launch_step4_coll<S, R, true>(L, tv, grid, chained, st);
         else launch_step4_coll<S, R, false>(L, tv, grid, chained, st);
         return;

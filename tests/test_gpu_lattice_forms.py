@@ -70,3 +70,37 @@ def test_fp16s_eight_and_four_cell_forms_agree_to_one_step(sfg, sample):
         total += d.size
     # both forms round stochastically: a good share of the values differ
     assert 0.1 < differ / total < 0.9, differ / total
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("coll", [0, 1, 2])
+@pytest.mark.parametrize("nx,ny,scalar", [(4, 9, False), (64, 20, True), (132, 37, True),
+                                          (260, 33, False), (1028, 12, False)])
+def test_one_and_four_cell_forms_are_bit_identical(sfg, precision, coll, nx, ny, scalar):
+    """FP32 and FP64: the context's size chooses between one cell a thread and
+    four a lane, so both must give the same bits (runs of 4 to 1,028 cells: one
+    lane, partial and several runs a row; fewer and more runs than warps)."""
+    import softflow_b200 as S
+    from softflow_b200 import workloads as W
+    p = W.channel_params(nx, ny, S.CollisionModel(coll), 0.83, 2e-5, 2, precision,
+                         0.05 if scalar else None)
+    caps = [(1, 6, 9, nx - 6, ny - 9, 3.0, 24, W.skalak(), 5)] if nx > 40 and ny > 18 else []
+    noise = np.random.default_rng(3).standard_normal((9, ny, nx))
+    f = W9[:, None, None] * (1 + 0.02 * noise)
+    out = {}
+    for variant in (1, 2):
+        e = _build([W.ChannelPlan(p, caps)], precision, variant)
+        e.field(0).set_distributions(f)
+        if scalar:
+            e.advectionDiffusion(0).setConcentration(np.abs(f[1]))
+        e.run(7)
+        out[variant] = [e.field(0).distributions()]
+        if scalar:
+            out[variant].append(e.advectionDiffusion(0).populations())
+        if caps:
+            out[variant].append(e.capsules(0).positions())
+        e.close()
+    rows = slice(1, ny - 1)
+    for a, b in zip(out[1], out[2]):
+        assert np.array_equal(a[..., rows, :] if a.ndim == 3 else a,
+                              b[..., rows, :] if b.ndim == 3 else b)
