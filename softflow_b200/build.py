@@ -5,7 +5,7 @@ Usage: python -m softflow_b200.build  (or softflow_b200.build.build()).
 Translation units and their floating-point contract:
   lattice_f64.cu, markers.cu  --fmad=false: FP64 paths keep the reference's
                               rounding (no fused multiply-add contraction);
-  lattice_f32.cu, scan.cu, context.cu: default contraction;
+  lattice_f32.cu, context.cu: default contraction;
   host_setup.cpp (g++)        -ffp-contract=off.
 """
 from __future__ import annotations
@@ -27,7 +27,6 @@ UNITS = [
     ("markers.cu", ["--fmad=false"]),
     ("spread_standalone.cu", ["--fmad=false"]),
     ("spread_noalloc.cu", []),
-    ("scan.cu", []),
     ("mlp.cu", []),
     ("learned_step.cu", ["--fmad=false"]),
     ("chemistry.cu", ["--fmad=false"]),

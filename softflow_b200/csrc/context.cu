@@ -635,7 +635,9 @@ static void apply_launch_config(sfg_context* c) {
     const int lat = c->lattice_cps > 0 ? std::min(c->lattice_cps, lat_max) : lat_max;
     const int spr = c->spread_cps > 0 ? std::min(c->spread_cps, spr_max) : spr_max;
     c->persistent_ctas = c->nsm * lat;
-    c->spread_grid = std::max(1, std::min((c->tb.max_slots + 7) / 8, c->nsm * spr));
+    const int per_cta = c->precision == SFG_FP64 ? 1 : 8;   // tiles a spread CTA works at a time
+    c->spread_grid =
+        std::max(1, std::min((c->tb.max_slots + per_cta - 1) / per_cta, c->nsm * spr));
     c->learned_grid = c->nsm * std::max(1, std::min(c->learned_cps, 6));
 }
 

@@ -16,6 +16,7 @@
 #include "sfg_internal.h"
 #include "ibm_interp.cuh"
 #include "launch.cuh"
+#include "spread_wide.cuh"
 
 namespace sfg {
 
@@ -653,7 +654,7 @@ __global__ void k_tile_fill(const ChannelDev* __restrict__ chans, int M, MarkerB
     int t[8];
     const int nt = stencil_tiles(ch, ix0, iy0, t);
     // one atomic per distinct tile and warp; the lanes of a tile take
-    // consecutive list entries (the order is restored by the sweep-0 sort)
+    // consecutive list entries (an FP64 spread restores the order)
     const int lane = threadIdx.x & 31;
     for (int a = 0; a < 8; ++a) {
         const int key = a < nt ? t[a] : -1;
@@ -683,133 +684,51 @@ __global__ void k_tile_fill(const ChannelDev* __restrict__ chans, int M, MarkerB
     o[1] = make_int4(s8[4], s8[5], s8[6], s8[7]);
 }
 
-// Stencil column of lattice column jx for a marker with origin ix0 (the
-// unwrapped index the reference uses in rx = x - ix); false if uncovered.
-__device__ __forceinline__ bool stencil_ix(int jx, int ix0, int nx, int& ix) {
-    int d = jx - ix0;
-    if (d >= -1 && d <= 2) { ix = jx; return true; }
-    d = jx - nx - ix0;
-    if (d >= -1 && d <= 2) { ix = jx - nx; return true; }
-    d = jx + nx - ix0;
-    if (d >= -1 && d <= 2) { ix = jx + nx; return true; }
-    return false;
-}
-
 constexpr int SPREAD_WARPS = 8;       // force tiles processed per CTA (one per warp)
-constexpr int SPREAD_LCAP = 256;      // list entries sorted in shared memory per warp
-                                      // (a power of two: the bitonic sort pads to one)
 constexpr int SPREAD_LIST_MAX = 4096; // longer lists are clamped and flagged
 
-// Shared memory of one spread warp: the tile's accumulators, the sort buffer
-// of its marker list (sweep 0) and a staged chunk of markers.
-constexpr int SPREAD_CHUNK = 16;      // markers staged per chunk
-// Channels narrower than a tile: the stencil data of each marker.
-struct SpreadChunkNarrow {
-    double2 f[SPREAD_CHUNK];
-    double ds[SPREAD_CHUNK];
-    double wx[SPREAD_CHUNK][4], wy[SPREAD_CHUNK][4];
-    int ix[SPREAD_CHUNK], iy[SPREAD_CHUNK], ok[SPREAD_CHUNK];
-};
-// Otherwise: each marker's 16 stencil contributions (f w ds, in the
-// reference's rounding order), the lanes that own a valid point of it, and
-// its stencil origin in tile coordinates.
-// (x, y) pair of the accumulation type: double2 in FP64 contexts (the
-// reference's arithmetic, bit for bit), float2 in the FP32-arithmetic modes.
-template <typename A> struct APair;
-template <> struct APair<double> {
-    using T = double2;
-    static __device__ __forceinline__ T make(double x, double y) { return make_double2(x, y); }
-};
-template <> struct APair<float> {
-    using T = float2;
-    static __device__ __forceinline__ T make(double x, double y) {
-        return make_float2((float)x, (float)y);
-    }
-};
-// Markers staged per chunk on the wide path: four lanes per marker, one
-// stencil row each.  A staged point goes to the slot of the lane that owns
-// its cell (lane (a, b) owns the tile cells whose column is a mod 8 and row
-// b mod 4): its contribution and its accumulator index.
-constexpr int WIDE_CHUNK = 8;
-template <typename A>
-struct SpreadChunkWide {
-    typename APair<A>::T v[WIDE_CHUNK][33];    // [marker][owner lane] (padded row)
-    unsigned short cell[WIDE_CHUNK][32];       // accumulator index of that point
-    unsigned mask[WIDE_CHUNK];                 // owner lanes holding a point
-};
-// The tile accumulators keep rows of TILE_W + 4 doubles: the 4 x 4 stencil
+// The tile accumulators keep rows of TILE_W + 4 cells: the 4 x 4 stencil
 // points of a marker (4 consecutive rows and columns) then fall on 16
-// distinct bank pairs (a row stride of 32 doubles puts all 4 rows on the same
-// banks: 4-way conflicts on every accumulation).
+// distinct banks (a row stride of 32 puts all 4 rows on the same banks).
 constexpr int ACC_W = TILE_W + 4;
 constexpr int ACC_CELLS = TILE_H * ACC_W;
 __device__ __forceinline__ int acc_at(int c) { return (c / TILE_W) * ACC_W + (c % TILE_W); }
-template <typename A>
-struct SpreadWarpSmem {
-    A ax[ACC_CELLS], ay[ACC_CELLS];
-    union {
-        int list[SPREAD_LCAP];                 // sweep 0: the bitonic sort of long lists
-        SpreadChunkNarrow n;                   // (the sort ends before the first chunk)
-        SpreadChunkWide<A> w;
-    } ck;
-};
-template <typename A>
-constexpr size_t spread_smem() { return sizeof(SpreadWarpSmem<A>) * SPREAD_WARPS; }
 
-// Deterministic spread into force tiles for MDF sweep `sweep`.  Sweep 0
-// spreads the membrane + contact forces (immersed_boundary.cpp:25-100);
-// sweep k >= 1 adds the corrections dF (:231-286).  One warp owns one tile:
-// it sorts the tile's marker list (ascending marker index = the reference's
-// loop order), then applies the markers one after the other, 16 lanes
-// covering the 4 x 4 stencil, so every cell receives its contributions in
-// the reference's order.  On a channel's last sweep the warp also adds the
-// body force on FLUID cells, applies the force cap and counts capped cells
-// (simulation.cpp:540-609), writing the final tile force `fin` (type R).
-// The tile accumulates in R; the step launches it for FP64 contexts (double,
-// bit for bit), the FP32-arithmetic modes run k_spread_fx.
-// Resident CTAs per SM asked of the compiler: 3 for the double form (4 for a
-// float instantiation).
-template <typename R>
-constexpr int spread_min_ctas() { return sizeof(R) == 4 ? 4 : 3; }
-
-template <typename R>
-__global__ void __launch_bounds__(SPREAD_WARPS * 32, spread_min_ctas<R>())
+// Deterministic spread into force tiles for MDF sweep `sweep` (FP64 contexts, bit
+// for bit; the FP32-arithmetic modes run k_spread_fx).  Sweep 0 spreads the
+// membrane + contact forces (immersed_boundary.cpp:25-100); sweep k >= 1 adds the
+// corrections dF (:231-286).  One CTA owns one tile, a warp a band of eight
+// columns (spread_wide.cuh), so every cell receives its contributions in the
+// reference's order.  On a channel's last sweep the warps also add the body force
+// on FLUID cells, apply the force cap and count capped cells
+// (simulation.cpp:540-609), writing the final tile force `fin`.  Tiles are dealt
+// to the CTAs in rounds over the work order (longest lists first, alternating
+// direction, so that each CTA's share sums to about the same work; a shared
+// claim counter serialises on one L2 address); the next tile's record is fetched
+// while the current one is processed.
+__global__ void __launch_bounds__(BAND_WARPS * 32, 6)
 k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot_info,
          const int* __restrict__ slot_order, const int* __restrict__ ctr, int max_slots,
          int* __restrict__ list, MarkerBufs mb, double* __restrict__ acc,
-         double* __restrict__ acc0, R* __restrict__ gsnap, R* __restrict__ fin, int sweep,
-         int mode, const unsigned* __restrict__ resid_gate,
+         double* __restrict__ acc0, double* __restrict__ gsnap, double* __restrict__ fin,
+         int sweep, int mode, const unsigned* __restrict__ resid_gate,
          const int* __restrict__ plain_needed, int* __restrict__ capped,
          int* __restrict__ fluid_touched, unsigned* status) {
     if (sweep > 0 && mode == MDF_PLAIN && plain_needed && !*plain_needed) return;
-    extern __shared__ __align__(16) unsigned char spread_smem[];
+    __shared__ BandSmem s_band[BAND_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    using A = R;
-    using A2 = typename APair<A>::T;
-    SpreadWarpSmem<A>& W = reinterpret_cast<SpreadWarpSmem<A>*>(spread_smem)[warp];
-    A* ax = W.ax;
-    A* ay = W.ay;
-    int* sl = W.ck.list;
+    BandSmem& B = s_band[warp];
     const int n_slots = ctr[CTR_SLOTS];
     const WorkOrder wo(ctr);
-    // slots are dealt to the warps in rounds over the work order (longest
-    // lists first, alternating direction, so each warp's share sums to
-    // about the same work; a shared claim counter serialises on one L2
-    // address); the next slot's record is fetched while the current one is
-    // processed
-    const int nwarps = gridDim.x * SPREAD_WARPS;
-    // round k takes work-order positions k nwarps .. (k + 1) nwarps - 1,
-    // the warps in reverse order on odd rounds
-    const int wid = blockIdx.x * SPREAD_WARPS + warp;
-    int round = 0, next = wid;
+    int round = 0, next = blockIdx.x;
     int nslot = next < n_slots ? wo.slot(slot_order, max_slots, next) : 0;
     SlotInfo nfo{};
     if (next < n_slots) nfo = slot_info[nslot];
-    while (next < n_slots) {
+    while (next < n_slots) {   // uniform in the CTA
         const int slot = nslot;
         const SlotInfo si = nfo;
         ++round;
-        next = round * nwarps + ((round & 1) ? nwarps - 1 - wid : wid);
+        next = round * gridDim.x + ((round & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
         if (next < n_slots) {
             nslot = wo.slot(slot_order, max_slots, next);
             nfo = slot_info[nslot];
@@ -817,275 +736,70 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
         const int chan = si.chan;
         const ChannelDev& ch = chans[chan];
         const int K = ch.ibm_iterations > 1 ? ch.ibm_iterations : 1;
-        if (sweep >= K) continue;  // warp-uniform
+        if (sweep >= K) continue;
         if (sweep > 0 && !mdf_active(ch, mode, resid_gate, chan)) continue;  // sweep 0: all
-        const int nx = si.nx, ny = si.ny;
-        const int x0 = si.x0, y0 = si.y0;
         int cnt = si.cnt;
-        const int off = si.off;
-        const int* lst;
-        // the lists are sorted by the step's first spread (sweep 0) and
-        // written back; later sweeps read them in order
-        const bool do_sort = (sweep == 0);
-        if (cnt <= SPREAD_LCAP && !do_sort) {
-            lst = list + off;
-        } else if (cnt <= 32) {
-            // bitonic sort across the warp's registers (ascending by lane)
-            int v = lane < cnt ? list[off + lane] : INT_MAX;
-#pragma unroll
-            for (int k = 2; k <= 32; k <<= 1)
-#pragma unroll
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    const int o = __shfl_xor_sync(0xffffffffu, v, j);
-                    const bool take_min = ((lane & j) == 0) == ((lane & k) == 0);
-                    v = take_min ? min(v, o) : max(v, o);
-                }
-            if (lane < cnt) list[off + lane] = v;
-            __syncwarp();
-            lst = list + off;
-        } else if (cnt <= SPREAD_LCAP) {
-            int pow2 = 1;
-            while (pow2 < cnt) pow2 <<= 1;
-            for (int i = lane; i < pow2; i += 32) sl[i] = i < cnt ? list[off + i] : INT_MAX;
-            __syncwarp();
-            for (int k = 2; k <= pow2; k <<= 1)
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    for (int i = lane; i < pow2; i += 32) {
-                        const int l = i ^ j;
-                        if (l > i) {
-                            const int a = sl[i], b = sl[l];
-                            if ((a > b) == ((i & k) == 0)) { sl[i] = b; sl[l] = a; }
-                        }
-                    }
-                    __syncwarp();
-                }
-            for (int i = lane; i < cnt; i += 32) list[off + i] = sl[i];
-            __syncwarp();
-            lst = list + off;
-        } else {
-            if (cnt > SPREAD_LIST_MAX) {
-                if (lane == 0) atomicOr(status, (unsigned)ST_LIST_OVERFLOW);
-                cnt = SPREAD_LIST_MAX;
-            }
-            if (lane == 0 && do_sort) {  // long lists are rare: sort in place
-                int* a = list + off;
-                for (int i = 1; i < cnt; ++i) {
-                    const int v = a[i];
-                    int j = i - 1;
-                    while (j >= 0 && a[j] > v) { a[j + 1] = a[j]; --j; }
-                    a[j + 1] = v;
-                }
-            }
-            __syncwarp();
-            lst = list + off;
+        if (cnt > SPREAD_LIST_MAX) {
+            if (threadIdx.x == 0) atomicOr(status, (unsigned)ST_LIST_OVERFLOW);
+            cnt = SPREAD_LIST_MAX;
         }
-        const size_t base = (size_t)slot * 2 * TILE_CELLS;
+        if (cnt > BAND_LIST && sweep == 0) {   // (sorted for the later sweeps too)
+            if (threadIdx.x == 0) long_list_sort(list + si.off, cnt);
+            __syncthreads();
+        }
         const bool last = mode == MDF_LEARNED ? true : (mode == MDF_SEED ? false : sweep == K - 1);
         // a learned channel's membrane-only force lives in acc0 only: the
         // seed sweep and a fallback's restart read it there.  The
         // accumulators hold (x, y) pairs per cell: [slot][TILE_CELLS] double2.
-        const A2* src = reinterpret_cast<const A2*>(
+        const double2* src = reinterpret_cast<const double2*>(
             (ch.learned && (mode == MDF_SEED || (mode == MDF_PLAIN && sweep == 1))) ? acc0 : acc);
-        const size_t base2 = (size_t)slot * TILE_CELLS;
-        for (int c = lane; c < TILE_CELLS; c += 32) {
-            const A2 a = sweep > 0 ? src[base2 + c] : APair<A>::make(0.0, 0.0);
-            const A vx = a.x, vy = a.y;
-            ax[acc_at(c)] = vx;
-            ay[acc_at(c)] = vy;
-            if (last && K > 1) {
-                gsnap[base + c] = (R)vx;
-                gsnap[base + TILE_CELLS + c] = (R)vy;
-            }
-        }
+        const size_t base = (size_t)slot * 2 * TILE_CELLS, base2 = (size_t)slot * TILE_CELLS;
+        const int x0 = si.x0 + BAND_W * warp;
+        // this lane's two cells: column a, rows b and b + 4 of the band
+        const int ca = lane & 7, cb = lane >> 3;
         __syncwarp();
-        const int la = lane & 7, lb = lane >> 3;
-        if (nx > TILE_W) {
-            // Markers in list order, WIDE_CHUNK at a time.  Staging: lanes
-            // 4j .. 4j + 3 take marker j of the chunk, one stencil row each
-            // (sy = lane & 3), and evaluate its four points: the weight
-            // w = phi(rx) phi(ry), the contribution (f w) ds and the lane that
-            // owns the point's cell, into whose slot the contribution and the
-            // cell's accumulator index go.  Lane (a, b) = (lane & 7, lane >> 3)
-            // owns the tile cells of column a mod 8 and row b mod 4; the 4 x 4
-            // stencil has 4 consecutive columns and rows, so its 16 points
-            // fall on 16 distinct lanes.  Then every lane adds its own point of
-            // each marker to its own cell, marker after marker, so every cell
-            // receives its terms in the reference's order.  A lane with no
-            // point of a marker adds zero to a padding cell of its own (the
-            // accumulator rows carry four padding columns: 8 x 4 = 32 cells,
-            // one per lane), so the additions carry no branches.
-            const int jm = lane >> 2, sy = lane & 3;
-            double2 rf = make_double2(0.0, 0.0), rw0 = rf, rw1 = rf;
-            double rds = 0.0, rwy = 0.0;
-            int rix = 0, riy = 0;
-            auto fetch = [&](int c) {
-                if (c + jm < cnt) {
-                    const int m = lst[c + jm];
-                    rf = sweep == 0 ? mb.frc[m] : mb.dF[m];
-                    rix = mb.org[m].x;
-                    riy = mb.org[m].y;
-                    rds = mb.ds[m];
-                    const double2* wx2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
-                    rw0 = wx2[0];
-                    rw1 = wx2[1];
-                    rwy = mb.wy[4 * (size_t)m + sy];
-                }
-            };
-            const int pad = (lane >> 2) * ACC_W + TILE_W + (lane & 3);   // this lane's padding cell
-            fetch(0);
-            for (int c0 = 0; c0 < cnt; c0 += WIDE_CHUNK) {
-                const int nb = cnt - c0 < WIDE_CHUNK ? cnt - c0 : WIDE_CHUNK;
-                __syncwarp();
-                unsigned bits = 0u;
-                if (jm < nb) {
-                    const bool ok = !(isnan(rf.x) || isnan(rf.y));
-                    const int cyl = riy - 1 + sy - y0, iy = riy - 1 + sy;
-                    const bool vrow = ok && cyl >= 0 && cyl < TILE_H && iy >= 0 && iy < ny;
-                    const double wxk[4] = {rw0.x, rw0.y, rw1.x, rw1.y};
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        int jx = rix - 1 + k;
-                        if (jx < 0) jx += nx;
-                        if (jx >= nx) jx -= nx;
-                        const int cl = jx - x0;
-                        const double w = wxk[k] * rwy;
-                        if (vrow && jx >= 0 && jx < nx && cl >= 0 && cl < TILE_W && w > 1e-15) {
-                            const int t = (cl & 7) + 8 * (cyl & 3);
-                            // FP64: (f w) ds in the reference's order; the
-                            // float form rounds f, w, ds once and works in float
-                            if constexpr (sizeof(A) == 8)
-                                W.ck.w.v[jm][t] = APair<A>::make(rf.x * w * rds, rf.y * w * rds);
-                            else
-                                W.ck.w.v[jm][t] = make_float2((float)rf.x * (float)w * (float)rds,
-                                                              (float)rf.y * (float)w * (float)rds);
-                            W.ck.w.cell[jm][t] = (unsigned short)(cyl * ACC_W + cl);
-                            bits |= 1u << t;
-                        }
-                    }
-                }
-                bits |= __shfl_xor_sync(0xffffffffu, bits, 1);
-                bits |= __shfl_xor_sync(0xffffffffu, bits, 2);
-                if (sy == 0 && jm < nb) W.ck.w.mask[jm] = bits;
-                __syncwarp();
-                fetch(c0 + WIDE_CHUNK);   // in flight while this chunk is added
-                const A2 zero = APair<A>::make(0.0, 0.0);
-                // this lane's point of marker j (or zero into its padding cell)
-                auto point = [&](int j, int& c, A2& v) {
-                    const bool h = (W.ck.w.mask[j] >> lane) & 1u;
-                    const int ci = W.ck.w.cell[j][lane];
-                    const A2 vi = W.ck.w.v[j][lane];
-                    c = h ? ci : pad;
-                    v = h ? vi : zero;
-                };
-                int j = 0;
-                // two markers at a time: both cells are read before either is
-                // written, the second addition taking the first's sum when
-                // both points are the same cell (same order, same rounding)
-                for (; j + 1 < nb; j += 2) {
-                    int c0i, c1i;
-                    A2 v0, v1;
-                    point(j, c0i, v0);
-                    point(j + 1, c1i, v1);
-                    A a0x = ax[c0i], a0y = ay[c0i];
-                    A a1x = ax[c1i], a1y = ay[c1i];
-                    a0x += v0.x;
-                    a0y += v0.y;
-                    ax[c0i] = a0x;
-                    ay[c0i] = a0y;
-                    const bool same = c1i == c0i;
-                    a1x = same ? a0x : a1x;
-                    a1y = same ? a0y : a1y;
-                    ax[c1i] = a1x + v1.x;
-                    ay[c1i] = a1y + v1.y;
-                }
-                if (j < nb) {
-                    int c;
-                    A2 v;
-                    point(j, c, v);
-                    ax[c] += v.x;
-                    ay[c] += v.y;
-                }
+        for (int h = 0; h < 2; ++h) {
+            const int r = cb + 4 * h, c = r * TILE_W + BAND_W * warp + ca;
+            const double2 a = sweep > 0 ? src[base2 + c] : make_double2(0.0, 0.0);
+            B.ax[r * BAND_ACC_W + ca] = a.x;
+            B.ay[r * BAND_ACC_W + ca] = a.y;
+            if (last && K > 1) {
+                gsnap[base + c] = a.x;
+                gsnap[base + TILE_CELLS + c] = a.y;
             }
-        } else {
-        // One tile holds both sides of the periodic seam: two stencil
-        // columns can share a residue, so a lane applies each of its points.
-        SpreadChunkNarrow& N = W.ck.n;
-        double2 rf = make_double2(0.0, 0.0), rw0 = rf, rw1 = rf, rv0 = rf, rv1 = rf;
-        double rds = 0.0;
-        int rix = 0, riy = 0;
-        auto fetch = [&](int c) {
-            if (lane < SPREAD_CHUNK && c + lane < cnt) {
-                const int m = lst[c + lane];
-                rf = sweep == 0 ? mb.frc[m] : mb.dF[m];
-                rix = mb.org[m].x;
-                riy = mb.org[m].y;
-                rds = mb.ds[m];
-                const double2* wx2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
-                const double2* wy2 = reinterpret_cast<const double2*>(mb.wy + 4 * (size_t)m);
-                rw0 = wx2[0]; rw1 = wx2[1]; rv0 = wy2[0]; rv1 = wy2[1];
-            }
+        }
+        const double2* frc = sweep == 0 ? mb.frc : mb.dF;
+        auto org_of = [&](int m) { return mb.org[m]; };
+        auto load = [&](int m, int sy, BandMarker& k) {
+            k.f = frc[m];
+            k.org = mb.org[m];
+            k.ds = mb.ds[m];
+            const double2* wx2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
+            const double2 wa = wx2[0], wb = wx2[1];
+            k.wx[0] = wa.x; k.wx[1] = wa.y; k.wx[2] = wb.x; k.wx[3] = wb.y;
+            k.wy = mb.wy[4 * (size_t)m + sy];
         };
-        fetch(0);
-        for (int c0 = 0; c0 < cnt; c0 += SPREAD_CHUNK) {
-            const int nb = cnt - c0 < SPREAD_CHUNK ? cnt - c0 : SPREAD_CHUNK;
-            __syncwarp();
-            if (lane < nb) {
-                N.f[lane] = rf;
-                N.ok[lane] = !(isnan(rf.x) || isnan(rf.y));
-                N.ds[lane] = rds;
-                N.ix[lane] = rix;
-                N.iy[lane] = riy;
-                N.wx[lane][0] = rw0.x; N.wx[lane][1] = rw0.y; N.wx[lane][2] = rw1.x; N.wx[lane][3] = rw1.y;
-                N.wy[lane][0] = rv0.x; N.wy[lane][1] = rv0.y; N.wy[lane][2] = rv1.x; N.wy[lane][3] = rv1.y;
-            }
-            __syncwarp();
-            fetch(c0 + SPREAD_CHUNK);   // in flight while this chunk is added
-            for (int j = 0; j < nb; ++j) {
-                if (!N.ok[j]) continue;  // warp-uniform
-                const int jx0 = N.ix[j] - 1;
-                const int r0n = N.iy[j] - 1 - y0;
-                const int syn = (lb - r0n) & 3;
-                const int cyn = r0n + syn;
-                if (cyn >= 0 && cyn < TILE_H && cyn + y0 >= 0 && cyn + y0 < ny) {
-                    for (int k = 0; k < 4; ++k) {
-                        int jx = jx0 + k;
-                        if (jx < 0) jx += nx;
-                        if (jx >= nx) jx -= nx;
-                        const int cl = jx - x0;
-                        if (cl < 0 || cl >= TILE_W || (cl & 7) != la) continue;
-                        const double w = N.wx[j][k] * N.wy[j][syn];
-                        if (w > 1e-15) {
-                            const double ds = N.ds[j];
-                            const double2 fo = N.f[j];
-                            const int c = cyn * ACC_W + cl;
-                            ax[c] += (A)(fo.x * w * ds);
-                            ay[c] += (A)(fo.y * w * ds);
-                        }
-                    }
-                }
-            }
-        }
-        }
-        __syncwarp();
+        band_spread(B, list + si.off, cnt, si.nx, si.ny, x0, si.y0, lane, org_of, load);
         if (!last) {
-            A2* out = reinterpret_cast<A2*>((sweep == 0 && ch.learned) ? acc0 : acc);
-            for (int c = lane; c < TILE_CELLS; c += 32) {
-                A2 o;
-                o.x = ax[acc_at(c)];
-                o.y = ay[acc_at(c)];
-                out[base2 + c] = o;
+            double2* out = reinterpret_cast<double2*>((sweep == 0 && ch.learned) ? acc0 : acc);
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int r = cb + 4 * h, i = r * BAND_ACC_W + ca;
+                out[base2 + r * TILE_W + BAND_W * warp + ca] = make_double2(B.ax[i], B.ay[i]);
             }
-            __syncwarp();
             continue;
         }
         // finalize: body force on FLUID cells, then the force cap
         int n_cap = 0, n_fluid = 0;
         const double Fm = ch.max_force, Fm2 = Fm * Fm;
         const bool body = (ch.body_fx != 0.0 || ch.body_fy != 0.0);
-        for (int c = lane; c < TILE_CELLS; c += 32) {
-            const int jx = x0 + (c % TILE_W), jy = y0 + (c / TILE_W);
-            double vx = (double)ax[acc_at(c)], vy = (double)ay[acc_at(c)];
-            if (jx < nx && jy < ny) {
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = cb + 4 * h, i = r * BAND_ACC_W + ca, c = r * TILE_W + BAND_W * warp + ca;
+            const int jx = x0 + ca, jy = si.y0 + r;
+            double vx = B.ax[i], vy = B.ay[i];
+            if (jx < si.nx && jy < si.ny) {
                 const bool fluid = cell_kind(ch, jx, jy) == CK_FLUID;
                 if (fluid && body) {
                     vx += ch.body_fx;
@@ -1101,18 +815,15 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
                 n_fluid += fluid ? 1 : 0;
             }
             // (no sweep reads acc after a channel's last one)
-            fin[base + c] = (R)vx;
-            fin[base + TILE_CELLS + c] = (R)vy;
+            fin[base + c] = vx;
+            fin[base + TILE_CELLS + c] = vy;
         }
-        for (int o = 16; o > 0; o >>= 1) {
-            n_cap += __shfl_down_sync(0xffffffffu, n_cap, o);
-            n_fluid += __shfl_down_sync(0xffffffffu, n_fluid, o);
-        }
+        n_cap = __reduce_add_sync(0xffffffffu, n_cap);
+        n_fluid = __reduce_add_sync(0xffffffffu, n_fluid);
         if (lane == 0) {
             if (n_cap) atomicAdd(&capped[chan], n_cap);
             if (n_fluid) atomicAdd(&fluid_touched[chan], n_fluid);
         }
-        __syncwarp();
     }
 }
 
@@ -1702,9 +1413,7 @@ size_t membrane_smem_bytes(int maxn) {
 int spread_blocks_per_sm(bool fp64) {
     int b = 0;
     const cudaError_t e =
-        fp64 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_spread<double>,
-                                                             SPREAD_WARPS * 32,
-                                                             spread_smem<double>())
+        fp64 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_spread, BAND_WARPS * 32, 0)
              : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_spread_fx,
                                                              SPREAD_WARPS * 32,
                                                              spread_fx_smem());
@@ -1713,13 +1422,8 @@ int spread_blocks_per_sm(bool fp64) {
 }
 
 cudaError_t prepare_spread() {
-    cudaError_t e = cudaFuncSetAttribute(k_spread<double>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)spread_smem<double>());
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_spread_fx, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)spread_fx_smem());
-    return e;
+    return cudaFuncSetAttribute(k_spread_fx, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)spread_fx_smem());
 }
 
 // ---------------- capsule geometry (thermo) ---------------------------------
@@ -2008,9 +1712,9 @@ void launch_spread(const ChannelDev* chans, const MarkerBufs& mb, TileBufs& tb, 
             static_cast<float*>(tb.gsnap), static_cast<float*>(tb.fin[parity]), sweep, mode,
             tb.resid_gate, tb.plain_needed, tb.capped, tb.fluid_touched, status);
     } else {
-        k_spread<R><<<grid, SPREAD_WARPS * 32, spread_smem<R>(), st>>>(
+        k_spread<<<grid, BAND_WARPS * 32, 0, st>>>(
             chans, tb.slot_info, tb.slot_order, tb.ctr, tb.max_slots, tb.list, mb, tb.acc,
-            tb.acc0, static_cast<R*>(tb.gsnap), static_cast<R*>(tb.fin[parity]), sweep, mode,
+            tb.acc0, static_cast<double*>(tb.gsnap), static_cast<double*>(tb.fin[parity]), sweep, mode,
             tb.resid_gate, tb.plain_needed, tb.capped, tb.fluid_touched, status);
     }
 }

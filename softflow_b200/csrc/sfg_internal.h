@@ -60,11 +60,6 @@ struct TileBufs {
     unsigned* resid_plain = nullptr;  // [nchan] plain iteration's last-sweep residual
 };
 
-// Exclusive prefix sum of n ints (three kernels, graph-capturable);
-// `total` (device int, may be null) receives the sum.
-void scan_exclusive(const int* in, int* out, int n, int* tmp, int* total, cudaStream_t st);
-size_t scan_tmp_ints(int n);
-
 // Capsules of up to maxn nodes; > 48 KB of shared memory needs opting in.
 size_t membrane_smem_bytes(int maxn);
 cudaError_t prepare_membrane(int maxn);

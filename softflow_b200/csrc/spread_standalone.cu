@@ -2,20 +2,23 @@
 // (reference immersed_boundary.cpp:25-100) on caller-provided device buffers.
 //
 // Deterministic gather without floating-point atomics: markers are binned by
-// the 32 x 8 force tiles their 4 x 4 stencil covers; one warp per tile sorts
-// the tile's marker list and applies the markers in ascending order, so every
-// cell sums its contributions in the reference's serial order.  The sum is
+// the 32 x 8 force tiles their 4 x 4 stencil covers (counts, list space taken by
+// atomics, fill); one CTA per tile applies its markers in ascending order,
+// so every cell sums its contributions in the reference's serial order.  The sum is
 // added to the caller's field as the reference's OpenMP reduction does
 // (F += sum, immersed_boundary.cpp:70-79).  Built with --fmad=false.
-#include <climits>
-#include <string>
 #include <algorithm>
+#include <climits>
 #include <cmath>
+#include <mutex>
+#include <string>
 
 #include "../../include/softflow_gpu.h"
 #include "markers.cuh"
 #include "sfg_internal.h"
+#include "launch.cuh"
 #include "spread_standalone.cuh"
+#include "spread_wide.cuh"
 
 namespace sfg_host {
 void set_error(const std::string& msg);
@@ -61,6 +64,7 @@ __device__ __forceinline__ int sa_tiles(int nx, int ny, int tiles_x, int ix0, in
 __global__ void k_sa_prep(int nx, int ny, int tiles_x, int ncaps, const int* __restrict__ off,
                           const double2* __restrict__ pos, const double2* __restrict__ frc, int M,
                           SpreadScratch sc) {
+    chain_begin();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M) return;
     // num_markers must equal off[ncaps]; a marker beyond the rings (a larger
@@ -105,12 +109,11 @@ __global__ void k_sa_prep(int nx, int ny, int tiles_x, int ncaps, const int* __r
 // built without contraction, so the table equals the host-built one of the
 // simulation contexts bit for bit.
 __global__ void k_sa_init(int T, SpreadScratch sc) {
+    chain_begin();
     const int n = T > 1025 ? T : 1025;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (i < T) {
-            sc.tile_cnt[i] = 0;
-            sc.cursor[i] = 0;
-        }
+        if (i < T) sc.tile_cnt[i] = 0;
+        if (i == 0) *sc.total = 0;
         if (i <= 1024) {
             const double ar = 2.0 * static_cast<double>(i) / 1024;
             double v = 0.0;
@@ -121,102 +124,79 @@ __global__ void k_sa_init(int T, SpreadScratch sc) {
     }
 }
 
+// List space of every tile, one atomic per warp (where a list lies does not
+// matter): tile_pos[t] is the next free entry, tile_off[t] the first.
+__global__ void k_sa_alloc(int T, SpreadScratch sc) {
+    chain_begin();
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const int cnt = t < T ? sc.tile_cnt[t] : 0;
+    int inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    int base = 0;
+    if (lane == 31 && inc > 0) base = atomicAdd(sc.total, inc);
+    base = __shfl_sync(0xffffffffu, base, 31) + inc - cnt;
+    if (cnt > 0) {
+        sc.tile_off[t] = base;
+        sc.tile_pos[t] = base;
+    }
+}
+
 __global__ void k_sa_fill(int nx, int ny, int tiles_x, int M, SpreadScratch sc) {
+    chain_begin();
     const int m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= M || sc.ix0[m] == INT_MIN) return;
     int t[8];
     const int nt = sa_tiles(nx, ny, tiles_x, sc.ix0[m], sc.iy0[m], t);
-    for (int i = 0; i < nt; ++i)
-        sc.list[sc.tile_off[t[i]] + atomicAdd(&sc.cursor[t[i]], 1)] = m;
+    for (int i = 0; i < nt; ++i) sc.list[atomicAdd(&sc.tile_pos[t[i]], 1)] = m;
 }
 
-constexpr int SA_WARPS = 8;
-constexpr int SA_LCAP = 256;  // a power of two: the bitonic sort pads to one
-
-__global__ void __launch_bounds__(SA_WARPS * 32)
+// One CTA per tile (spread_wide.cuh).  The staging lanes evaluate their markers'
+// weights.  Marker by marker, with two loads and the table lookups in a row for
+// each, one warp a tile, 500 rings of 40 markers on 1000 x 700 took 112 us.
+__global__ void __launch_bounds__(BAND_WARPS * 32)
 k_sa_gather(int nx, int ny, int tiles_x, int T, const double2* __restrict__ pos,
             const double2* __restrict__ frc, const double* __restrict__ phi_tbl,
             SpreadScratch sc, double* __restrict__ Fx, double* __restrict__ Fy) {
-    __shared__ double s_acc[SA_WARPS][2][TILE_CELLS];
-    __shared__ int s_list[SA_WARPS][SA_LCAP];
+    __shared__ BandSmem s_band[BAND_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    double* ax = s_acc[warp][0];
-    double* ay = s_acc[warp][1];
-    int* sl = s_list[warp];
-    const int sx = lane & 3, sy = (lane >> 2) & 3;
-    for (int t = blockIdx.x * SA_WARPS + warp; t < T; t += gridDim.x * SA_WARPS) {
-        int cnt = sc.tile_cnt[t];
+    BandSmem& B = s_band[warp];
+    chain_begin();
+    for (int t = blockIdx.x; t < T; t += gridDim.x) {   // uniform in the CTA
+        const int cnt = sc.tile_cnt[t];
         if (cnt == 0) continue;
-        const int off = sc.tile_off[t];
-        const int x0 = (t % tiles_x) * TILE_W, y0 = (t / tiles_x) * TILE_H;
-        const int* lst;
-        if (cnt <= SA_LCAP) {
-            int pow2 = 1;
-            while (pow2 < cnt) pow2 <<= 1;
-            for (int i = lane; i < pow2; i += 32) sl[i] = i < cnt ? sc.list[off + i] : INT_MAX;
-            __syncwarp();
-            for (int k = 2; k <= pow2; k <<= 1)
-                for (int j = k >> 1; j > 0; j >>= 1) {
-                    for (int i = lane; i < pow2; i += 32) {
-                        const int l = i ^ j;
-                        if (l > i) {
-                            const int a = sl[i], b = sl[l];
-                            if ((a > b) == ((i & k) == 0)) { sl[i] = b; sl[l] = a; }
-                        }
-                    }
-                    __syncwarp();
-                }
-            lst = sl;
-        } else {
-            if (lane == 0) {
-                int* a = sc.list + off;
-                for (int i = 1; i < cnt; ++i) {
-                    const int v = a[i];
-                    int j = i - 1;
-                    while (j >= 0 && a[j] > v) { a[j + 1] = a[j]; --j; }
-                    a[j + 1] = v;
-                }
-            }
-            __syncwarp();
-            lst = sc.list + off;
-        }
-        for (int c = lane; c < TILE_CELLS; c += 32) {
-            ax[c] = 0.0;
-            ay[c] = 0.0;
+        int* list = sc.list + sc.tile_off[t];
+        const int x0 = (t % tiles_x) * TILE_W + BAND_W * warp, y0 = (t / tiles_x) * TILE_H;
+        if (cnt > BAND_LIST) {
+            if (threadIdx.x == 0) long_list_sort(list, cnt);
+            __syncthreads();
         }
         __syncwarp();
-        for (int i = 0; i < cnt; ++i) {
-            const int m = lst[i];
-            if (lane < 16) {
-                const int ix = sc.ix0[m] - 1 + sx, iy = sc.iy0[m] - 1 + sy;
-                int jx = ix;
-                if (jx < 0) jx += nx;
-                if (jx >= nx) jx -= nx;
-                const int cxl = jx - x0, cyl = iy - y0;
-                if (iy >= 0 && iy < ny && cxl >= 0 && cxl < TILE_W && cyl >= 0 && cyl < TILE_H) {
-                    const double2 p = pos[m];
-                    const double w = phi_lut(phi_tbl, p.x - (double)ix) *
-                                     phi_lut(phi_tbl, p.y - (double)iy);
-                    if (w > 1e-15) {
-                        const double2 f = frc[m];
-                        const double ds = sc.ds[m];
-                        const int c = cyl * TILE_W + cxl;
-                        ax[c] += f.x * w * ds;
-                        ay[c] += f.y * w * ds;
-                    }
-                }
-            }
-            __syncwarp();
-        }
-        for (int c = lane; c < TILE_CELLS; c += 32) {
-            const int jx = x0 + (c % TILE_W), jy = y0 + (c / TILE_W);
+        for (int c = lane; c < BAND_ACC; c += 32) B.ax[c] = B.ay[c] = 0.0;
+        auto org_of = [&](int m) { return make_int2(sc.ix0[m], sc.iy0[m]); };
+        auto load = [&](int m, int sy, BandMarker& k) {
+            const double2 p = pos[m];
+            k.f = frc[m];
+            k.org = make_int2(sc.ix0[m], sc.iy0[m]);
+            k.ds = sc.ds[m];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) k.wx[q] = phi_lut(phi_tbl, p.x - (double)(k.org.x - 1 + q));
+            k.wy = phi_lut(phi_tbl, p.y - (double)(k.org.y - 1 + sy));
+        };
+        band_spread(B, list, cnt, nx, ny, x0, y0, lane, org_of, load);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int r = (lane >> 3) + 4 * h, a = r * BAND_ACC_W + (lane & 7);
+            const int jx = x0 + (lane & 7), jy = y0 + r;
             if (jx < nx && jy < ny) {
                 const size_t n = (size_t)jy * nx + jx;
-                Fx[n] = Fx[n] + ax[c];
-                Fy[n] = Fy[n] + ay[c];
+                Fx[n] = Fx[n] + B.ax[a];
+                Fy[n] = Fy[n] + B.ay[a];
             }
         }
-        __syncwarp();
     }
 }
 
@@ -224,7 +204,7 @@ size_t spread_scratch_bytes(int M, int T) {
     const size_t a = 256;
     auto up = [a](size_t b) { return (b + a - 1) / a * a; };
     return up(sizeof(double) * M) + 2 * up(sizeof(int) * M) + up(sizeof(int) * 8 * (size_t)M) +
-           3 * up(sizeof(int) * T) + up(sizeof(int) * scan_tmp_ints(T)) + up(sizeof(double) * 1025);
+           3 * up(sizeof(int) * T) + up(sizeof(int)) + up(sizeof(double) * 1025);
 }
 
 SpreadScratch carve_spread_scratch(void* base, int M, int T) {
@@ -238,8 +218,8 @@ SpreadScratch carve_spread_scratch(void* base, int M, int T) {
     sc.list = reinterpret_cast<int*>(p);          p += up(sizeof(int) * 8 * (size_t)M);
     sc.tile_cnt = reinterpret_cast<int*>(p);      p += up(sizeof(int) * T);
     sc.tile_off = reinterpret_cast<int*>(p);      p += up(sizeof(int) * T);
-    sc.cursor = reinterpret_cast<int*>(p);        p += up(sizeof(int) * T);
-    sc.scan_tmp = reinterpret_cast<int*>(p);      p += up(sizeof(int) * scan_tmp_ints(T));
+    sc.tile_pos = reinterpret_cast<int*>(p);      p += up(sizeof(int) * T);
+    sc.total = reinterpret_cast<int*>(p);         p += up(sizeof(int));
     sc.phi = reinterpret_cast<double*>(p);
     return sc;
 }
@@ -259,17 +239,14 @@ int run_spread(int nx, int ny, int ncaps, const int* off, const double* pos, con
     }
     const int B = 256, G = (M + B - 1) / B;
     const int Gi = std::min((std::max(T, 1025) + B - 1) / B, nsm * 8);
-    k_sa_init<<<Gi, B, 0, st>>>(T, sc);
-    k_sa_prep<<<G, B, 0, st>>>(nx, ny, tiles_x, ncaps, off,
-                               reinterpret_cast<const double2*>(pos),
-                               reinterpret_cast<const double2*>(frc), M, sc);
-    scan_exclusive(sc.tile_cnt, sc.tile_off, T, sc.scan_tmp, nullptr, st);
-    k_sa_fill<<<G, B, 0, st>>>(nx, ny, tiles_x, M, sc);
-    const int grid = std::max(1, std::min((T + SA_WARPS - 1) / SA_WARPS, nsm * 4));
-    k_sa_gather<<<grid, SA_WARPS * 32, 0, st>>>(nx, ny, tiles_x, T,
-                                                reinterpret_cast<const double2*>(pos),
-                                                reinterpret_cast<const double2*>(frc), sc.phi, sc,
-                                                Fx, Fy);
+    const double2 *p2 = reinterpret_cast<const double2*>(pos), *f2 = reinterpret_cast<const double2*>(frc);
+    const int grid = std::max(1, std::min(T, nsm * 6));
+    launch_chain(false, k_sa_init, Gi, B, 0, st, T, sc);
+    launch_chain(true, k_sa_prep, G, B, 0, st, nx, ny, tiles_x, ncaps, off, p2, f2, M, sc);
+    launch_chain(true, k_sa_alloc, (T + B - 1) / B, B, 0, st, T, sc);
+    launch_chain(true, k_sa_fill, G, B, 0, st, nx, ny, tiles_x, M, sc);
+    launch_chain(true, k_sa_gather, grid, BAND_WARPS * 32, 0, st, nx, ny, tiles_x, T, p2, f2,
+                 (const double*)sc.phi, sc, Fx, Fy);
     e = cudaGetLastError();
     if (e != cudaSuccess) {
         sfg_host::set_error(std::string("spread: ") + cudaGetErrorString(e));
@@ -295,6 +272,48 @@ int check_spread_args(int nx, int ny, int ncaps, const int* off, const double* p
 
 using namespace sfg;
 
+namespace {
+
+// Scratch memory of sfg_spread_forces: a pool of its own per device that keeps at
+// most 32 MiB (one chunk of the driver's) between calls.  The device's default pool gives its memory back
+// whenever the stream is waited for, and the next call maps it anew: a caller
+// that waits for each spread paid 600 us for 140 us of work.  Null while a stream is
+// being captured (the call's allocation then becomes a node of the graph, from
+// the default pool, as ever) or when the pool cannot be made.
+cudaMemPool_t scratch_pool(cudaStream_t st) {
+    constexpr int kMaxDevices = 64;
+    static std::mutex mutex;
+    static cudaMemPool_t pools[kMaxDevices] = {};
+    static bool failed[kMaxDevices] = {};
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    int dev = 0;
+    if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
+        cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    std::lock_guard<std::mutex> lock(mutex);
+    if (!pools[dev] && !failed[dev]) {
+        cudaMemPoolProps props = {};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        unsigned long long keep = 32ull << 20;
+        cudaMemPool_t pool = nullptr;
+        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+            cudaGetLastError();
+            if (pool) cudaMemPoolDestroy(pool);
+            failed[dev] = true;
+        } else {
+            pools[dev] = pool;
+        }
+    }
+    return pools[dev];
+}
+
+}  // namespace
+
 extern "C" int sfg_spread_forces(int nx, int ny, int ncaps, const int* d_offsets,
                                  const double* d_pos, const double* d_force, double* d_Fx,
                                  double* d_Fy, int num_markers, void* stream) {
@@ -306,7 +325,10 @@ extern "C" int sfg_spread_forces(int nx, int ny, int ncaps, const int* d_offsets
     const int tiles_x = (nx + TILE_W - 1) / TILE_W, tiles_y = (ny + TILE_H - 1) / TILE_H;
     const int T = tiles_x * tiles_y, M = num_markers;
     void* base = nullptr;
-    cudaError_t e = cudaMallocAsync(&base, spread_scratch_bytes(M, T), st);
+    const cudaMemPool_t pool = scratch_pool(st);
+    const size_t bytes = spread_scratch_bytes(M, T);
+    cudaError_t e = pool ? cudaMallocFromPoolAsync(&base, bytes, pool, st)
+                         : cudaMallocAsync(&base, bytes, st);
     if (e != cudaSuccess) {
         sfg_host::set_error(std::string("sfg_spread_forces: ") + cudaGetErrorString(e));
         return SFG_ERR_CUDA;

@@ -13,9 +13,9 @@ struct SpreadScratch {
     int* iy0 = nullptr;         // [M]
     int* list = nullptr;        // [8 M] markers per covered tile
     int* tile_cnt = nullptr;    // [T]
-    int* tile_off = nullptr;    // [T]
-    int* cursor = nullptr;      // [T]
-    int* scan_tmp = nullptr;
+    int* tile_off = nullptr;    // [T] first list entry
+    int* tile_pos = nullptr;    // [T] next free list entry
+    int* total = nullptr;       // [1] list entries
     double* phi = nullptr;      // [1025] Peskin table
 };
 

@@ -96,3 +96,17 @@ def test_spread_momentum_conservation(sfg, oracle_mod, nx, ny, center, R, Nn, f)
                                lambda p: np.tile(np.array(f), (len(p), 1)))
     F = _gpu_spread(nx, ny, o.offsets(), pos, frc)
     assert _residual(F, pos, f, nx) < 1e-12
+
+
+@pytest.mark.parametrize("nx", [12, 33, 64])
+@pytest.mark.parametrize("copies", [1, 2, 12, 14])
+def test_spread_list_lengths(sfg, oracle_mod, nx, copies):
+    """Tile lists of up to 32 entries (sorted in registers), up to 256 (in shared
+    memory) and beyond (in place), in channels narrower than a tile, with a last
+    tile of one column, and of whole tiles: bit for bit the serial sum."""
+    rng = np.random.default_rng(11)
+    rings = [(6.4 + 0.01 * k, 11.7, 2.5, 20) for k in range(copies)]
+    o, pos, frc = _ring_system(nx, 24, rings, lambda p: rng.normal(0, 1e-3, p.shape))
+    Fx, Fy = o.spread()
+    gx, gy = _gpu_spread(nx, 24, o.offsets(), pos, frc)
+    assert np.array_equal(gx, Fx) and np.array_equal(gy, Fy)
