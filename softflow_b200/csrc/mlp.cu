@@ -5,7 +5,10 @@
 // per 128 samples: forward, backward and the CTA's partial weight gradients,
 // all GEMMs as tcgen05.mma with BF16 operands and FP32 accumulators in tensor
 // memory) and k_mlp_adam (sums the partials in a fixed order, so training is
-// deterministic, and applies Adam to the FP32 master weights).
+// deterministic, and applies Adam to the FP32 master weights and their BF16
+// operand image).  The batches of a call are one chain of launches that are
+// set up while their predecessors run; a row list (the shuffled order of an
+// epoch) is followed by the tile's own loads, without a shuffled copy.
 //
 // Loss: mean over samples and outputs of (y - t)^2 on normalised targets; the
 // per-sample output gradient 2 (y - t) / 2 and the batch mean follow the
@@ -15,6 +18,7 @@
 #include <vector>
 
 #include "../../include/softflow_gpu.h"
+#include "launch.cuh"
 #include "mlp.cuh"
 
 namespace sfg_host {
@@ -24,20 +28,32 @@ void set_error(const std::string& msg);
 namespace sfg {
 namespace mlp {
 
-constexpr int NB = 96;  // width of the weight-gradient GEMM (H1^T, X^T, ones, zeros)
+constexpr int HXW = 96;             // width of [H1 | X | 1 | 0]
+constexpr int DZW = 2 * N_H;        // width of [dZ2 | dZ1]
+constexpr int TRAIN_THREADS = 2 * ROWS;
+constexpr int PART_STRIDE = (N_PARAMS + 3) / 4 * 4;  // 16-byte rows of partial gradients
+constexpr unsigned ST_TIMEOUT = 1u, ST_BAD_ROW = 2u;
 
-struct __align__(1024) BwdSmem {
-    __nv_bfloat16 dY[ROWS * K1];     // [128 x 16] A of dH2 (columns 0, 1)
-    __nv_bfloat16 W3T[N_H * K1];     // [64 x 16]  B of dH2: (n, k) = W3[k][n]
-    __nv_bfloat16 W2T[N_H * N_H];    // [64 x 64]  B of dH1: (n, k) = W2[k][n]
-    __nv_bfloat16 dZ2[ROWS * N_H];   // [128 x 64] A of dH1
-    __nv_bfloat16 AT[ROWS * ROWS];   // [128 x 128] rows 0..63 dZ2^T, 64..127 dZ1^T
-    __nv_bfloat16 BT[NB * ROWS];     // [96 x 128] rows 0..63 H1^T, 64..79 X^T, 80 ones
-    float dYf[ROWS * N_OUT];
+// Shared-memory image of a training tile.  Every operand is stored once and
+// read both ways: along its columns by the layers, and transposed (the sample
+// index as K, opdesc_t) by the weight-gradient GEMM; W2 and W3 likewise serve
+// the forward and the backward pass.
+struct __align__(1024) TrainSmem {
+    __nv_bfloat16 HX[ROWS * HXW];    // 24 KB: H1 (0..63), X (64..79), ones (80), zeros
+    __nv_bfloat16 DZ[ROWS * DZW];    // 32 KB: dZ2 (0..63), dZ1 (64..127)
+    __nv_bfloat16 H2[ROWS * N_H];    // 16 KB
+    __nv_bfloat16 dY[ROWS * K1];     // 4 KB: columns 0, 1
+    __nv_bfloat16 W1[N_H * K1];      // 2 KB
+    __nv_bfloat16 W3[N3 * N_H];      // 2 KB
+    __nv_bfloat16 W2[N_H * N_H];     // 8 KB
+    float2 dYf[ROWS];
+    float b2[N_H], b3[N_OUT];
+    float in_mean[N_IN], in_inv_std[N_IN], out_mean[N_OUT], out_std[N_OUT];
     float red[ROWS / 32];
+    uint64_t bar;
+    uint32_t taddr;
+    int error;
 };
-
-constexpr size_t TRAIN_SMEM = sizeof(FwdSmem) + sizeof(BwdSmem);
 
 // norm layout: in_mean[8], in_inv_std[8], out_mean[2], out_std[2]
 __global__ void k_build_model(const float* __restrict__ p, const float* __restrict__ norm,
@@ -69,182 +85,295 @@ k_mlp_forward(const ModelDev* __restrict__ md, const float* __restrict__ x, int 
             y[(size_t)i * 2 + 1] = out[1] * s.out_std[1] + s.out_mean[1];
         }
     }
-    if (finish_tiles(s, phase, 128) && threadIdx.x == 0) atomicOr(status, 1u);
+    if (finish_tiles(s, phase, 128) && threadIdx.x == 0) atomicOr(status, ST_TIMEOUT);
 }
 
-// One CTA: samples [128 b, 128 b + 128) of the batch.  Writes the CTA's
+// The gradient through a layer's ReLU: the 16 accumulator columns v where the
+// activations H (columns h .. h + 15 of row r) are positive, else 0, into
+// columns d .. d + 15 of DZ.
+__device__ __forceinline__ void put_gated16(__nv_bfloat16* DZ, int d, const __nv_bfloat16* H,
+                                            int h, int HW, int r, float* v) {
+#pragma unroll
+    for (int half = 0; half < 16; half += 8) {
+        const uint4 u = *reinterpret_cast<const uint4*>(H + kmaj(r, h + half, HW));
+        const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const uint32_t bits = (i & 1) ? (w[i >> 1] & 0xffff0000u) : (w[i >> 1] << 16);
+            v[half + i] = __uint_as_float(bits) > 0.0f ? v[half + i] : 0.0f;
+        }
+        put8(DZ, r, d + half, DZW, v + half);
+    }
+}
+
+// One CTA: samples [128 b, 128 b + 128) of the batch, sample i being row
+// rows[i] of the data (row first + i without a row list).  Writes the CTA's
 // partial gradient (N_PARAMS floats) and partial squared error.
-__global__ void __launch_bounds__(ROWS)
-k_mlp_train_tile(const float* __restrict__ p, const float* __restrict__ norm,
-                 const float* __restrict__ x, const float* __restrict__ t, int n, float inv_n,
-                 float* __restrict__ part, float* __restrict__ part_loss,
-                 unsigned* __restrict__ status) {
+//
+// Bound: one tile's chain of latencies (six rounds of MMAs with their barriers
+// and TMEM reads); a batch of 8192 samples is 64 CTAs.  So the weights arrive
+// ready-made in the operand layouts (k_mlp_adam keeps the image), no operand
+// is transposed through shared memory, warps 4-7 do the layer-3 gradients
+// beside the backward rounds of warps 0-3, and the samples are loaded before
+// the wait for the previous step.  Batch of 8192, cold caches: 26.0 us with conversion,
+// transposed copies and layer 3 at the end, 10.7 us so.
+__global__ void __launch_bounds__(TRAIN_THREADS)
+k_mlp_train_tile(const ModelDev* __restrict__ md, const float* __restrict__ x,
+                 const float* __restrict__ t, const long long* __restrict__ rows, long long first,
+                 long long n_rows, int n, float inv_n, float* __restrict__ part,
+                 float* __restrict__ part_loss, unsigned* __restrict__ status) {
     extern __shared__ __align__(1024) unsigned char smem_raw[];
-    FwdSmem& s = *reinterpret_cast<FwdSmem*>(smem_raw);
-    BwdSmem& b = *reinterpret_cast<BwdSmem*>(smem_raw + sizeof(FwdSmem));
+    TrainSmem& s = *reinterpret_cast<TrainSmem*>(smem_raw);
     const int r = threadIdx.x;
-    // weights in operand layouts, straight from the FP32 master copy
-    for (int i = r; i < N_H * N_H; i += ROWS) {
-        const int o = i / N_H, k = i % N_H;
-        const float w = p[P_W2 + i];
-        s.W2[kmaj(o, k, N_H)] = __float2bfloat16_rn(w);
-        b.W2T[kmaj(k, o, N_H)] = __float2bfloat16_rn(w);
+    const bool chain = r < ROWS;  // warps 0-3: one sample each
+    const int i = blockIdx.x * ROWS + r;
+    // The samples are no kernel of the chain's work (the chain's first kernel
+    // is launched without overlap): they may be read before the wait.
+    bool valid = chain && i < n, bad = false;
+    float f[N_IN] = {}, tr[N_OUT] = {};
+    if (valid) {
+        const long long row = rows ? rows[first + i] : first + i;
+        bad = row < 0 || row >= n_rows;
+        valid = !bad;
+        if (valid) {
+#pragma unroll
+            for (int k = 0; k < N_IN; ++k) f[k] = x[row * N_IN + k];
+#pragma unroll
+            for (int k = 0; k < N_OUT; ++k) tr[k] = t[row * N_OUT + k];
+        }
     }
-    for (int i = r; i < N_H * K1; i += ROWS) {
-        const int o = i / K1, k = i % K1;
-        float v = 0.0f;
-        if (k < N_IN) v = p[P_W1 + o * N_IN + k];
-        else if (k == N_IN) v = p[P_B1 + o];
-        s.W1[kmaj(o, k, K1)] = __float2bfloat16_rn(v);
-        // W3T: (n = o, k) = W3[k][o] for k < 2
-        b.W3T[kmaj(o, k, K1)] = __float2bfloat16_rn(k < N_OUT ? p[P_W3 + k * N_H + o] : 0.0f);
-    }
-    for (int i = r; i < N3 * N_H; i += ROWS) {
-        const int o = i / N_H, k = i % N_H;
-        s.W3[kmaj(o, k, N_H)] = __float2bfloat16_rn(o < N_OUT ? p[P_W3 + o * N_H + k] : 0.0f);
-    }
-    if (r < N_H) s.b2[r] = p[P_B2 + r];
-    if (r < N_OUT) {
-        s.b3[r] = p[P_B3 + r];
-        s.out_mean[r] = norm[16 + r];
-        s.out_std[r] = norm[18 + r];
-    }
-    if (r < N_IN) {
-        s.in_mean[r] = norm[r];
-        s.in_inv_std[r] = norm[8 + r];
-    }
-    // rows 80..95 of BT: ones (bias gradient of layer 2), then zeros
-    for (int k = 80; k < NB; ++k) b.BT[kmaj(k, r, ROWS)] = __float2bfloat16_rn(k == 80 ? 1.0f : 0.0f);
-    __syncthreads();
+    chain_begin();
+    load_model<TRAIN_THREADS>(s, md);
+    // only now: a later step's CTAs must not hold tensor memory that this
+    // step's still wait for
     start_tiles(s, 256);
     uint32_t phase = 0;
-    const int i = blockIdx.x * ROWS + r;
-    const bool valid = i < n;
-    float f[N_IN];
-#pragma unroll
-    for (int k = 0; k < N_IN; ++k) f[k] = valid ? x[(size_t)i * N_IN + k] : 0.0f;
-    put_input_row(s, f, valid);
-    float y[2];
-    bool ok = forward_tile(s, s.taddr, phase, y);
-    float dy0 = 0.0f, dy1 = 0.0f, se = 0.0f;
-    if (valid) {
-        const float t0 = (t[(size_t)i * 2 + 0] - s.out_mean[0]) / s.out_std[0];
-        const float t1 = (t[(size_t)i * 2 + 1] - s.out_mean[1]) / s.out_std[1];
-        const float e0 = y[0] - t0, e1 = y[1] - t1;
-        se = e0 * e0 + e1 * e1;
-        dy0 = e0 * inv_n;
-        dy1 = e1 * inv_n;
-    }
-    b.dYf[r * 2 + 0] = dy0;
-    b.dYf[r * 2 + 1] = dy1;
-#pragma unroll
-    for (int k = 0; k < K1; ++k)
-        b.dY[kmaj(r, k, K1)] = __float2bfloat16_rn(k == 0 ? dy0 : (k == 1 ? dy1 : 0.0f));
-    // transposed copies of this row's H1 and X for the weight-gradient GEMM
-#pragma unroll 8
-    for (int c = 0; c < N_H; ++c) b.BT[kmaj(c, r, ROWS)] = s.H1[kmaj(r, c, N_H)];
-#pragma unroll
-    for (int k = 0; k < K1; ++k) b.BT[kmaj(N_H + k, r, ROWS)] = s.X[kmaj(r, k, K1)];
     const uint32_t tb = s.taddr;
-    // dH2 = dY W3 -> columns [0, 64)
-    if (ok) ok = layer<K1>(s, tb, b.dY, b.W3T, idesc_bf16(ROWS, N_H), phase);
-    if (ok) {
-        float v[16];
-#pragma unroll
-        for (int c = 0; c < N_H; c += 16) {
-            tmem_ld16(tmem_row(tb, c), v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const bool on = __bfloat162float(s.H2[kmaj(r, c + j, N_H)]) > 0.0f;
-                const __nv_bfloat16 d = __float2bfloat16_rn(on ? v[j] : 0.0f);
-                b.dZ2[kmaj(r, c + j, N_H)] = d;
-                b.AT[kmaj(c + j, r, ROWS)] = d;
-            }
+    float* gp = part + (size_t)blockIdx.x * PART_STRIDE;
+    bool ok = true;
+    if (chain) {
+        if (bad) atomicOr(status, ST_BAD_ROW);
+        put_input_cols(s, s.HX, N_H, HXW, f, valid);
+        {
+            // the ones column (bias gradient of layer 2), then zeros
+            float v[8] = {1.0f};
+            put8(s.HX, r, 80, HXW, v);
+            v[0] = 0.0f;
+            put8(s.HX, r, 88, HXW, v);
         }
-    }
-    // dH1 = dZ2 W2 -> columns [64, 128)
-    if (ok) ok = layer<N_H>(s, tb + 64, b.dZ2, b.W2T, idesc_bf16(ROWS, N_H), phase);
-    if (ok) {
         float v[16];
+        ok = mma_round<true>(s, phase, [&] {
+            mma(tb, opdesc(s.HX + kmaj(0, N_H, HXW), HXW, 0), opdesc(s.W1, K1, 0),
+                idesc_bf16(ROWS, N_H), 0u);
+        });
+        if (ok) {
 #pragma unroll
-        for (int c = 0; c < N_H; c += 16) {
-            tmem_ld16(tmem_row(tb, 64 + c), v);
-#pragma unroll
-            for (int j = 0; j < 16; ++j) {
-                const bool on = __bfloat162float(s.H1[kmaj(r, c + j, N_H)]) > 0.0f;
-                b.AT[kmaj(N_H + c + j, r, ROWS)] = __float2bfloat16_rn(on ? v[j] : 0.0f);
+            for (int c = 0; c < N_H; c += 16) {
+                tmem_ld16(tmem_row(tb, c), v);
+                put_relu16(s.HX, r, c, HXW, v, nullptr);
             }
+            ok = mma_round<true>(s, phase, [&] {
+#pragma unroll
+                for (int kk = 0; kk < N_H / 16; ++kk)
+                    mma(tb + 64, opdesc(s.HX, HXW, kk), opdesc(s.W2, N_H, kk),
+                        idesc_bf16(ROWS, N_H), kk > 0 ? 1u : 0u);
+            });
         }
+        if (ok) {
+#pragma unroll
+            for (int c = 0; c < N_H; c += 16) {
+                tmem_ld16(tmem_row(tb, 64 + c), v);
+                put_relu16(s.H2, r, c, N_H, v, s.b2 + c);
+            }
+            ok = mma_round<true>(s, phase, [&] {
+#pragma unroll
+                for (int kk = 0; kk < N_H / 16; ++kk)
+                    mma(tb, opdesc(s.H2, N_H, kk), opdesc(s.W3, N_H, kk), idesc_bf16(ROWS, N3),
+                        kk > 0 ? 1u : 0u);
+            });
+        }
+        float y[2] = {0.0f, 0.0f};
+        if (ok) {
+            tmem_ld16(tmem_row(tb, 0), v);
+            y[0] = v[0] + s.b3[0];
+            y[1] = v[1] + s.b3[1];
+        }
+        float dy0 = 0.0f, dy1 = 0.0f, se = 0.0f;
+        if (valid) {
+            const float t0 = (tr[0] - s.out_mean[0]) / s.out_std[0];
+            const float t1 = (tr[1] - s.out_mean[1]) / s.out_std[1];
+            const float e0 = y[0] - t0, e1 = y[1] - t1;
+            se = e0 * e0 + e1 * e1;
+            dy0 = e0 * inv_n;
+            dy1 = e1 * inv_n;
+        }
+        s.dYf[r] = make_float2(dy0, dy1);
+        {
+            float d[8] = {dy0, dy1};
+            put8(s.dY, r, 0, K1, d);
+            d[0] = d[1] = 0.0f;
+            put8(s.dY, r, 8, K1, d);
+        }
+        // squared error of the CTA
+        for (int o = 16; o > 0; o >>= 1) se += __shfl_down_sync(0xffffffffu, se, o);
+        if ((r & 31) == 0) s.red[r >> 5] = se;
     }
-    // [dZ2^T; dZ1^T] [H1^T; X^T; 1]^T -> columns [128, 224)
-    if (ok) ok = layer<ROWS>(s, tb + 128, b.AT, b.BT, idesc_bf16(ROWS, NB), phase);
-    float* gp = part + (size_t)blockIdx.x * N_PARAMS;
-    if (ok) {
+    __syncthreads();  // dYf, H2 and red are complete
+    if (!chain) {
+        // layer-3 gradients on the CUDA cores: dW3 = dY^T H2, db3 = sum dY,
+        // each one sum over the samples in order
+        const int u = r - ROWS;
+        if (u < N_H) {
+            float a0 = 0.0f, a1 = 0.0f;
+#pragma unroll 16
+            for (int q = 0; q < ROWS; ++q) {
+                const float h = __bfloat162float(s.H2[kmaj(q, u, N_H)]);
+                const float2 d = s.dYf[q];
+                a0 = fmaf(d.x, h, a0);
+                a1 = fmaf(d.y, h, a1);
+            }
+            gp[P_W3 + u] = a0;
+            gp[P_W3 + N_H + u] = a1;
+        } else if (u == N_H) {
+            float d0 = 0.0f, d1 = 0.0f;
+#pragma unroll 16
+            for (int q = 0; q < ROWS; ++q) {
+                const float2 d = s.dYf[q];
+                d0 += d.x;
+                d1 += d.y;
+            }
+            gp[P_B3 + 0] = d0;
+            gp[P_B3 + 1] = d1;
+        } else if (u == N_H + 32) {
+            part_loss[blockIdx.x] = s.red[0] + s.red[1] + s.red[2] + s.red[3];
+        }
+    } else {
         float v[16];
-        if (r < N_H) {
+        // dH2 = dY W3 -> columns [0, 64)
+        if (ok)
+            ok = mma_round<true>(s, phase, [&] {
+                mma(tb, opdesc(s.dY, K1, 0), opdesc_t(s.W3, N_H, 0),
+                    idesc_bf16(ROWS, N_H) | B_MN_MAJOR, 0u);
+            });
+        if (ok) {
+#pragma unroll
+            for (int c = 0; c < N_H; c += 16) {
+                tmem_ld16(tmem_row(tb, c), v);
+                put_gated16(s.DZ, c, s.H2, c, N_H, r, v);
+            }
+            // dH1 = dZ2 W2 -> columns [64, 128)
+            ok = mma_round<true>(s, phase, [&] {
+#pragma unroll
+                for (int kk = 0; kk < N_H / 16; ++kk)
+                    mma(tb + 64, opdesc(s.DZ, DZW, kk), opdesc_t(s.W2, N_H, kk),
+                        idesc_bf16(ROWS, N_H) | B_MN_MAJOR, kk > 0 ? 1u : 0u);
+            });
+        }
+        if (ok) {
+#pragma unroll
+            for (int c = 0; c < N_H; c += 16) {
+                tmem_ld16(tmem_row(tb, 64 + c), v);
+                put_gated16(s.DZ, N_H + c, s.HX, c, HXW, r, v);
+            }
+            // [dZ2 | dZ1]^T [H1 | X | 1] -> columns [128, 224)
+            ok = mma_round<true>(s, phase, [&] {
+#pragma unroll
+                for (int kk = 0; kk < ROWS / 16; ++kk)
+                    mma(tb + 128, opdesc_t(s.DZ, DZW, kk), opdesc_t(s.HX, HXW, kk),
+                        idesc_bf16(ROWS, HXW) | A_MN_MAJOR | B_MN_MAJOR, kk > 0 ? 1u : 0u);
+            });
+        }
+        if (ok && r < N_H) {
+            float4* g2 = reinterpret_cast<float4*>(gp + P_W2 + r * N_H);
 #pragma unroll
             for (int c = 0; c < N_H; c += 16) {
                 tmem_ld16(tmem_row(tb, 128 + c), v);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) gp[P_W2 + r * N_H + c + j] = v[j];
+                for (int j = 0; j < 16; j += 4)
+                    g2[(c + j) / 4] = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
             }
             tmem_ld16(tmem_row(tb, 128 + 80), v);
             gp[P_B2 + r] = v[0];
-        } else {
+        } else if (ok) {
             // warps 2 and 3: rows 64..127 are dW1 (columns 64..71) and db1 (72)
             const int o = r - N_H;
             tmem_ld16(tmem_row(tb, 128 + 64), v);
-#pragma unroll
-            for (int k = 0; k < N_IN; ++k) gp[P_W1 + o * N_IN + k] = v[k];
+            float4* g1 = reinterpret_cast<float4*>(gp + P_W1 + o * N_IN);
+            g1[0] = make_float4(v[0], v[1], v[2], v[3]);
+            g1[1] = make_float4(v[4], v[5], v[6], v[7]);
             gp[P_B1 + o] = v[N_IN];
         }
     }
-    // layer-3 gradients on the CUDA cores: dW3 = dY^T H2, db3 = sum dY
-    __syncthreads();
-    {
-        const int o = r >> 6, j = r & 63;
-        float acc = 0.0f;
-        for (int q = 0; q < ROWS; ++q)
-            acc = fmaf(b.dYf[q * 2 + o], __bfloat162float(s.H2[kmaj(q, j, N_H)]), acc);
-        gp[P_W3 + o * N_H + j] = acc;
-        if (r < N_OUT) {
-            float d = 0.0f;
-            for (int q = 0; q < ROWS; ++q) d += b.dYf[q * 2 + r];
-            gp[P_B3 + r] = d;
-        }
-    }
-    // squared error of the CTA
-    for (int o = 16; o > 0; o >>= 1) se += __shfl_down_sync(0xffffffffu, se, o);
-    if ((r & 31) == 0) b.red[r >> 5] = se;
-    if (finish_tiles(s, phase, 256) && r == 0) atomicOr(status, 1u);
-    if (r == 0) part_loss[blockIdx.x] = b.red[0] + b.red[1] + b.red[2] + b.red[3];
+    if (finish_tiles(s, phase, 256) && r == 0) atomicOr(status, ST_TIMEOUT);
 }
 
-// Sums the CTA partials in CTA order; then Adam (step > 0) or the plain
-// gradient into g_out (step == 0).
-__global__ void k_mlp_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
-                           const float* __restrict__ part, int nparts, int step, float lr,
-                           float* __restrict__ g_out, const float* __restrict__ part_loss,
-                           float loss_scale, float* __restrict__ loss_out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i == 0 && loss_out) {
+// The parameter's place in the operand image.
+__device__ __forceinline__ void put_param(ModelDev* md, int i, float w) {
+    const __nv_bfloat16 h = __float2bfloat16_rn(w);
+    if (i < P_B1) md->W1[kmaj(i / N_IN, i % N_IN, K1)] = h;
+    else if (i < P_W2) md->W1[kmaj(i - P_B1, N_IN, K1)] = h;
+    else if (i < P_B2) md->W2[kmaj((i - P_W2) / N_H, (i - P_W2) % N_H, N_H)] = h;
+    else if (i < P_W3) md->b2[i - P_B2] = w;
+    else if (i < P_B3) md->W3[kmaj((i - P_W3) / N_H, (i - P_W3) % N_H, N_H)] = h;
+    else md->b3[i - P_B3] = w;
+}
+
+// Sums the CTA partials in CTA order; then Adam (step > 0), which also renews
+// the parameter in the operand image, or the plain gradient into g_out
+// (step == 0).  The last warp of the grid adds up the loss, also in CTA order.
+//
+// Bound: the latency of the loads (4866 sums over 64 partials for a batch of
+// 8192), so 32 loads are in flight per thread, the threads lie on 77 CTAs, and the
+// loss's partials are loaded by 32 lanes: 7.3 us -> 5.5 us (of that the loss alone,
+// by one thread, had taken longer than all else).
+constexpr int ADAM_THREADS = 64, ADAM_LOADS = 32;
+constexpr int ADAM_BLOCKS = (N_PARAMS + ADAM_THREADS - 1) / ADAM_THREADS + 1;
+__global__ void __launch_bounds__(ADAM_THREADS)
+k_mlp_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
+           const float* __restrict__ part, int nparts, int step, float lr,
+           float* __restrict__ g_out, const float* __restrict__ part_loss, float loss_scale,
+           float* __restrict__ loss_out, ModelDev* __restrict__ md) {
+    chain_begin();
+    if (blockIdx.x == gridDim.x - 1) {
+        const int lane = threadIdx.x;
+        if (lane >= 32 || !loss_out) return;
         float l = 0.0f;
-        for (int c = 0; c < nparts; ++c) l += part_loss[c];
-        *loss_out = l * loss_scale;
+        for (int c0 = 0; c0 < nparts; c0 += 32) {
+            const float q = c0 + lane < nparts ? part_loss[c0 + lane] : 0.0f;
+            const int cnt = min(32, nparts - c0);
+            for (int c = 0; c < cnt; ++c) l += __shfl_sync(0xffffffffu, q, c);
+        }
+        if (lane == 0) *loss_out = l * loss_scale;
+        return;
     }
+    const int i = blockIdx.x * ADAM_THREADS + threadIdx.x;
     if (i >= N_PARAMS) return;
+    const float m0 = m[i], v0 = v[i], p0 = p[i];
     float g = 0.0f;
-    for (int c = 0; c < nparts; ++c) g += part[(size_t)c * N_PARAMS + i];
+    int c = 0;
+    for (; c + ADAM_LOADS <= nparts; c += ADAM_LOADS) {
+        float q[ADAM_LOADS];
+#pragma unroll
+        for (int j = 0; j < ADAM_LOADS; ++j) q[j] = part[(size_t)(c + j) * PART_STRIDE + i];
+#pragma unroll
+        for (int j = 0; j < ADAM_LOADS; ++j) g += q[j];
+    }
+#pragma unroll 4
+    for (; c < nparts; ++c) g += part[(size_t)c * PART_STRIDE + i];
     if (g_out) g_out[i] = g;
     if (step <= 0) return;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
-    const float mi = b1 * m[i] + (1.0f - b1) * g;
-    const float vi = b2 * v[i] + (1.0f - b2) * g * g;
+    // the rounding is written out: left to the compiler, which product is fused
+    // depends on where the loads stand
+    const float mi = fmaf(1.0f - b1, g, b1 * m0);
+    const float vi = fmaf((1.0f - b2) * g, g, b2 * v0);
     m[i] = mi;
     v[i] = vi;
     const float mh = mi / (1.0f - powf(b1, (float)step));
     const float vh = vi / (1.0f - powf(b2, (float)step));
-    p[i] -= lr * mh / (sqrtf(vh) + eps);
+    const float w = p0 - lr * mh / (sqrtf(vh) + eps);
+    p[i] = w;
+    put_param(md, i, w);
 }
 
 }  // namespace mlp
@@ -260,7 +389,8 @@ struct sfg_mlp {
     float* d_m = nullptr;
     float* d_v = nullptr;
     float* d_norm = nullptr;
-    sfg::mlp::ModelDev* d_model = nullptr;
+    sfg::mlp::ModelDev* d_model = nullptr;  // forward's and the step's, built on demand
+    sfg::mlp::ModelDev* d_train = nullptr;  // the training steps' own, renewed by each
     float* d_part = nullptr;
     float* d_part_loss = nullptr;
     float* d_loss = nullptr;
@@ -291,7 +421,7 @@ int ensure_parts(sfg_mlp* m, int nparts) {
     if (m->d_part_loss) cudaFree(m->d_part_loss);
     m->d_part = nullptr;
     m->d_part_loss = nullptr;
-    MCU(cudaMalloc(&m->d_part, sizeof(float) * (size_t)nparts * N_PARAMS));
+    MCU(cudaMalloc(&m->d_part, sizeof(float) * (size_t)nparts * PART_STRIDE));
     MCU(cudaMalloc(&m->d_part_loss, sizeof(float) * nparts));
     m->part_cap = nparts;
     return SFG_OK;
@@ -301,7 +431,12 @@ int check_status(sfg_mlp* m, cudaStream_t st, const char* who) {
     unsigned s = 0;
     MCU(cudaMemcpyAsync(&s, m->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
     MCU(cudaStreamSynchronize(st));
-    if (s) return fail(SFG_ERR_CUDA, std::string(who) + ": a tensor-core wait timed out");
+    if (s & ST_TIMEOUT)
+        return fail(SFG_ERR_CUDA, std::string(who) + ": a tensor-core wait timed out");
+    if (s & ST_BAD_ROW) {
+        MCU(cudaMemset(m->d_status, 0, sizeof(unsigned)));
+        return fail(SFG_ERR_ARG, std::string(who) + ": row index out of range");
+    }
     return SFG_OK;
 }
 
@@ -310,28 +445,43 @@ int prepare_kernels(int device) {
     const unsigned long long bit = (device >= 0 && device < 64) ? (1ull << device) : 0ull;
     if (bit && (done & bit)) return SFG_OK;
     MCU(cudaFuncSetAttribute(k_mlp_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)TRAIN_SMEM));
+                             (int)sizeof(TrainSmem)));
     MCU(cudaFuncSetAttribute(k_mlp_forward, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sizeof(FwdSmem)));
     done |= bit;
     return SFG_OK;
 }
 
-// one batch: partial gradients, then the reduction (+ Adam when step > 0)
-int batch_step(sfg_mlp* m, const float* x, const float* t, int n, int step, float lr,
-               float* g_out, float* loss_out, cudaStream_t st) {
+struct Samples {
+    const float *x, *t;
+    const long long* rows;  // null: consecutive rows
+    long long n_rows;
+};
+
+// one batch: partial gradients, then the reduction (+ Adam when step > 0).
+// `chained`: the stream's previous operation is the batch before it.
+int batch_step(sfg_mlp* m, const Samples& d, long long first, int n, int step, float lr,
+               float* g_out, float* loss_out, bool chained, cudaStream_t st) {
     const int nparts = (n + ROWS - 1) / ROWS;
-    int rc = ensure_parts(m, nparts);
-    if (rc) return rc;
-    k_mlp_train_tile<<<nparts, ROWS, TRAIN_SMEM, st>>>(m->d_params, m->d_norm, x, t, n,
-                                                        1.0f / (float)n, m->d_part,
-                                                        m->d_part_loss, m->d_status);
+    sfg::launch_chain(chained, k_mlp_train_tile, nparts, TRAIN_THREADS, sizeof(TrainSmem), st,
+                      m->d_train, d.x, d.t, d.rows, first, d.n_rows, n, 1.0f / (float)n,
+                      m->d_part, m->d_part_loss, m->d_status);
     MCU(cudaGetLastError());
-    k_mlp_adam<<<(N_PARAMS + 255) / 256, 256, 0, st>>>(
-        m->d_params, m->d_m, m->d_v, m->d_part, nparts, step, lr, g_out, m->d_part_loss,
-        1.0f / (2.0f * (float)n), loss_out);
+    sfg::launch_chain(true, k_mlp_adam, ADAM_BLOCKS, ADAM_THREADS, 0, st, m->d_params, m->d_m,
+                      m->d_v, m->d_part, nparts, step, lr, g_out, m->d_part_loss,
+                      1.0f / (2.0f * (float)n), loss_out, m->d_train);
     MCU(cudaGetLastError());
     if (step > 0) m->model_dirty = true;
+    return SFG_OK;
+}
+
+// The training image of the current parameters and normalisation, and room
+// for one batch's partial gradients.
+int begin_training(sfg_mlp* m, int n, cudaStream_t st) {
+    int rc = ensure_parts(m, (n + ROWS - 1) / ROWS);
+    if (rc) return rc;
+    k_build_model<<<(N_H * N_H + 255) / 256, 256, 0, st>>>(m->d_params, m->d_norm, m->d_train);
+    MCU(cudaGetLastError());
     return SFG_OK;
 }
 
@@ -352,6 +502,7 @@ extern "C" int sfg_mlp_create(int device, sfg_mlp** out) {
     if (e == cudaSuccess) e = cudaMalloc(&m->d_grad, sizeof(float) * N_PARAMS);
     if (e == cudaSuccess) e = cudaMalloc(&m->d_norm, sizeof(float) * 20);
     if (e == cudaSuccess) e = cudaMalloc(&m->d_model, sizeof(sfg::mlp::ModelDev));
+    if (e == cudaSuccess) e = cudaMalloc(&m->d_train, sizeof(sfg::mlp::ModelDev));
     if (e == cudaSuccess) e = cudaMalloc(&m->d_loss, sizeof(float) * 4096);
     if (e == cudaSuccess) e = cudaMalloc(&m->d_status, sizeof(unsigned));
     if (e == cudaSuccess) e = cudaMemset(m->d_params, 0, sizeof(float) * N_PARAMS);
@@ -375,7 +526,7 @@ extern "C" int sfg_mlp_destroy(sfg_mlp* m) {
     if (!m) return SFG_OK;
     cudaSetDevice(m->device);
     for (void* p : {(void*)m->d_params, (void*)m->d_m, (void*)m->d_v, (void*)m->d_norm,
-                    (void*)m->d_model, (void*)m->d_part, (void*)m->d_part_loss,
+                    (void*)m->d_model, (void*)m->d_train, (void*)m->d_part, (void*)m->d_part_loss,
                     (void*)m->d_loss, (void*)m->d_grad, (void*)m->d_status})
         if (p) cudaFree(p);
     delete m;
@@ -459,7 +610,9 @@ extern "C" int sfg_mlp_gradients(sfg_mlp* m, const float* d_x, const float* d_t,
     if (n <= 0) return fail(SFG_ERR_ARG, "sfg_mlp_gradients: empty batch");
     MCU(cudaSetDevice(m->device));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int rc = batch_step(m, d_x, d_t, n, 0, 0.0f, m->d_grad, m->d_loss, st);
+    int rc = begin_training(m, n, st);
+    if (rc) return rc;
+    rc = batch_step(m, {d_x, d_t, nullptr, n}, 0, n, 0, 0.0f, m->d_grad, m->d_loss, false, st);
     if (rc) return rc;
     if ((rc = check_status(m, st, "sfg_mlp_gradients"))) return rc;
     MCU(cudaMemcpy(grad, m->d_grad, sizeof(float) * N_PARAMS, cudaMemcpyDeviceToHost));
@@ -467,21 +620,23 @@ extern "C" int sfg_mlp_gradients(sfg_mlp* m, const float* d_x, const float* d_t,
     return SFG_OK;
 }
 
-extern "C" int sfg_mlp_train(sfg_mlp* m, const float* d_x, const float* d_t, int n, int batch,
-                             float lr, float* losses, void* stream) {
+extern "C" int sfg_mlp_train_rows(sfg_mlp* m, const float* d_x, const float* d_t,
+                                  const long long* d_rows, int n, int batch, float lr,
+                                  float* losses, void* stream) {
     if (!m || !d_x || !d_t) return fail(SFG_ERR_ARG, "sfg_mlp_train: null argument");
     if (n <= 0 || batch <= 0) return fail(SFG_ERR_ARG, "sfg_mlp_train: empty data or batch");
     MCU(cudaSetDevice(m->device));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nb = n / batch;
     if (nb < 1) return fail(SFG_ERR_ARG, "sfg_mlp_train: fewer samples than one batch");
-    std::vector<float> hl;
+    int rc = begin_training(m, batch, st);
+    if (rc) return rc;
+    const Samples d{d_x, d_t, d_rows, n};
     for (int b0 = 0; b0 < nb; b0 += 4096) {
         const int cnt = nb - b0 < 4096 ? nb - b0 : 4096;
         for (int k = 0; k < cnt; ++k) {
-            const size_t off = (size_t)(b0 + k) * batch;
-            int rc = batch_step(m, d_x + off * N_IN, d_t + off * N_OUT, batch, ++m->step, lr,
-                                nullptr, m->d_loss + k, st);
+            rc = batch_step(m, d, (long long)(b0 + k) * batch, batch, ++m->step, lr, nullptr,
+                            m->d_loss + k, k > 0, st);
             if (rc) return rc;
         }
         if (losses) {
@@ -490,6 +645,11 @@ extern "C" int sfg_mlp_train(sfg_mlp* m, const float* d_x, const float* d_t, int
         }
     }
     return check_status(m, st, "sfg_mlp_train");
+}
+
+extern "C" int sfg_mlp_train(sfg_mlp* m, const float* d_x, const float* d_t, int n, int batch,
+                             float lr, float* losses, void* stream) {
+    return sfg_mlp_train_rows(m, d_x, d_t, nullptr, n, batch, lr, losses, stream);
 }
 
 extern "C" int sfg_mlp_step_count(sfg_mlp* m, int* steps) {

@@ -49,6 +49,17 @@ __host__ __device__ __forceinline__ int kmaj(int r, int k, int K) {
     return ((((r >> 3) * (K >> 3)) + (k >> 3)) << 6) + ((r & 7) << 3) + (k & 7);
 }
 
+// Eight columns k .. k + 7 (k a multiple of 8) of row r in BF16: they are 16
+// contiguous bytes of the operand, so one store writes them, and the lanes of
+// a warp (rows r) fill whole core matrices.  Written one by one, the 2-byte
+// stores of a warp hit the same four banks four times over.
+__device__ __forceinline__ void put8(__nv_bfloat16* base, int r, int k, int K, const float* v) {
+    __nv_bfloat162 h[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) h[i] = __floats2bfloat162_rn(v[2 * i], v[2 * i + 1]);
+    *reinterpret_cast<uint4*>(base + kmaj(r, k, K)) = *reinterpret_cast<const uint4*>(h);
+}
+
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
@@ -64,6 +75,16 @@ __device__ __forceinline__ uint64_t sdesc(uint32_t saddr, uint32_t lbo, uint32_t
 __device__ __forceinline__ uint64_t opdesc(const __nv_bfloat16* base, int K, int kk) {
     return sdesc(smem_u32(base) + (uint32_t)kk * 256u, 128u, (uint32_t)(K >> 3) * 128u);
 }
+
+// The same matrix read transposed: of an operand stored as kmaj(r, c, W), the
+// K index is r and the M or N index is c (MN-major).  K-step kk is rows
+// 16 kk .. 16 kk + 15; the leading offset steps the 8-row groups (K), the
+// stride offset the 8-column groups (M or N).
+__device__ __forceinline__ uint64_t opdesc_t(const __nv_bfloat16* base, int W, int kk) {
+    const uint32_t group = (uint32_t)(W >> 3) * 128u;
+    return sdesc(smem_u32(base) + (uint32_t)kk * 2u * group, group, 128u);
+}
+constexpr uint32_t A_MN_MAJOR = 1u << 15, B_MN_MAJOR = 1u << 16;
 
 // Instruction descriptor of kind::f16: FP32 accumulator, BF16 A and B, both
 // K-major, shape M x N.
@@ -179,7 +200,7 @@ struct __align__(1024) FwdSmem {
 };
 
 // Copies the model (already in operand layout) into shared memory.
-template <typename SM>
+template <int NT = ROWS, typename SM>
 __device__ __forceinline__ void load_model(SM& s, const ModelDev* __restrict__ md) {
     const int t = threadIdx.x;
     const uint4* w1 = reinterpret_cast<const uint4*>(md->W1);
@@ -188,9 +209,9 @@ __device__ __forceinline__ void load_model(SM& s, const ModelDev* __restrict__ m
     uint4* s1 = reinterpret_cast<uint4*>(s.W1);
     uint4* s2 = reinterpret_cast<uint4*>(s.W2);
     uint4* s3 = reinterpret_cast<uint4*>(s.W3);
-    for (int i = t; i < N_H * K1 / 8; i += ROWS) s1[i] = w1[i];
-    for (int i = t; i < N_H * N_H / 8; i += ROWS) s2[i] = w2[i];
-    for (int i = t; i < N3 * N_H / 8; i += ROWS) s3[i] = w3[i];
+    for (int i = t; i < N_H * K1 / 8; i += NT) s1[i] = w1[i];
+    for (int i = t; i < N_H * N_H / 8; i += NT) s2[i] = w2[i];
+    for (int i = t; i < N3 * N_H / 8; i += NT) s3[i] = w3[i];
     if (t < N_H) s.b2[t] = md->b2[t];
     if (t < N_OUT) {
         s.b3[t] = md->b3[t];
@@ -203,42 +224,72 @@ __device__ __forceinline__ void load_model(SM& s, const ModelDev* __restrict__ m
     }
 }
 
-// Writes this thread's row of X: normalised features, 1 (bias), zeros.
+// Writes this thread's row of X into columns c .. c + 15 of an operand of
+// width W: normalised features, 1 (bias), zeros.
 template <typename SM>
-__device__ __forceinline__ void put_input_row(SM& s, const float* feat, bool valid) {
+__device__ __forceinline__ void put_input_cols(SM& s, __nv_bfloat16* X, int c, int W,
+                                               const float* feat, bool valid) {
     const int r = threadIdx.x;
+    float v[8];
 #pragma unroll
-    for (int k = 0; k < K1; ++k) {
-        float v = 0.0f;
-        if (valid && k < N_IN) v = (feat[k] - s.in_mean[k]) * s.in_inv_std[k];
-        if (valid && k == N_IN) v = 1.0f;
-        s.X[kmaj(r, k, K1)] = __float2bfloat16_rn(v);
-    }
+    for (int k = 0; k < N_IN; ++k)
+        v[k] = valid ? (feat[k] - s.in_mean[k]) * s.in_inv_std[k] : 0.0f;
+    put8(X, r, c, W, v);
+#pragma unroll
+    for (int k = 0; k < N_IN; ++k) v[k] = (valid && k == 0) ? 1.0f : 0.0f;
+    put8(X, r, c + 8, W, v);
 }
 
-// One layer: makes the operands written by the threads visible to the tensor
-// cores, issues the K/16 MMAs from thread 0 and waits for their commit.
-// After a timed-out wait the CTA issues nothing more (s.error, read after
-// the next barrier) and finish_tile waits once more before freeing.
-template <int K, typename SM>
-__device__ __forceinline__ bool layer(SM& s, uint32_t tmem_d, const __nv_bfloat16* A,
-                                      const __nv_bfloat16* B, uint32_t idesc,
-                                      uint32_t& phase) {
+template <typename SM>
+__device__ __forceinline__ void put_input_row(SM& s, const float* feat, bool valid) {
+    put_input_cols(s, s.X, 0, K1, feat, valid);
+}
+
+// ReLU of 16 accumulator columns (plus bias, if any) into columns c .. c + 15
+// of row r, in BF16.
+__device__ __forceinline__ void put_relu16(__nv_bfloat16* H, int r, int c, int W, float* v,
+                                           const float* bias) {
+#pragma unroll
+    for (int i = 0; i < 16; ++i) v[i] = fmaxf(bias ? v[i] + bias[i] : v[i], 0.0f);
+    put8(H, r, c, W, v);
+    put8(H, r, c + 8, W, v + 8);
+}
+
+// One round of MMAs: makes the operands written by the threads visible to the
+// tensor cores, issues issue()'s MMAs from thread 0 and waits for their
+// commit.  After a timed-out wait the CTA issues nothing more (s.error, read
+// after the next barrier) and finish_tiles waits once more before freeing.
+// PART: only the first ROWS threads of the CTA take part.
+template <bool PART, typename SM, typename Issue>
+__device__ __forceinline__ bool mma_round(SM& s, uint32_t& phase, Issue issue) {
     fence_async_smem();
     tc_fence_before();
-    __syncthreads();
-    if (s.error) return false;  // uniform: read after the barrier
+    if constexpr (PART)
+        asm volatile("bar.sync 1, %0;" : : "n"(ROWS) : "memory");
+    else
+        __syncthreads();
+    if (*static_cast<volatile int*>(&s.error)) return false;  // uniform: read after the barrier
     if (threadIdx.x == 0) {
         tc_fence_after();
-#pragma unroll
-        for (int kk = 0; kk < K / 16; ++kk)
-            mma(tmem_d, opdesc(A, K, kk), opdesc(B, K, kk), idesc, kk > 0 ? 1u : 0u);
+        issue();
         mma_commit(&s.bar);
     }
     if (!mbar_wait(&s.bar, phase)) s.error = 1;
     phase ^= 1u;
     tc_fence_after();
     return true;
+}
+
+// One layer: D = A B^T over K columns, both operands K wide.
+template <int K, typename SM>
+__device__ __forceinline__ bool layer(SM& s, uint32_t tmem_d, const __nv_bfloat16* A,
+                                      const __nv_bfloat16* B, uint32_t idesc,
+                                      uint32_t& phase) {
+    return mma_round<false>(s, phase, [&] {
+#pragma unroll
+        for (int kk = 0; kk < K / 16; ++kk)
+            mma(tmem_d, opdesc(A, K, kk), opdesc(B, K, kk), idesc, kk > 0 ? 1u : 0u);
+    });
 }
 
 // Forward pass of a tile whose X rows are written.  Tensor-memory columns:
@@ -255,9 +306,7 @@ __device__ __forceinline__ bool forward_tile(FwdSmem& s, uint32_t tbase, uint32_
 #pragma unroll
         for (int c = 0; c < N_H; c += 16) {
             tmem_ld16(tmem_row(tbase, c), v);
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                s.H1[kmaj(r, c + i, N_H)] = __float2bfloat16_rn(fmaxf(v[i], 0.0f));
+            put_relu16(s.H1, r, c, N_H, v, nullptr);
         }
     }
     if (!layer<N_H>(s, tbase + 64, s.H1, s.W2, idesc_bf16(ROWS, N_H), phase)) return false;
@@ -266,9 +315,7 @@ __device__ __forceinline__ bool forward_tile(FwdSmem& s, uint32_t tbase, uint32_
 #pragma unroll
         for (int c = 0; c < N_H; c += 16) {
             tmem_ld16(tmem_row(tbase, 64 + c), v);
-#pragma unroll
-            for (int i = 0; i < 16; ++i)
-                s.H2[kmaj(r, c + i, N_H)] = __float2bfloat16_rn(fmaxf(v[i] + s.b2[c + i], 0.0f));
+            put_relu16(s.H2, r, c, N_H, v, s.b2 + c);
         }
     }
     if (!layer<N_H>(s, tbase, s.H2, s.W3, idesc_bf16(ROWS, N3), phase)) return false;
@@ -308,14 +355,7 @@ constexpr uint32_t DUAL_TMEM_COLS = 128;
 // put_input_row into input buffer `b` of the dual image.
 __device__ __forceinline__ void put_input_row_dual(FwdSmemDual& s, int b, const float* feat,
                                                    bool valid) {
-    const int r = threadIdx.x;
-#pragma unroll
-    for (int k = 0; k < K1; ++k) {
-        float v = 0.0f;
-        if (valid && k < N_IN) v = (feat[k] - s.in_mean[k]) * s.in_inv_std[k];
-        if (valid && k == N_IN) v = 1.0f;
-        s.X[b][kmaj(r, k, K1)] = __float2bfloat16_rn(v);
-    }
+    put_input_cols(s, s.X[b], 0, K1, feat, valid);
 }
 
 // layer() for both inputs of the dual image: the MMAs of A0 into d0 and of
@@ -325,24 +365,14 @@ __device__ __forceinline__ bool layer_dual(FwdSmemDual& s, uint32_t d0, uint32_t
                                            const __nv_bfloat16* A0, const __nv_bfloat16* A1,
                                            const __nv_bfloat16* B, uint32_t idesc,
                                            uint32_t& phase) {
-    fence_async_smem();
-    tc_fence_before();
-    __syncthreads();
-    if (s.error) return false;  // uniform: read after the barrier
-    if (threadIdx.x == 0) {
-        tc_fence_after();
+    return mma_round<false>(s, phase, [&] {
 #pragma unroll
         for (int kk = 0; kk < K / 16; ++kk)
             mma(d0, opdesc(A0, K, kk), opdesc(B, K, kk), idesc, kk > 0 ? 1u : 0u);
 #pragma unroll
         for (int kk = 0; kk < K / 16; ++kk)
             mma(d1, opdesc(A1, K, kk), opdesc(B, K, kk), idesc, kk > 0 ? 1u : 0u);
-        mma_commit(&s.bar);
-    }
-    if (!mbar_wait(&s.bar, phase)) s.error = 1;
-    phase ^= 1u;
-    tc_fence_after();
-    return true;
+    });
 }
 
 // The forward pass of both inputs: outputs of this thread's row in y
@@ -360,9 +390,7 @@ __device__ __forceinline__ bool forward_tile_dual(FwdSmemDual& s, uint32_t tbase
 #pragma unroll
             for (int c = 0; c < N_H; c += 16) {
                 tmem_ld16(tmem_row(b ? t1 : tbase, c), v);
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    s.H1[b][kmaj(r, c + i, N_H)] = __float2bfloat16_rn(fmaxf(v[i], 0.0f));
+                put_relu16(s.H1[b], r, c, N_H, v, nullptr);
             }
     }
     if (!layer_dual<N_H>(s, tbase, t1, s.H1[0], s.H1[1], s.W2, idesc_bf16(ROWS, N_H), phase))
@@ -376,10 +404,7 @@ __device__ __forceinline__ bool forward_tile_dual(FwdSmemDual& s, uint32_t tbase
 #pragma unroll
             for (int c = 0; c < N_H; c += 16) {
                 tmem_ld16(tmem_row(b ? t1 : tbase, c), v);
-#pragma unroll
-                for (int i = 0; i < 16; ++i)
-                    s.H1[b][kmaj(r, c + i, N_H)] =
-                        __float2bfloat16_rn(fmaxf(v[i] + s.b2[c + i], 0.0f));
+                put_relu16(s.H1[b], r, c, N_H, v, s.b2 + c);
             }
     }
     if (!layer_dual<N_H>(s, tbase, t1, s.H1[0], s.H1[1], s.W3, idesc_bf16(ROWS, N3), phase))

@@ -161,13 +161,12 @@ class MDFNetwork:
         losses = []
         for _ in range(int(epochs)):
             perm = torch.randperm(n, device=x.device, generator=gen)
-            xs = x[perm].contiguous()
-            ts = t[perm].contiguous()
             nb = n // batch
             out = np.zeros(nb, np.float32)
-            L.check(self._lib.sfg_mlp_train(self._h, C.c_void_p(xs.data_ptr()),
-                                            C.c_void_p(ts.data_ptr()), int(n), int(batch),
-                                            float(lr), _fptr(out), self._stream()))
+            L.check(self._lib.sfg_mlp_train_rows(
+                self._h, C.c_void_p(x.data_ptr()), C.c_void_p(t.data_ptr()),
+                C.c_void_p(perm.data_ptr()), int(n), int(batch), float(lr), _fptr(out),
+                self._stream()))
             losses.append(out)
         return np.concatenate(losses) if losses else np.zeros(0, np.float32)
 

@@ -94,3 +94,57 @@ def test_training_reduces_loss_and_is_deterministic(sfg):
     Xv, Tv = _data(4096, 8)
     yv = a.forward(Xv).cpu().numpy()
     assert np.mean((yv - Tv) ** 2) < 0.5 * np.mean((Q.forward_exact(Q.he_init(7), Xv)[0] - Tv) ** 2)
+
+
+@pytest.mark.parametrize("n,batch", [(1, 1), (129, 129), (1000, 300), (8192, 4100)])
+def test_training_by_row_list_equals_training_on_copies(sfg, n, batch):
+    """A row list is the same as rows copied into its order, bit for bit; the
+    sizes leave a last tile of 1, 1, 44 and 4 samples, and rows unused."""
+    import ctypes as C
+    import torch
+    X, T = _data(n, 12)
+    x, t = torch.tensor(X, device="cuda"), torch.tensor(T, device="cuda")
+    rows = torch.randperm(n, device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    ptr = lambda a: C.c_void_p(a.data_ptr())
+    out = []
+    for copied in (False, True):
+        net = _net(9)
+        loss = np.zeros(n // batch, np.float32)
+        lp = loss.ctypes.data_as(C.POINTER(C.c_float))
+        lib, st = net._lib, C.c_void_p(torch.cuda.current_stream().cuda_stream)
+        for _ in range(2):
+            if copied:
+                xs, ts = x[rows].contiguous(), t[rows].contiguous()
+                rc = lib.sfg_mlp_train(net.handle, ptr(xs), ptr(ts), n, batch, 1e-3, lp, st)
+            else:
+                rc = lib.sfg_mlp_train_rows(net.handle, ptr(x), ptr(t), ptr(rows), n, batch,
+                                            1e-3, lp, st)
+            assert rc == 0
+        out.append((net.params(), loss, net.forward(X).cpu().numpy()))
+    for a, b in zip(*out):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
+    first = Q.loss_exact(Q.he_init(9), X, T) if n == batch else None
+    if first is not None:
+        net = _net(9)
+        one = net.train(X, T, epochs=1, batch=batch, lr=1e-3, seed=0)
+        assert abs(one[0] - first) / first < 2e-2
+
+
+def test_row_list_out_of_range_is_an_error(sfg):
+    import ctypes as C
+    import torch
+    X, T = _data(256, 13)
+    x, t = torch.tensor(X, device="cuda"), torch.tensor(T, device="cuda")
+    rows = torch.arange(256, device="cuda")
+    ptr = lambda a: C.c_void_p(a.data_ptr())
+    net = _net(9)
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    run = lambda: net._lib.sfg_mlp_train_rows(net.handle, ptr(x), ptr(t), ptr(rows), 256, 256,
+                                              1e-3, None, st)
+    rows[7] = 256
+    assert run() == 1
+    assert b"row index" in net._lib.sfg_last_error()
+    rows[7] = -1
+    assert run() == 1
+    rows[7] = 7
+    assert run() == 0
