@@ -1268,113 +1268,119 @@ __global__ void k_interp_move(const ChannelDev* __restrict__ chans, int M, Marke
     move_marker(ch, mb, cb, m, u);
 }
 
-// The marker move of the FP32-arithmetic modes, one warp per capsule: the
-// warp first forms, for every cell of the box that holds its markers'
-// stencils, the new state's moments (rho, jx, jy; zero on SOLID cells) and
-// the cell's final force, into shared memory, the lanes running along the
+// The marker move of the FP32-arithmetic modes, one block per capsule: the
+// block first forms, for every cell of the box that holds the capsule's
+// stencils, the new state's velocity (0 on SOLID cells) from its moments and
+// the cell's final force, into shared memory, the threads running along the
 // box's rows (each cell's nine populations are read once, coalesced, where
-// the markers' stencils overlap); then each lane interpolates its markers
-// from there with the terms, order and arithmetic of interp_u_acc (the same
-// values, so the same result bit for bit), and moves them.  A capsule whose
-// box exceeds MOVE_BOX_MAX cells interpolates from global memory as
-// k_interp_move does.
-// (out of line: the rare large capsule keeps its registers out of the box path)
+// the markers' stencils overlap, and divided once); then one thread per
+// marker interpolates from there with the terms, order and arithmetic of
+// interp_u_acc (the same values, so the same result bit for bit), and moves
+// it.  A capsule whose box exceeds MOVE_BOX_MAX cells interpolates from global
+// memory as k_interp_move does.
+//
+// Bound: latency, of few capsules as of many (each thread's loads depend on the
+// marker's cell, then on the cell's tile); so all of a cell's loads are issued at
+// once and few registers are held, and the block is as wide as the capsule has
+// cells (100-130 of 24 markers) where all blocks are resident at once, half of
+// that where they are not and every warp's own forming of the box counts.  One
+// warp per capsule, with five floats a cell in shared memory and 126 registers,
+// then blocks of 128 threads, of 64 and of 32 (us):
+//   30 capsules, FP32         13.5   9.4  10.3
+//   40 capsules, FP16S        21.0  11.1  12.6
+//   2000 capsules, FP32       33.4  23.3  22.5  27.9
+//   8522 capsules, FP16S      68.0  54.9  44.3  41.7
+
+// The new state's velocity of a cell, jy in [0, ny).
 template <typename S>
-__device__ __noinline__ double2 interp_u_acc_global(const ChannelDev& ch, const MarkerBufs& mb,
-                                                    int m, const S* __restrict__ f,
-                                                    const int* __restrict__ tile_slot,
-                                                    const float* __restrict__ fin) {
-    return interp_u_acc<S, float, float>(ch, mb, m, f, tile_slot, fin);
+__device__ __forceinline__ float2 new_velocity(const ChannelDev& ch, int jx, int jy,
+                                               const S* __restrict__ f,
+                                               const int* __restrict__ tile_slot,
+                                               const float* __restrict__ fin) {
+    const long long nn = (long long)jy * ch.pitch + jx;
+    float v[9];
+#pragma unroll
+    for (int q = 0; q < 9; ++q) v[q] = PopIO<S, float>::ld(f + ch.f_off + q * ch.plane + nn, q);
+    const int sl = tile_slot[ch.tile_base + (jy / TILE_H) * ch.tiles_x + jx / TILE_W];
+    if (cell_kind(ch, jx, jy) == CK_SOLID) return make_float2(0.f, 0.f);
+    float gx = 0.f, gy = 0.f, rho, a, b;
+    if (sl >= 0) {
+        const int cell = (jy % TILE_H) * TILE_W + (jx % TILE_W);
+        gx = fin[(size_t)sl * 2 * TILE_CELLS + cell];
+        gy = fin[(size_t)sl * 2 * TILE_CELLS + TILE_CELLS + cell];
+    }
+    lattice_moments(v, rho, a, b);
+    if (!(rho > 1e-15f)) return make_float2(0.f, 0.f);
+    const float inv = __frcp_rn(rho);
+    return make_float2((a + 0.5f * gx) * inv, (b + 0.5f * gy) * inv);
 }
-constexpr int MOVE_WARPS = 4;
+
 constexpr int MOVE_BOX_MAX = 512;
-struct MoveBox {
-    float rho[MOVE_BOX_MAX], jx[MOVE_BOX_MAX], jy[MOVE_BOX_MAX];
-    float fx[MOVE_BOX_MAX], fy[MOVE_BOX_MAX];
-};
-template <typename S>
-__global__ void __launch_bounds__(MOVE_WARPS * 32)
-k_interp_move_caps(const CapsuleDev* __restrict__ caps, int ncaps,
-                   const ChannelDev* __restrict__ chans, MarkerBufs mb, ContactBufs cb,
-                   const S* __restrict__ f, const int* __restrict__ tile_slot,
-                   const float* __restrict__ fin) {
-    extern __shared__ __align__(16) unsigned char move_smem[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int c = blockIdx.x * MOVE_WARPS + warp;
-    if (c >= ncaps) return;
-    MoveBox& B = reinterpret_cast<MoveBox*>(move_smem)[warp];
-    const CapsuleDev cp = caps[c];
+constexpr int MOVE_WIDE_CAPS = 1024;
+template <typename S, int MOVE_THREADS>
+__global__ void __launch_bounds__(MOVE_THREADS)
+k_interp_move_caps(const CapsuleDev* __restrict__ caps, const ChannelDev* __restrict__ chans,
+                   MarkerBufs mb, ContactBufs cb, const S* __restrict__ f,
+                   const int* __restrict__ tile_slot, const float* __restrict__ fin) {
+    __shared__ float2 uv[MOVE_BOX_MAX];
+    const int tid = threadIdx.x, lane = tid & 31;
+    const CapsuleDev cp = caps[blockIdx.x];
     const ChannelDev& ch = chans[cp.chan];
     const int nx = ch.nx, ny = ch.ny, n = cp.n, off = cp.off;
-    // the stencils' box: x relative to the first marker (minimum image)
-    int ref = 0;
-    for (int k = 0; k < n; ++k)
-        if (mb.valid[off + k]) { ref = mb.org[off + k].x; break; }
-    int dmin = INT_MAX, dmax = INT_MIN, ymin = INT_MAX, ymax = INT_MIN;
-    for (int k = lane; k < n; k += 32) {
-        if (!mb.valid[off + k]) continue;
-        const int2 og = mb.org[off + k];
-        int d = og.x - ref;
-        if (2 * d > nx) d -= nx;
-        if (2 * d < -nx) d += nx;
-        const int y = og.y;
-        dmin = min(dmin, d);
-        dmax = max(dmax, d);
-        ymin = min(ymin, y);
-        ymax = max(ymax, y);
+    // the stencils' box: x relative to the first valid marker (minimum
+    // image); every warp forms it for itself
+    int ref = 0, dmin = INT_MAX, dmax = INT_MIN, ymin = INT_MAX, ymax = INT_MIN;
+    bool have = false;
+    for (int k0 = 0; k0 < n; k0 += 32) {
+        const int k = k0 + lane;
+        const bool v = k < n && mb.valid[off + k];
+        const int2 og = v ? mb.org[off + k] : make_int2(0, 0);
+        const unsigned vm = __ballot_sync(0xffffffffu, v);
+        if (!have && vm) {
+            ref = __shfl_sync(0xffffffffu, og.x, __ffs(vm) - 1);
+            have = true;
+        }
+        if (v) {
+            int d = og.x - ref;
+            if (2 * d > nx) d -= nx;
+            if (2 * d < -nx) d += nx;
+            dmin = min(dmin, d);
+            dmax = max(dmax, d);
+            ymin = min(ymin, og.y);
+            ymax = max(ymax, og.y);
+        }
     }
     dmin = __reduce_min_sync(0xffffffffu, dmin);
     dmax = __reduce_max_sync(0xffffffffu, dmax);
     ymin = __reduce_min_sync(0xffffffffu, ymin);
     ymax = __reduce_max_sync(0xffffffffu, ymax);
-    const bool any = dmin <= dmax;
     const int bw = dmax - dmin + 4, bh = ymax - ymin + 4;
-    const bool boxed = any && (long long)bw * bh <= MOVE_BOX_MAX;
+    const bool boxed = have && (long long)bw * bh <= MOVE_BOX_MAX;
     if (boxed) {
         const int bx0 = ref + dmin - 1, by0 = ymin - 1;
-        for (int i = lane; i < bw * bh; i += 32) {
+        for (int i = tid; i < bw * bh; i += MOVE_THREADS) {
             const int by = i / bw, bx = i - by * bw;
             int jx = (bx0 + bx) % nx;
             if (jx < 0) jx += nx;
             const int jy = by0 + by;
-            float r = 0.f, a = 0.f, b = 0.f, gx = 0.f, gy = 0.f;
-            if (jy >= 0 && jy < ny && cell_kind(ch, jx, jy) != CK_SOLID) {
-                const long long nn = (long long)jy * ch.pitch + jx;
-                float v[9];
-#pragma unroll
-                for (int q = 0; q < 9; ++q)
-                    v[q] = PopIO<S, float>::ld(f + ch.f_off + q * ch.plane + nn, q);
-                lattice_moments(v, r, a, b);
-                const int t = ch.tile_base + (jy / TILE_H) * ch.tiles_x + jx / TILE_W;
-                const int sl = tile_slot[t];
-                if (sl >= 0) {
-                    const int cell = (jy % TILE_H) * TILE_W + (jx % TILE_W);
-                    gx = fin[(size_t)sl * 2 * TILE_CELLS + cell];
-                    gy = fin[(size_t)sl * 2 * TILE_CELLS + TILE_CELLS + cell];
-                }
-            }
-            B.rho[i] = r;
-            B.jx[i] = a;
-            B.jy[i] = b;
-            B.fx[i] = gx;
-            B.fy[i] = gy;
+            float2 u = make_float2(0.f, 0.f);
+            if (jy >= 0 && jy < ny) u = new_velocity(ch, jx, jy, f, tile_slot, fin);
+            uv[i] = u;
         }
-        __syncwarp();
     }
-    for (int k = lane; k < n; k += 32) {
+    __syncthreads();
+    for (int k = tid; k < n; k += MOVE_THREADS) {
         const int m = off + k;
         double2 u = make_double2(0.0, 0.0);
         if (mb.valid[m]) {
-            if (!boxed) {
-                u = interp_u_acc_global<S>(ch, mb, m, f, tile_slot, fin);
-            } else {
-                const int ix0 = mb.org[m].x, iy0 = mb.org[m].y;
+            const int ix0 = mb.org[m].x, iy0 = mb.org[m].y;
+            float wxs[4], wys[4];
+            stencil_weights(mb, m, wxs, wys);
+            float ux = 0.f, uy = 0.f;
+            if (boxed) {
                 int d = ix0 - ref;
                 if (2 * d > nx) d -= nx;
                 if (2 * d < -nx) d += nx;
-                float wxs[4], wys[4];
-                stencil_weights(mb, m, wxs, wys);
-                float ux = 0.f, uy = 0.f;
 #pragma unroll
                 for (int sy = 0; sy < 4; ++sy) {
                     const int jy = iy0 - 1 + sy;
@@ -1384,21 +1390,28 @@ k_interp_move_caps(const CapsuleDev* __restrict__ caps, int ncaps,
                     for (int sx = 0; sx < 4; ++sx) {
                         const float w = wxs[sx] * wys[sy];
                         if (w > 1e-15f) {
-                            const int i = row + sx;
-                            const float rho = B.rho[i];
-                            float cu = 0.f, cv = 0.f;
-                            if (rho > 1e-15f) {
-                                const float inv = __frcp_rn(rho);
-                                cu = (B.jx[i] + 0.5f * B.fx[i]) * inv;
-                                cv = (B.jy[i] + 0.5f * B.fy[i]) * inv;
-                            }
-                            ux += cu * w;
-                            uy += cv * w;
+                            const float2 c = uv[row + sx];
+                            ux += c.x * w;
+                            uy += c.y * w;
                         }
                     }
                 }
-                u = make_double2((double)ux, (double)uy);
+            } else {
+#pragma unroll 1
+                for (int tap = 0; tap < 16; ++tap) {
+                    const int sy = tap >> 2, sx = tap & 3, jy = iy0 - 1 + sy;
+                    const float wx = sx < 2 ? (sx ? wxs[1] : wxs[0]) : (sx == 2 ? wxs[2] : wxs[3]);
+                    const float wy = sy < 2 ? (sy ? wys[1] : wys[0]) : (sy == 2 ? wys[2] : wys[3]);
+                    const float w = wx * wy;
+                    if (jy < 0 || jy >= ny || !(w > 1e-15f)) continue;
+                    int jx = (ix0 - 1 + sx) % nx;
+                    if (jx < 0) jx += nx;
+                    const float2 c = new_velocity(ch, jx, jy, f, tile_slot, fin);
+                    ux += c.x * w;
+                    uy += c.y * w;
+                }
             }
+            u = make_double2((double)ux, (double)uy);
         }
         move_marker(ch, mb, cb, m, u);
     }
@@ -1751,10 +1764,13 @@ void launch_interp_move(const ChannelDev* chans, const CapsuleDev* caps, int nca
     if constexpr (sizeof(R) == 4) {
         (void)phi_tbl;
         if (ncaps == 0) return;
-        k_interp_move_caps<S><<<(ncaps + MOVE_WARPS - 1) / MOVE_WARPS, MOVE_WARPS * 32,
-                                MOVE_WARPS * sizeof(MoveBox), st>>>(
-            caps, ncaps, chans, mb, cb, f, tb.tile_slot[parity],
-            static_cast<const float*>(tb.fin[parity]));
+        const float* fin = static_cast<const float*>(tb.fin[parity]);
+        if (ncaps <= MOVE_WIDE_CAPS)
+            k_interp_move_caps<S, 128><<<ncaps, 128, 0, st>>>(caps, chans, mb, cb, f,
+                                                              tb.tile_slot[parity], fin);
+        else
+            k_interp_move_caps<S, 64><<<ncaps, 64, 0, st>>>(caps, chans, mb, cb, f,
+                                                            tb.tile_slot[parity], fin);
     } else {
         const int B = tb.marker_block, G = (M + B - 1) / B;
         k_interp_move<S, R><<<G, B, 0, st>>>(chans, M, mb, cb, f, tb.tile_slot[parity],
