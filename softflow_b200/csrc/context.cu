@@ -628,14 +628,19 @@ static cudaError_t dalloc(T** p, size_t n) {
 // ------------------------------------------------------------------------
 // initialize
 // ------------------------------------------------------------------------
+static int resident_spread_ctas(const sfg_context* c) {
+    return spread_blocks_per_sm(c->precision == SFG_FP64, spread_wide(c->tb.max_slots));
+}
+
 // Grid sizes from the tuned CTAs-per-SM counts (0 = the resident maximum).
 static void apply_launch_config(sfg_context* c) {
     const int lat_max = lattice_ctas_per_sm(c->precision, c->any_adr && !c->any_chem, c->use_vec8);
-    const int spr_max = spread_blocks_per_sm(c->precision == SFG_FP64);
+    const int spr_max = resident_spread_ctas(c);
     const int lat = c->lattice_cps > 0 ? std::min(c->lattice_cps, lat_max) : lat_max;
     const int spr = c->spread_cps > 0 ? std::min(c->spread_cps, spr_max) : spr_max;
     c->persistent_ctas = c->nsm * lat;
-    const int per_cta = c->precision == SFG_FP64 ? 1 : 8;   // tiles a spread CTA works at a time
+    // tiles a spread CTA works at a time
+    const int per_cta = c->precision == SFG_FP64 || spread_wide(c->tb.max_slots) ? 1 : 8;
     c->spread_grid =
         std::max(1, std::min((c->tb.max_slots + per_cta - 1) / per_cta, c->nsm * spr));
     c->learned_grid = c->nsm * std::max(1, std::min(c->learned_cps, 6));
@@ -1462,7 +1467,7 @@ extern "C" int sfg_autotune(sfg_context* c, int steps_per_trial, int* steps_run)
     };
     std::vector<Knob> knobs;
     const int lat_max = lattice_ctas_per_sm(c->precision, c->any_adr && !c->any_chem, c->use_vec8);
-    const int spr_max = spread_blocks_per_sm(c->precision == SFG_FP64);
+    const int spr_max = resident_spread_ctas(c);
     std::vector<int> lat, spr;
     for (int k = 1; k <= lat_max; ++k) lat.push_back(k);
     for (int k = 1; k <= spr_max; ++k) spr.push_back(k);
@@ -1506,7 +1511,7 @@ extern "C" int sfg_get_launch_config(sfg_context* c, int* lattice_cps, int* spre
     if (!c) return fail(SFG_ERR_ARG, "sfg_get_launch_config: null context");
     // the chosen counts (the spread grid is further capped by the slot count)
     const int lat_max = lattice_ctas_per_sm(c->precision, c->any_adr && !c->any_chem, c->use_vec8);
-    const int spr_max = spread_blocks_per_sm(c->precision == SFG_FP64);
+    const int spr_max = resident_spread_ctas(c);
     if (lattice_cps) *lattice_cps = c->lattice_cps > 0 ? std::min(c->lattice_cps, lat_max) : lat_max;
     if (spread_cps) *spread_cps = c->spread_cps > 0 ? std::min(c->spread_cps, spr_max) : spr_max;
     if (marker_block) *marker_block = c->tb.marker_block;

@@ -863,7 +863,21 @@ struct SpreadFxWarp {
     unsigned char hit[ACC_CELLS];     // touched this tile
     unsigned short idx[TILE_CELLS];   // the touched cells, compacted
 };
-constexpr size_t spread_fx_smem() { return sizeof(SpreadFxWarp) * SPREAD_WARPS; }
+// A tile is one warp's work, eight tiles a CTA, or (WIDE) a CTA's of four warps.
+// Where the tiles are few, the sweep takes as long as one tile's chain of marker
+// passes and cells, which four warps cut by four; where they are many, the
+// narrow form keeps more tiles in flight, and its waits cost less.  The line lies at
+// the context's tile count (spread phase of a step of five sweeps, one warp /
+// two / four / eight a tile, us):
+//   400 x 80, 130 tiles                  66.4  53.1  44.9  44.4
+//   12 ragged channels, about 1,000      76.3  54.8  50.1  49.6
+//   16 channels of 512 x 104, 3,300      83.7  57.4  53.1  56.3
+//   32 channels, 6,600                   93.0  67.3  75.9  82.0
+//   64 channels, 13,000                  98.1  99.8 105.3 120.4
+//   4096 x 1024, 16,384 (one sweep)      20.3        29.0
+constexpr int FX_WIDE_WARPS = 4, FX_WIDE_SLOTS = 8192;
+template <bool WIDE> constexpr int fx_threads = 32 * (WIDE ? FX_WIDE_WARPS : SPREAD_WARPS);
+template <bool WIDE> constexpr size_t fx_smem = sizeof(SpreadFxWarp) * (WIDE ? 1 : SPREAD_WARPS);
 __device__ __forceinline__ long long fx_quant(float v) { return __float2ll_rn(v * FX_SCALE); }
 __device__ __forceinline__ unsigned fx_lo(long long q) {
     return (unsigned)(q & ((1LL << FX_LO_BITS) - 1));
@@ -873,7 +887,8 @@ __device__ __forceinline__ float fx_value(unsigned lo, int hi) {
     return __ll2float_rn((long long)hi * (1LL << FX_LO_BITS) + (long long)lo) * FX_UNSCALE;
 }
 
-__global__ void __launch_bounds__(SPREAD_WARPS * 32, 4)
+template <bool WIDE>
+__global__ void __launch_bounds__(fx_threads<WIDE>, WIDE ? 8 : 4)
 k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot_info,
             const int* __restrict__ slot_order, const int* __restrict__ ctr, int max_slots,
             const int* __restrict__ list, MarkerBufs mb,
@@ -883,20 +898,26 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
             int* __restrict__ fluid_touched, unsigned* status) {
     if (sweep > 0 && mode == MDF_PLAIN && plain_needed && !*plain_needed) return;
     extern __shared__ __align__(16) unsigned char spread_fx_raw[];
+    // the group of WPT warps that works on a tile, its warp `wg` and thread `gl`
+    constexpr int WPT = WIDE ? FX_WIDE_WARPS : 1, GROUPS = fx_threads<WIDE> / (32 * WPT);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    SpreadFxWarp& W = reinterpret_cast<SpreadFxWarp*>(spread_fx_raw)[warp];
-    for (int i = lane; i < ACC_CELLS; i += 32) {
+    const int group = warp / WPT, wg = warp % WPT, gl = 32 * wg + lane;
+    auto group_sync = [] {
+        if constexpr (WIDE) __syncthreads(); else __syncwarp();
+    };
+    SpreadFxWarp& W = reinterpret_cast<SpreadFxWarp*>(spread_fx_raw)[group];
+    for (int i = gl; i < ACC_CELLS; i += 32 * WPT) {
         W.lo[0][i] = W.lo[1][i] = 0u;
         W.hi[0][i] = W.hi[1][i] = 0;
         W.hit[i] = 0;
     }
-    __syncwarp();
+    group_sync();
     const int n_slots = ctr[CTR_SLOTS];
     const WorkOrder wo(ctr);
-    const int nwarps = gridDim.x * SPREAD_WARPS;
-    // round k takes work-order positions k nwarps .. (k + 1) nwarps - 1,
-    // the warps in reverse order on odd rounds
-    const int wid = blockIdx.x * SPREAD_WARPS + warp;
+    const int ngroups = gridDim.x * GROUPS;
+    // round k takes work-order positions k ngroups .. (k + 1) ngroups - 1,
+    // the groups in reverse order on odd rounds
+    const int wid = blockIdx.x * GROUPS + group;
     int round = 0, next = wid;
     int nslot = next < n_slots ? wo.slot(slot_order, max_slots, next) : 0;
     SlotInfo nfo{};
@@ -905,7 +926,7 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
         const int slot = nslot;
         const SlotInfo si = nfo;
         ++round;
-        next = round * nwarps + ((round & 1) ? nwarps - 1 - wid : wid);
+        next = round * ngroups + ((round & 1) ? ngroups - 1 - wid : wid);
         if (next < n_slots) {
             nslot = wo.slot(slot_order, max_slots, next);
             nfo = slot_info[nslot];
@@ -913,13 +934,13 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
         const int chan = si.chan;
         const ChannelDev& ch = chans[chan];
         const int K = ch.ibm_iterations > 1 ? ch.ibm_iterations : 1;
-        if (sweep >= K) continue;  // warp-uniform
+        if (sweep >= K) continue;  // uniform in the group
         if (sweep > 0 && !mdf_active(ch, mode, resid_gate, chan)) continue;  // sweep 0: all
         const int nx = si.nx, ny = si.ny;
         const int x0 = si.x0, y0 = si.y0;
         int cnt = si.cnt;
         if (cnt > SPREAD_LIST_MAX) {
-            if (lane == 0) atomicOr(status, (unsigned)ST_LIST_OVERFLOW);
+            if (gl == 0) atomicOr(status, (unsigned)ST_LIST_OVERFLOW);
             cnt = SPREAD_LIST_MAX;
         }
         const int* lst = list + si.off;
@@ -929,7 +950,7 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
         const float2* src = reinterpret_cast<const float2*>(
             (ch.learned && (mode == MDF_SEED || (mode == MDF_PLAIN && sweep == 1))) ? acc0 : acc);
         const size_t base2 = (size_t)slot * TILE_CELLS;
-        // four lanes per marker, one stencil row each, eight markers a pass;
+        // four lanes per marker, one stencil row each, eight markers a warp and pass;
         // the next pass's marker data is loaded before this pass's points.
         // Neighbouring list entries are neighbouring markers, whose stencils
         // overlap: the lanes of marker jm take their four columns in an order
@@ -937,7 +958,7 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
         // fewer of each other's cells (same-address shared atomics serialise;
         // along a vertical piece of membrane all eight markers share their
         // columns)
-        const int jm = lane >> 2, sy = lane & 3;
+        const int jm = gl >> 2, sy = gl & 3;
         const bool rot1 = jm & 1, rot2 = jm & 2;
         struct Mk {
             float4 w;
@@ -956,8 +977,8 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
         };
         Mk cur{}, nxt{};
         fetch(0, cur);
-        for (int c0 = 0; c0 < cnt; c0 += 8) {
-            fetch(c0 + 8, nxt);
+        for (int c0 = 0; c0 < cnt; c0 += 8 * WPT) {
+            fetch(c0 + 8 * WPT, nxt);
             const int iy = cur.org.y - 1 + sy, cyl = iy - y0;
             if (c0 + jm < cnt && cyl >= 0 && cyl < TILE_H && iy >= 0 && iy < ny) {
                 const bool ok = !(isnan(cur.f.x) || isnan(cur.f.y));
@@ -989,21 +1010,23 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
             }
             cur = nxt;
         }
-        __syncwarp();
+        group_sync();
         if (!last) {
-            // the touched cells, compacted row by row
+            // the touched cells of the warp's rows, compacted row by row
+            unsigned short* idx = W.idx + wg * (TILE_CELLS / WPT);
             int n = 0;
 #pragma unroll
-            for (int r = 0; r < TILE_H; ++r) {
+            for (int rr = 0; rr < TILE_H / WPT; ++rr) {
+                const int r = wg * (TILE_H / WPT) + rr;
                 const bool h = W.hit[r * ACC_W + lane] != 0;
                 const unsigned b = __ballot_sync(0xffffffffu, h);
-                if (h) W.idx[n + __popc(b & ((1u << lane) - 1u))] = (unsigned short)(r * TILE_W + lane);
+                if (h) idx[n + __popc(b & ((1u << lane) - 1u))] = (unsigned short)(r * TILE_W + lane);
                 n += __popc(b);
             }
             __syncwarp();
             float2* out = reinterpret_cast<float2*>((sweep == 0 && ch.learned) ? acc0 : acc);
             for (int k = lane; k < n; k += 32) {
-                const int c = W.idx[k], i = acc_at(c);
+                const int c = idx[k], i = acc_at(c);
                 float2 v = make_float2(fx_value(W.lo[0][i], W.hi[0][i]),
                                        fx_value(W.lo[1][i], W.hi[1][i]));
                 if (sweep > 0) {
@@ -1016,7 +1039,7 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
                 W.hi[0][i] = W.hi[1][i] = 0;
                 W.hit[i] = 0;
             }
-            __syncwarp();
+            group_sync();
             continue;
         }
         // finalize every cell, two adjacent cells a lane: the value before
@@ -1031,7 +1054,7 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
         const bool row_kinds = ch.mask == nullptr && ch.bc_x != 0 && ch.bc_x != 2;
         const float2 zero = make_float2(0.f, 0.f);
 #pragma unroll 2
-        for (int it = 0; it < TILE_H / 2; ++it) {
+        for (int it = wg; it < TILE_H / 2; it += WPT) {
             const int r = 2 * it + (lane >> 4), cx = 2 * (lane & 15);
             const int c = r * TILE_W + cx, i = r * ACC_W + cx;
             const int jx = x0 + cx, jy = y0 + r;
@@ -1094,7 +1117,7 @@ k_spread_fx(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ s
             if (n_cap) atomicAdd(&capped[chan], n_cap);
             if (n_fluid) atomicAdd(&fluid_touched[chan], n_fluid);
         }
-        __syncwarp();
+        group_sync();
     }
 }
 
@@ -1423,20 +1446,23 @@ size_t membrane_smem_bytes(int maxn) {
     return (size_t)MEM_WARPS * MEM_DOUBLES_PER_NODE * maxn * sizeof(double);
 }
 
-int spread_blocks_per_sm(bool fp64) {
+bool spread_wide(int max_slots) { return max_slots <= FX_WIDE_SLOTS; }
+
+int spread_blocks_per_sm(bool fp64, bool wide) {
     int b = 0;
     const cudaError_t e =
         fp64 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_spread, BAND_WARPS * 32, 0)
-             : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_spread_fx,
-                                                             SPREAD_WARPS * 32,
-                                                             spread_fx_smem());
+        : wide ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_spread_fx<true>,
+                                                               fx_threads<true>, fx_smem<true>)
+               : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_spread_fx<false>,
+                                                               fx_threads<false>, fx_smem<false>);
     if (e != cudaSuccess || b < 1) b = 1;
     return b;
 }
 
 cudaError_t prepare_spread() {
-    return cudaFuncSetAttribute(k_spread_fx, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)spread_fx_smem());
+    return cudaFuncSetAttribute(k_spread_fx<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)fx_smem<false>);
 }
 
 // ---------------- capsule geometry (thermo) ---------------------------------
@@ -1720,10 +1746,14 @@ template <typename R>
 void launch_spread(const ChannelDev* chans, const MarkerBufs& mb, TileBufs& tb, int parity,
                    int sweep, int mode, int grid, unsigned* status, cudaStream_t st) {
     if constexpr (sizeof(R) == 4) {
-        k_spread_fx<<<grid, SPREAD_WARPS * 32, spread_fx_smem(), st>>>(
+        auto run = [&](auto kernel, int threads, size_t smem) {
+            kernel<<<grid, threads, smem, st>>>(
             chans, tb.slot_info, tb.slot_order, tb.ctr, tb.max_slots, tb.list, mb, tb.acc, tb.acc0,
             static_cast<float*>(tb.gsnap), static_cast<float*>(tb.fin[parity]), sweep, mode,
             tb.resid_gate, tb.plain_needed, tb.capped, tb.fluid_touched, status);
+        };
+        if (spread_wide(tb.max_slots)) run(k_spread_fx<true>, fx_threads<true>, fx_smem<true>);
+        else run(k_spread_fx<false>, fx_threads<false>, fx_smem<false>);
     } else {
         k_spread<<<grid, BAND_WARPS * 32, 0, st>>>(
             chans, tb.slot_info, tb.slot_order, tb.ctr, tb.max_slots, tb.list, mb, tb.acc,

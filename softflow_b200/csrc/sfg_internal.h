@@ -66,7 +66,8 @@ cudaError_t prepare_membrane(int maxn);
 // Opts the spread kernels into their shared-memory size (once per device).
 cudaError_t prepare_spread();
 // Resident spread CTAs per SM (after prepare_spread).
-int spread_blocks_per_sm(bool fp64);
+int spread_blocks_per_sm(bool fp64, bool wide);
+bool spread_wide(int max_slots);   // FP32 spreads: four warps a tile
 void launch_membrane(const CapsuleDev* caps, int ncaps, const MarkerBufs& mb, int* has_prev,
                      int maxn, unsigned* status, cudaStream_t st);
 // Pair and wall contact forces, added to the membrane forces (after the

@@ -42,3 +42,38 @@ def test_few_and_many_markers_agree(sfg, precision, nodes):
         assert np.array_equal(a, b)
     assert np.array_equal(few.capsules(0).positions(), many.capsules(0).positions())
     assert np.array_equal(few.capsules(0).velocities(), many.capsules(0).velocities())
+
+
+@pytest.mark.parametrize("precision", ["fp32", "fp16s"])
+@pytest.mark.parametrize("sweeps", [1, 4])
+@pytest.mark.parametrize("nodes", [9, 33, 200])
+def test_few_and_many_tiles_agree(sfg, precision, sweeps, nodes):
+    """The FP32 spread gives a tile one warp, or four in contexts of at most 8,192
+    tiles: again the same channel on both sides of that line, bit for bit.  The
+    tiles' lists hold from a few markers to far more than one pass of four warps
+    (32), and the tiles at the right and upper edge are partly outside."""
+    import softflow_b200 as S
+    ctx = []
+    for many in (False, True):
+        ens = S.Ensemble(precision=precision)
+        for nx, ny in ((77, 43),) + (((1056, 2048),) if many else ()):
+            p = S.SimulationParams(nx=nx, ny=ny, ibm_iterations=sweeps, precision=precision)
+            p.fluid.boundary_type = S.BoundaryType.PERIODIC
+            p.fluid.collision_model = S.CollisionModel.BGK
+            p.fluid.body_force_x = 2e-5
+            i = ens.add_channel(p)
+            mp = S.MembraneParams(model=S.MembraneModel.NEO_HOOKEAN, G_s=0.05)
+            if i == 0:
+                for c in ((1.2, 20.3), (30.4, 9.1), (70.8, 33.9)):
+                    ens.addCapsule(i, c, 4.0, nodes, mp)
+            else:
+                for k in range(40):
+                    ens.addCapsule(i, (20 + 25 * k, 40 + 45 * k), 4.0, 32, mp)
+        ens.initialize()
+        ens.run(5)
+        ctx.append(ens)
+    few, many = ctx
+    for a, b in zip(few.field(0).macroscopic(), many.field(0).macroscopic()):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
+    assert np.array_equal(few.capsules(0).positions(), many.capsules(0).positions())
+    assert np.array_equal(few.capsules(0).velocities(), many.capsules(0).velocities())
