@@ -338,7 +338,70 @@ __device__ __forceinline__ double2 quad_interp(const ChannelDev& ch, const Marke
     return make_double2((double)ux, (double)uy);
 }
 
-// Whether a per-marker interpolation takes four lanes a marker.  Few markers
+// interp_u_acc by four lanes of a warp, lane `row` a stencil row, as quad_interp.
+template <typename S, typename R, typename A>
+__device__ __forceinline__ double2 quad_interp_acc(const ChannelDev& ch, const MarkerBufs& mb,
+                                                   int m, bool on, int row,
+                                                   const S* __restrict__ f,
+                                                   const A* __restrict__ acc) {
+    static_assert(sizeof(R) == 8, "the FP32-arithmetic modes move markers by capsule");
+    double tx[4], ty[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) tx[i] = ty[i] = 0;
+    if (on) {
+        const int2 og = mb.org[m];
+        const int jy = og.y - 1 + row, ty0 = max(og.y - 1, 0) / TILE_H;
+        const int4 sl4 =
+            reinterpret_cast<const int4*>(mb.slot8 + 8 * (size_t)m)[jy / TILE_H != ty0 ? 1 : 0];
+        const int sl[4] = {sl4.x, sl4.y, sl4.z, sl4.w};
+        const double2* x2 = reinterpret_cast<const double2*>(mb.wx + 4 * (size_t)m);
+        const double2 xa = x2[0], xb = x2[1];
+        const double wx[4] = {xa.x, xa.y, xb.x, xb.y}, wy = mb.wy[4 * (size_t)m + row];
+        double v[4][9], fx[4], fy[4];
+        bool use[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            int jx = og.x - 1 + i;
+            if (jx < 0) jx += ch.nx;
+            if (jx >= ch.nx) jx -= ch.nx;
+            use[i] = jy >= 0 && jy < ch.ny && jx >= 0 && jx < ch.nx &&
+                     cell_kind(ch, jx, jy) != CK_SOLID;
+            if (use[i]) {
+                const long long n = (long long)jy * ch.pitch + jx;
+#pragma unroll
+                for (int q = 0; q < 9; ++q)
+                    v[i][q] = PopIO<S, R>::ld(f + ch.f_off + q * ch.plane + n, q);
+                const size_t ci =
+                    (size_t)sl[i] * 2 * TILE_CELLS + (jy % TILE_H) * TILE_W + (jx % TILE_W);
+                fx[i] = acc[ci];
+                fy[i] = acc[ci + TILE_CELLS];
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const double w = wx[i] * wy;
+            if (use[i] && w > 1e-15) {
+                double rho, jxm, jym;
+                lattice_moments(v[i], rho, jxm, jym);
+                if (rho > 1e-15) {
+                    tx[i] = (jxm + 0.5 * fx[i]) / rho * w;
+                    ty[i] = (jym + 0.5 * fy[i]) / rho * w;
+                }
+            }
+        }
+    }
+    double ux = 0, uy = 0;
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {   // (see quad_interp)
+        const double sx = (((ux + tx[0]) + tx[1]) + tx[2]) + tx[3];
+        const double sy = (((uy + ty[0]) + ty[1]) + ty[2]) + ty[3];
+        ux = __shfl_sync(0xffffffffu, sx, r, 4);
+        uy = __shfl_sync(0xffffffffu, sy, r, 4);
+    }
+    return make_double2(ux, uy);
+}
+
+// Whether a per-marker kernel takes four lanes a marker.  Few markers
 // cannot fill the chip and every kernel is one warp's chain of dependent loads
 // and instructions, which the quad shortens (1,455 instructions a warp to a
 // third; 720 markers: 8.6 -> 5.2 us a sweep); with many the one-thread form

@@ -373,63 +373,142 @@ __device__ __forceinline__ void contact_cells(int m, int M, const ChannelDev* __
     cb.cell[c] = make_int2(base, n);
 }
 
-// One thread per marker.  The nine cell records of its 3 x 3 neighbourhood
-// are loaded together; an entry of the same capsule (most of them) costs one
-// 8-byte load, another capsule's entry also the position copied into the
-// list.  Velocities are read only where damping or friction use them.
-__global__ void k_contact_force(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
-                                ContactBufs cb) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    const ChannelDev& ch = chans[mb.mk_chan[m]];
-    const int cap = mb.mk_cap[m];
-    const double2 pa = mb.pos[m], va = mb.vel[m];
-    double2 F = mb.frc[m];
-    int count = 0;
-    if (ch.brute_contact) {
-        for (int b = ch.mk_begin; b < ch.mk_end; ++b) {
-            if (mb.mk_cap[b] == cap) continue;
-            const double2 f = pair_force(ch, pa, va, mb.pos[b], mb.vel[b]);
-            F.x = F.x + f.x;
-            F.y = F.y + f.y;
-            ++count;
-        }
-    } else {
+// The nine cell records of a marker's 3 x 3 neighbourhood (x in [0, ncx)
+// wrapped, rows outside empty), cells k0 .. k1 - 1, row by row.
+struct ContactCells {
+    int2 rec[9];
+    __device__ __forceinline__ ContactCells(const ChannelDev& ch, const ContactBufs& cb, int m,
+                                            int k0, int k1) {
         const int ci = cb.cell_of[m] - ch.cell_base;
         const int cx = ci % ch.ncx, cy = ci / ch.ncx;
-        const bool moving = ch.rep_damping > 0.0 || ch.rep_friction > 0.0;
-        int2 rec[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
             const int yy = cy + k / 3 - 1;
             int xx = cx + k % 3 - 1;
             if (xx < 0) xx += ch.ncx;
             if (xx >= ch.ncx) xx -= ch.ncx;
-            rec[k] = yy < 0 || yy >= ch.ncy ? make_int2(0, 0)
-                                            : cb.cell[ch.cell_base + yy * ch.ncx + xx];
+            rec[k] = k < k0 || k >= k1 || yy < 0 || yy >= ch.ncy
+                         ? make_int2(0, 0)
+                         : cb.cell[ch.cell_base + yy * ch.ncx + xx];
         }
+    }
+    // add(f) for every marker of another capsule, in the cells' order; an
+    // entry of the same capsule (most of them) costs one 8-byte load, another
+    // capsule's entry also the position copied into the list.  Velocities are
+    // read only where damping or friction use them.
+    template <typename Add>
+    __device__ __forceinline__ void each(const ChannelDev& ch, const MarkerBufs& mb,
+                                         const ContactBufs& cb, int cap, double2 pa, double2 va,
+                                         Add add) const {
+        const bool moving = ch.rep_damping > 0.0 || ch.rep_friction > 0.0;
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
             for (int e = rec[k].x; e < rec[k].x + rec[k].y; ++e) {
                 const int2 o = cb.list[e];   // marker, capsule
                 if (o.y == cap) continue;
-                const double2 f = pair_force(ch, pa, va, cb.lpos[e],
-                                             moving ? mb.vel[o.x] : make_double2(0.0, 0.0));
-                F.x = F.x + f.x;
-                F.y = F.y + f.y;
-                ++count;
+                add(pair_force(ch, pa, va, cb.lpos[e],
+                               moving ? mb.vel[o.x] : make_double2(0.0, 0.0)));
             }
         }
     }
+};
+
+__device__ __forceinline__ void add2(double2& F, double2 f) {
+    F.x = F.x + f.x;
+    F.y = F.y + f.y;
+}
+
+// The whole of a marker's contact force by one thread.
+__device__ __forceinline__ int contact_serial(const ChannelDev& ch, const MarkerBufs& mb,
+                                              const ContactBufs& cb, int m, int cap, double2 pa,
+                                              double2 va, double2& F) {
+    int count = 0;
+    if (ch.brute_contact) {
+        for (int b = ch.mk_begin; b < ch.mk_end; ++b) {
+            if (mb.mk_cap[b] == cap) continue;
+            add2(F, pair_force(ch, pa, va, mb.pos[b], mb.vel[b]));
+            ++count;
+        }
+    } else {
+        ContactCells(ch, cb, m, 0, 9).each(ch, mb, cb, cap, pa, va, [&](double2 f) {
+            add2(F, f);
+            ++count;
+        });
+    }
+    return count;
+}
+
+// Contact and wall forces of a marker, by one thread or (QUAD) by four lanes,
+// which take two or three of the nine cells each and a wall each.  The forces
+// that are not zero (a few at most, as the cut-off is below the cells' width)
+// are kept by the lanes and added in the cells' order by all four, so the sum
+// is the one thread's; a lane that finds more than QUAD_PAIRS of them leaves
+// the marker to one thread.  By interp_by_quads: with 720 to 2400 markers
+// 17.1 -> 15.4 us, with two capsules in the cell-free form 19.1 -> 14.9; with
+// 72,000 markers 18.9 -> 35.1 and 204,528 30.4 -> 85.9, whose chip is full.
+constexpr int QUAD_PAIRS = 4;
+template <bool QUAD>
+__global__ void k_contact_force(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
+                                ContactBufs cb) {
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, m = QUAD ? t >> 2 : t;
+    if (!QUAD && m >= M) return;
+    const bool on = m < M;   // (lanes beyond the last marker only take part)
+    const ChannelDev& ch = chans[on ? mb.mk_chan[m] : 0];
+    const int cap = on ? mb.mk_cap[m] : 0;
     const double2 z = make_double2(0.0, 0.0);
-    double2 f = pair_force(ch, pa, va, make_double2(pa.x, ch.y_bot), z);
-    F.x = F.x + f.x;
-    F.y = F.y + f.y;
-    f = pair_force(ch, pa, va, make_double2(pa.x, ch.y_top), z);
-    F.x = F.x + f.x;
-    F.y = F.y + f.y;
-    mb.frc[m] = F;
-    mb.pair_count[m] = count;
+    const double2 pa = on ? mb.pos[m] : z, va = on ? mb.vel[m] : z;
+    double2 F = on ? mb.frc[m] : z;
+    const double2 bot = make_double2(pa.x, ch.y_bot), top = make_double2(pa.x, ch.y_top);
+    if constexpr (!QUAD) {
+        const int count = contact_serial(ch, mb, cb, m, cap, pa, va, F);
+        add2(F, pair_force(ch, pa, va, bot, z));
+        add2(F, pair_force(ch, pa, va, top, z));
+        mb.frc[m] = F;
+        mb.pair_count[m] = count;
+    } else {
+        const int q = t & 3;
+        double2 keep[QUAD_PAIRS];
+#pragma unroll
+        for (int i = 0; i < QUAD_PAIRS; ++i) keep[i] = z;
+        int n = 0, count = 0;
+        if (on && !ch.brute_contact) {
+            ContactCells(ch, cb, m, q == 0 ? 0 : 2 * q + 1, 2 * q + 3)
+                .each(ch, mb, cb, cap, pa, va, [&](double2 f) {
+                    ++count;
+                    if (f.x == 0.0 && f.y == 0.0) return;
+#pragma unroll
+                    for (int i = 0; i < QUAD_PAIRS; ++i)
+                        if (i == n) keep[i] = f;
+                    ++n;
+                });
+        }
+        const double2 wall = pair_force(ch, pa, va, (q & 1) ? top : bot, z);
+        int most = n;
+        most = max(most, __shfl_xor_sync(0xffffffffu, most, 1));
+        most = max(most, __shfl_xor_sync(0xffffffffu, most, 2));
+        count += __shfl_xor_sync(0xffffffffu, count, 1);
+        count += __shfl_xor_sync(0xffffffffu, count, 2);
+        const bool serial = on && (ch.brute_contact || most > QUAD_PAIRS);
+        if (serial && q == 0) count = contact_serial(ch, mb, cb, m, cap, pa, va, F);
+        if (count > 0 && !serial) add2(F, z);   // (the zero forces: -0 becomes +0)
+        for (int l = 0; l < 4; ++l) {
+            const int got = __shfl_sync(0xffffffffu, n, l, 4), nl = serial ? 0 : got;
+#pragma unroll
+            for (int i = 0; i < QUAD_PAIRS; ++i) {
+                if (!__any_sync(0xffffffffu, i < nl)) break;   // uniform in the warp
+                const double fx = __shfl_sync(0xffffffffu, keep[i].x, l, 4);
+                const double fy = __shfl_sync(0xffffffffu, keep[i].y, l, 4);
+                if (i < nl) add2(F, make_double2(fx, fy));
+            }
+        }
+        const double tx = __shfl_sync(0xffffffffu, wall.x, 1, 4);
+        const double ty = __shfl_sync(0xffffffffu, wall.y, 1, 4);
+        if (!on || q != 0) return;
+        add2(F, wall);
+        add2(F, make_double2(tx, ty));
+        mb.frc[m] = F;
+        mb.pair_count[m] = count;
+    }
 }
 
 // ====================== immersed-boundary force tiles ======================
@@ -459,92 +538,151 @@ __device__ __forceinline__ int stencil_tiles(const ChannelDev& ch, int ix0, int 
     return n;
 }
 
+// Counts (FILL false) or list places (true) of a marker's stencil tiles among
+// the lanes of a warp that share them: one atomic per distinct tile and warp.
+// All lanes of the warp call it, lanes without a tile with key -1.  Returns the
+// lane's place in the tile's list.
+__device__ __forceinline__ int warp_tile_add(int* __restrict__ at, int key) {
+    const int lane = threadIdx.x & 31;
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    const int leader = __ffs(peers) - 1;
+    int base = 0;
+    if (key >= 0 && lane == leader) base = atomicAdd(&at[key], __popc(peers));
+    return __shfl_sync(0xffffffffu, base, leader) + __popc(peers & ((1u << lane) - 1u));
+}
+
 // Per-marker preparation: contact cell, arc length ds (min-image,
 // immersed_boundary.cpp:164-173), stencil origin, validity, and the tile
 // occupancy counts.  Also starts the step's counters and per-channel
 // results at zero (nothing else of the step runs before it, and the previous
 // step's have been read): as memsets these were five graph nodes in a row.
-template <typename R>
+// One thread per marker, or (QUAD, by interp_by_quads) four: a column and a
+// row of the stencil each, one of the two neighbours' distances, and every
+// fourth tile, as in k_tile_fill.  Both and the slots between them: 720 markers
+// 28.5 -> 24.4 us, 72,000 37.8 -> 43.7, 204,528 52.6 -> 73.2.
+template <typename R, bool QUAD>
 __global__ void k_marker_prep(const ChannelDev* __restrict__ chans, int nch,
                               const CapsuleDev* __restrict__ caps, int M, MarkerBufs mb,
                               const double* __restrict__ phi_tbl, TileBufs tb, ContactBufs cb,
                               unsigned* status) {
     chain_begin();
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int c = m; c < nch; c += gridDim.x * blockDim.x) {
+    constexpr int LANES = QUAD ? 4 : 1;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, m = t / LANES, q = t % LANES;
+    for (int c = t; c < nch; c += gridDim.x * blockDim.x) {
         tb.capped[c] = 0;
         tb.fluid_touched[c] = 0;
         tb.resid_gate[c] = 0u;
         tb.resid_plain[c] = 0u;
     }
-    if (m < NUM_STEP_CTR) tb.ctr[m] = 0;
-    if (m >= M) return;
-    const ChannelDev& ch = chans[mb.mk_chan[m]];
-    if (!ch.brute_contact) {
-        const int c = ch.cell_base + contact_cell(ch, mb.pos[m]);
+    if (t < NUM_STEP_CTR) tb.ctr[t] = 0;
+    const bool in = m < M;   // (lanes beyond the last marker only take part)
+    const ChannelDev& ch = chans[in ? mb.mk_chan[m] : 0];
+    const double2 p = in ? mb.pos[m] : make_double2(0.0, 0.0);
+    if (in && q == LANES - 1 && !ch.brute_contact) {
+        const int c = ch.cell_base + contact_cell(ch, p);
         cb.cell_of[m] = c;
         cb.next[m] = atomicExch(&cb.cell[c].x, m + 1);
     }
-    const CapsuleDev& cp = caps[mb.mk_cap[m]];
-    const int k = m - cp.off, n = cp.n;
-    const int kp = cp.off + (k - 1 + n) % n, kn = cp.off + (k + 1) % n;
-    const double Lx = (double)ch.nx;
-    const double2 p = mb.pos[m];
-    const double dp = norm_d(min_image_d(p, mb.pos[kp], Lx));
-    const double dn = norm_d(min_image_d(mb.pos[kn], p, Lx));
-    const double ds = 0.5 * (dp + dn);
-    int ok = finite2(p);
+    double ds = 0.0;
+    {
+        double dp = 0.0, dn = 0.0;
+        if (in) {
+            const CapsuleDev& cp = caps[mb.mk_cap[m]];
+            const int k = m - cp.off, n = cp.n;
+            const int kp = cp.off + (k - 1 + n) % n, kn = cp.off + (k + 1) % n;
+            const double Lx = (double)ch.nx;
+            if constexpr (QUAD) {
+                const double2 o = mb.pos[(q & 1) ? kn : kp];
+                dp = norm_d((q & 1) ? min_image_d(o, p, Lx) : min_image_d(p, o, Lx));
+            } else {
+                dp = norm_d(min_image_d(p, mb.pos[kp], Lx));
+                dn = norm_d(min_image_d(mb.pos[kn], p, Lx));
+            }
+        }
+        if constexpr (QUAD) {
+            dn = __shfl_sync(0xffffffffu, dp, 1, 4);
+            dp = __shfl_sync(0xffffffffu, dp, 0, 4);
+        }
+        ds = 0.5 * (dp + dn);
+    }
+    bool ok = in && finite2(p);
     int ix0 = 0, iy0 = 0;
     if (ok) {
         // markers more than one period outside the lattice are skipped (the
         // reference indexes out of range there); wrapped x stays in [0, nx)
-        if (p.x < -(double)ch.nx + 2.0 || p.x >= 2.0 * (double)ch.nx - 3.0) ok = 0;
-        if (fabs(p.y) > 1e9) ok = 0;
-    }
-    if (ok) {
-        ix0 = (int)floor(p.x);
-        iy0 = (int)floor(p.y);
-        if (iy0 < -2 || iy0 >= ch.ny + 2) ok = 0;
-    } else if (!finite2(p)) {
+        if (p.x < -(double)ch.nx + 2.0 || p.x >= 2.0 * (double)ch.nx - 3.0) ok = false;
+        if (fabs(p.y) > 1e9) ok = false;
+        if (ok) {
+            ix0 = (int)floor(p.x);
+            iy0 = (int)floor(p.y);
+            if (iy0 < -2 || iy0 >= ch.ny + 2) ok = false;
+        }
+    } else if (in && q == 0) {
         atomicOr(status, (unsigned)ST_NAN_MARKER);
     }
-    mb.org[m] = make_int2(ix0, iy0);
-    mb.valid[m] = ok;
-    if (!ok) return;
+    if (in && q == 0) {
+        mb.org[m] = make_int2(ix0, iy0);
+        mb.valid[m] = ok;
+    }
     // Peskin weights of the stencil, evaluated once per step (delta_function.h:44-59)
     double wx[4], wy[4];
+    if constexpr (QUAD) {
+        const double ax = ok ? phi_lut(phi_tbl, p.x - (double)(ix0 - 1 + q)) : 0.0;
+        wy[0] = ok ? phi_lut(phi_tbl, p.y - (double)(iy0 - 1 + q)) : 0.0;   // this lane's row
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        wx[k] = phi_lut(phi_tbl, p.x - (double)(ix0 - 1 + k));
-        wy[k] = phi_lut(phi_tbl, p.y - (double)(iy0 - 1 + k));
-    }
-    if constexpr (sizeof(R) == 8) {
-        mb.ds[m] = ds;
+        for (int k = 0; k < 4; ++k) wx[k] = __shfl_sync(0xffffffffu, ax, k, 4);
+        if (ok) {
+            if constexpr (sizeof(R) == 8) {
+                if (q == 0) mb.ds[m] = ds;
+                mb.wx[t] = ax;
+                mb.wy[t] = wy[0];
+            } else {
+                if (q == 0) mb.dsf[m] = (float)ds;
+                reinterpret_cast<float*>(mb.wxf)[t] = (float)ax;
+                reinterpret_cast<float*>(mb.wyf)[t] = (float)wy[0];
+            }
+        }
+    } else if (ok) {
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
-            mb.wx[4 * (size_t)m + k] = wx[k];
-            mb.wy[4 * (size_t)m + k] = wy[k];
+            wx[k] = phi_lut(phi_tbl, p.x - (double)(ix0 - 1 + k));
+            wy[k] = phi_lut(phi_tbl, p.y - (double)(iy0 - 1 + k));
         }
-    } else {
-        mb.dsf[m] = (float)ds;
-        mb.wxf[m] = make_float4((float)wx[0], (float)wx[1], (float)wx[2], (float)wx[3]);
-        mb.wyf[m] = make_float4((float)wy[0], (float)wy[1], (float)wy[2], (float)wy[3]);
-        auto point = [&](int k, int j) {
-            const double w = wx[k] * wy[j];
-            return w > 1e-15 ? (float)w : (w > 0.5e-15 ? WF_TOUCH_ONLY : WF_NONE);
-        };
+        if constexpr (sizeof(R) == 8) {
+            mb.ds[m] = ds;
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-            mb.wf[4 * (size_t)m + j] = make_float4(point(0, j), point(1, j), point(2, j), point(3, j));
+            for (int k = 0; k < 4; ++k) {
+                mb.wx[4 * (size_t)m + k] = wx[k];
+                mb.wy[4 * (size_t)m + k] = wy[k];
+            }
+        } else {
+            mb.dsf[m] = (float)ds;
+            mb.wxf[m] = make_float4((float)wx[0], (float)wx[1], (float)wx[2], (float)wx[3]);
+            mb.wyf[m] = make_float4((float)wy[0], (float)wy[1], (float)wy[2], (float)wy[3]);
+        }
     }
-    int t[8];
-    const int nt = stencil_tiles(ch, ix0, iy0, t);
-    // consecutive markers share tiles: one atomic per distinct tile and warp
-    for (int a = 0; a < 8; ++a) {
-        const int key = a < nt ? t[a] : -1;
-        const unsigned peers = __match_any_sync(__activemask(), key);
-        if (key >= 0 && (threadIdx.x & 31) == __ffs(peers) - 1)
-            atomicAdd(&tb.tile_cnt[key], __popc(peers));
+    if constexpr (sizeof(R) == 4) {
+        if (ok) {
+            auto point = [&](int k, int j) {
+                const double w = wx[k] * wy[j];
+                return w > 1e-15 ? (float)w : (w > 0.5e-15 ? WF_TOUCH_ONLY : WF_NONE);
+            };
+#pragma unroll
+            for (int j = 0; j < 4 / LANES; ++j)   // (QUAD: the lane's own row)
+                mb.wf[4 * (size_t)m + q + j] =
+                    make_float4(point(0, j), point(1, j), point(2, j), point(3, j));
+        }
+    }
+    int tiles[8];
+    const int nt = ok ? stencil_tiles(ch, ix0, iy0, tiles) : 0;
+#pragma unroll
+    for (int a = 0; a < 8; a += LANES) {
+        int key = -1;
+#pragma unroll
+        for (int l = 0; l < LANES; ++l)
+            if (l == q && a + l < nt) key = tiles[a + l];
+        // (most stencils lie in one or two tiles)
+        if (__any_sync(0xffffffffu, key >= 0)) warp_tile_add(tb.tile_cnt, key);
     }
 }
 
@@ -643,45 +781,57 @@ struct WorkOrder {
     }
 };
 
+template <bool QUAD>
 __global__ void k_tile_fill(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
                             int* __restrict__ tile_pos, int* __restrict__ list,
                             const int* __restrict__ tile_slot) {
     chain_begin();
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M || !mb.valid[m]) return;
-    const ChannelDev& ch = chans[mb.mk_chan[m]];
-    const int ix0 = mb.org[m].x, iy0 = mb.org[m].y;
-    int t[8];
-    const int nt = stencil_tiles(ch, ix0, iy0, t);
-    // one atomic per distinct tile and warp; the lanes of a tile take
-    // consecutive list entries (an FP64 spread restores the order)
-    const int lane = threadIdx.x & 31;
-    for (int a = 0; a < 8; ++a) {
-        const int key = a < nt ? t[a] : -1;
-        const unsigned peers = __match_any_sync(__activemask(), key);
-        const int leader = __ffs(peers) - 1;
-        int base = 0;
-        if (key >= 0 && lane == leader) base = atomicAdd(&tile_pos[key], __popc(peers));
-        base = __shfl_sync(peers, base, leader);
-        if (key >= 0) list[base + __popc(peers & ((1u << lane) - 1u))] = m;
+    constexpr int LANES = QUAD ? 4 : 1;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, m = t / LANES, q = t % LANES;
+    const bool ok = m < M && mb.valid[m];   // (the others only take part)
+    const ChannelDev& ch = chans[ok ? mb.mk_chan[m] : 0];
+    const int2 og = ok ? mb.org[m] : make_int2(0, 0);
+    // the lanes of a tile take consecutive list entries (an FP64 spread
+    // restores the order)
+    int tiles[8];
+    const int nt = ok ? stencil_tiles(ch, og.x, og.y, tiles) : 0;
+#pragma unroll
+    for (int a = 0; a < 8; a += LANES) {
+        int key = -1;
+#pragma unroll
+        for (int l = 0; l < LANES; ++l)
+            if (l == q && a + l < nt) key = tiles[a + l];
+        if (__any_sync(0xffffffffu, key >= 0)) {
+            const int at = warp_tile_add(tile_pos, key);
+            if (key >= 0) list[at] = m;
+        }
     }
     // the slot of every stencil cell, by row tile and stencil column, for the
     // interpolations of the step (one 32-byte record instead of 16 lookups)
-    int s8[8];
-    const int ty0 = max(iy0 - 1, 0) / TILE_H, ty1 = min(iy0 + 2, ch.ny - 1) / TILE_H;
+    if (ok) {
+        const int ty0 = max(og.y - 1, 0) / TILE_H, ty1 = min(og.y + 2, ch.ny - 1) / TILE_H;
+        int s8[8];
 #pragma unroll
-    for (int sx = 0; sx < 4; ++sx) {
-        int jx = ix0 - 1 + sx;
-        if (jx < 0) jx += ch.nx;
-        if (jx >= ch.nx) jx -= ch.nx;
-        const bool in = jx >= 0 && jx < ch.nx;
-        const int tx = in ? jx / TILE_W : 0;
-        s8[sx] = in ? tile_slot[ch.tile_base + ty0 * ch.tiles_x + tx] : -1;
-        s8[4 + sx] = in ? tile_slot[ch.tile_base + ty1 * ch.tiles_x + tx] : -1;
+        for (int sx = 0; sx < 4; ++sx) {
+            if (QUAD && sx != q) continue;
+            int jx = og.x - 1 + sx;
+            if (jx < 0) jx += ch.nx;
+            if (jx >= ch.nx) jx -= ch.nx;
+            const bool in = jx >= 0 && jx < ch.nx;
+            const int tx = in ? jx / TILE_W : 0;
+            s8[sx] = in ? tile_slot[ch.tile_base + ty0 * ch.tiles_x + tx] : -1;
+            s8[4 + sx] = in ? tile_slot[ch.tile_base + ty1 * ch.tiles_x + tx] : -1;
+            if constexpr (QUAD) {
+                mb.slot8[8 * (size_t)m + sx] = s8[sx];
+                mb.slot8[8 * (size_t)m + 4 + sx] = s8[4 + sx];
+            }
+        }
+        if constexpr (!QUAD) {
+            int4* o = reinterpret_cast<int4*>(mb.slot8 + 8 * (size_t)m);
+            o[0] = make_int4(s8[0], s8[1], s8[2], s8[3]);
+            o[1] = make_int4(s8[4], s8[5], s8[6], s8[7]);
+        }
     }
-    int4* o = reinterpret_cast<int4*>(mb.slot8 + 8 * (size_t)m);
-    o[0] = make_int4(s8[0], s8[1], s8[2], s8[3]);
-    o[1] = make_int4(s8[4], s8[5], s8[6], s8[7]);
 }
 
 constexpr int SPREAD_WARPS = 8;       // force tiles processed per CTA (one per warp)
@@ -1278,17 +1428,25 @@ __device__ __forceinline__ void move_marker(const ChannelDev& ch, const MarkerBu
 }
 
 // Interpolate the new velocity and move the markers (FP64 contexts), one
-// thread per marker.
-template <typename S, typename R>
+// thread per marker or (QUAD) four, by interp_by_quads: 2400 markers 14.7 us a
+// launch with one thread, 6.7 with four (divisions and 144 loads in a row).
+template <typename S, typename R, bool QUAD>
 __global__ void k_interp_move(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
                               ContactBufs cb, const S* __restrict__ f, const int* __restrict__ tile_slot,
                               const R* __restrict__ fin, const double* __restrict__ phi_tbl) {
-    const int m = blockIdx.x * blockDim.x + threadIdx.x;
-    if (m >= M) return;
-    const ChannelDev& ch = chans[mb.mk_chan[m]];
-    double2 u = make_double2(0.0, 0.0);
-    if (mb.valid[m]) u = interp_u_acc<S, R, R>(ch, mb, m, f, tile_slot, fin);
-    move_marker(ch, mb, cb, m, u);
+    const int t = blockIdx.x * blockDim.x + threadIdx.x, m = QUAD ? t >> 2 : t;
+    if constexpr (QUAD) {
+        const ChannelDev& ch = chans[m < M ? mb.mk_chan[m] : 0];
+        const double2 u =
+            quad_interp_acc<S, R>(ch, mb, m, m < M && mb.valid[m], t & 3, f, fin);
+        if (m < M && (t & 3) == 0) move_marker(ch, mb, cb, m, u);
+    } else {
+        if (m >= M) return;
+        const ChannelDev& ch = chans[mb.mk_chan[m]];
+        double2 u = make_double2(0.0, 0.0);
+        if (mb.valid[m]) u = interp_u_acc<S, R, R>(ch, mb, m, f, tile_slot, fin);
+        move_marker(ch, mb, cb, m, u);
+    }
 }
 
 // The marker move of the FP32-arithmetic modes, one block per capsule: the
@@ -1716,8 +1874,9 @@ void launch_obstacle_repulsion(const ChannelDev* chans, int M, const MarkerBufs&
 void launch_contact_force(const ChannelDev* chans, int M, const MarkerBufs& mb,
                           const ContactBufs& cb, cudaStream_t st) {
     if (M == 0) return;
-    const int B = 256, G = (M + B - 1) / B;
-    k_contact_force<<<G, B, 0, st>>>(chans, M, mb, cb);
+    const bool quads = interp_by_quads(M);
+    const int B = 256, G = ((quads ? 4 * M : M) + B - 1) / B;
+    (quads ? k_contact_force<true> : k_contact_force<false>)<<<G, B, 0, st>>>(chans, M, mb, cb);
 }
 
 template <typename R>
@@ -1726,13 +1885,15 @@ void launch_tiles(const ChannelDev* chans, int nch, const CapsuleDev* caps, int 
                   const double* phi_tbl, unsigned* status, cudaStream_t st,
                   cudaEvent_t slots_ready) {
     const int B = 256, G = (M + B - 1) / B, TB = (tb.T + B - 1) / B;
-    launch_chain(false, k_marker_prep<R>, G, B, 0, st, chans, nch, caps, M, mb, phi_tbl, tb, cb,
-                 status);
+    const bool quads = interp_by_quads(M);
+    const int GM = ((quads ? 4 * M : M) + B - 1) / B;
+    launch_chain(false, quads ? k_marker_prep<R, true> : k_marker_prep<R, false>, GM, B, 0, st,
+                 chans, nch, caps, M, mb, phi_tbl, tb, cb, status);
     launch_chain(true, k_tile_slots, TB + (ncells > 0 ? G : 0), B, 0, st, chans, M, mb, tb,
                  tb.tile_slot[parity], cb, TB);
     if (slots_ready) cudaEventRecord(slots_ready, st);
-    launch_chain(true, k_tile_fill, G, B, 0, st, chans, M, mb, tb.tile_pos, tb.list,
-                 tb.tile_slot[parity]);
+    launch_chain(true, quads ? k_tile_fill<true> : k_tile_fill<false>, GM, B, 0, st, chans, M,
+                 mb, tb.tile_pos, tb.list, tb.tile_slot[parity]);
 }
 
 template void launch_tiles<double>(const ChannelDev*, int, const CapsuleDev*, int, const MarkerBufs&,
@@ -1802,9 +1963,11 @@ void launch_interp_move(const ChannelDev* chans, const CapsuleDev* caps, int nca
             k_interp_move_caps<S, 64><<<ncaps, 64, 0, st>>>(caps, chans, mb, cb, f,
                                                             tb.tile_slot[parity], fin);
     } else {
-        const int B = tb.marker_block, G = (M + B - 1) / B;
-        k_interp_move<S, R><<<G, B, 0, st>>>(chans, M, mb, cb, f, tb.tile_slot[parity],
-                                             static_cast<const R*>(tb.fin[parity]), phi_tbl);
+        const bool quads = interp_by_quads(M);
+        const int B = tb.marker_block, G = ((quads ? 4 * M : M) + B - 1) / B;
+        (quads ? k_interp_move<S, R, true> : k_interp_move<S, R, false>)<<<G, B, 0, st>>>(
+            chans, M, mb, cb, f, tb.tile_slot[parity], static_cast<const R*>(tb.fin[parity]),
+            phi_tbl);
     }
 }
 

@@ -77,3 +77,43 @@ def test_few_and_many_tiles_agree(sfg, precision, sweeps, nodes):
         assert np.isfinite(a).all() and np.array_equal(a, b)
     assert np.array_equal(few.capsules(0).positions(), many.capsules(0).positions())
     assert np.array_equal(few.capsules(0).velocities(), many.capsules(0).velocities())
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("nodes", [12, 80])
+def test_crowded_contact_agrees(sfg, precision, nodes):
+    """Capsules whose membranes touch: a lane of a marker's four keeps up to four
+    forces that are not zero, and with 80 nodes a capsule far more lie within the
+    cut-off, so that one thread adds them; alone and among many markers alike."""
+    import softflow_b200 as S
+    out = []
+    for n_many in (0, 5):
+        ens = S.Ensemble(precision=precision)
+        for k in range(1 + n_many):
+            p = S.SimulationParams(nx=72 if k == 0 else 320, ny=44 if k == 0 else 200,
+                                   ibm_iterations=1, precision=precision)
+            p.fluid.boundary_type = S.BoundaryType.PERIODIC
+            p.fluid.collision_model = S.CollisionModel.BGK
+            i = ens.add_channel(p)
+            mp = S.MembraneParams(model=S.MembraneModel.NEO_HOOKEAN, G_s=0.05)
+            if k == 0:
+                # a touching pair across the seam, one capsule at the wall
+                for c in ((2.0, 20.3), (68.0, 21.1), (30.4, 6.2)):
+                    ens.addCapsule(i, c, 4.0, nodes, mp)
+            else:
+                for cy in range(12, 190, 16):
+                    for cx in range(10, 316, 16):
+                        ens.addCapsule(i, (cx, cy), 4.0, 32, mp)
+        ens.initialize()
+        a, b = (ens.capsules(0).positions().reshape(-1, 2)[k * nodes:(k + 1) * nodes]
+                for k in (0, 1))
+        d = a[:, None] - b[None]
+        d[..., 0] -= 72 * np.round(d[..., 0] / 72)
+        near = (np.hypot(d[..., 0], d[..., 1]) < p.repulsion.r_cut).sum(1).max()
+        assert 0 < near if nodes == 12 else near > 16   # more than four lanes keep
+        ens.run(2)
+        out.append((ens.num_markers(), ens.capsules(0).positions().copy(),
+                    ens.capsules(0).velocities().copy()))
+    assert out[0][0] <= 32768 < out[1][0]
+    for x, y in zip(out[0][1:], out[1][1:]):
+        assert np.isfinite(x).all() and np.array_equal(x, y)
