@@ -651,9 +651,9 @@ static void apply_launch_config(sfg_context* c) {
 // cells is then the step's length: FP32 400 x 80 3.8 us a step with four cells a
 // lane against 2.6 with one, 1024 x 256 equal (5.5), 2048 x 512 13.6 against 16.3;
 // FP64 BGK 512 x 200 7.0 against 5.3, 1024 x 256 11.9 against 9.9, 2048 x 512 39.8
-// against 42.7.  FP64 regularized, bound by its divisions, keeps too few warps
-// resident with four cells in registers at any size (4096 x 1024: 969 us against
-// 585).  FP32 and FP64 give the same bits either way; the FP16-shifted kernels
+// against 42.7, MRT 1024 x 512 25.2 against 19.9, 4096 x 1024 171 against 177.  FP64
+// regularized, bound by its arithmetic, keeps too few warps resident with four
+// cells in registers at any size (4096 x 1024: 223 us against 200).  FP32 and FP64 give the same bits either way; the FP16-shifted kernels
 // draw other dither bits, so their form follows from nx alone.
 static bool one_cell_lattice(const sfg_context* c, long long cells) {
     if (c->precision == SFG_FP32) return cells <= 200 * 1024;
