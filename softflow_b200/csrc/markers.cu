@@ -375,6 +375,11 @@ __device__ __forceinline__ void contact_cells(int m, int M, const ChannelDev* __
 
 // The nine cell records of a marker's 3 x 3 neighbourhood (x in [0, ncx)
 // wrapped, rows outside empty), cells k0 .. k1 - 1, row by row.
+// List entries of a cell loaded at once (nearly all are of the marker's own
+// capsule, and one by one each waited for its load: contact phase of 720 markers
+// 16.1 us one by one, 15.0 by four, 14.9 by eight; a step of 12 ragged channels 89.4,
+// 88.7, 87.7, of 256 channels 499, 494, 492).
+constexpr int CONTACT_AHEAD = 8;
 struct ContactCells {
     int2 rec[9];
     __device__ __forceinline__ ContactCells(const ChannelDev& ch, const ContactBufs& cb, int m,
@@ -393,7 +398,7 @@ struct ContactCells {
         }
     }
     // add(f) for every marker of another capsule, in the cells' order; an
-    // entry of the same capsule (most of them) costs one 8-byte load, another
+    // entry of the same capsule costs one 8-byte load, another
     // capsule's entry also the position copied into the list.  Velocities are
     // read only where damping or friction use them.
     template <typename Add>
@@ -403,11 +408,18 @@ struct ContactCells {
         const bool moving = ch.rep_damping > 0.0 || ch.rep_friction > 0.0;
 #pragma unroll
         for (int k = 0; k < 9; ++k) {
-            for (int e = rec[k].x; e < rec[k].x + rec[k].y; ++e) {
-                const int2 o = cb.list[e];   // marker, capsule
-                if (o.y == cap) continue;
-                add(pair_force(ch, pa, va, cb.lpos[e],
-                               moving ? mb.vel[o.x] : make_double2(0.0, 0.0)));
+            const int end = rec[k].x + rec[k].y;
+            for (int e0 = rec[k].x; e0 < end; e0 += CONTACT_AHEAD) {
+                // list entries are (marker, capsule)
+                unsigned others = 0;
+#pragma unroll
+                for (int j = 0; j < CONTACT_AHEAD; ++j)
+                    if (cb.list[min(e0 + j, end - 1)].y != cap && e0 + j < end) others |= 1u << j;
+                for (; others; others &= others - 1) {
+                    const int e = e0 + __ffs(others) - 1;
+                    add(pair_force(ch, pa, va, cb.lpos[e],
+                                   moving ? mb.vel[cb.list[e].x] : make_double2(0.0, 0.0)));
+                }
             }
         }
     }
