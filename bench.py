@@ -246,7 +246,7 @@ def scalar_bytes_per_cell(precision: str) -> int:
     return 144 if precision == "fp64" else 72
 
 
-SPREAD_ENTRY_BYTES = 100   # per list entry: force 16, arc length 8, origin 8, weights 64, index 4
+SPREAD_ENTRY_BYTES = 96    # per list entry: force 16, arc length 4, origin 8, weights 64, index 4
 SLOT_FINAL_BYTES = 4096    # per force tile, last sweep: final force and force before it, 2 x 2 KB
 
 
@@ -301,14 +301,20 @@ def spread_roofline(ens, plans, spread_ms, sweeps, peak, peak_kind):
 def lattice_kernel_name(plans, precision):
     """The lattice kernel instantiation a workload runs: the eight-cell
     FP16-shifted kernel when the storage is FP16S, there is no scalar and
-    every nx % 8 == 0, otherwise the four-cell kernel (storage, arithmetic,
-    scalar fused or not); the template's last argument is the collision
-    model."""
+    every nx % 8 == 0, the one-cell kernel on small FP32 and FP64 lattices, in
+    FP64 regularized and where an nx % 4 != 0, otherwise the four-cell kernel
+    (storage, arithmetic, scalar fused or not; the last argument is the
+    collision model)."""
     adr = int(any(p.params.scalar.enabled for p in plans))
     coll = "|".join(map(str, sorted({int(p.params.fluid.collision_model) for p in plans})))
     if precision == "fp16s" and not adr and all(p.params.nx % 8 == 0 for p in plans):
         return f"k_lattice_step8h<{coll}>"
     st = {"fp64": "double, double", "fp32": "float, float", "fp16s": "__half, float"}[precision]
+    cells = sum(p.params.nx * p.params.ny for p in plans)
+    one = {"fp32": cells <= 200 * 1024, "fp16s": False,
+           "fp64": coll == "2" or cells <= 512 * 1024}[precision]
+    if one or any(p.params.nx % 4 for p in plans):
+        return f"k_lattice_step<{st}, {adr}>"
     return f"k_lattice_step4<{st}, {adr}, {coll}>"
 
 
