@@ -181,9 +181,9 @@ __device__ __forceinline__ R div_const(R a, R d) {
 }
 
 // Whether every input of a cell's collision is zero or of magnitude 2^-200 to
-// 2^200: then every intermediate that is divided (products of up to four of them
-// and sums, whose terms are multiples of the inputs' last places) is zero or far
-// inside the exponent range.
+// 2^200 (the rates of MRT are checked once per channel): then every intermediate that is divided (products
+// of up to four of them and sums, whose terms are multiples of the inputs' last
+// places) is zero or far inside the exponent range.
 __device__ __forceinline__ bool ordinary(double v) {
     const unsigned hi = (unsigned)__double2hiint(v);
     return ((hi >> 20) & 0x7ffu) - 823u <= 400u || ((hi << 1) | (unsigned)__double2loint(v)) == 0u;
@@ -322,8 +322,8 @@ __device__ __noinline__ void mrt_divide(R* f, R r, R vx, R vy, R fx, R fy, R sn,
 
 template <typename R>
 __device__ __forceinline__ void collide_mrt(R f[9], R r, R vx, R vy, R fx, R fy, R sn, R s1, R s2,
-                                            R s4) {
-    if (ordinary_cell(f, vx, vy, fx, fy)) {
+                                            R s4, bool divides) {
+    if (!divides && ordinary_cell(f, vx, vy, fx, fy)) {
         mrt_cell<true>(f, r, vx, vy, fx, fy, sn, s1, s2, s4);
     } else {
         R g[9];
@@ -526,7 +526,7 @@ __device__ __forceinline__ void mrt_collide_v(V d[9], V rho, V vx, V vy, V fx, V
 template <>
 __device__ __forceinline__ void collide_mrt<float>(float f[9], float r, float vx, float vy,
                                                    float fx, float fy, float sn, float s1,
-                                                   float s2, float s4) {
+                                                   float s2, float s4, bool) {
     mrt_collide_v(f, r, vx, vy, fx, fy, mrt_const<float>(sn, s1, s2, s4));
 }
 

@@ -52,6 +52,7 @@ struct ChannelDev {
     long long g_off;            // = 9 * cell_off: plane 0 in the scalar buffers
     int collision;              // 0 BGK, 1 MRT, 2 regularized
     int ibm_iterations;
+    int mrt_divides;            // a rate is outside 2^-200 .. 2^200 (div_const)
     double omega, tau;
     double mrt_se, mrt_s_eps, mrt_sq;
     double body_fx, body_fy;

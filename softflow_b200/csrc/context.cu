@@ -704,6 +704,9 @@ extern "C" int sfg_initialize(sfg_context* c) {
         d.mrt_se = p.mrt_se;
         d.mrt_s_eps = p.mrt_s_eps;
         d.mrt_sq = p.mrt_sq;
+        d.mrt_divides = 0;
+        for (double s : {d.omega, d.mrt_se, d.mrt_s_eps, d.mrt_sq})
+            if (s != 0.0 && !(std::fabs(s) >= 0x1p-200 && std::fabs(s) <= 0x1p200)) d.mrt_divides = 1;
         d.body_fx = p.body_fx;
         d.body_fy = p.body_fy;
         d.max_force = p.max_lattice_force;

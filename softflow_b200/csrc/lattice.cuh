@@ -245,7 +245,7 @@ k_lattice_step(const RowItem* __restrict__ items, int n_items, const ChannelDev*
         collide_regularized(f, rho, ux, uy, cf.Fx, cf.Fy, R(ch.omega));
     } else if (coll == 1) {
         collide_mrt(f, rho, ux, uy, cf.Fx, cf.Fy, R(ch.omega), R(ch.mrt_se), R(ch.mrt_s_eps),
-                    R(ch.mrt_sq));
+                    R(ch.mrt_sq), ch.mrt_divides != 0);
     } else {
         collide_bgk(f, rho, ux, uy, cf.Fx, cf.Fy, R(ch.omega));
     }
@@ -333,7 +333,7 @@ k_lattice_step_bc(const RowItem* __restrict__ items, int n_items,
             collide_regularized(f, rho, ux, uy, cf.Fx, cf.Fy, R(ch.omega));
         } else if (coll == 1) {
             collide_mrt(f, rho, ux, uy, cf.Fx, cf.Fy, R(ch.omega), R(ch.mrt_se),
-                        R(ch.mrt_s_eps), R(ch.mrt_sq));
+                        R(ch.mrt_s_eps), R(ch.mrt_sq), ch.mrt_divides != 0);
         } else {
             collide_bgk(f, rho, ux, uy, cf.Fx, cf.Fy, R(ch.omega));
         }
@@ -888,7 +888,7 @@ __device__ __forceinline__ void collide_cell(R c[9], R rho, R ux, R uy, R Fx, R 
         collide_regularized(c, rho, ux, uy, Fx, Fy, R(ch.omega));
     else if (coll == 1)
         collide_mrt(c, rho, ux, uy, Fx, Fy, R(ch.omega), R(ch.mrt_se), R(ch.mrt_s_eps),
-                    R(ch.mrt_sq));
+                    R(ch.mrt_sq), ch.mrt_divides != 0);
     else
         collide_bgk(c, rho, ux, uy, Fx, Fy, R(ch.omega));
 }

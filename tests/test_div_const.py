@@ -141,3 +141,63 @@ def test_cells_outside_the_method_divide(sfg, kind, nx):
     with np.errstate(all="ignore"):
         want = _regularized(f, 1.0 / 0.8)
     assert np.array_equal(got, np.broadcast_to(want[:, None, None], got.shape), equal_nan=True)
+
+
+def _mrt(f, rates):
+    """collide of the FP64 MRT cell without forces, numpy's divisions."""
+    sn, s1, s2, s4 = rates
+    r, vx, vy = _velocity(f)
+    m = [f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8],
+         -4 * f[0] - f[1] - f[2] - f[3] - f[4] + 2 * f[5] + 2 * f[6] + 2 * f[7] + 2 * f[8],
+         4 * f[0] - 2 * f[1] - 2 * f[2] - 2 * f[3] - 2 * f[4] + f[5] + f[6] + f[7] + f[8],
+         f[1] - f[3] + f[5] - f[6] - f[7] + f[8],
+         -2 * f[1] + 2 * f[3] + f[5] - f[6] - f[7] + f[8],
+         f[2] - f[4] + f[5] + f[6] - f[7] - f[8],
+         -2 * f[2] + 2 * f[4] + f[5] + f[6] - f[7] - f[8],
+         f[1] - f[2] + f[3] - f[4], f[5] - f[6] + f[7] - f[8]]
+    uu = vx * vx + vy * vy
+    eq = {1: -2 * r + 3 * r * uu, 2: r - 3 * r * uu, 4: -r * vx, 6: -r * vy,
+          7: r * (vx * vx - vy * vy), 8: r * vx * vy}
+    for k, s in ((1, s1), (2, s2), (4, s4), (6, s4), (7, sn), (8, sn)):
+        m[k] = m[k] - s * (m[k] - eq[k]) + 0.0
+    m0, m1, m2, m3, m4, m5, m6, m7, m8 = m
+    return np.array([
+        m0 / 9 - m1 / 9 + m2 / 9,
+        m0 / 9 - m1 / 36 - m2 / 18 + m3 / 6 - m4 / 6 + m7 / 4,
+        m0 / 9 - m1 / 36 - m2 / 18 + m5 / 6 - m6 / 6 - m7 / 4,
+        m0 / 9 - m1 / 36 - m2 / 18 - m3 / 6 + m4 / 6 + m7 / 4,
+        m0 / 9 - m1 / 36 - m2 / 18 - m5 / 6 + m6 / 6 - m7 / 4,
+        m0 / 9 + m1 / 18 + m2 / 36 + m3 / 6 + m4 / 12 + m5 / 6 + m6 / 12 + m8 / 4,
+        m0 / 9 + m1 / 18 + m2 / 36 - m3 / 6 - m4 / 12 + m5 / 6 + m6 / 12 - m8 / 4,
+        m0 / 9 + m1 / 18 + m2 / 36 - m3 / 6 - m4 / 12 - m5 / 6 - m6 / 12 + m8 / 4,
+        m0 / 9 + m1 / 18 + m2 / 36 + m3 / 6 + m4 / 12 - m5 / 6 - m6 / 12 - m8 / 4])
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nx", [64, 63])
+@pytest.mark.parametrize("kind", ["plain", "edge", "tiny", "subnormal", "one_tiny", "inf", "rate"])
+def test_mrt_cells_outside_the_method_divide(sfg, kind, nx):
+    import softflow_b200 as S
+    rng = np.random.default_rng(9)
+    f = W * (1 + 0.1 * rng.uniform(-1, 1, 9))
+    f = f * {"edge": 2.0 ** -199, "tiny": 1e-70, "subnormal": 1e-310}.get(kind, 1.0)
+    if kind in ("one_tiny", "inf"):
+        f[3] = {"one_tiny": 1e-200, "inf": np.inf}[kind]
+    ens = S.Ensemble(precision="fp64")
+    p = S.SimulationParams(nx=nx, ny=12, precision="fp64")
+    p.fluid.boundary_type = S.BoundaryType.PERIODIC
+    p.fluid.collision_model = S.CollisionModel.MRT
+    p.fluid.tau = 0.8
+    p.fluid.periodic_y = True
+    if kind == "rate":
+        p.fluid.mrt_se = 1e-290
+        f = W.copy()   # moments that vanish, but for rounding
+    i = ens.add_channel(p)
+    ens.initialize()
+    ens.field(i).set_distributions(np.broadcast_to(f[:, None, None], (9, 12, nx)))
+    ens.run(1)
+    got = ens.field(i).distributions()
+    fl = p.fluid
+    with np.errstate(all="ignore"):
+        want = _mrt(f, (1.0 / 0.8, fl.mrt_se, fl.mrt_s_eps, fl.mrt_sq))
+    assert np.array_equal(got, np.broadcast_to(want[:, None, None], got.shape), equal_nan=True)
