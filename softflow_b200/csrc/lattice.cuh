@@ -53,9 +53,9 @@ struct PopIO;
 // d = f - w for FP32 arithmetic (FP32 and FP16 storage both keep d).
 template <>
 struct PopIO<double, double> {
-    static __device__ __forceinline__ double ld(const double* p, int) { return __ldg(p); }
+    static __device__ __forceinline__ double ld(const double* p, int) { return *p; }
     static __device__ __forceinline__ void st_sr(double* p, int, double v, uint32_t) { *p = v; }
-    static __device__ __forceinline__ double load(const double* p, int) { return __ldg(p); }
+    static __device__ __forceinline__ double load(const double* p, int) { return *p; }
     static __device__ __forceinline__ void store(double* p, int, double v) { *p = v; }
 };
 // FP32 storage keeps the deviation f - w (the populations stay close to
@@ -64,24 +64,24 @@ struct PopIO<double, double> {
 template <>
 struct PopIO<float, float> {
     static __device__ __forceinline__ float load(const float* p, int q) {
-        return float(w_of(q)) + __ldg(p);
+        return float(w_of(q)) + *p;
     }
     static __device__ __forceinline__ void store(float* p, int q, float v) {
         *p = v - float(w_of(q));
     }
-    static __device__ __forceinline__ float ld(const float* p, int) { return __ldg(p); }
+    static __device__ __forceinline__ float ld(const float* p, int) { return *p; }
     static __device__ __forceinline__ void st_sr(float* p, int, float v, uint32_t) { *p = v; }
 };
 template <>
 struct PopIO<__half, float> {
     static __device__ __forceinline__ float load(const __half* p, int q) {
-        return float(w_of(q)) + __half2float(__ldg(p)) * FP16S_UNSCALE;
+        return float(w_of(q)) + __half2float(*p) * FP16S_UNSCALE;
     }
     static __device__ __forceinline__ void store(__half* p, int q, float v) {
         *p = __float2half_rn((v - float(w_of(q))) * FP16S_SCALE);
     }
     static __device__ __forceinline__ float ld(const __half* p, int) {
-        return __half2float(__ldg(p)) * FP16S_UNSCALE;
+        return __half2float(*p) * FP16S_UNSCALE;
     }
     // r: per-cell seed; each direction draws its own 13 dither bits
     static __device__ __forceinline__ void st_sr(__half* p, int q, float v, uint32_t r) {
@@ -217,8 +217,8 @@ __device__ __forceinline__ void push_cell(S* __restrict__ fd, const R f[9], int 
 template <typename S, typename R, bool ADR>
 __global__ void __launch_bounds__(256)
 k_lattice_step(const RowItem* __restrict__ items, int n_items, const ChannelDev* __restrict__ chans,
-               const S* __restrict__ src, S* __restrict__ dst, const R* __restrict__ gsrc,
-               R* __restrict__ gdst, const R* __restrict__ cfield, TileView tv, StepFlagArgs fa) {
+               const S* src, S* __restrict__ dst, const R* gsrc, R* __restrict__ gdst,
+               const R* __restrict__ cfield, TileView tv, StepFlagArgs fa) {
     chain_begin();
     advance_flags(chans, fa);
     const int item = blockIdx.x * ITEMS_PER_CTA + (threadIdx.x >> 5);
@@ -230,7 +230,7 @@ k_lattice_step(const RowItem* __restrict__ items, int n_items, const ChannelDev*
     const int nx = ch.nx, ny = ch.ny, pitch = ch.pitch, plane = (int)ch.plane;
     const int x = it.x0 + lane, y = it.y;
     const int n = y * pitch + x;
-    const S* __restrict__ fs = src + ch.f_off + n;
+    const S* fs = src + ch.f_off + n;
     R f[9];
 #pragma unroll
     for (int q = 0; q < 9; ++q) f[q] = PopIO<S, R>::ld(fs + q * plane, q);
@@ -303,8 +303,8 @@ __device__ __forceinline__ R wall_correction(int q, R rho, double vel) {
 template <typename S, typename R>
 __global__ void __launch_bounds__(256)
 k_lattice_step_bc(const RowItem* __restrict__ items, int n_items,
-                  const ChannelDev* __restrict__ chans, const S* __restrict__ src,
-                  S* __restrict__ dst, TileView tv, StepFlagArgs fa) {
+                  const ChannelDev* __restrict__ chans, const S* src, S* __restrict__ dst,
+                  TileView tv, StepFlagArgs fa) {
     chain_begin();
     advance_flags(chans, fa);
     const int item = blockIdx.x * ITEMS_PER_CTA + (threadIdx.x >> 5);
@@ -318,7 +318,7 @@ k_lattice_step_bc(const RowItem* __restrict__ items, int n_items,
     const int kind = cell_kind(ch, x, y);
     if (kind == CK_SOLID) return;
     const int n = y * pitch + x;
-    const S* __restrict__ fs = src + ch.f_off + n;
+    const S* fs = src + ch.f_off + n;
     R f[9];
 #pragma unroll
     for (int q = 0; q < 9; ++q) f[q] = PopIO<S, R>::ld(fs + q * plane, q);
@@ -382,8 +382,7 @@ k_lattice_step_bc(const RowItem* __restrict__ items, int n_items,
 // formula.
 template <typename S, typename R>
 __global__ void k_ibb(const IbbLink* __restrict__ links, int n,
-                      const ChannelDev* __restrict__ chans, S* __restrict__ dst,
-                      const unsigned* __restrict__ step_ctr) {
+                      const ChannelDev* __restrict__ chans, S* dst, const unsigned* step_ctr) {
     chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
@@ -391,7 +390,7 @@ __global__ void k_ibb(const IbbLink* __restrict__ links, int n,
     const ChannelDev& ch = chans[L.chan];
     const int nx = ch.nx, ny = ch.ny, plane = (int)ch.plane, pitch = ch.pitch;
     const int q = L.q, o = opp_of(q);
-    S* __restrict__ fd = dst + ch.f_off;
+    S* fd = dst + ch.f_off;
     const R fq = PopIO<S, R>::ld(fd + q * plane + L.y * pitch + L.x, q);
     R v;
     if (L.qf < 0.5) {
@@ -421,8 +420,8 @@ __global__ void k_ibb(const IbbLink* __restrict__ links, int n,
 // weights sum to 1 and opposite weights cancel.
 template <typename S, typename R>
 __global__ void k_zou_he(const RowItem* __restrict__ rows, int n_rows,
-                         const ChannelDev* __restrict__ chans, S* __restrict__ dst,
-                         const unsigned* __restrict__ step_ctr) {
+                         const ChannelDev* __restrict__ chans, S* dst,
+                         const unsigned* step_ctr) {
     chain_begin();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n_rows) return;
@@ -430,7 +429,7 @@ __global__ void k_zou_he(const RowItem* __restrict__ rows, int n_rows,
     const ChannelDev& ch = chans[it.chan];
     const int y = it.y, ny = ch.ny, plane = (int)ch.plane;
     const R base = sizeof(R) == sizeof(double) ? R(0) : R(1);
-    S* __restrict__ fd = dst + ch.f_off;
+    S* fd = dst + ch.f_off;
     const uint32_t seed = mix32((uint32_t)y ^ mix32(*step_ctr + 0x2E5BF271u));
     {   // inlet
         const int n = y * ch.pitch;
@@ -484,7 +483,7 @@ struct Vec;
 template <>
 struct Vec<float> {
     static __device__ __forceinline__ void load4(const float* p, float v[4]) {
-        const float4 a = __ldg(reinterpret_cast<const float4*>(p));
+        const float4 a = *reinterpret_cast<const float4*>(p);
         v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
     }
     static __device__ __forceinline__ void store4(float* p, float a, float b, float c, float d) {
@@ -497,8 +496,8 @@ struct Vec<float> {
 template <>
 struct Vec<double> {
     static __device__ __forceinline__ void load4(const double* p, double v[4]) {
-        const double2 a = __ldg(reinterpret_cast<const double2*>(p));
-        const double2 b = __ldg(reinterpret_cast<const double2*>(p) + 1);
+        const double2 a = reinterpret_cast<const double2*>(p)[0];
+        const double2 b = reinterpret_cast<const double2*>(p)[1];
         v[0] = a.x; v[1] = a.y; v[2] = b.x; v[3] = b.y;
     }
     static __device__ __forceinline__ void store4(double* p, double a, double b, double c,
@@ -513,7 +512,7 @@ struct Vec<double> {
 template <>
 struct Vec<__half> {
     static __device__ __forceinline__ void load4(const __half* p, __half v[4]) {
-        const uint2 a = __ldg(reinterpret_cast<const uint2*>(p));
+        const uint2 a = *reinterpret_cast<const uint2*>(p);
         const __half2 lo = *reinterpret_cast<const __half2*>(&a.x);
         const __half2 hi = *reinterpret_cast<const __half2*>(&a.y);
         v[0] = __low2half(lo); v[1] = __high2half(lo);
@@ -900,13 +899,13 @@ template <typename S>
 __device__ __forceinline__ void load_pairs(const S* p, F2& a, F2& b);
 template <>
 __device__ __forceinline__ void load_pairs<float>(const float* p, F2& a, F2& b) {
-    const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+    const float4 v = *reinterpret_cast<const float4*>(p);
     a = mk2(v.x, v.y);
     b = mk2(v.z, v.w);
 }
 template <>
 __device__ __forceinline__ void load_pairs<__half>(const __half* p, F2& a, F2& b) {
-    const uint2 w = __ldg(reinterpret_cast<const uint2*>(p));
+    const uint2 w = *reinterpret_cast<const uint2*>(p);
     F2 u, v;
     u.v = __half22float2(*reinterpret_cast<const __half2*>(&w.x));
     v.v = __half22float2(*reinterpret_cast<const __half2*>(&w.y));
@@ -941,8 +940,8 @@ __device__ __forceinline__ void store_pairs<float>(float* row, F2 a, F2 b, int, 
 // per paired instruction.
 template <typename S, bool ADR, int COLL>
 __device__ __forceinline__ void lattice_run4f(const RowItem& it, const ChannelDev& ch, int st,
-                                              const S* __restrict__ src, S* __restrict__ dst,
-                                              const float* __restrict__ gsrc,
+                                              const S* src, S* __restrict__ dst,
+                                              const float* gsrc,
                                               float* __restrict__ gdst,
                                               const float* __restrict__ cfield,
                                               const TileView& tv, bool adr_on, bool fresh,
@@ -1047,8 +1046,8 @@ __device__ __forceinline__ void lattice_run4f(const RowItem& it, const ChannelDe
 
 template <typename S, typename R, bool ADR, int COLL>
 __device__ __forceinline__ void lattice_run4(const RowItem& it, const ChannelDev& ch, int st,
-                                             const S* __restrict__ src, S* __restrict__ dst,
-                                             const R* __restrict__ gsrc, R* __restrict__ gdst,
+                                             const S* src, S* __restrict__ dst,
+                                             const R* gsrc, R* __restrict__ gdst,
                                              const R* __restrict__ cfield, const TileView& tv,
                                              bool adr_on, bool fresh, uint32_t step_mix,
                                              int lane) {
@@ -1233,7 +1232,7 @@ struct QuadForces {
     float4 Fx, Fy, Gx, Gy;
 };
 __device__ __forceinline__ float4 ld4f(const float* p) {
-    return __ldg(reinterpret_cast<const float4*>(p));
+    return *reinterpret_cast<const float4*>(p);
 }
 __device__ __forceinline__ float4 splat4(float a) { return make_float4(a, a, a, a); }
 __device__ __forceinline__ QuadForces quad_forces(const ChannelDev& ch, const RunTiles& rt, int i,
@@ -1289,8 +1288,8 @@ __device__ __forceinline__ F2 quad_pair(const float4& v, int p) {
 // together write exactly what pass 0 writes.
 template <int COLL>
 __device__ __forceinline__ void lattice_run8h(const RowItem& it, const ChannelDev& ch, int st,
-                                              const __half* __restrict__ src,
-                                              __half* __restrict__ dst, const TileView& tv,
+                                              const __half* src, __half* __restrict__ dst,
+                                              const TileView& tv,
                                               uint32_t step_mix, int lane, int pass,
                                               unsigned* __restrict__ status) {
     bool in_run = 8 * lane < it.len;
@@ -1321,7 +1320,7 @@ __device__ __forceinline__ void lattice_run8h(const RowItem& it, const ChannelDe
         const __half* fs = src + ch.f_off + n;
 #pragma unroll
         for (int q = 0; q < 9; ++q)
-            w[q] = active ? __ldg(reinterpret_cast<const uint4*>(fs + (size_t)q * plane))
+            w[q] = active ? *reinterpret_cast<const uint4*>(fs + (size_t)q * plane)
                           : make_uint4(0u, 0u, 0u, 0u);
     }
     const uint32_t seed = mix32((uint32_t)n ^ step_mix);
@@ -1371,7 +1370,7 @@ template <int COLL>
 __global__ void __launch_bounds__(256, 2)
 k_lattice_step8h(const RowItem* __restrict__ items, int n_items,
                  const ChannelDev* __restrict__ chans, int n_chans,
-                 const __half* __restrict__ src, __half* __restrict__ dst, TileView tv,
+                 const __half* src, __half* __restrict__ dst, TileView tv,
                  StepFlagArgs fa, int pass, unsigned* __restrict__ status) {
     chain_begin();
     if (pass != 1) advance_flags(chans, fa);
@@ -1405,8 +1404,8 @@ constexpr int lattice_min_ctas() { return sizeof(R) == 8 ? 1 : (ADR ? 2 : 3); }
 template <typename S, typename R, bool ADR, int COLL>
 __global__ void __launch_bounds__(256, lattice_min_ctas<R, ADR>())
 k_lattice_step4(const RowItem* __restrict__ items, int n_items,
-                const ChannelDev* __restrict__ chans, const S* __restrict__ src,
-                S* __restrict__ dst, const R* __restrict__ gsrc, R* __restrict__ gdst,
+                const ChannelDev* __restrict__ chans, const S* src, S* __restrict__ dst,
+                const R* gsrc, R* __restrict__ gdst,
                 const R* __restrict__ cfield, TileView tv, StepFlagArgs fa) {
     chain_begin();
     advance_flags(chans, fa);

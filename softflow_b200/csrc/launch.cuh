@@ -9,6 +9,14 @@
 // not return before that call, so that completion of a kernel implies completion
 // of everything before it in the chain.
 //
+// What another kernel of the chain writes is read with ordinary loads through
+// parameters without __restrict__, never with __ldg: a waiting kernel is resident
+// while its predecessors write, so the memory is not constant over its lifetime as
+// the read-only path requires, and a load that the compiler may take for invariant
+// could also be moved above the wait.  __restrict__ stays on what is constant over
+// the chain (work items, channel records, the caller's data) and on what a kernel
+// only writes.
+//
 // Used where one stream runs kernel after kernel with nothing beside it: the
 // steps of a context without markers (400 x 80: 6.2 -> 4.0 us a step) and the
 // step's bookkeeping kernels (512 x 160 with 40 capsules: 31.7 -> 27.6 us).  Not on

@@ -326,7 +326,7 @@ __device__ __forceinline__ double2 pair_force(const ChannelDev& ch, double2 pa, 
 constexpr int CONTACT_BUF = 32;   // markers of a cell sorted in thread-local memory
 __device__ __forceinline__ void contact_cells(int m, int M, const ChannelDev* __restrict__ chans,
                                               const MarkerBufs& mb, const ContactBufs& cb,
-                                              int* __restrict__ total) {
+                                              int* total) {
     bool owner = m < M;
     int c = 0, n = 0, head = 0;
     int buf[CONTACT_BUF];
@@ -554,7 +554,7 @@ __device__ __forceinline__ int stencil_tiles(const ChannelDev& ch, int ix0, int 
 // the lanes of a warp that share them: one atomic per distinct tile and warp.
 // All lanes of the warp call it, lanes without a tile with key -1.  Returns the
 // lane's place in the tile's list.
-__device__ __forceinline__ int warp_tile_add(int* __restrict__ at, int key) {
+__device__ __forceinline__ int warp_tile_add(int* at, int key) {
     const int lane = threadIdx.x & 31;
     const unsigned peers = __match_any_sync(0xffffffffu, key);
     const int leader = __ffs(peers) - 1;
@@ -708,7 +708,7 @@ __global__ void k_marker_prep(const ChannelDev* __restrict__ chans, int nch,
 // Each slot is also entered under its list-length class (slot_order), for the
 // spread's work order.  The blocks after the tiles' build the contact cells.
 __global__ void k_tile_slots(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
-                             TileBufs tb, int* __restrict__ tile_slot, ContactBufs cb,
+                             TileBufs tb, int* tile_slot, ContactBufs cb,
                              int tile_blocks) {
     chain_begin();
     if ((int)blockIdx.x >= tile_blocks) {
@@ -795,8 +795,7 @@ struct WorkOrder {
 
 template <bool QUAD>
 __global__ void k_tile_fill(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
-                            int* __restrict__ tile_pos, int* __restrict__ list,
-                            const int* __restrict__ tile_slot) {
+                            int* tile_pos, int* __restrict__ list, const int* tile_slot) {
     chain_begin();
     constexpr int LANES = QUAD ? 4 : 1;
     const int t = blockIdx.x * blockDim.x + threadIdx.x, m = t / LANES, q = t % LANES;

@@ -70,7 +70,7 @@ __device__ __forceinline__ void stencil_weights(const MarkerBufs& mb, int m, flo
 
 // ---------------- Peskin 4-point delta via the 1024-bin table --------------
 // reference delta_function.h:44-54 (table built on the host from :18-26)
-__device__ __forceinline__ double phi_lut(const double* __restrict__ tbl, double r) {
+__device__ __forceinline__ double phi_lut(const double* tbl, double r) {
     double ar = fabs(r);
     if (ar >= 2.0) return 0.0;
     double idx = ar * (1024 * 0.5);

@@ -118,7 +118,7 @@ __device__ __forceinline__ void put_gated16(__nv_bfloat16* DZ, int d, const __nv
 // the wait for the previous step.  Batch of 8192, cold caches: 26.0 us with conversion,
 // transposed copies and layer 3 at the end, 10.7 us so.
 __global__ void __launch_bounds__(TRAIN_THREADS)
-k_mlp_train_tile(const ModelDev* __restrict__ md, const float* __restrict__ x,
+k_mlp_train_tile(const ModelDev* md, const float* __restrict__ x,
                  const float* __restrict__ t, const long long* __restrict__ rows, long long first,
                  long long n_rows, int n, float inv_n, float* __restrict__ part,
                  float* __restrict__ part_loss, unsigned* __restrict__ status) {
@@ -329,9 +329,8 @@ __device__ __forceinline__ void put_param(ModelDev* md, int i, float w) {
 constexpr int ADAM_THREADS = 64, ADAM_LOADS = 32;
 constexpr int ADAM_BLOCKS = (N_PARAMS + ADAM_THREADS - 1) / ADAM_THREADS + 1;
 __global__ void __launch_bounds__(ADAM_THREADS)
-k_mlp_adam(float* __restrict__ p, float* __restrict__ m, float* __restrict__ v,
-           const float* __restrict__ part, int nparts, int step, float lr,
-           float* __restrict__ g_out, const float* __restrict__ part_loss, float loss_scale,
+k_mlp_adam(float* p, float* m, float* v, const float* part, int nparts, int step, float lr,
+           float* __restrict__ g_out, const float* part_loss, float loss_scale,
            float* __restrict__ loss_out, ModelDev* __restrict__ md) {
     chain_begin();
     if (blockIdx.x == gridDim.x - 1) {

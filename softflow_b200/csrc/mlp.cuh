@@ -201,7 +201,7 @@ struct __align__(1024) FwdSmem {
 
 // Copies the model (already in operand layout) into shared memory.
 template <int NT = ROWS, typename SM>
-__device__ __forceinline__ void load_model(SM& s, const ModelDev* __restrict__ md) {
+__device__ __forceinline__ void load_model(SM& s, const ModelDev* md) {
     const int t = threadIdx.x;
     const uint4* w1 = reinterpret_cast<const uint4*>(md->W1);
     const uint4* w2 = reinterpret_cast<const uint4*>(md->W2);

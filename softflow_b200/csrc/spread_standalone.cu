@@ -159,8 +159,8 @@ __global__ void k_sa_fill(int nx, int ny, int tiles_x, int M, SpreadScratch sc) 
 // each, one warp a tile, 500 rings of 40 markers on 1000 x 700 took 112 us.
 __global__ void __launch_bounds__(BAND_WARPS * 32)
 k_sa_gather(int nx, int ny, int tiles_x, int T, const double2* __restrict__ pos,
-            const double2* __restrict__ frc, const double* __restrict__ phi_tbl,
-            SpreadScratch sc, double* __restrict__ Fx, double* __restrict__ Fy) {
+            const double2* __restrict__ frc, const double* phi_tbl, SpreadScratch sc,
+            double* __restrict__ Fx, double* __restrict__ Fy) {
     __shared__ BandSmem s_band[BAND_WARPS];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     BandSmem& B = s_band[warp];

@@ -77,7 +77,7 @@ __device__ __forceinline__ void band_sort(int* a, int cnt, int lane) {
 }
 
 // Sorts a list longer than BAND_LIST in place, by one thread (rare).
-__device__ __forceinline__ void long_list_sort(int* __restrict__ a, int cnt) {
+__device__ __forceinline__ void long_list_sort(int* a, int cnt) {
     for (int i = 1; i < cnt; ++i) {
         const int v = a[i];
         int j = i - 1;
@@ -99,7 +99,7 @@ struct BandMarker {
 // first row of the tile.  org_of(m): stencil origin; load(m, sy, k): the marker's
 // data for stencil row sy.  Lists longer than BAND_LIST are already sorted.
 template <typename OrgOf, typename Load>
-__device__ __forceinline__ void band_spread(BandSmem& B, const int* __restrict__ list, int cnt,
+__device__ __forceinline__ void band_spread(BandSmem& B, const int* list, int cnt,
                                             int nx, int ny, int x0, int y0, int lane, OrgOf org_of,
                                             Load load) {
     const int pad = (lane >> 2) * BAND_ACC_W + BAND_W + (lane & 3);   // this lane's padding cell
