@@ -5,6 +5,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "tile_rows.h"
+
 namespace sfg {
 
 // D2Q9 velocity set in the reference's numbering (src/lbm/lattice.h:12-27):
@@ -26,11 +28,8 @@ __host__ __device__ constexpr double w_of(int q) {
 static_assert(opp_of(1) == 3 && opp_of(2) == 4 && opp_of(3) == 1 && opp_of(4) == 2, "opp");
 static_assert(opp_of(5) == 7 && opp_of(6) == 8 && opp_of(7) == 5 && opp_of(8) == 6, "opp");
 
-// Force-tile geometry: lattice forces from the immersed boundary live in
-// 32 x 8 tiles that are only materialised where markers touch the lattice.
-constexpr int TILE_W = 32;
-constexpr int TILE_H = 8;
-constexpr int TILE_CELLS = TILE_W * TILE_H;
+// Lattice forces from the immersed boundary live in force tiles (tile_rows.h)
+// that are only materialised where markers touch the lattice.
 // Classes of force tiles by list length for the spread's work order: the
 // passes of 8 markers a tile takes, the last class open-ended.
 constexpr int SLOT_CLASSES = 16;

@@ -16,12 +16,12 @@ namespace sfg {
 struct StencilSlots {
     int s[8];
     int ty0;
-    __device__ __forceinline__ StencilSlots(const MarkerBufs& mb, int m, int iy0) {
+    __device__ __forceinline__ StencilSlots(const MarkerBufs& mb, int m, int iy0, int ny) {
         const int4* p = reinterpret_cast<const int4*>(mb.slot8 + 8 * (size_t)m);
         const int4 a = p[0], b = p[1];
         s[0] = a.x; s[1] = a.y; s[2] = a.z; s[3] = a.w;
         s[4] = b.x; s[5] = b.y; s[6] = b.z; s[7] = b.w;
-        ty0 = max(iy0 - 1, 0) / TILE_H;
+        ty0 = first_tile_row(iy0, ny);
     }
     __device__ __forceinline__ int slot(int sx, int jy) const {
         return s[(jy / TILE_H != ty0 ? 4 : 0) + sx];
@@ -39,7 +39,7 @@ __device__ __forceinline__ double2 interp_u_acc(const ChannelDev& ch, const Mark
     using C = typename std::conditional<sizeof(R) == 8, double, float>::type;
     const int2 og = mb.org[m];
     const int ix0 = og.x, iy0 = og.y;
-    const StencilSlots ss(mb, m, iy0);
+    const StencilSlots ss(mb, m, iy0, ch.ny);
     C wxs[4], wys[4];
     stencil_weights(mb, m, wxs, wys);
     int jxs[4];
@@ -137,7 +137,7 @@ __device__ __forceinline__ double2 interp_u_mom(const ChannelDev& ch, const Mark
     using C = typename std::conditional<sizeof(R) == 8, double, float>::type;
     const int2 og = mb.org[m];
     const int ix0 = og.x, iy0 = og.y;
-    const StencilSlots ss(mb, m, iy0);
+    const StencilSlots ss(mb, m, iy0, ch.ny);
     C wxs[4], wys[4];
     stencil_weights(mb, m, wxs, wys);
     int jxs[4];
@@ -252,7 +252,7 @@ __device__ __forceinline__ double2 quad_interp(const ChannelDev& ch, const Marke
         C wx[4], wy;
         int4 sl4;
         {
-            const int ty0 = max(og.y - 1, 0) / TILE_H;
+            const int ty0 = first_tile_row(og.y, ch.ny);
             sl4 = reinterpret_cast<const int4*>(mb.slot8 + 8 * (size_t)m)[jy / TILE_H != ty0 ? 1 : 0];
         }
         if constexpr (sizeof(R) == 8) {
@@ -350,7 +350,7 @@ __device__ __forceinline__ double2 quad_interp_acc(const ChannelDev& ch, const M
     for (int i = 0; i < 4; ++i) tx[i] = ty[i] = 0;
     if (on) {
         const int2 og = mb.org[m];
-        const int jy = og.y - 1 + row, ty0 = max(og.y - 1, 0) / TILE_H;
+        const int jy = og.y - 1 + row, ty0 = first_tile_row(og.y, ch.ny);
         const int4 sl4 =
             reinterpret_cast<const int4*>(mb.slot8 + 8 * (size_t)m)[jy / TILE_H != ty0 ? 1 : 0];
         const int sl[4] = {sl4.x, sl4.y, sl4.z, sl4.w};

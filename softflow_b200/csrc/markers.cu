@@ -820,7 +820,7 @@ __global__ void k_tile_fill(const ChannelDev* __restrict__ chans, int M, MarkerB
     // the slot of every stencil cell, by row tile and stencil column, for the
     // interpolations of the step (one 32-byte record instead of 16 lookups)
     if (ok) {
-        const int ty0 = max(og.y - 1, 0) / TILE_H, ty1 = min(og.y + 2, ch.ny - 1) / TILE_H;
+        const int ty0 = first_tile_row(og.y, ch.ny), ty1 = last_tile_row(og.y, ch.ny);
         int s8[8];
 #pragma unroll
         for (int sx = 0; sx < 4; ++sx) {
