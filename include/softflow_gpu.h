@@ -286,10 +286,19 @@ int sfg_get_contact_counts(sfg_context* ctx, int channel, int* counts);
  *                ring are skipped, never read)
  * Deterministic: each cell sums its contributions in ascending marker order
  * (the reference's serial order) without floating-point atomics.  Scratch
- * memory is taken with cudaMallocAsync on the stream and released on it. */
+ * memory (48 bytes a marker, 12 a force tile and 10 KB) is taken and released on
+ * the stream from a pool of the library's own, one per device context, which
+ * keeps up to 32 MiB for the next call; sfg_release_scratch gives that back.
+ * While `stream` is being captured the memory comes from the device's default
+ * pool and nothing is kept. */
 int sfg_spread_forces(int nx, int ny, int ncaps, const int* d_offsets, const double* d_pos,
                       const double* d_force, double* d_Fx, double* d_Fy, int num_markers,
                       void* stream);
+
+/* Returns the memory that sfg_spread_forces keeps on the current device to the
+ * driver: all that no spread in flight uses (wait for their streams first to
+ * get all of it).  Any thread may call it at any time, and spreads may follow. */
+int sfg_release_scratch(void);
 
 /* The spread of sfg_spread_forces for callers that cannot allocate device
  * memory inside a call (a host engine or framework that owns the device

@@ -13,6 +13,8 @@
 #include <mutex>
 #include <string>
 
+#include <cuda.h>
+
 #include "../../include/softflow_gpu.h"
 #include "markers.cuh"
 #include "sfg_internal.h"
@@ -274,42 +276,78 @@ using namespace sfg;
 
 namespace {
 
-// Scratch memory of sfg_spread_forces: a pool of its own per device that keeps at
-// most 32 MiB (one chunk of the driver's) between calls.  The device's default pool gives its memory back
+// Scratch memory of sfg_spread_forces: a pool of its own per device context that
+// keeps at most 32 MiB (one chunk of the driver's) between calls, until
+// sfg_release_scratch.  The device's default pool gives its memory back
 // whenever the stream is waited for, and the next call maps it anew: a caller
-// that waits for each spread paid 600 us for 140 us of work.  Null while a stream is
-// being captured (the call's allocation then becomes a node of the graph, from
-// the default pool, as ever) or when the pool cannot be made.
+// that waits for each spread paid 600 us for 140 us of work.
+struct ScratchPool {
+    unsigned long long context = 0;   // cuCtxGetId: no two contexts of a process share one
+    cudaMemPool_t pool = nullptr;     // null: it could not be made
+};
+constexpr int MAX_POOLS = 64;
+std::mutex g_pool_mutex;
+ScratchPool g_pools[MAX_POOLS];
+int g_num_pools = 0;
+
+// The current context's id, 0 without one.  A pool ends with its context
+// (cudaDeviceReset); by the id its handle is never used in the next one.
+unsigned long long context_id() {
+    using GetId = CUresult (*)(CUcontext, unsigned long long*);
+    static const GetId get = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+        if (cudaGetDriverEntryPointByVersion("cuCtxGetId", &f, 12000, cudaEnableDefault, &found) !=
+                cudaSuccess || found != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            f = nullptr;
+        }
+        return reinterpret_cast<GetId>(f);
+    }();
+    unsigned long long id = 0;
+    return get && get(nullptr, &id) == CUDA_SUCCESS ? id : 0;
+}
+
+// The current context's entry, null without one (all callers hold the mutex).
+ScratchPool* find_pool(unsigned long long context) {
+    for (int i = 0; i < g_num_pools; ++i)
+        if (g_pools[i].context == context) return &g_pools[i];
+    return nullptr;
+}
+
+// Null while the stream is being captured (the call's allocation then becomes a
+// node of the graph, from the default pool) or when the pool cannot be made.
 cudaMemPool_t scratch_pool(cudaStream_t st) {
-    constexpr int kMaxDevices = 64;
-    static std::mutex mutex;
-    static cudaMemPool_t pools[kMaxDevices] = {};
-    static bool failed[kMaxDevices] = {};
     cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
     int dev = 0;
     if (cudaStreamIsCapturing(st, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone ||
-        cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
+        cudaGetDevice(&dev) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    std::lock_guard<std::mutex> lock(mutex);
-    if (!pools[dev] && !failed[dev]) {
-        cudaMemPoolProps props = {};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = dev;
-        unsigned long long keep = 32ull << 20;
-        cudaMemPool_t pool = nullptr;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
-            cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
-            cudaGetLastError();
-            if (pool) cudaMemPoolDestroy(pool);
-            failed[dev] = true;
-        } else {
-            pools[dev] = pool;
-        }
+    const unsigned long long context = context_id();
+    if (context == 0) return nullptr;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (ScratchPool* known = find_pool(context)) return known->pool;
+    if (g_num_pools == MAX_POOLS) return nullptr;
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    unsigned long long keep = 32ull << 20;
+    cudaMemPool_t pool = nullptr;
+    // (another thread's stream capture forbids neither call to this one)
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess ||
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        if (pool) cudaMemPoolDestroy(pool);
+        pool = nullptr;
     }
-    return pools[dev];
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    g_pools[g_num_pools++] = {context, pool};
+    return pool;
 }
 
 }  // namespace
@@ -327,8 +365,11 @@ extern "C" int sfg_spread_forces(int nx, int ny, int ncaps, const int* d_offsets
     void* base = nullptr;
     const cudaMemPool_t pool = scratch_pool(st);
     const size_t bytes = spread_scratch_bytes(M, T);
-    cudaError_t e = pool ? cudaMallocFromPoolAsync(&base, bytes, pool, st)
-                         : cudaMallocAsync(&base, bytes, st);
+    cudaError_t e = pool ? cudaMallocFromPoolAsync(&base, bytes, pool, st) : cudaErrorMemoryAllocation;
+    if (e == cudaErrorMemoryAllocation) {   // the default pool may still hold enough
+        if (pool) cudaGetLastError();
+        e = cudaMallocAsync(&base, bytes, st);
+    }
     if (e != cudaSuccess) {
         sfg_host::set_error(std::string("sfg_spread_forces: ") + cudaGetErrorString(e));
         return SFG_ERR_CUDA;
@@ -341,4 +382,16 @@ extern "C" int sfg_spread_forces(int nx, int ny, int ncaps, const int* d_offsets
         return SFG_ERR_CUDA;
     }
     return rc;
+}
+
+extern "C" int sfg_release_scratch(void) {
+    const unsigned long long context = context_id();
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    const ScratchPool* known = context ? find_pool(context) : nullptr;
+    const cudaError_t e = known && known->pool ? cudaMemPoolTrimTo(known->pool, 0) : cudaSuccess;
+    if (e != cudaSuccess) {
+        sfg_host::set_error(std::string("sfg_release_scratch: ") + cudaGetErrorString(e));
+        return SFG_ERR_CUDA;
+    }
+    return SFG_OK;
 }
