@@ -199,28 +199,52 @@ struct __align__(1024) FwdSmem {
     int error;
 };
 
-// Copies the model (already in operand layout) into shared memory.
+// Copies the model (already in operand layout) into shared memory: all of a
+// thread's loads, then its stores.  They are ordinary loads, which the compiler does
+// not move over stores: 32 batches of 8192 with predictions 620 us one after the
+// other, 586 so.
 template <int NT = ROWS, typename SM>
 __device__ __forceinline__ void load_model(SM& s, const ModelDev* md) {
     const int t = threadIdx.x;
-    const uint4* w1 = reinterpret_cast<const uint4*>(md->W1);
-    const uint4* w2 = reinterpret_cast<const uint4*>(md->W2);
-    const uint4* w3 = reinterpret_cast<const uint4*>(md->W3);
-    uint4* s1 = reinterpret_cast<uint4*>(s.W1);
-    uint4* s2 = reinterpret_cast<uint4*>(s.W2);
-    uint4* s3 = reinterpret_cast<uint4*>(s.W3);
-    for (int i = t; i < N_H * K1 / 8; i += NT) s1[i] = w1[i];
-    for (int i = t; i < N_H * N_H / 8; i += NT) s2[i] = w2[i];
-    for (int i = t; i < N3 * N_H / 8; i += NT) s3[i] = w3[i];
-    if (t < N_H) s.b2[t] = md->b2[t];
+    constexpr int C1 = N_H * K1 / 8, C2 = N_H * N_H / 8, C3 = N3 * N_H / 8;   // 16-byte chunks
+    constexpr int P1 = (C1 + NT - 1) / NT, P2 = (C2 + NT - 1) / NT, P3 = (C3 + NT - 1) / NT;
+    uint4 a1[P1], a2[P2], a3[P3];
+    auto load = [&](uint4* a, const __nv_bfloat16* from, int n, int passes) {
+#pragma unroll
+        for (int p = 0; p < passes; ++p)
+            if (p * NT + t < n) a[p] = reinterpret_cast<const uint4*>(from)[p * NT + t];
+    };
+    auto store = [&](__nv_bfloat16* to, const uint4* a, int n, int passes) {
+#pragma unroll
+        for (int p = 0; p < passes; ++p)
+            if (p * NT + t < n) reinterpret_cast<uint4*>(to)[p * NT + t] = a[p];
+    };
+    load(a1, md->W1, C1, P1);
+    load(a2, md->W2, C2, P2);
+    load(a3, md->W3, C3, P3);
+    const float b2 = t < N_H ? md->b2[t] : 0.0f;
+    float out[3] = {}, in[2] = {};
     if (t < N_OUT) {
-        s.b3[t] = md->b3[t];
-        s.out_mean[t] = md->out_mean[t];
-        s.out_std[t] = md->out_std[t];
+        out[0] = md->b3[t];
+        out[1] = md->out_mean[t];
+        out[2] = md->out_std[t];
     }
     if (t < N_IN) {
-        s.in_mean[t] = md->in_mean[t];
-        s.in_inv_std[t] = md->in_inv_std[t];
+        in[0] = md->in_mean[t];
+        in[1] = md->in_inv_std[t];
+    }
+    store(s.W1, a1, C1, P1);
+    store(s.W2, a2, C2, P2);
+    store(s.W3, a3, C3, P3);
+    if (t < N_H) s.b2[t] = b2;
+    if (t < N_OUT) {
+        s.b3[t] = out[0];
+        s.out_mean[t] = out[1];
+        s.out_std[t] = out[2];
+    }
+    if (t < N_IN) {
+        s.in_mean[t] = in[0];
+        s.in_inv_std[t] = in[1];
     }
 }
 
