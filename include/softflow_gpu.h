@@ -348,8 +348,10 @@ int sfg_mlp_gradients(sfg_mlp* m, const float* d_x, const float* d_t, int n, flo
  * batch loss. */
 int sfg_mlp_train(sfg_mlp* m, const float* d_x, const float* d_t, int n, int batch, float lr,
                   float* losses, void* stream);
-/* The same over the rows d_rows[0], d_rows[1], ... (device, n entries in
- * [0, n); an entry outside is an error) of the data instead of rows 0, 1, ... */
+/* The same over the rows d_rows[0], d_rows[1], ... (device, n entries) of the
+ * data instead of rows 0, 1, ...  Where one of the entries that make up whole
+ * batches is outside [0, n), SFG_ERR_ARG is returned and the network (parameters,
+ * moments, step count) is as it was; `losses` then means nothing. */
 int sfg_mlp_train_rows(sfg_mlp* m, const float* d_x, const float* d_t, const long long* d_rows,
                        int n, int batch, float lr, float* losses, void* stream);
 int sfg_mlp_step_count(sfg_mlp* m, int* steps);

@@ -13,6 +13,7 @@
 // Loss: mean over samples and outputs of (y - t)^2 on normalised targets; the
 // per-sample output gradient 2 (y - t) / 2 and the batch mean follow the
 // reference surrogate network (src/ml/simple_nn.cpp:195-198, :236).
+#include <algorithm>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -32,7 +33,9 @@ constexpr int HXW = 96;             // width of [H1 | X | 1 | 0]
 constexpr int DZW = 2 * N_H;        // width of [dZ2 | dZ1]
 constexpr int TRAIN_THREADS = 2 * ROWS;
 constexpr int PART_STRIDE = (N_PARAMS + 3) / 4 * 4;  // 16-byte rows of partial gradients
-constexpr unsigned ST_TIMEOUT = 1u, ST_BAD_ROW = 2u;
+// Words of the status array: failed waits, and the number of the last training
+// call whose row list has an entry out of range.
+constexpr int ST_TIMEOUT = 0, ST_BAD_ROW = 1, ST_WORDS = 2;
 
 // Shared-memory image of a training tile.  Every operand is stored once and
 // read both ways: along its columns by the layers, and transposed (the sample
@@ -55,9 +58,23 @@ struct __align__(1024) TrainSmem {
     int error;
 };
 
+// The row list's entries that a training call uses, looked at before its first
+// update: an entry out of range fails the call with the network as it was.
+struct RowCheck {
+    const long long* rows;
+    long long used, n_rows;
+    unsigned* bad_call;
+    unsigned call;
+};
+
 // norm layout: in_mean[8], in_inv_std[8], out_mean[2], out_std[2]
 __global__ void k_build_model(const float* __restrict__ p, const float* __restrict__ norm,
-                              ModelDev* __restrict__ md) {
+                              ModelDev* __restrict__ md, RowCheck rc) {
+    bool bad = false;
+    for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < rc.used;
+         i += (long long)gridDim.x * blockDim.x)
+        bad = bad || rc.rows[i] < 0 || rc.rows[i] >= rc.n_rows;
+    if (bad) *rc.bad_call = rc.call;   // (all that meet here store the same)
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i < N_H * N_H) build_model_elem(md, p, norm, i);
 }
@@ -85,7 +102,7 @@ k_mlp_forward(const ModelDev* __restrict__ md, const float* __restrict__ x, int 
             y[(size_t)i * 2 + 1] = out[1] * s.out_std[1] + s.out_mean[1];
         }
     }
-    if (finish_tiles(s, phase, 128) && threadIdx.x == 0) atomicOr(status, ST_TIMEOUT);
+    if (finish_tiles(s, phase, 128) && threadIdx.x == 0) status[ST_TIMEOUT] = 1u;
 }
 
 // The gradient through a layer's ReLU: the 16 accumulator columns v where the
@@ -129,12 +146,11 @@ k_mlp_train_tile(const ModelDev* md, const float* __restrict__ x,
     const int i = blockIdx.x * ROWS + r;
     // The samples are no kernel of the chain's work (the chain's first kernel
     // is launched without overlap): they may be read before the wait.
-    bool valid = chain && i < n, bad = false;
+    bool valid = chain && i < n;
     float f[N_IN] = {}, tr[N_OUT] = {};
     if (valid) {
         const long long row = rows ? rows[first + i] : first + i;
-        bad = row < 0 || row >= n_rows;
-        valid = !bad;
+        valid = row >= 0 && row < n_rows;   // (the others fail the call: RowCheck)
         if (valid) {
 #pragma unroll
             for (int k = 0; k < N_IN; ++k) f[k] = x[row * N_IN + k];
@@ -152,7 +168,6 @@ k_mlp_train_tile(const ModelDev* md, const float* __restrict__ x,
     float* gp = part + (size_t)blockIdx.x * PART_STRIDE;
     bool ok = true;
     if (chain) {
-        if (bad) atomicOr(status, ST_BAD_ROW);
         put_input_cols(s, s.HX, N_H, HXW, f, valid);
         {
             // the ones column (bias gradient of layer 2), then zeros
@@ -304,7 +319,7 @@ k_mlp_train_tile(const ModelDev* md, const float* __restrict__ x,
             gp[P_B1 + o] = v[N_IN];
         }
     }
-    if (finish_tiles(s, phase, 256) && r == 0) atomicOr(status, ST_TIMEOUT);
+    if (finish_tiles(s, phase, 256) && r == 0) status[ST_TIMEOUT] = 1u;
 }
 
 // The parameter's place in the operand image.
@@ -331,7 +346,8 @@ constexpr int ADAM_BLOCKS = (N_PARAMS + ADAM_THREADS - 1) / ADAM_THREADS + 1;
 __global__ void __launch_bounds__(ADAM_THREADS)
 k_mlp_adam(float* p, float* m, float* v, const float* part, int nparts, int step, float lr,
            float* __restrict__ g_out, const float* part_loss, float loss_scale,
-           float* __restrict__ loss_out, ModelDev* __restrict__ md) {
+           float* __restrict__ loss_out, ModelDev* __restrict__ md, const unsigned* bad_call,
+           unsigned call) {
     chain_begin();
     if (blockIdx.x == gridDim.x - 1) {
         const int lane = threadIdx.x;
@@ -348,6 +364,7 @@ k_mlp_adam(float* p, float* m, float* v, const float* part, int nparts, int step
     const int i = blockIdx.x * ADAM_THREADS + threadIdx.x;
     if (i >= N_PARAMS) return;
     const float m0 = m[i], v0 = v[i], p0 = p[i];
+    const bool keep = *bad_call == call;   // the call will fail: nothing is updated
     float g = 0.0f;
     int c = 0;
     for (; c + ADAM_LOADS <= nparts; c += ADAM_LOADS) {
@@ -360,7 +377,7 @@ k_mlp_adam(float* p, float* m, float* v, const float* part, int nparts, int step
 #pragma unroll 4
     for (; c < nparts; ++c) g += part[(size_t)c * PART_STRIDE + i];
     if (g_out) g_out[i] = g;
-    if (step <= 0) return;
+    if (step <= 0 || keep) return;
     const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
     // the rounding is written out: left to the compiler, which product is fused
     // depends on where the loads stand
@@ -394,7 +411,8 @@ struct sfg_mlp {
     float* d_part_loss = nullptr;
     float* d_loss = nullptr;
     float* d_grad = nullptr;
-    unsigned* d_status = nullptr;
+    unsigned* d_status = nullptr;   // [ST_WORDS]
+    unsigned call = 0;              // training and gradient calls so far (never 0 in one)
     int part_cap = 0;
     int step = 0;
     bool model_dirty = true;
@@ -426,16 +444,14 @@ int ensure_parts(sfg_mlp* m, int nparts) {
     return SFG_OK;
 }
 
-int check_status(sfg_mlp* m, cudaStream_t st, const char* who) {
-    unsigned s = 0;
-    MCU(cudaMemcpyAsync(&s, m->d_status, sizeof(unsigned), cudaMemcpyDeviceToHost, st));
+int check_status(sfg_mlp* m, cudaStream_t st, const char* who, bool training = false) {
+    unsigned s[ST_WORDS] = {0};
+    MCU(cudaMemcpyAsync(s, m->d_status, sizeof s, cudaMemcpyDeviceToHost, st));
     MCU(cudaStreamSynchronize(st));
-    if (s & ST_TIMEOUT)
+    if (s[ST_TIMEOUT])
         return fail(SFG_ERR_CUDA, std::string(who) + ": a tensor-core wait timed out");
-    if (s & ST_BAD_ROW) {
-        MCU(cudaMemset(m->d_status, 0, sizeof(unsigned)));
+    if (training && s[ST_BAD_ROW] == m->call)
         return fail(SFG_ERR_ARG, std::string(who) + ": row index out of range");
-    }
     return SFG_OK;
 }
 
@@ -468,18 +484,24 @@ int batch_step(sfg_mlp* m, const Samples& d, long long first, int n, int step, f
     MCU(cudaGetLastError());
     sfg::launch_chain(true, k_mlp_adam, ADAM_BLOCKS, ADAM_THREADS, 0, st, m->d_params, m->d_m,
                       m->d_v, m->d_part, nparts, step, lr, g_out, m->d_part_loss,
-                      1.0f / (2.0f * (float)n), loss_out, m->d_train);
+                      1.0f / (2.0f * (float)n), loss_out, m->d_train, m->d_status + ST_BAD_ROW, m->call);
     MCU(cudaGetLastError());
     if (step > 0) m->model_dirty = true;
     return SFG_OK;
 }
 
-// The training image of the current parameters and normalisation, and room
-// for one batch's partial gradients.
-int begin_training(sfg_mlp* m, int n, cudaStream_t st) {
-    int rc = ensure_parts(m, (n + ROWS - 1) / ROWS);
+// The training image of the current parameters and normalisation, room for one
+// batch's partial gradients, and the check of the first `used` entries of the row
+// list (if any) into data of n_rows.
+int begin_training(sfg_mlp* m, int batch, const long long* rows, long long used, long long n_rows,
+                   cudaStream_t st) {
+    int rc = ensure_parts(m, (batch + ROWS - 1) / ROWS);
     if (rc) return rc;
-    k_build_model<<<(N_H * N_H + 255) / 256, 256, 0, st>>>(m->d_params, m->d_norm, m->d_train);
+    if (++m->call == 0u) m->call = 1u;
+    const RowCheck check{rows, rows ? used : 0, n_rows, m->d_status + ST_BAD_ROW, m->call};
+    const long long grid = std::max((long long)(N_H * N_H + 255) / 256,
+                                    std::min(256LL, (check.used + 255) / 256));
+    k_build_model<<<(unsigned)grid, 256, 0, st>>>(m->d_params, m->d_norm, m->d_train, check);
     MCU(cudaGetLastError());
     return SFG_OK;
 }
@@ -503,11 +525,11 @@ extern "C" int sfg_mlp_create(int device, sfg_mlp** out) {
     if (e == cudaSuccess) e = cudaMalloc(&m->d_model, sizeof(sfg::mlp::ModelDev));
     if (e == cudaSuccess) e = cudaMalloc(&m->d_train, sizeof(sfg::mlp::ModelDev));
     if (e == cudaSuccess) e = cudaMalloc(&m->d_loss, sizeof(float) * 4096);
-    if (e == cudaSuccess) e = cudaMalloc(&m->d_status, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMalloc(&m->d_status, sizeof(unsigned) * ST_WORDS);
     if (e == cudaSuccess) e = cudaMemset(m->d_params, 0, sizeof(float) * N_PARAMS);
     if (e == cudaSuccess) e = cudaMemset(m->d_m, 0, sizeof(float) * N_PARAMS);
     if (e == cudaSuccess) e = cudaMemset(m->d_v, 0, sizeof(float) * N_PARAMS);
-    if (e == cudaSuccess) e = cudaMemset(m->d_status, 0, sizeof(unsigned));
+    if (e == cudaSuccess) e = cudaMemset(m->d_status, 0, sizeof(unsigned) * ST_WORDS);
     if (e == cudaSuccess) {
         float norm[20];
         for (int i = 0; i < 20; ++i) norm[i] = (i < 8 || (i >= 16 && i < 18)) ? 0.0f : 1.0f;
@@ -576,7 +598,8 @@ extern "C" int sfg_mlp_set_normalization(sfg_mlp* m, const float* in_mean, const
 // normalisation changed); used by the forward kernel and the step.
 int sfg_mlp_model_device(sfg_mlp* m, const void** model, cudaStream_t st) {
     if (m->model_dirty) {
-        k_build_model<<<(N_H * N_H + 255) / 256, 256, 0, st>>>(m->d_params, m->d_norm, m->d_model);
+        k_build_model<<<(N_H * N_H + 255) / 256, 256, 0, st>>>(m->d_params, m->d_norm, m->d_model,
+                                                               RowCheck{});
         MCU(cudaGetLastError());
         m->model_dirty = false;
     }
@@ -609,7 +632,7 @@ extern "C" int sfg_mlp_gradients(sfg_mlp* m, const float* d_x, const float* d_t,
     if (n <= 0) return fail(SFG_ERR_ARG, "sfg_mlp_gradients: empty batch");
     MCU(cudaSetDevice(m->device));
     cudaStream_t st = static_cast<cudaStream_t>(stream);
-    int rc = begin_training(m, n, st);
+    int rc = begin_training(m, n, nullptr, 0, n, st);
     if (rc) return rc;
     rc = batch_step(m, {d_x, d_t, nullptr, n}, 0, n, 0, 0.0f, m->d_grad, m->d_loss, false, st);
     if (rc) return rc;
@@ -628,8 +651,9 @@ extern "C" int sfg_mlp_train_rows(sfg_mlp* m, const float* d_x, const float* d_t
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     const int nb = n / batch;
     if (nb < 1) return fail(SFG_ERR_ARG, "sfg_mlp_train: fewer samples than one batch");
-    int rc = begin_training(m, batch, st);
+    int rc = begin_training(m, batch, d_rows, (long long)nb * batch, n, st);
     if (rc) return rc;
+    const int step0 = m->step;
     const Samples d{d_x, d_t, d_rows, n};
     for (int b0 = 0; b0 < nb; b0 += 4096) {
         const int cnt = nb - b0 < 4096 ? nb - b0 : 4096;
@@ -643,7 +667,9 @@ extern "C" int sfg_mlp_train_rows(sfg_mlp* m, const float* d_x, const float* d_t
                                 cudaMemcpyDeviceToHost, st));
         }
     }
-    return check_status(m, st, "sfg_mlp_train");
+    rc = check_status(m, st, "sfg_mlp_train", true);
+    if (rc == SFG_ERR_ARG) m->step = step0;   // (no batch was applied)
+    return rc;
 }
 
 extern "C" int sfg_mlp_train(sfg_mlp* m, const float* d_x, const float* d_t, int n, int batch,

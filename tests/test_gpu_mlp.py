@@ -148,3 +148,38 @@ def test_row_list_out_of_range_is_an_error(sfg):
     assert run() == 1
     rows[7] = 7
     assert run() == 0
+
+
+@pytest.mark.parametrize("n,batch,where", [(1024, 128, 1000), (1024, 128, 0), (1000, 300, 899)])
+def test_row_list_out_of_range_leaves_the_network_alone(sfg, n, batch, where):
+    """A bad row in the last batch (or the first) fails the call before any update:
+    parameters, step count and moments, and so all later training and predictions,
+    are those of a network that never saw the call.  A row that no whole batch uses
+    is not looked at."""
+    import ctypes as C
+    import torch
+    X, T = _data(n, 14)
+    x, t = torch.tensor(X, device="cuda"), torch.tensor(T, device="cuda")
+    ptr = lambda a: C.c_void_p(a.data_ptr())
+    st = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+
+    def run(net, rows):
+        return net._lib.sfg_mlp_train_rows(net.handle, ptr(x), ptr(t), ptr(rows), n, batch, 1e-3,
+                                           None, st)
+
+    a, b = _net(9), _net(9)
+    good = torch.randperm(n, device="cuda", generator=torch.Generator("cuda").manual_seed(4))
+    assert run(a, good) == 0 and run(b, good) == 0
+    before = a.params()
+    for value in (n, -1, 1 << 40):
+        bad = good.clone()
+        bad[where] = value
+        assert run(a, bad) == 1
+        assert b"row index" in a._lib.sfg_last_error()
+        assert np.array_equal(a.params(), before) and a.steps() == b.steps()
+        assert np.array_equal(a.forward(X).cpu().numpy(), b.forward(X).cpu().numpy())
+    unused = good.clone()
+    if n % batch:
+        unused[n - 1] = n + 5
+    assert run(a, unused) == 0 and run(b, good) == 0
+    assert np.array_equal(a.params(), b.params()) and a.steps() == b.steps()
