@@ -289,6 +289,10 @@ __device__ __forceinline__ double2 pair_force(const ChannelDev& ch, double2 pa, 
         if (diff.x > 0.5 * Lx) diff.x -= Lx;
         if (diff.x < -0.5 * Lx) diff.x += Lx;
     }
+    // far pairs without the square root: beyond r_cut^2 by more than its rounding,
+    // r >= r_cut follows (an infinite r_cut^2 rejects nothing)
+    if (diff.x * diff.x + diff.y * diff.y > ch.rep_r_cut * ch.rep_r_cut * (1.0 + 1e-14))
+        return make_double2(0.0, 0.0);
     const double r = norm_d(diff);
     if (r < 1e-15 || r >= ch.rep_r_cut) return make_double2(0.0, 0.0);
     const double2 nrm = make_double2(diff.x / r, diff.y / r);
@@ -313,7 +317,7 @@ __device__ __forceinline__ double2 pair_force(const ChannelDev& ch, double2 pa, 
 }
 
 // The cell list without a scan: k_marker_prep pushes every marker onto its
-// cell's linked list (CellRec.head, CellRec::next by marker); here the marker
+// cell's linked list (the cell's head, ContactBufs::next by marker); here the marker
 // that reached its empty cell first walks that list, takes list space for the
 // cell (one atomic per warp), sorts the cell's markers into the reference's
 // insertion order (capsule-major, node-minor = ascending marker index) and
@@ -323,7 +327,11 @@ __device__ __forceinline__ double2 pair_force(const ChannelDev& ch, double2 pa, 
 // records of visited cells are cleared again by the marker move, so nothing
 // runs over all cells: on 30 capsules the binning, three-kernel scan, fill
 // and sort with their two memsets were nine graph nodes in a row.
-constexpr int CONTACT_BUF = 32;   // markers of a cell sorted in thread-local memory
+//
+// Up to CONTACT_BUF markers one thread sorts in its own memory; a more crowded cell
+// (fine membranes, a long cut-off) is ranked by its warp.  By one thread the lists
+// phase of 7,000 markers with cells of 30 to 250 took 84 to 721 us, so 29 to 54.
+constexpr int CONTACT_BUF = 12;
 __device__ __forceinline__ void contact_cells(int m, int M, const ChannelDev* __restrict__ chans,
                                               const MarkerBufs& mb, const ContactBufs& cb,
                                               int* total) {
@@ -351,54 +359,75 @@ __device__ __forceinline__ void contact_cells(int m, int M, const ChannelDev* __
     int base = 0;
     if (lane == 31 && inc > 0) base = atomicAdd(total, inc);
     base = __shfl_sync(0xffffffffu, base, 31) + inc - n;
-    if (!owner) return;
-    if (n <= CONTACT_BUF) {
+    if (owner) cb.cell[c] = make_int2(base, n);
+    if (owner && n <= CONTACT_BUF) {
         for (int i = 1; i < n; ++i) {
             const int v = buf[i];
             int j = i - 1;
             while (j >= 0 && buf[j] > v) { buf[j + 1] = buf[j]; --j; }
             buf[j + 1] = v;
         }
-        for (int i = 0; i < n; ++i) cb.list[base + i] = make_int2(buf[i], mb.mk_cap[buf[i]]);
-    } else {   // a crowded cell: sorted in place
-        int k = 0;
-        for (int i = head; i != 0; i = cb.next[i - 1], ++k) {
-            const int v = i - 1;
-            int j = k - 1;
-            while (j >= 0 && cb.list[base + j].x > v) { cb.list[base + j + 1] = cb.list[base + j]; --j; }
-            cb.list[base + j + 1] = make_int2(v, mb.mk_cap[v]);
+        for (int i = 0; i < n; ++i) {
+            cb.list[base + i] = make_int2(buf[i], mb.mk_cap[buf[i]]);
+            cb.lpos[base + i] = mb.pos[buf[i]];
         }
     }
-    for (int i = 0; i < n; ++i) cb.lpos[base + i] = mb.pos[cb.list[base + i].x];
-    cb.cell[c] = make_int2(base, n);
+    // crowded cells, one after the other by the whole warp: the owner has left the
+    // markers as they came in the memory of the cell's positions, every lane counts
+    // how many precede its own
+    const bool crowded = owner && n > CONTACT_BUF;
+    if (crowded) {
+        int* came = reinterpret_cast<int*>(cb.lpos + base);
+        for (int i = head, k = 0; i != 0; i = cb.next[i - 1], ++k) came[k] = i - 1;
+    }
+    __syncwarp();
+    for (unsigned left = __ballot_sync(0xffffffffu, crowded); left; left &= left - 1) {
+        const int o = __ffs(left) - 1;
+        const int at = __shfl_sync(0xffffffffu, base, o), cnt = __shfl_sync(0xffffffffu, n, o);
+        const int* came = reinterpret_cast<const int*>(cb.lpos + at);
+        for (int e = lane; e < cnt; e += 32) {
+            const int v = came[e];
+            int rank = 0;
+#pragma unroll 8
+            for (int k = 0; k < cnt; ++k) rank += came[k] < v ? 1 : 0;
+            cb.list[at + rank] = make_int2(v, mb.mk_cap[v]);
+        }
+        __syncwarp();
+        for (int e = lane; e < cnt; e += 32) cb.lpos[at + e] = mb.pos[cb.list[at + e].x];
+        __syncwarp();
+    }
 }
 
-// The nine cell records of a marker's 3 x 3 neighbourhood (x in [0, ncx)
-// wrapped, rows outside empty), cells k0 .. k1 - 1, row by row.
 // List entries of a cell loaded at once (nearly all are of the marker's own
 // capsule, and one by one each waited for its load: contact phase of 720 markers
 // 16.1 us one by one, 15.0 by four, 14.9 by eight; a step of 12 ragged channels 89.4,
 // 88.7, 87.7, of 256 channels 499, 494, 492).
 constexpr int CONTACT_AHEAD = 8;
+
+// The cells k0 .. k1 - 1 of a marker's 3 x 3 neighbourhood, row by row (x in
+// [0, ncx) wrapped, rows outside empty).  One after the other in a loop that is not
+// unrolled, the next record loaded ahead: nine copies of the pair force did not
+// stay in the instruction cache (516,096 markers with a cut-off of 14: contact phase
+// 1,373 us with nine copies, 1,081 so; 7,000 markers 401 -> 233).
 struct ContactCells {
-    int2 rec[9];
+    int cx, cy, k0, k1;
     __device__ __forceinline__ ContactCells(const ChannelDev& ch, const ContactBufs& cb, int m,
-                                            int k0, int k1) {
+                                            int first, int end)
+        : k0(first), k1(end) {
         const int ci = cb.cell_of[m] - ch.cell_base;
-        const int cx = ci % ch.ncx, cy = ci / ch.ncx;
-#pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const int yy = cy + k / 3 - 1;
-            int xx = cx + k % 3 - 1;
-            if (xx < 0) xx += ch.ncx;
-            if (xx >= ch.ncx) xx -= ch.ncx;
-            rec[k] = k < k0 || k >= k1 || yy < 0 || yy >= ch.ncy
-                         ? make_int2(0, 0)
-                         : cb.cell[ch.cell_base + yy * ch.ncx + xx];
-        }
+        cx = ci % ch.ncx;
+        cy = ci / ch.ncx;
     }
-    // add(f) for every marker of another capsule, in the cells' order; an
-    // entry of the same capsule costs one 8-byte load, another
+    __device__ __forceinline__ int2 rec(const ChannelDev& ch, const ContactBufs& cb, int k) const {
+        const int yy = cy + k / 3 - 1;
+        int xx = cx + k % 3 - 1;
+        if (xx < 0) xx += ch.ncx;
+        if (xx >= ch.ncx) xx -= ch.ncx;
+        return k >= k1 || yy < 0 || yy >= ch.ncy ? make_int2(0, 0)
+                                                 : cb.cell[ch.cell_base + yy * ch.ncx + xx];
+    }
+    // add(f) for every marker of another capsule, in the cells' order, until it
+    // returns false; an entry of the same capsule costs one 8-byte load, another
     // capsule's entry also the position copied into the list.  Velocities are
     // read only where damping or friction use them.
     template <typename Add>
@@ -406,10 +435,13 @@ struct ContactCells {
                                          const ContactBufs& cb, int cap, double2 pa, double2 va,
                                          Add add) const {
         const bool moving = ch.rep_damping > 0.0 || ch.rep_friction > 0.0;
-#pragma unroll
-        for (int k = 0; k < 9; ++k) {
-            const int end = rec[k].x + rec[k].y;
-            for (int e0 = rec[k].x; e0 < end; e0 += CONTACT_AHEAD) {
+        int2 next = rec(ch, cb, k0);
+#pragma unroll 1
+        for (int k = k0; k < k1; ++k) {
+            const int2 now = next;
+            next = rec(ch, cb, k + 1);
+            const int end = now.x + now.y;
+            for (int e0 = now.x; e0 < end; e0 += CONTACT_AHEAD) {
                 // list entries are (marker, capsule)
                 unsigned others = 0;
 #pragma unroll
@@ -417,8 +449,9 @@ struct ContactCells {
                     if (cb.list[min(e0 + j, end - 1)].y != cap && e0 + j < end) others |= 1u << j;
                 for (; others; others &= others - 1) {
                     const int e = e0 + __ffs(others) - 1;
-                    add(pair_force(ch, pa, va, cb.lpos[e],
-                                   moving ? mb.vel[cb.list[e].x] : make_double2(0.0, 0.0)));
+                    if (!add(pair_force(ch, pa, va, cb.lpos[e],
+                                        moving ? mb.vel[cb.list[e].x] : make_double2(0.0, 0.0))))
+                        return;
                 }
             }
         }
@@ -445,6 +478,7 @@ __device__ __forceinline__ int contact_serial(const ChannelDev& ch, const Marker
         ContactCells(ch, cb, m, 0, 9).each(ch, mb, cb, cap, pa, va, [&](double2 f) {
             add2(F, f);
             ++count;
+            return true;
         });
     }
     return count;
@@ -458,10 +492,14 @@ __device__ __forceinline__ int contact_serial(const ChannelDev& ch, const Marker
 // the marker to one thread.  By interp_by_quads: with 720 to 2400 markers
 // 17.1 -> 15.4 us, with two capsules in the cell-free form 19.1 -> 14.9; with
 // 72,000 markers 18.9 -> 35.1 and 204,528 30.4 -> 85.9, whose chip is full.
+// A lane that has found more stops there, as the one thread counts them anew.  One
+// thread a marker is bound by the latency of dependent FP64 instructions: three
+// blocks resident (80 registers) where 88 registers kept two; 516,096 markers with
+// a cut-off of 14 1,312 -> 1,081 us.
 constexpr int QUAD_PAIRS = 4;
 template <bool QUAD>
-__global__ void k_contact_force(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
-                                ContactBufs cb) {
+__global__ void __launch_bounds__(256, QUAD ? 2 : 3)
+k_contact_force(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb, ContactBufs cb) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x, m = QUAD ? t >> 2 : t;
     if (!QUAD && m >= M) return;
     const bool on = m < M;   // (lanes beyond the last marker only take part)
@@ -487,11 +525,11 @@ __global__ void k_contact_force(const ChannelDev* __restrict__ chans, int M, Mar
             ContactCells(ch, cb, m, q == 0 ? 0 : 2 * q + 1, 2 * q + 3)
                 .each(ch, mb, cb, cap, pa, va, [&](double2 f) {
                     ++count;
-                    if (f.x == 0.0 && f.y == 0.0) return;
+                    if (f.x == 0.0 && f.y == 0.0) return true;
 #pragma unroll
                     for (int i = 0; i < QUAD_PAIRS; ++i)
                         if (i == n) keep[i] = f;
-                    ++n;
+                    return ++n <= QUAD_PAIRS;
                 });
         }
         const double2 wall = pair_force(ch, pa, va, (q & 1) ? top : bot, z);

@@ -40,3 +40,35 @@ def test_lists_against_oracle(sfg, oracle_mod, nx, ny, rings):
         assert rel_l2(sim.capsules().forces(), o.forces()) < 1e-8
         assert np.max(np.abs(sim.capsules().positions() - o.positions())) < 1e-9
         assert rel_l2(sim.field().force_x(), o.Fx()) < 1e-8
+
+
+@pytest.mark.parametrize("precision", ["fp64", "fp32"])
+@pytest.mark.parametrize("r_cut,n", [(3.5, 160), (9.0, 64), (25.0, 64)])
+def test_cells_of_many_markers_against_oracle(sfg, oracle_mod, precision, r_cut, n):
+    """Cells of more than 12 markers, ranked by a warp, and of several capsules each,
+    where a marker's lane finds far more than four forces; few markers (four lanes each)
+    and, with a second channel, many (one thread).  Pair counts are integers; forces
+    in the tolerances of the other cases (FP32 keeps positions and contact in double)."""
+    import softflow_b200 as S
+    from cases import add_case_capsules, gpu_params
+    case = _case(96, 60, [(14.0 + 17 * k, 20.3 + 16 * j, 6.0, n)
+                          for k in range(5) for j in range(2)], 1)
+    case["spec"].update(rep_r_cut=r_cut, rep_epsilon=1e-4)
+    o = build_oracle(case)
+    o.step(1)
+    for copies in (0, 4):
+        ens = S.Ensemble(precision=precision)
+        ens.add_channel(gpu_params(case, precision))
+        add_case_capsules(ens, 0, case)
+        for _ in range(copies):
+            p = S.SimulationParams(nx=1024, ny=128, precision=precision)
+            p.fluid.boundary_type = S.BoundaryType.PERIODIC
+            j = ens.add_channel(p)
+            mp = S.MembraneParams(model=S.MembraneModel.NEO_HOOKEAN, G_s=0.05)
+            for cy in range(16, 120, 20):
+                for cx in range(16, 1010, 20):
+                    ens.addCapsule(j, (cx, cy), 4.0, 34, mp)
+        ens.initialize()
+        ens.run(1)
+        assert np.array_equal(ens.capsules(0).contact_counts(), o.contact_pairs()[0])
+        assert rel_l2(ens.capsules(0).forces(), o.forces()) < 1e-8
