@@ -629,7 +629,7 @@ static cudaError_t dalloc(T** p, size_t n) {
 // initialize
 // ------------------------------------------------------------------------
 static int resident_spread_ctas(const sfg_context* c) {
-    return spread_blocks_per_sm(c->precision == SFG_FP64, spread_wide(c->tb.max_slots));
+    return spread_blocks_per_sm(c->precision == SFG_FP64, c->tb.wide);
 }
 
 // Grid sizes from the tuned CTAs-per-SM counts (0 = the resident maximum).
@@ -640,10 +640,31 @@ static void apply_launch_config(sfg_context* c) {
     const int spr = c->spread_cps > 0 ? std::min(c->spread_cps, spr_max) : spr_max;
     c->persistent_ctas = c->nsm * lat;
     // tiles a spread CTA works at a time
-    const int per_cta = c->precision == SFG_FP64 || spread_wide(c->tb.max_slots) ? 1 : 8;
+    const int per_cta = c->tb.wide ? 1 : 8;
     c->spread_grid =
         std::max(1, std::min((c->tb.max_slots + per_cta - 1) / per_cta, c->nsm * spr));
     c->learned_grid = c->nsm * std::max(1, std::min(c->learned_cps, 6));
+}
+
+// Force tiles that the markers' stencils reach at their positions `pos` (x, y).
+static int touched_tiles(const sfg_context* c, const std::vector<double>& pos,
+                         const std::vector<int>& mk_chan, int tiles) {
+    std::vector<char> seen((size_t)tiles, 0);
+    int count = 0;
+    for (size_t m = 0; m < mk_chan.size(); ++m) {
+        const ChannelDev& d = c->ch[mk_chan[m]].d;
+        const double x = pos[2 * m], y = pos[2 * m + 1];
+        if (!(x >= -d.nx && x < 2.0 * d.nx && y > -3.0 && y < d.ny + 3.0)) continue;
+        const int ix = (int)std::floor(x) + d.nx, iy = (int)std::floor(y);
+        for (int k = 0; k < 4; ++k) {   // the corners of the 4 x 4 stencil
+            const int jx = (ix + (k & 1 ? 2 : -1) + d.nx) % d.nx;
+            const int jy = std::min(std::max(iy + (k & 2 ? 2 : -1), 0), d.ny - 1);
+            char& t = seen[(size_t)d.tile_base + (size_t)(jy / TILE_H) * d.tiles_x + jx / TILE_W];
+            count += t == 0;
+            t = 1;
+        }
+    }
+    return count;
 }
 
 // Whether the one-cell-per-thread lattice kernel is the faster one for `cells`
@@ -1070,6 +1091,8 @@ extern "C" int sfg_initialize(sfg_context* c) {
     TileBufs& tb = c->tb;
     tb.T = tile_base;
     tb.max_slots = M > 0 ? (int)std::min<long long>(tile_base, 8LL * M) : 1;
+    tb.wide = spread_wide(c->precision == SFG_FP64, tb.max_slots,
+                          c->precision == SFG_FP64 ? touched_tiles(c, pos, mk_chan, tb.T) : 0);
     const int T = tb.T;
     CU(dalloc(&tb.tile_chan, T));
     CU(cudaMemcpy(tb.tile_chan, tile_chan.data(), sizeof(int) * T, cudaMemcpyHostToDevice));

@@ -896,16 +896,36 @@ __device__ __forceinline__ int acc_at(int c) { return (c / TILE_W) * ACC_W + (c 
 // Deterministic spread into force tiles for MDF sweep `sweep` (FP64 contexts, bit
 // for bit; the FP32-arithmetic modes run k_spread_fx).  Sweep 0 spreads the
 // membrane + contact forces (immersed_boundary.cpp:25-100); sweep k >= 1 adds the
-// corrections dF (:231-286).  One CTA owns one tile, a warp a band of eight
-// columns (spread_wide.cuh), so every cell receives its contributions in the
-// reference's order.  On a channel's last sweep the warps also add the body force
-// on FLUID cells, apply the force cap and count capped cells
-// (simulation.cpp:540-609), writing the final tile force `fin`.  Tiles are dealt
-// to the CTAs in rounds over the work order (longest lists first, alternating
-// direction, so that each CTA's share sums to about the same work; a shared
+// corrections dF (:231-286).  A warp owns a tile, or (WIDE) a band of eight of its
+// columns, a CTA of four warps the tile (spread_wide.cuh): either way every cell
+// receives its contributions in the reference's order.  On a channel's last sweep the
+// warps also add the body force on FLUID cells, apply the force cap and count capped
+// cells (simulation.cpp:540-609), writing the final tile force `fin`.  Tiles are dealt
+// to the warps or CTAs in rounds over the work order (longest lists first, alternating
+// direction, so that each share sums to about the same work; a shared
 // claim counter serialises on one L2 address); the next tile's record is fetched
 // while the current one is processed.
-__global__ void __launch_bounds__(BAND_WARPS * 32, 6)
+//
+// Few tiles leave the chip idle, and a tile's chain is then the kernel's length, which
+// four warps cut; with many tiles the bands' passes over each list are only more work.
+// The line lies where the warps with a tile each (24 an SM) run in one round and the
+// bands' CTAs (6 an SM) in three.  It goes by the tiles touched when the context is
+// initialized, as large lattices with few markers have many tiles too.  Spread
+// phase of a step of five sweeps, a warp a tile / bands, us, by touched tiles:
+//   200 to 800 x 40 to 160 channels    103   73  55     1161 100  76     2528 125 114
+//                                     4985  142 185     9055 224 294    17342 372 546
+//   lattices of 1024 x 256 and more    132   96  62      832  99  83     1664 115 116
+//                                     2128  156 136     3264 158 192     4128 188 226
+//   four capsules of 300 nodes          15  206 148 (lists of up to 300)
+constexpr int BAND_TILES = 2800;
+template <bool WIDE> using SpreadTile = typename std::conditional<WIDE, BandTile, WarpTile>::type;
+template <bool WIDE> constexpr int spread_warps = WIDE ? BAND_WARPS : SPREAD_WARPS;
+template <bool WIDE>
+constexpr size_t spread_smem =
+    sizeof(SpreadTile<WIDE>) * spread_warps<WIDE> + (WIDE ? sizeof(int) * SORT_SMEM : 0);
+
+template <bool WIDE>
+__global__ void __launch_bounds__(32 * spread_warps<WIDE>, WIDE ? 6 : 3)
 k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot_info,
          const int* __restrict__ slot_order, const int* __restrict__ ctr, int max_slots,
          int* __restrict__ list, MarkerBufs mb, double* __restrict__ acc,
@@ -914,20 +934,27 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
          const int* __restrict__ plain_needed, int* __restrict__ capped,
          int* __restrict__ fluid_touched, unsigned* status) {
     if (sweep > 0 && mode == MDF_PLAIN && plain_needed && !*plain_needed) return;
-    __shared__ BandSmem s_band[BAND_WARPS];
+    using Tile = SpreadTile<WIDE>;
+    constexpr int THREADS = WIDE ? 32 * BAND_WARPS : 32;   // of the group that has a tile
+    extern __shared__ __align__(16) unsigned char spread_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    BandSmem& B = s_band[warp];
+    Tile& B = reinterpret_cast<Tile*>(spread_raw)[warp];
+    int* sort = WIDE ? reinterpret_cast<int*>(reinterpret_cast<Tile*>(spread_raw) + BAND_WARPS)
+                     : reinterpret_cast<int*>(B.v);
+    const int group = WIDE ? blockIdx.x : blockIdx.x * SPREAD_WARPS + warp;
+    const int groups = WIDE ? gridDim.x : gridDim.x * SPREAD_WARPS;
+    const int gt = WIDE ? threadIdx.x : lane;
     const int n_slots = ctr[CTR_SLOTS];
     const WorkOrder wo(ctr);
-    int round = 0, next = blockIdx.x;
+    int round = 0, next = group;
     int nslot = next < n_slots ? wo.slot(slot_order, max_slots, next) : 0;
     SlotInfo nfo{};
     if (next < n_slots) nfo = slot_info[nslot];
-    while (next < n_slots) {   // uniform in the CTA
+    while (next < n_slots) {   // uniform in the group
         const int slot = nslot;
         const SlotInfo si = nfo;
         ++round;
-        next = round * gridDim.x + ((round & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x);
+        next = round * groups + ((round & 1) ? groups - 1 - group : group);
         if (next < n_slots) {
             nslot = wo.slot(slot_order, max_slots, next);
             nfo = slot_info[nslot];
@@ -939,13 +966,13 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
         if (sweep > 0 && !mdf_active(ch, mode, resid_gate, chan)) continue;  // sweep 0: all
         int cnt = si.cnt;
         if (cnt > SPREAD_LIST_MAX) {
-            if (threadIdx.x == 0) atomicOr(status, (unsigned)ST_LIST_OVERFLOW);
+            if (gt == 0) atomicOr(status, (unsigned)ST_LIST_OVERFLOW);
             cnt = SPREAD_LIST_MAX;
         }
-        if (cnt > BAND_LIST && sweep == 0) {   // (sorted for the later sweeps too)
-            if (threadIdx.x == 0) long_list_sort(list + si.off, cnt);
-            __syncthreads();
-        }
+        int* lst = list + si.off;
+        const int first = sweep == 0
+                              ? tile_list_sort<THREADS>(lst, cnt, sort, gt, !WIDE || K > 1)
+                              : (lane < cnt ? lst[lane] : 0);
         const bool last = mode == MDF_LEARNED ? true : (mode == MDF_SEED ? false : sweep == K - 1);
         // a learned channel's membrane-only force lives in acc0 only: the
         // seed sweep and a fallback's restart read it there.  The
@@ -953,16 +980,19 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
         const double2* src = reinterpret_cast<const double2*>(
             (ch.learned && (mode == MDF_SEED || (mode == MDF_PLAIN && sweep == 1))) ? acc0 : acc);
         const size_t base = (size_t)slot * 2 * TILE_CELLS, base2 = (size_t)slot * TILE_CELLS;
-        const int x0 = si.x0 + BAND_W * warp;
-        // this lane's two cells: column a, rows b and b + 4 of the band
-        const int ca = lane & 7, cb = lane >> 3;
+        // this lane's cells: column a, rows b and b + 4 of the band, or a column of
+        // the tile
+        constexpr int MINE = WIDE ? 2 : TILE_H;
+        const int mine_x = WIDE ? BAND_W * warp + (lane & 7) : lane;
+        auto row_of = [&](int h) { return WIDE ? (lane >> 3) + 4 * h : h; };
+        auto at = [&](int r) { return r * Tile::ROW + (WIDE ? lane & 7 : lane); };
         __syncwarp();
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = cb + 4 * h, c = r * TILE_W + BAND_W * warp + ca;
+        for (int h = 0; h < MINE; ++h) {
+            const int r = row_of(h), c = r * TILE_W + mine_x;
             const double2 a = sweep > 0 ? src[base2 + c] : make_double2(0.0, 0.0);
-            B.ax[r * BAND_ACC_W + ca] = a.x;
-            B.ay[r * BAND_ACC_W + ca] = a.y;
+            B.ax[at(r)] = a.x;
+            B.ay[at(r)] = a.y;
             if (last && K > 1) {
                 gsnap[base + c] = a.x;
                 gsnap[base + TILE_CELLS + c] = a.y;
@@ -979,13 +1009,23 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
             k.wx[0] = wa.x; k.wx[1] = wa.y; k.wx[2] = wb.x; k.wx[3] = wb.y;
             k.wy = mb.wy[4 * (size_t)m + sy];
         };
-        band_spread(B, list + si.off, cnt, si.nx, si.ny, x0, si.y0, lane, org_of, load);
+        if constexpr (WIDE) {
+            band_spread<true>(B, lst, cnt, first, si.nx, si.ny, si.x0 + BAND_W * warp, 0, si.y0,
+                              lane, org_of, load);
+        } else if (si.nx > TILE_W) {
+            band_spread<false>(B, lst, cnt, first, si.nx, si.ny, si.x0, 0, si.y0, lane, org_of,
+                               load);
+        } else {
+            for (int col = 0; col < TILE_W; col += BAND_W)
+                band_spread<true>(B, lst, cnt, first, si.nx, si.ny, si.x0 + col, col, si.y0, lane,
+                                  org_of, load);
+        }
         if (!last) {
             double2* out = reinterpret_cast<double2*>((sweep == 0 && ch.learned) ? acc0 : acc);
 #pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                const int r = cb + 4 * h, i = r * BAND_ACC_W + ca;
-                out[base2 + r * TILE_W + BAND_W * warp + ca] = make_double2(B.ax[i], B.ay[i]);
+            for (int h = 0; h < MINE; ++h) {
+                const int r = row_of(h);
+                out[base2 + r * TILE_W + mine_x] = make_double2(B.ax[at(r)], B.ay[at(r)]);
             }
             continue;
         }
@@ -994,10 +1034,10 @@ k_spread(const ChannelDev* __restrict__ chans, const SlotInfo* __restrict__ slot
         const double Fm = ch.max_force, Fm2 = Fm * Fm;
         const bool body = (ch.body_fx != 0.0 || ch.body_fy != 0.0);
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int r = cb + 4 * h, i = r * BAND_ACC_W + ca, c = r * TILE_W + BAND_W * warp + ca;
-            const int jx = x0 + ca, jy = si.y0 + r;
-            double vx = B.ax[i], vy = B.ay[i];
+        for (int h = 0; h < MINE; ++h) {
+            const int r = row_of(h), c = r * TILE_W + mine_x;
+            const int jx = si.x0 + mine_x, jy = si.y0 + r;
+            double vx = B.ax[at(r)], vy = B.ay[at(r)];
             if (jx < si.nx && jy < si.ny) {
                 const bool fluid = cell_kind(ch, jx, jy) == CK_FLUID;
                 if (fluid && body) {
@@ -1653,12 +1693,17 @@ size_t membrane_smem_bytes(int maxn) {
     return (size_t)MEM_WARPS * MEM_DOUBLES_PER_NODE * maxn * sizeof(double);
 }
 
-bool spread_wide(int max_slots) { return max_slots <= FX_WIDE_SLOTS; }
+bool spread_wide(bool fp64, int max_slots, int touched) {
+    return fp64 ? touched <= BAND_TILES : max_slots <= FX_WIDE_SLOTS;
+}
 
 int spread_blocks_per_sm(bool fp64, bool wide) {
     int b = 0;
     const cudaError_t e =
-        fp64 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_spread, BAND_WARPS * 32, 0)
+        fp64 && wide ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                           &b, k_spread<true>, 32 * spread_warps<true>, spread_smem<true>)
+        : fp64 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                     &b, k_spread<false>, 32 * spread_warps<false>, spread_smem<false>)
         : wide ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_spread_fx<true>,
                                                                fx_threads<true>, fx_smem<true>)
                : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_spread_fx<false>,
@@ -1668,8 +1713,12 @@ int spread_blocks_per_sm(bool fp64, bool wide) {
 }
 
 cudaError_t prepare_spread() {
-    return cudaFuncSetAttribute(k_spread_fx<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)fx_smem<false>);
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_spread_fx<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)fx_smem<false>);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(k_spread<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)spread_smem<false>);
 }
 
 // ---------------- capsule geometry (thermo) ---------------------------------
@@ -1955,20 +2004,18 @@ template void launch_tiles<float>(const ChannelDev*, int, const CapsuleDev*, int
 template <typename R>
 void launch_spread(const ChannelDev* chans, const MarkerBufs& mb, TileBufs& tb, int parity,
                    int sweep, int mode, int grid, unsigned* status, cudaStream_t st) {
-    if constexpr (sizeof(R) == 4) {
-        auto run = [&](auto kernel, int threads, size_t smem) {
-            kernel<<<grid, threads, smem, st>>>(
+    auto run = [&](auto kernel, int threads, size_t smem) {
+        kernel<<<grid, threads, smem, st>>>(
             chans, tb.slot_info, tb.slot_order, tb.ctr, tb.max_slots, tb.list, mb, tb.acc, tb.acc0,
-            static_cast<float*>(tb.gsnap), static_cast<float*>(tb.fin[parity]), sweep, mode,
-            tb.resid_gate, tb.plain_needed, tb.capped, tb.fluid_touched, status);
-        };
-        if (spread_wide(tb.max_slots)) run(k_spread_fx<true>, fx_threads<true>, fx_smem<true>);
+            static_cast<R*>(tb.gsnap), static_cast<R*>(tb.fin[parity]), sweep, mode, tb.resid_gate,
+            tb.plain_needed, tb.capped, tb.fluid_touched, status);
+    };
+    if constexpr (sizeof(R) == 4) {
+        if (tb.wide) run(k_spread_fx<true>, fx_threads<true>, fx_smem<true>);
         else run(k_spread_fx<false>, fx_threads<false>, fx_smem<false>);
     } else {
-        k_spread<<<grid, BAND_WARPS * 32, 0, st>>>(
-            chans, tb.slot_info, tb.slot_order, tb.ctr, tb.max_slots, tb.list, mb, tb.acc,
-            tb.acc0, static_cast<double*>(tb.gsnap), static_cast<double*>(tb.fin[parity]), sweep, mode,
-            tb.resid_gate, tb.plain_needed, tb.capped, tb.fluid_touched, status);
+        if (tb.wide) run(k_spread<true>, 32 * spread_warps<true>, spread_smem<true>);
+        else run(k_spread<false>, 32 * spread_warps<false>, spread_smem<false>);
     }
 }
 template void launch_spread<double>(const ChannelDev*, const MarkerBufs&, TileBufs&, int, int,

@@ -35,6 +35,7 @@ struct SlotInfo {
 struct TileBufs {
     int T = 0;                  // force tiles over all channels
     int max_slots = 0;
+    bool wide = false;          // spread_wide
     int* tile_chan = nullptr;   // [T]
     int* tile_cnt = nullptr;    // [T] markers whose stencil covers the tile (0 between steps)
     int* tile_pos = nullptr;    // [T] next free list entry of the tile
@@ -67,7 +68,9 @@ cudaError_t prepare_membrane(int maxn);
 cudaError_t prepare_spread();
 // Resident spread CTAs per SM (after prepare_spread).
 int spread_blocks_per_sm(bool fp64, bool wide);
-bool spread_wide(int max_slots);   // FP32 spreads: four warps a tile
+// Whether the spreads give a tile four warps: by the slots a context may need, in
+// FP64 by the force tiles its markers touch at the start.
+bool spread_wide(bool fp64, int max_slots, int touched);
 void launch_membrane(const CapsuleDev* caps, int ncaps, const MarkerBufs& mb, int* has_prev,
                      int maxn, unsigned* status, cudaStream_t st);
 // Pair and wall contact forces, added to the membrane forces (after the

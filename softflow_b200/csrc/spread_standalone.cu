@@ -163,21 +163,19 @@ __global__ void __launch_bounds__(BAND_WARPS * 32)
 k_sa_gather(int nx, int ny, int tiles_x, int T, const double2* __restrict__ pos,
             const double2* __restrict__ frc, const double* phi_tbl, SpreadScratch sc,
             double* __restrict__ Fx, double* __restrict__ Fy) {
-    __shared__ BandSmem s_band[BAND_WARPS];
+    __shared__ BandTile s_band[BAND_WARPS];
+    __shared__ __align__(16) int s_sort[SORT_SMEM];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    BandSmem& B = s_band[warp];
+    BandTile& B = s_band[warp];
     chain_begin();
     for (int t = blockIdx.x; t < T; t += gridDim.x) {   // uniform in the CTA
         const int cnt = sc.tile_cnt[t];
         if (cnt == 0) continue;
         int* list = sc.list + sc.tile_off[t];
         const int x0 = (t % tiles_x) * TILE_W + BAND_W * warp, y0 = (t / tiles_x) * TILE_H;
-        if (cnt > BAND_LIST) {
-            if (threadIdx.x == 0) long_list_sort(list, cnt);
-            __syncthreads();
-        }
+        const int first = tile_list_sort<32 * BAND_WARPS>(list, cnt, s_sort, threadIdx.x, false);
         __syncwarp();
-        for (int c = lane; c < BAND_ACC; c += 32) B.ax[c] = B.ay[c] = 0.0;
+        for (int c = lane; c < BandTile::CELLS; c += 32) B.ax[c] = B.ay[c] = 0.0;
         auto org_of = [&](int m) { return make_int2(sc.ix0[m], sc.iy0[m]); };
         auto load = [&](int m, int sy, BandMarker& k) {
             const double2 p = pos[m];
@@ -188,10 +186,10 @@ k_sa_gather(int nx, int ny, int tiles_x, int T, const double2* __restrict__ pos,
             for (int q = 0; q < 4; ++q) k.wx[q] = phi_lut(phi_tbl, p.x - (double)(k.org.x - 1 + q));
             k.wy = phi_lut(phi_tbl, p.y - (double)(k.org.y - 1 + sy));
         };
-        band_spread(B, list, cnt, nx, ny, x0, y0, lane, org_of, load);
+        band_spread<true>(B, list, cnt, first, nx, ny, x0, 0, y0, lane, org_of, load);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int r = (lane >> 3) + 4 * h, a = r * BAND_ACC_W + (lane & 7);
+            const int r = (lane >> 3) + 4 * h, a = r * BandTile::ROW + (lane & 7);
             const int jx = x0 + (lane & 7), jy = y0 + r;
             if (jx < nx && jy < ny) {
                 const size_t n = (size_t)jy * nx + jx;

@@ -117,3 +117,41 @@ def test_crowded_contact_agrees(sfg, precision, nodes):
     assert out[0][0] <= 32768 < out[1][0]
     for x, y in zip(out[0][1:], out[1][1:]):
         assert np.isfinite(x).all() and np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("nx,ny,r,nodes,sweeps", [
+    (9, 24, 2.0, 12, 3),        # narrower than a stencil's residues, over the seam
+    (32, 24, 4.0, 24, 2),       # one tile wide
+    (33, 24, 4.0, 24, 2),       # a second tile of one column
+    (77, 43, 4.0, 9, 4), (77, 43, 4.0, 150, 1), (77, 43, 4.0, 150, 4),
+    (77, 43, 3.0, 600, 3),      # lists beyond 256 entries
+])
+def test_fp64_few_and_many_touched_tiles_agree(sfg, nx, ny, r, nodes, sweeps):
+    """The FP64 spread gives a tile four warps, or one in contexts whose markers touch
+    more than 2,800 tiles: the same channel on both sides of that line, bit for bit."""
+    import softflow_b200 as S
+    ctx = []
+    for many in (False, True):
+        ens = S.Ensemble(precision="fp64")
+        for w, h in ((nx, ny),) + (((2048, 512),) if many else ()):
+            p = S.SimulationParams(nx=w, ny=h, ibm_iterations=sweeps, precision="fp64")
+            p.fluid.boundary_type = S.BoundaryType.PERIODIC
+            p.fluid.collision_model = S.CollisionModel.BGK
+            p.fluid.body_force_x = 2e-5
+            i = ens.add_channel(p)
+            mp = S.MembraneParams(model=S.MembraneModel.NEO_HOOKEAN, G_s=0.05)
+            if i == 0:
+                for c in ((1.2, 11.3),) + (((30.4, 12.1), (70.8, 30.9)) if nx > 40 else ()):
+                    ens.addCapsule(i, c, r, nodes, mp)
+            else:
+                for cy in range(10, 505, 16):
+                    for cx in range(10, 2040, 16):
+                        ens.addCapsule(i, (cx, cy), 4.0, 12, mp)
+        ens.initialize()
+        ens.run(3)
+        ctx.append(ens)
+    few, many = ctx
+    for a, b in zip(few.field(0).macroscopic(), many.field(0).macroscopic()):
+        assert np.isfinite(a).all() and np.array_equal(a, b)
+    assert np.array_equal(few.capsules(0).positions(), many.capsules(0).positions())
+    assert np.array_equal(few.capsules(0).velocities(), many.capsules(0).velocities())

@@ -110,3 +110,16 @@ def test_spread_list_lengths(sfg, oracle_mod, nx, copies):
     Fx, Fy = o.spread()
     gx, gy = _gpu_spread(nx, 24, o.offsets(), pos, frc)
     assert np.array_equal(gx, Fx) and np.array_equal(gy, Fy)
+
+
+@pytest.mark.parametrize("nx", [12, 70])
+@pytest.mark.parametrize("copies", [3, 13, 26, 52, 205])
+def test_spread_long_lists(sfg, oracle_mod, nx, copies):
+    """Lists sorted in place, between and beyond powers of two (60 to 4,100 markers, all of
+    them in one or two tiles): bit for bit the serial sum."""
+    rng = np.random.default_rng(12)
+    rings = [(6.4 + 0.002 * k, 11.7 + 0.001 * k, 2.5, 20) for k in range(copies)]
+    o, pos, frc = _ring_system(nx, 24, rings, lambda p: rng.normal(0, 1e-3, p.shape))
+    Fx, Fy = o.spread()
+    gx, gy = _gpu_spread(nx, 24, o.offsets(), pos, frc)
+    assert np.array_equal(gx, Fx) and np.array_equal(gy, Fy)
