@@ -40,8 +40,8 @@ KERNELS = {
 # functions that chained kernels pass other kernels' output to
 FUNCTIONS = {"lattice_run4f": {"dst", "gdst", "cfield"}, "lattice_run4": {"dst", "gdst", "cfield"},
              "lattice_run8h": {"dst", "status"}, "contact_cells": {"chans"},
-             "warp_tile_add": set(), "band_spread": set(), "long_list_sort": set(),
-             "phi_lut": set(), "load_model": set()}
+             "warp_tile_add": set(), "band_spread": set(), "group_sort": set(),
+             "tile_list_sort": set(), "phi_lut": set(), "load_model": set()}
 
 
 def _sources():
