@@ -386,12 +386,18 @@ int sfg_get_harvest(sfg_context* ctx, float* features, float* labels, int* valid
  * sfg_autotune times whole steps (CUDA events) for each candidate launch
  * shape -- CTAs per SM of the persistent lattice kernel, of the spread and of
  * the learned seed, and the block size of the per-marker kernels -- one
- * tunable at a time, and keeps the fastest.  The trials are real steps: the
- * context advances by *steps_run steps (call it in place of warm-up steps).
+ * tunable at a time, and keeps the fastest.  Only what the context runs is
+ * tried (the one-cell lattice kernels have no such count; see
+ * sfg_get_lattice_form).  The trials are real steps, at least 16 where there are
+ * no markers: the context advances by *steps_run steps, 0 if there is nothing to
+ * tune (call it in place of warm-up steps).
  * No reference counterpart (the reference has no launch shapes). */
 int sfg_autotune(sfg_context* ctx, int steps_per_trial, int* steps_run);
 int sfg_get_launch_config(sfg_context* ctx, int* lattice_ctas_per_sm, int* spread_ctas_per_sm,
                           int* marker_block, int* learned_ctas_per_sm);
+/* Cells per thread of the lattice kernel the context's steps run: 8, 4 or 1
+ * (chosen at sfg_initialize, see sfg_set_lattice_variant). */
+int sfg_get_lattice_form(sfg_context* ctx, int* cells_per_thread);
 
 /* ---- thermo: device-side reductions of the state -------------------------
  * One record per channel, reduced on the device over the state after the

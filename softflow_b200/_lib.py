@@ -157,6 +157,7 @@ SIGNATURES = {
     "sfg_mlp_train": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int, C.c_int, C.c_float,
                                 _P(C.c_float), C.c_void_p]),
     "sfg_release_scratch": (C.c_int, []),
+    "sfg_get_lattice_form": (C.c_int, [C.c_void_p, _P(C.c_int)]),
     "sfg_mlp_train_rows": (C.c_int, [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int,
                                      C.c_int, C.c_float, _P(C.c_float), C.c_void_p]),
     "sfg_mlp_step_count": (C.c_int, [C.c_void_p, _P(C.c_int)]),

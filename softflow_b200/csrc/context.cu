@@ -1465,9 +1465,11 @@ static void drop_graphs(sfg_context* c) {
 // ------------------------------------------------------------------------
 // launch-shape autotuner
 // ------------------------------------------------------------------------
-static int time_steps(sfg_context* c, int n, float* ms_per_step) {
+// One trial: `warm` steps, which build every graph that the timed ones launch,
+// then n timed.
+static int time_steps(sfg_context* c, int warm, int n, float* ms_per_step) {
     drop_graphs(c);
-    int rc = sfg_step(c, 2);
+    int rc = sfg_step(c, warm);
     if (rc) return rc;
     CU(cudaStreamSynchronize(c->stream));
     if ((rc = sfg_step(c, n))) return rc;
@@ -1497,7 +1499,8 @@ extern "C" int sfg_autotune(sfg_context* c, int steps_per_trial, int* steps_run)
     std::vector<int> lat, spr;
     for (int k = 1; k <= lat_max; ++k) lat.push_back(k);
     for (int k = 1; k <= spr_max; ++k) spr.push_back(k);
-    knobs.push_back({&c->lattice_cps, lat});
+    // (the one-cell kernels' grid follows from the lattice)
+    if (c->use_vec4) knobs.push_back({&c->lattice_cps, lat});
     if (c->M > 0) {
         knobs.push_back({&c->spread_cps, spr});
         knobs.push_back({&c->tb.marker_block, {64, 128, 256}});
@@ -1505,6 +1508,9 @@ extern "C" int sfg_autotune(sfg_context* c, int steps_per_trial, int* steps_run)
     }
     if (c->lattice_cps == 0) c->lattice_cps = lat_max;
     if (c->spread_cps == 0) c->spread_cps = spr_max;
+    // without markers a run's steps go by graphs of MULTI_STEPS, the timed ones too
+    const int n = c->M > 0 ? steps_per_trial : std::max(steps_per_trial, MULTI_STEPS);
+    const int warm = c->M > 0 ? 2 : n;
     for (auto& k : knobs) {
         int best = *k.v;
         float best_ms = 1e30f;
@@ -1512,8 +1518,8 @@ extern "C" int sfg_autotune(sfg_context* c, int steps_per_trial, int* steps_run)
             *k.v = v;
             apply_launch_config(c);
             float ms = 0.f;
-            int rc = time_steps(c, steps_per_trial, &ms);
-            run += 2 + steps_per_trial;
+            int rc = time_steps(c, warm, n, &ms);
+            run += warm + n;
             if (rc) {
                 c->profiling = prof;
                 return rc;
@@ -1542,6 +1548,13 @@ extern "C" int sfg_get_launch_config(sfg_context* c, int* lattice_cps, int* spre
     if (spread_cps) *spread_cps = c->spread_cps > 0 ? std::min(c->spread_cps, spr_max) : spr_max;
     if (marker_block) *marker_block = c->tb.marker_block;
     if (learned_cps) *learned_cps = std::max(1, std::min(c->learned_cps, 6));
+    return SFG_OK;
+}
+
+extern "C" int sfg_get_lattice_form(sfg_context* c, int* cells_per_thread) {
+    if (!c || !cells_per_thread) return fail(SFG_ERR_ARG, "sfg_get_lattice_form: null argument");
+    if (!c->initialized) return fail(SFG_ERR_STATE, "sfg_get_lattice_form: context not initialized");
+    *cells_per_thread = c->use_vec8 && !(c->any_adr && !c->any_chem) ? 8 : (c->use_vec4 ? 4 : 1);
     return SFG_OK;
 }
 

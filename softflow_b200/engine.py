@@ -996,8 +996,11 @@ class Ensemble:
         ctx = self._need()
         v = [C.c_int() for _ in range(4)]
         L.check(ctx._lib.sfg_get_launch_config(ctx._h, *[C.byref(x) for x in v]))
+        form = C.c_int()
+        L.check(ctx._lib.sfg_get_lattice_form(ctx._h, C.byref(form)))
         return dict(lattice_ctas_per_sm=v[0].value, spread_ctas_per_sm=v[1].value,
-                    marker_block=v[2].value, learned_ctas_per_sm=v[3].value)
+                    marker_block=v[2].value, learned_ctas_per_sm=v[3].value,
+                    lattice_cells_per_thread=form.value)
 
     # ---- learned multi-direct forcing
     def setLearnedMDF(self, net=None, threshold: float = 1e-4):
