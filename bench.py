@@ -298,22 +298,17 @@ def spread_roofline(ens, plans, spread_ms, sweeps, peak, peak_kind):
                     "that return at once; tiles and cells from the final marker positions"}
 
 
-def lattice_kernel_name(plans, precision):
-    """The lattice kernel instantiation a workload runs: the eight-cell
-    FP16-shifted kernel when the storage is FP16S, there is no scalar and
-    every nx % 8 == 0, the one-cell kernel on small FP32 and FP64 lattices, in
-    FP64 regularized and where an nx % 4 != 0, otherwise the four-cell kernel
-    (storage, arithmetic, scalar fused or not; the last argument is the
-    collision model)."""
+def lattice_kernel_name(cells_per_thread, plans, precision):
+    """The lattice kernel instantiation a context of `plans` runs, by the form the
+    library says it chose (Ensemble.launchConfig): eight cells a thread in
+    FP16-shifted storage without the scalar, four, or one (storage, arithmetic,
+    scalar fused or not; the last argument is the collision model)."""
     adr = int(any(p.params.scalar.enabled for p in plans))
     coll = "|".join(map(str, sorted({int(p.params.fluid.collision_model) for p in plans})))
-    if precision == "fp16s" and not adr and all(p.params.nx % 8 == 0 for p in plans):
+    if cells_per_thread == 8:
         return f"k_lattice_step8h<{coll}>"
     st = {"fp64": "double, double", "fp32": "float, float", "fp16s": "__half, float"}[precision]
-    cells = sum(p.params.nx * p.params.ny for p in plans)
-    one = {"fp32": cells <= 200 * 1024, "fp16s": False,
-           "fp64": coll == "2" or cells <= 512 * 1024}[precision]
-    if one or any(p.params.nx % 4 for p in plans):
+    if cells_per_thread == 1:
         return f"k_lattice_step<{st}, {adr}>"
     return f"k_lattice_step4<{st}, {adr}, {coll}>"
 
@@ -348,7 +343,8 @@ def measure_form(plans, precision, steps, warmup, local, prof_steps=20):
             "capsule_steps_per_s": caps * steps / sec, "mlups": cells * steps / sec / 1e6,
             "marker_updates_per_s": markers * steps / sec,
             "fluid_cells": cells, "capsules": caps, "markers": markers, "launch_shapes": tuned,
-            "lattice": {"kernel": lattice_kernel_name(plans, precision), "ms": lat_ms,
+            "lattice": {"kernel": lattice_kernel_name(tuned["lattice_cells_per_thread"], plans,
+                                                      precision), "ms": lat_ms,
                         "algorithmic_bytes": alg, "achieved_gbs": ach, "peak_gbs": peak,
                         "frac": ach / peak, "peak_source": kind},
             "phase_ms_per_step": {k: v / prof_steps for k, v in phases.items() if v > 0}}
@@ -537,7 +533,8 @@ def run_product(args, world, rank, local, pg):
         "marker_updates_per_s": mk_upd,
         "gpu_launches": launches * args.steps,
         "phase_ms_per_step": {k: v / prof_steps for k, v in phases.items()},
-        "roofline": {"kernel": lattice_kernel_name(plans, args.precision), "bound": "hbm",
+        "roofline": {"kernel": lattice_kernel_name(tuned["lattice_cells_per_thread"], plans,
+                                                   args.precision), "bound": "hbm",
                      "achieved": achieved,
                      "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "peak_source": peak_kind,
