@@ -181,8 +181,8 @@ __device__ __forceinline__ R div_const(R a, R d) {
 }
 
 // Whether every input of a cell's collision is zero or of magnitude 2^-200 to
-// 2^200 (the rates of MRT are checked once per channel): then every intermediate that is divided (products
-// of up to four of them and sums, whose terms are multiples of the inputs' last
+// 2^200 (the rates of MRT are checked once per channel): then every intermediate
+// that is divided (products of up to four of them and sums, whose terms are multiples of the inputs' last
 // places) is zero or far inside the exponent range.
 __device__ __forceinline__ bool ordinary(double v) {
     const unsigned hi = (unsigned)__double2hiint(v);

@@ -410,7 +410,8 @@ static void free_all(sfg_context* c) {
     F(c->mb.wxf); F(c->mb.wyf); F(c->mb.wf); F(c->mb.dsf);
     F(c->tb.tile_chan); F(c->tb.tile_cnt); F(c->tb.tile_pos); F(c->tb.ctr);
     F(c->tb.list); F(c->tb.acc); F(c->tb.gsnap); F(c->tb.capped);
-    F(c->tb.fluid_touched); F(c->tb.acc0); F(c->tb.mom); F(c->tb.slot_info); F(c->tb.slot_order); F(c->tb.resid_gate); F(c->tb.resid_plain);
+    F(c->tb.fluid_touched); F(c->tb.acc0); F(c->tb.mom); F(c->tb.slot_info);
+    F(c->tb.slot_order); F(c->tb.resid_gate); F(c->tb.resid_plain);
     F(c->mb.u0); F(c->mb.dFsum); F(c->mb.dFprev); F(c->mb.slot8);
     F(c->d_model); F(c->d_learned_steps); F(c->d_fallbacks);
     F(c->d_hfeat); F(c->d_hlab); F(c->d_hvalid); F(c->d_feat); F(c->d_frame); F(c->d_plain_needed);
@@ -1200,7 +1201,8 @@ static int enqueue_step_t(sfg_context* c, int p, bool within) {
     int launches = 0;
     mark(c, -1);
     LatticeLaunch L{c->d_items, c->n_items, c->d_chans, c->f[p], c->f[1 - p], c->g[p],
-                    c->g[1 - p], c->cfield, c->flag_args(p), c->any_adr && !c->any_chem, c->d_items4, c->n_items4, c->use_vec4,
+                    c->g[1 - p], c->cfield, c->flag_args(p), c->any_adr && !c->any_chem, c->d_items4,
+                    c->n_items4, c->use_vec4,
                     c->persistent_ctas, c->shared_collision, c->any_bc, c->d_zh_rows,
                     c->n_zh, c->d_ibb, c->ibb_level_start.data(),
                     (int)c->ibb_level_start.size() - 1, c->d_items8, c->n_items8, c->use_vec8,
@@ -1280,8 +1282,8 @@ static int enqueue_step_t(sfg_context* c, int p, bool within) {
         if (c->any_learned) {
             // seed, one plain sweep, gate; the plain sweeps below run only for
             // channels above the threshold
-            launch_mdf_learned<R>(c->d_chans, c->d_caps, c->M, c->mb, c->tb, c->d_model, c->d_feat, c->d_frame, c->learned_grid,
-                                     c->d_status, st);
+            launch_mdf_learned<R>(c->d_chans, c->d_caps, c->M, c->mb, c->tb, c->d_model,
+                                  c->d_feat, c->d_frame, c->learned_grid, c->d_status, st);
             mark(c, SFG_PHASE_MDF_LEARNED);
             launch_spread<R>(c->d_chans, c->mb, c->tb, p, 1, MDF_SEED, c->spread_grid,
                              c->d_status, st);
@@ -1341,7 +1343,7 @@ static int enqueue_step_t(sfg_context* c, int p, bool within) {
     launches += 1;
     if (c->M > 0) {
         launch_interp_move<S, R>(c->d_chans, c->d_caps, c->NC, c->M, c->mb, c->cb,
-                                 static_cast<const S*>(c->f[1 - p]), c->tb, p, c->d_phi, st);
+                                 static_cast<const S*>(c->f[1 - p]), c->tb, p, st);
         mark(c, SFG_PHASE_INTERP_MOVE);
         launches += 1;
     }

@@ -9,9 +9,6 @@
 
 namespace sfg {
 
-// u = (j + F/2)/rho at the marker's 4 x 4 stencil with the accumulated force
-// acc (immersed_boundary.cpp:174-229 with the stencil weights of the step;
-// SOLID rows and rho <= 1e-15 contribute zero).
 // Slot of stencil cell (sx, jy) from the marker's slot record (k_tile_fill).
 struct StencilSlots {
     int s[8];
@@ -28,19 +25,17 @@ struct StencilSlots {
     }
 };
 
-template <typename S, typename R, typename A = double>
+// u = (j + F/2)/rho at the marker's 4 x 4 stencil with the final force acc
+// (immersed_boundary.cpp:174-229 with the stencil weights of the step; SOLID rows and
+// rho <= 1e-15 contribute zero).  FP64 contexts; the FP32-arithmetic modes move
+// markers by capsule.
 __device__ __forceinline__ double2 interp_u_acc(const ChannelDev& ch, const MarkerBufs& mb, int m,
-                                               const S* __restrict__ f,
-                                               const int* __restrict__ tile_slot,
-                                               const A* __restrict__ acc) {
-    (void)tile_slot;
-    // compute type: double in FP64 contexts (the reference's arithmetic),
-    // float in the FP32-arithmetic modes
-    using C = typename std::conditional<sizeof(R) == 8, double, float>::type;
+                                               const double* __restrict__ f,
+                                               const double* __restrict__ acc) {
     const int2 og = mb.org[m];
     const int ix0 = og.x, iy0 = og.y;
     const StencilSlots ss(mb, m, iy0, ch.ny);
-    C wxs[4], wys[4];
+    double wxs[4], wys[4];
     stencil_weights(mb, m, wxs, wys);
     int jxs[4];
 #pragma unroll
@@ -50,14 +45,13 @@ __device__ __forceinline__ double2 interp_u_acc(const ChannelDev& ch, const Mark
         if (jx >= ch.nx) jx -= ch.nx;
         jxs[sx] = jx;
     }
-    C ux = 0, uy = 0;
+    double ux = 0, uy = 0;
     // one stencil row at a time: the populations and forces of its four
     // cells are loaded together, then its terms are added in order
 #pragma unroll
     for (int sy = 0; sy < 4; ++sy) {
         const int jy = iy0 - 1 + sy;
-        R v[4][9];
-        A fx[4], fy[4];
+        double v[4][9], fx[4], fy[4];
         bool in[4], solid[4];
 #pragma unroll
         for (int sx = 0; sx < 4; ++sx) {
@@ -68,7 +62,7 @@ __device__ __forceinline__ double2 interp_u_acc(const ChannelDev& ch, const Mark
                 const long long n = (long long)jy * ch.pitch + jx;
 #pragma unroll
                 for (int q = 0; q < 9; ++q)
-                    v[sx][q] = PopIO<S, R>::ld(f + ch.f_off + q * ch.plane + n, q);
+                    v[sx][q] = PopIO<double, double>::ld(f + ch.f_off + q * ch.plane + n, q);
                 const size_t ci = (size_t)ss.slot(sx, jy) * 2 * TILE_CELLS +
                                   (jy % TILE_H) * TILE_W + (jx % TILE_W);
                 fx[sx] = acc[ci];
@@ -78,33 +72,20 @@ __device__ __forceinline__ double2 interp_u_acc(const ChannelDev& ch, const Mark
 #pragma unroll
         for (int sx = 0; sx < 4; ++sx) {
             if (!in[sx]) continue;
-            const C w = wxs[sx] * wys[sy];
-            if (w > (C)1e-15) {
-                C rho = 0, jxm = 0, jym = 0;
-                if (!solid[sx]) {
-                    R r, a, b;
-                    lattice_moments(v[sx], r, a, b);
-                    rho = (C)r;
-                    jxm = (C)a;
-                    jym = (C)b;
-                }
-                C cu = 0, cv = 0;
-                if (!solid[sx] && rho > (C)1e-15) {
-                    if constexpr (sizeof(R) == 8) {
-                        cu = (jxm + 0.5 * (double)fx[sx]) / rho;
-                        cv = (jym + 0.5 * (double)fy[sx]) / rho;
-                    } else {
-                        const float inv = __frcp_rn(rho);
-                        cu = (jxm + 0.5f * (float)fx[sx]) * inv;
-                        cv = (jym + 0.5f * (float)fy[sx]) * inv;
-                    }
+            const double w = wxs[sx] * wys[sy];
+            if (w > 1e-15) {
+                double rho = 0, jxm = 0, jym = 0, cu = 0, cv = 0;
+                if (!solid[sx]) lattice_moments(v[sx], rho, jxm, jym);
+                if (!solid[sx] && rho > 1e-15) {
+                    cu = (jxm + 0.5 * fx[sx]) / rho;
+                    cv = (jym + 0.5 * fy[sx]) / rho;
                 }
                 ux += cu * w;
                 uy += cv * w;
             }
         }
     }
-    return make_double2((double)ux, (double)uy);
+    return make_double2(ux, uy);
 }
 
 // Moments (rho, jx, jy) of a force tile's cells, computed once per step
@@ -117,9 +98,9 @@ template <> struct Mom4<double> { using T = double4; };
 template <> struct Mom4<float> { using T = float4; };
 
 // interp_u_acc with the step's tile moments and the accumulated force acc
-// ([slot][TILE_CELLS] (x, y) pairs): the same terms in the same order.  The loads of a stencil row (moments and force of four cells) are
-// issued together before any of their terms is formed, so a marker waits
-// for one round of gathers per row instead of one per cell.  FP64
+// ([slot][TILE_CELLS] (x, y) pairs): the same terms in the same order.  The loads of
+// a stencil row (moments and force of four cells) are issued together before any of
+// their terms is formed, so a marker waits for one round of gathers per row instead of one per cell.  FP64
 // divides by rho as the reference does (bit for bit); FP32-arithmetic modes
 // multiply by one reciprocal per cell.  With NEAR, also the density
 // at the node nearest to the marker (immersed_boundary.cpp:262-270: the
@@ -339,12 +320,10 @@ __device__ __forceinline__ double2 quad_interp(const ChannelDev& ch, const Marke
 }
 
 // interp_u_acc by four lanes of a warp, lane `row` a stencil row, as quad_interp.
-template <typename S, typename R, typename A>
 __device__ __forceinline__ double2 quad_interp_acc(const ChannelDev& ch, const MarkerBufs& mb,
                                                    int m, bool on, int row,
-                                                   const S* __restrict__ f,
-                                                   const A* __restrict__ acc) {
-    static_assert(sizeof(R) == 8, "the FP32-arithmetic modes move markers by capsule");
+                                                   const double* __restrict__ f,
+                                                   const double* __restrict__ acc) {
     double tx[4], ty[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) tx[i] = ty[i] = 0;
@@ -370,7 +349,7 @@ __device__ __forceinline__ double2 quad_interp_acc(const ChannelDev& ch, const M
                 const long long n = (long long)jy * ch.pitch + jx;
 #pragma unroll
                 for (int q = 0; q < 9; ++q)
-                    v[i][q] = PopIO<S, R>::ld(f + ch.f_off + q * ch.plane + n, q);
+                    v[i][q] = PopIO<double, double>::ld(f + ch.f_off + q * ch.plane + n, q);
                 const size_t ci =
                     (size_t)sl[i] * 2 * TILE_CELLS + (jy % TILE_H) * TILE_W + (jx % TILE_W);
                 fx[i] = acc[ci];

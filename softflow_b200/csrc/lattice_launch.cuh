@@ -22,10 +22,10 @@ inline TileView to_view(const TileViewArgs& a) {
 template <typename S, typename R, bool ADR, int COLL>
 static void launch_step4(const LatticeLaunch& L, const TileViewArgs& tv, int grid, bool chained,
                          cudaStream_t st) {
-    launch_chain(
-        chained, k_lattice_step4<S, R, ADR, COLL>, grid, 32 * ITEMS_PER_CTA, 0, st, L.items4, L.n_items4, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
-        static_cast<const R*>(L.gsrc), static_cast<R*>(L.gdst), static_cast<const R*>(L.cfield),
-        to_view(tv), L.flags);
+    launch_chain(chained, k_lattice_step4<S, R, ADR, COLL>, grid, 32 * ITEMS_PER_CTA, 0, st,
+                 L.items4, L.n_items4, L.chans, static_cast<const S*>(L.src),
+                 static_cast<S*>(L.dst), static_cast<const R*>(L.gsrc), static_cast<R*>(L.gdst),
+                 static_cast<const R*>(L.cfield), to_view(tv), L.flags);
 }
 
 template <typename S, typename R, bool ADR>
@@ -46,10 +46,10 @@ void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, bool ch
         // boundary-aware kernel (no scalar transport in such contexts), then
         // the Zou-He columns on the streamed populations
         if (L.n_items == 0) return;
-        launch_chain(
-            chained, k_lattice_step_bc<S, R>, (L.n_items + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA,
-            32 * ITEMS_PER_CTA, 0, st, L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
-            to_view(tv), L.flags);
+        launch_chain(chained, k_lattice_step_bc<S, R>,
+                     (L.n_items + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA, 32 * ITEMS_PER_CTA, 0, st,
+                     L.items, L.n_items, L.chans, static_cast<const S*>(L.src),
+                     static_cast<S*>(L.dst), to_view(tv), L.flags);
         for (int lv = 0; lv < L.n_ibb_levels; ++lv) {
             const int a = L.ibb_level_start[lv], n = L.ibb_level_start[lv + 1] - a;
             if (n > 0)
@@ -87,14 +87,16 @@ void launch_lattice_step(const LatticeLaunch& L, const TileViewArgs& tv, bool ch
     if (L.n_items == 0) return;
     const int grid = (L.n_items + ITEMS_PER_CTA - 1) / ITEMS_PER_CTA;
     if (L.any_adr)
-        launch_chain(
-            chained, k_lattice_step<S, R, true>, grid, 32 * ITEMS_PER_CTA, 0, st, L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
-            static_cast<const R*>(L.gsrc), static_cast<R*>(L.gdst),
-            static_cast<const R*>(L.cfield), to_view(tv), L.flags);
+        launch_chain(chained, k_lattice_step<S, R, true>, grid, 32 * ITEMS_PER_CTA, 0, st,
+                     L.items, L.n_items, L.chans, static_cast<const S*>(L.src),
+                     static_cast<S*>(L.dst), static_cast<const R*>(L.gsrc),
+                     static_cast<R*>(L.gdst), static_cast<const R*>(L.cfield), to_view(tv),
+                     L.flags);
     else
-        launch_chain(
-            chained, k_lattice_step<S, R, false>, grid, 32 * ITEMS_PER_CTA, 0, st, L.items, L.n_items, L.chans, static_cast<const S*>(L.src), static_cast<S*>(L.dst),
-            (const R*)nullptr, (R*)nullptr, (const R*)nullptr, to_view(tv), L.flags);
+        launch_chain(chained, k_lattice_step<S, R, false>, grid, 32 * ITEMS_PER_CTA, 0, st,
+                     L.items, L.n_items, L.chans, static_cast<const S*>(L.src),
+                     static_cast<S*>(L.dst), (const R*)nullptr, (R*)nullptr, (const R*)nullptr,
+                     to_view(tv), L.flags);
 }
 
 template <typename S, typename R>

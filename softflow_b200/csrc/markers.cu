@@ -1479,9 +1479,8 @@ __global__ void k_tile_moments(const ChannelDev* __restrict__ chans,
     }
 }
 
-// Move marker m with its interpolated velocity u (simulation.cpp:656-675,
-// capsule.cpp:267-297).
-// The record of the marker's contact cell goes back to empty for the next
+// Moves marker m with its interpolated velocity u (simulation.cpp:656-675,
+// capsule.cpp:267-297) and empties the record of its contact cell for the next
 // step (every marker of a cell stores the same zeros).
 __device__ __forceinline__ void move_marker(const ChannelDev& ch, const MarkerBufs& mb,
                                             const ContactBufs& cb, int m, double2 u) {
@@ -1519,21 +1518,20 @@ __device__ __forceinline__ void move_marker(const ChannelDev& ch, const MarkerBu
 // Interpolate the new velocity and move the markers (FP64 contexts), one
 // thread per marker or (QUAD) four, by interp_by_quads: 2400 markers 14.7 us a
 // launch with one thread, 6.7 with four (divisions and 144 loads in a row).
-template <typename S, typename R, bool QUAD>
+template <bool QUAD>
 __global__ void k_interp_move(const ChannelDev* __restrict__ chans, int M, MarkerBufs mb,
-                              ContactBufs cb, const S* __restrict__ f, const int* __restrict__ tile_slot,
-                              const R* __restrict__ fin, const double* __restrict__ phi_tbl) {
+                              ContactBufs cb, const double* __restrict__ f,
+                              const double* __restrict__ fin) {
     const int t = blockIdx.x * blockDim.x + threadIdx.x, m = QUAD ? t >> 2 : t;
     if constexpr (QUAD) {
         const ChannelDev& ch = chans[m < M ? mb.mk_chan[m] : 0];
-        const double2 u =
-            quad_interp_acc<S, R>(ch, mb, m, m < M && mb.valid[m], t & 3, f, fin);
+        const double2 u = quad_interp_acc(ch, mb, m, m < M && mb.valid[m], t & 3, f, fin);
         if (m < M && (t & 3) == 0) move_marker(ch, mb, cb, m, u);
     } else {
         if (m >= M) return;
         const ChannelDev& ch = chans[mb.mk_chan[m]];
         double2 u = make_double2(0.0, 0.0);
-        if (mb.valid[m]) u = interp_u_acc<S, R, R>(ch, mb, m, f, tile_slot, fin);
+        if (mb.valid[m]) u = interp_u_acc(ch, mb, m, f, fin);
         move_marker(ch, mb, cb, m, u);
     }
 }
@@ -2047,9 +2045,8 @@ void launch_tile_moments(const ChannelDev* chans, const S* f, TileBufs& tb, int 
 template <typename S, typename R>
 void launch_interp_move(const ChannelDev* chans, const CapsuleDev* caps, int ncaps, int M,
                         const MarkerBufs& mb, const ContactBufs& cb, const S* f, TileBufs& tb,
-                        int parity, const double* phi_tbl, cudaStream_t st) {
+                        int parity, cudaStream_t st) {
     if constexpr (sizeof(R) == 4) {
-        (void)phi_tbl;
         if (ncaps == 0) return;
         const float* fin = static_cast<const float*>(tb.fin[parity]);
         if (ncaps <= MOVE_WIDE_CAPS)
@@ -2061,9 +2058,8 @@ void launch_interp_move(const ChannelDev* chans, const CapsuleDev* caps, int nca
     } else {
         const bool quads = interp_by_quads(M);
         const int B = tb.marker_block, G = ((quads ? 4 * M : M) + B - 1) / B;
-        (quads ? k_interp_move<S, R, true> : k_interp_move<S, R, false>)<<<G, B, 0, st>>>(
-            chans, M, mb, cb, f, tb.tile_slot[parity], static_cast<const R*>(tb.fin[parity]),
-            phi_tbl);
+        (quads ? k_interp_move<true> : k_interp_move<false>)<<<G, B, 0, st>>>(
+            chans, M, mb, cb, f, static_cast<const double*>(tb.fin[parity]));
     }
 }
 
@@ -2072,7 +2068,7 @@ void launch_interp_move(const ChannelDev* chans, const CapsuleDev* caps, int nca
                                             cudaStream_t);                                      \
     template void launch_interp_move<S, R>(const ChannelDev*, const CapsuleDev*, int, int,     \
                                            const MarkerBufs&, const ContactBufs&, const S*,    \
-                                           TileBufs&, int, const double*, cudaStream_t);
+                                           TileBufs&, int, cudaStream_t);
 SFG_INST(double, double)
 SFG_INST(float, float)
 SFG_INST(__half, float)

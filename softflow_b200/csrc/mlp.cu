@@ -484,7 +484,8 @@ int batch_step(sfg_mlp* m, const Samples& d, long long first, int n, int step, f
     MCU(cudaGetLastError());
     sfg::launch_chain(true, k_mlp_adam, ADAM_BLOCKS, ADAM_THREADS, 0, st, m->d_params, m->d_m,
                       m->d_v, m->d_part, nparts, step, lr, g_out, m->d_part_loss,
-                      1.0f / (2.0f * (float)n), loss_out, m->d_train, m->d_status + ST_BAD_ROW, m->call);
+                      1.0f / (2.0f * (float)n), loss_out, m->d_train,
+                      m->d_status + ST_BAD_ROW, m->call);
     MCU(cudaGetLastError());
     if (step > 0) m->model_dirty = true;
     return SFG_OK;

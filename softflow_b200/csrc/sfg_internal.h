@@ -103,8 +103,8 @@ void launch_mdf_interp(const ChannelDev* chans, int M, const MarkerBufs& mb, Til
 // channel.  `model` is a mlp::ModelDev.
 template <typename R>
 void launch_mdf_learned(const ChannelDev* chans, const CapsuleDev* caps, int M,
-                        const MarkerBufs& mb, TileBufs& tb, const void* model, float* feat, double2* frame, int grid,
-                        unsigned* status, cudaStream_t st);
+                        const MarkerBufs& mb, TileBufs& tb, const void* model, float* feat,
+                        double2* frame, int grid, unsigned* status, cudaStream_t st);
 // Training data of the step: inputs [M x 8], labels [M x 2] (the step's total
 // correction in the local frame), valid [M].
 void launch_harvest(const ChannelDev* chans, const CapsuleDev* caps, int M, const MarkerBufs& mb,
@@ -119,7 +119,7 @@ void launch_tile_moments(const ChannelDev* chans, const S* f, TileBufs& tb, int 
 template <typename S, typename R>
 void launch_interp_move(const ChannelDev* chans, const CapsuleDev* caps, int ncaps, int M,
                         const MarkerBufs& mb, const ContactBufs& cb, const S* f, TileBufs& tb,
-                        int parity, const double* phi_tbl, cudaStream_t st);
+                        int parity, cudaStream_t st);
 
 // Lattice kernels (lattice_f64.cu / lattice_f32.cu).
 struct LatticeLaunch {

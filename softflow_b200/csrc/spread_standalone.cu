@@ -239,7 +239,8 @@ int run_spread(int nx, int ny, int ncaps, const int* off, const double* pos, con
     }
     const int B = 256, G = (M + B - 1) / B;
     const int Gi = std::min((std::max(T, 1025) + B - 1) / B, nsm * 8);
-    const double2 *p2 = reinterpret_cast<const double2*>(pos), *f2 = reinterpret_cast<const double2*>(frc);
+    const double2* p2 = reinterpret_cast<const double2*>(pos);
+    const double2* f2 = reinterpret_cast<const double2*>(frc);
     const int grid = std::max(1, std::min(T, nsm * 6));
     launch_chain(false, k_sa_init, Gi, B, 0, st, T, sc);
     launch_chain(true, k_sa_prep, G, B, 0, st, nx, ny, tiles_x, ncaps, off, p2, f2, M, sc);
