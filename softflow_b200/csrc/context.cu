@@ -668,17 +668,24 @@ static int touched_tiles(const sfg_context* c, const std::vector<double>& pos,
     return count;
 }
 
-// Whether the one-cell-per-thread lattice kernel is the faster one for `cells`
-// lattice cells.  Few cells leave the chip idle, and a thread's chain of four
-// cells is then the step's length: FP32 400 x 80 3.8 us a step with four cells a
-// lane against 2.6 with one, 1024 x 256 equal (5.5), 2048 x 512 13.6 against 16.3;
-// FP64 BGK 512 x 200 7.0 against 5.3, 1024 x 256 11.9 against 9.9, 2048 x 512 39.8
-// against 42.7, MRT 1024 x 512 25.2 against 19.9, 4096 x 1024 171 against 177.  FP64
-// regularized, bound by its arithmetic, keeps too few warps resident with four
-// cells in registers at any size (4096 x 1024: 223 us against 200).  FP32 and FP64 give the same bits either way; the FP16-shifted kernels
-// draw other dither bits, so their form follows from nx alone.
+// Whether the one-cell-per-thread lattice kernel runs for `cells` lattice cells (rows
+// padded to 32).  Few cells leave the chip idle, and a thread's chain of four cells is
+// then the step's length; the line lies where the one-cell blocks no longer all fit at
+// once (FP32: five an SM, 185 Ki cells, with the scalar four, 148 Ki).  FP64 regularized,
+// bound by its arithmetic, keeps too few warps resident with four cells in registers at
+// any size.  us a step, one cell a thread / four a lane, then the same with the scalar:
+//   FP32 MRT         512 x 160   3.4  3.6   5.0  5.3      512 x 256  3.7  4.0   4.9  5.3
+//                    640 x 256   3.8  4.0   6.4  5.9      768 x 256  4.8  4.1   6.7  6.5
+//                   1024 x 256   5.5  4.6   8.2  6.7
+//   FP64 BGK         512 x 160   5.0  5.8   7.5  9.1     1024 x 384 13.3 16.6  27.4 30.9
+//                   2048 x 512  42.8 40.4  68.3 73.9     4096 x 1024          264  285
+//   FP64 MRT        1024 x 384  15.4 19.7  28.9 33.7     2048 x 512 46.4 46.9  71.1 79.7
+//   FP64 regularized 1024 x 384 19.5 25.2  32.3 39.6     4096 x 1024 199  220   302  356
+// FP32 and FP64 give the same bits either way; the FP16-shifted kernels draw other
+// dither bits, so their form follows from nx alone.
 static bool one_cell_lattice(const sfg_context* c, long long cells) {
-    if (c->precision == SFG_FP32) return cells <= 200 * 1024;
+    if (c->precision == SFG_FP32)
+        return cells <= (c->any_adr && !c->any_chem ? 144 : 180) * 1024;
     if (c->precision != SFG_FP64) return false;
     for (const ChanHost& h : c->ch)
         if (h.p.collision != 2) return cells <= 512 * 1024;
