@@ -1105,9 +1105,12 @@ struct SpreadFxWarp {
 // A tile is one warp's work, eight tiles a CTA, or (WIDE) a CTA's of four warps.
 // Where the tiles are few, the sweep takes as long as one tile's chain of marker
 // passes and cells, which four warps cut by four; where they are many, the
-// narrow form keeps more tiles in flight, and its waits cost less.  The line lies at
-// the context's tile count (spread phase of a step of five sweeps, one warp /
-// two / four / eight a tile, us):
+// narrow form keeps more tiles in flight, and its waits cost less.  The line goes by
+// the slots a context may need, its lattice tiles or 8 a marker, of contexts with
+// capsules all over; a large lattice with few markers stays with one warp, which was
+// its only form before (4096 x 1024 with 10 capsules, five sweeps, 134 us a step).
+// Spread phase of a step of five sweeps, one warp / two / four / eight a tile, us, by
+// lattice tiles:
 //   400 x 80, 130 tiles                  66.4  53.1  44.9  44.4
 //   12 ragged channels, about 1,000      76.3  54.8  50.1  49.6
 //   16 channels of 512 x 104, 3,300      83.7  57.4  53.1  56.3
