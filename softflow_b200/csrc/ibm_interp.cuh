@@ -435,8 +435,8 @@ __device__ __forceinline__ void atomic_max_resid(unsigned* slot, double r) {
 
 // atomic_max_resid for the active lanes of a warp (each calls it once, `on`
 // lanes carry a residual; lanes that left the kernel take no part): lanes of
-// one channel are reduced first and one lane per channel updates the slot (the max of non-negative floats is the max of their bit
-// patterns, NaN mapped above every finite value as in atomic_max_resid).
+// one channel are reduced first and one lane per channel updates the slot (the max
+// of non-negative floats is the max of their bit patterns, NaN mapped above every finite value as in atomic_max_resid).
 __device__ __forceinline__ void warp_max_resid(unsigned* slots, int chan, bool on, double r) {
     const float rf = (float)r;
     const unsigned v = on ? (isnan(rf) ? 0x7fc00000u : __float_as_uint(rf)) : 0u;
