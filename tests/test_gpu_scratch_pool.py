@@ -46,9 +46,11 @@ def test_release_returns_what_a_call_keeps(sfg):
     free = lambda: torch.cuda.mem_get_info()[0]
     small, big = Rings(256, 128, 40, 32, 1), Rings(4096, 4096, 40000, 32, 2)   # 0.1 and 60 MB
     small.spread(lib, st)
+    want = small.F.clone()
+    assert torch.equal(small.F, want)             # (torch's own memory is in place now)
     torch.cuda.synchronize()
     assert lib.sfg_release_scratch() == 0
-    before, want = free(), small.F.clone()
+    before = free()
     for r in (small, big, small):
         r.F.zero_()
         r.spread(lib, st)
